@@ -18,6 +18,7 @@ UNITS = [
     ("fsg_kernels64.cu", ["-fmad=false"]),
     ("fsg_mag.cu", ["-fmad=false"]),
     ("fsg_fast.cu", ["-fmad=true"]),
+    ("fsg_accum64.cu", ["-fmad=true"]),
     ("fsg_api.cu", ["-fmad=false"]),
     ("fsg_noalloc.cu", ["-fmad=false"]),
     ("fsg_adjoint.cu", ["-fmad=false"]),

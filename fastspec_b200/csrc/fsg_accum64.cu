@@ -1,0 +1,214 @@
+// fsg_accum64.cu -- plain FP64 line opacity: LineOpacity1 (opacity.f90:297-346) and the wide lines
+// (synth.f90:981-1001) on wavelength tiles.
+//
+//   LineOpac(t, p) += sum over lines l with Ileft(l) <= p <= Iright(l) of HVoigt(a(l,t), v) LinCop(l,t)
+//
+// A warp owns 32 * P wavelengths (lanes) x D depths and takes the lines of its tile in list order, so
+// every point sums its lines in the reference's order whatever the tile or the wavelength range of the
+// call.  Warps share nothing: each reads the windows of the tile's candidate lines 32 at a time, queues
+// those that touch the tile and works through the queue A64_G lines at a time.  For a group the lanes
+// first turn the lines' (LinCop, LinVvgt, LinAvgt) at the warp's depths into the wing form's
+// coefficients, one (line, depth) per lane, in shared memory; then every lane evaluates its points:
+//   outside the line's core range (s >= 196 at every depth, voigt.f90:100-101)
+//     val = c1 (t + 1) / (t^2 + 2 a^2),  t = dl^2 LinVvgt^2 + a^2 - 1/2,  c1 = LinCop a / sqrt(pi)
+//     -- three FMAs, a reciprocal of three more, one FMA into the sum;
+//   inside it the same form where t >= 195.5, else the table lerp or the continued fraction of HVoigt.
+// He I lines with a Stark shift per depth take the point-by-point form over their whole window.
+//
+// Bound by the FP64 pipe: 7.5 FP64 instructions per wing evaluation (64 lanes/clk/SM: 2.5e12
+// evaluations/s).  P = 2 and D = 4 keep the per-line work (offsets, window test, 8 shared loads) under a
+// tenth of the evaluations' and leave registers for five 4-warp CTAs per SM.
+#include "fsg_fp64.cuh"
+
+#define A64_P 2
+#define A64_D 4
+#define A64_G (32 / A64_D)          // lines per group: one (line, depth) pair per lane
+#define A64_TW (32 * A64_P)
+#define A64_W 4                     // warps per CTA
+
+// 1 / d for normal d in FP64: the hardware's approximate reciprocal r (relative error e, |e| < 2^-19)
+// and one third-order step r (1 + e + e^2), e = 1 - d r, which leaves e^3
+__device__ __forceinline__ double rcp64(double d) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    double e = fma(-d, r, 1.0);
+    e = fma(e, e, e);
+    return fma(r, e, r);
+}
+
+struct Wing64 { double vv2, c2m1, twoA, c1; };
+struct Core64 { double vv, a, ua, cop; int ia, pad; };
+
+__device__ __forceinline__ double wing64(double t, const Wing64 &w) {
+    return fma(w.c1, t, w.c1) * rcp64(fma(t, t, w.twoA));
+}
+
+// HVoigt (voigt.f90:81-107) where s < 196, table row and weight of a given
+__device__ __forceinline__ double core64(const float *__restrict__ vtab, const Core64 &c, double av) {
+    if (c.ia > 0 && av < 8.0) {
+        const double fv = av * 125.0;
+        const int iv = min((int)fv, FSG_NVV - 1);
+        const double tv = fv - (double)iv;
+        const float *p0 = vtab + (c.ia - 1) * FSG_NV1 + iv, *p1 = p0 + FSG_NV1;
+        const float t00 = __ldg(p0), t01 = __ldg(p0 + 1), t10 = __ldg(p1), t11 = __ldg(p1 + 1);
+        const double c0 = (double)t00 + tv * (double)(t01 - t00), c1 = (double)t10 + tv * (double)(t11 - t10);
+        return (c0 + c.ua * (c1 - c0)) * c.cop;
+    }
+    const double a2 = c.a * c.a, v2 = av * av, p = v2 - a2 - 1.5, q = 2.0 * av * c.a;
+    const double dr = av * p - c.a * q, di = av * q + c.a * p;
+    return FSG_SQRTPIINV * ((p + 0.5) * di - q * dr) / (dr * dr + di * di) * c.cop;
+}
+
+struct Accum64Job {
+    int ntau, nwl, w0, w1;              // wavelengths w0 .. w1 (1-based) are filled
+    int tile0, ntiles, ngrp;            // first tile, tiles, depth groups of A64_D
+    const double *wave;
+    const LineHdr64 *hdr;
+    const double3 *p64;
+    const int *lo, *hi;                 // candidate rows of each tile of the grid
+    const double *heshf, *contstd, *anode, *aida;
+    const float *vtab;
+    double *lineopac;
+};
+
+__global__ void __launch_bounds__(32 * A64_W, 5) k_accum64(Accum64Job J) {
+    __shared__ int queue_s[A64_W][64];
+    __shared__ __align__(16) LineHdr64 hdr_s[A64_W][A64_G];
+    __shared__ __align__(16) Wing64 wing_s[A64_W][A64_G][A64_D];
+    __shared__ Core64 core_s[A64_W][A64_G][A64_D];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t item = (int64_t)blockIdx.x * A64_W + warp;
+    if (item >= (int64_t)J.ntiles * J.ngrp) return;      // warps are independent: no CTA barrier below
+    const int tile = J.tile0 + (int)(item / J.ngrp), t0 = (int)(item % J.ngrp) * A64_D;
+    const int ntau = J.ntau, lo = J.lo[tile], hi = J.hi[tile];
+    if (lo > hi) return;
+    const int first = max(tile * A64_TW + 1, J.w0), last = min(tile * A64_TW + A64_TW, J.w1);
+    int *queue = queue_s[warp];
+    double wv[A64_P], acc[A64_P][A64_D];
+    int pix[A64_P];                                      // 1-based
+#pragma unroll
+    for (int k = 0; k < A64_P; k++) {
+        pix[k] = tile * A64_TW + lane + 32 * k + 1;
+        wv[k] = J.wave[min(pix[k], J.nwl) - 1];
+#pragma unroll
+        for (int d = 0; d < A64_D; d++) acc[k][d] = 0.0;
+    }
+    const int tq = lane / A64_D, td = lane % A64_D;      // this lane's (line, depth) of a group
+    auto group = [&](int head, int n) {                  // n <= A64_G queued lines from head on
+        const bool mine = tq < n;
+        const int row = mine ? queue[(head + tq) & 63] : 0;
+        LineHdr64 h;
+        if (mine) {
+            h = J.hdr[row];
+            if (td == 0) hdr_s[warp][tq] = h;
+            Wing64 w = { 0.0, 1.0e3, 0.0, 0.0 };         // past the last depth: a term of 0
+            if (t0 + td < ntau) {
+                const double3 p = J.p64[(size_t)row * ntau + t0 + td];
+                const double a2 = p.z * p.z;
+                w.vv2 = p.y * p.y; w.c2m1 = a2 - 0.5; w.twoA = 2.0 * a2; w.c1 = p.x * p.z * FSG_SQRTPIINV;
+                if (h.ihe > 0 || (h.cl <= h.cr && h.cr >= first && h.cl <= last)) {
+                    Core64 c;
+                    c.vv = p.y; c.a = p.z; c.cop = p.x; c.pad = 0;
+                    // table row and weight as HVoigt takes them (voigt.f90:84-92); ia = 0: a >= 8
+                    if (!(p.z < 8.0)) { c.ia = 0; c.ua = 0.0; }
+                    else if (p.z < J.anode[1]) { c.ia = 1; c.ua = p.z * J.aida[0]; }
+                    else {
+                        c.ia = min((int)(sqrt(p.z) * (1.0 / (2.8284271247461903 / 400.0))) + 1, FSG_NVA);
+                        c.ua = (p.z - J.anode[c.ia - 1]) * J.aida[c.ia - 1];
+                    }
+                    core_s[warp][tq][td] = c;
+                }
+            }
+            wing_s[warp][tq][td] = w;
+        }
+        __syncwarp();
+        for (int q = 0; q < n; q++) {
+            const LineHdr64 g = hdr_s[warp][q];
+            double dl[A64_P], x[A64_P];
+#pragma unroll
+            for (int k = 0; k < A64_P; k++) { dl[k] = wv[k] - g.wlc; x[k] = dl[k] * dl[k]; }
+            if (g.ihe > 0 || (g.cl <= g.cr && g.cr >= first && g.cl <= last)) {
+                const int nd = min(A64_D, ntau - t0);
+#pragma unroll
+                for (int d = 0; d < A64_D; d++) {
+                    if (d >= nd) break;
+                    const Wing64 w = wing_s[warp][q][d];
+                    const double sh = g.ihe > 0 ? J.heshf[(size_t)(g.ihe - 1) * ntau + t0 + d] : 0.0;
+#pragma unroll
+                    for (int k = 0; k < A64_P; k++) {
+                        if (pix[k] < g.il || pix[k] > g.ir) continue;
+                        const double dk = dl[k] - sh, t = fma(dk * dk, w.vv2, w.c2m1);
+                        const Core64 &c = core_s[warp][q][d];
+                        if (t >= 195.5) acc[k][d] += wing64(t, w);
+                        else acc[k][d] += core64(J.vtab, c, fabs(dk) * c.vv);
+                    }
+                }
+            } else if (g.il <= first && g.ir >= last) {
+#pragma unroll
+                for (int d = 0; d < A64_D; d++) {
+                    const Wing64 w = wing_s[warp][q][d];
+#pragma unroll
+                    for (int k = 0; k < A64_P; k++) acc[k][d] += wing64(fma(x[k], w.vv2, w.c2m1), w);
+                }
+            } else {
+                bool in[A64_P];
+#pragma unroll
+                for (int k = 0; k < A64_P; k++) in[k] = pix[k] >= g.il && pix[k] <= g.ir;
+#pragma unroll
+                for (int d = 0; d < A64_D; d++) {
+                    const Wing64 w = wing_s[warp][q][d];
+#pragma unroll
+                    for (int k = 0; k < A64_P; k++) {
+                        const double v = wing64(fma(x[k], w.vv2, w.c2m1), w);
+                        if (in[k]) acc[k][d] += v;
+                    }
+                }
+            }
+        }
+        __syncwarp();                                    // the group's shared records may be replaced
+    };
+    int head = 0, cnt = 0;
+    for (int base = lo; base <= hi; base += 32) {
+        const int j = base + lane;
+        bool sel = false;
+        if (j <= hi) {
+            const int2 w = *(const int2 *)&J.hdr[j].il;
+            sel = w.x <= w.y && w.x <= last && w.y >= first;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, sel);
+        if (!m) continue;
+        if (sel) queue[(head + cnt + __popc(m & ((1u << lane) - 1u))) & 63] = j;
+        cnt += __popc(m);
+        __syncwarp();
+        while (cnt >= A64_G) { group(head, A64_G); head += A64_G; cnt -= A64_G; }
+    }
+    if (cnt > 0) group(head, cnt);
+#pragma unroll
+    for (int k = 0; k < A64_P; k++) {
+        if (pix[k] < J.w0 || pix[k] > J.w1) continue;
+        double *dst = J.lineopac + (size_t)(pix[k] - 1) * ntau + t0;
+#pragma unroll
+        for (int d = 0; d < A64_D; d++)
+            if (t0 + d < ntau) dst[d] += J.contstd ? acc[k][d] / J.contstd[t0 + d] : acc[k][d];
+    }
+}
+
+int fsg_accum64_tile() { return A64_TW; }
+
+// rows hdr / p64 with the tile ranges lo / hi (tiles of fsg_accum64_tile() wavelengths of the whole grid) onto
+// LineOpac at the wavelengths w0 .. w1 (1-based, inclusive)
+int fsg_launch_accum64(cudaStream_t s, const AtmView &A, const LineHdr64 *hdr, const double3 *p64, const int *lo,
+                       const int *hi, int w0, int w1, const VoigtTables &T, double *lineopac) {
+    if (w1 < w0) return FSG_OK;
+    Accum64Job J;
+    J.ntau = A.ntau; J.nwl = A.nwl; J.w0 = w0; J.w1 = w1;
+    J.tile0 = (w0 - 1) / A64_TW;
+    J.ntiles = (w1 - 1) / A64_TW - J.tile0 + 1;
+    J.ngrp = (A.ntau + A64_D - 1) / A64_D;
+    J.wave = A.wave; J.hdr = hdr; J.p64 = p64; J.lo = lo; J.hi = hi;
+    J.heshf = A.heshf; J.contstd = A.motype == 1 ? A.contstd : nullptr;
+    J.anode = T.anode; J.aida = T.aida; J.vtab = T.vtab; J.lineopac = lineopac;
+    const int64_t items = (int64_t)J.ntiles * J.ngrp;
+    k_accum64<<<(unsigned)((items + A64_W - 1) / A64_W), 32 * A64_W, 0, s>>>(J);
+    return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
+}

@@ -83,15 +83,13 @@ void fsg_launch_center(cudaStream_t, const AtmView &, const LineView &, const Vo
 void fsg_launch_params_fast(cudaStream_t, const AtmView &, const LineView &, const int64_t *, int64_t, int64_t,
                             int64_t, const int32_t *, const int32_t *, const int32_t *, const VoigtTables &,
                             WingRec *, CoreRec *, LineHdr *);
-void fsg_launch_params_fp64(cudaStream_t, const AtmView &, const LineView &, int64_t, int64_t, const int32_t *,
-                            double3 *);
+void fsg_launch_params_fp64(cudaStream_t, const AtmView &, const LineView &, const int64_t *, int64_t, int64_t, int,
+                            const int32_t *, const int32_t *, const int32_t *, double3 *, LineHdr64 *);
+int fsg_launch_tile_span64(cudaStream_t, int, int, int64_t, const LineHdr64 *, int *, int *, void *, size_t);
+int fsg_accum64_tile();
+int fsg_launch_accum64(cudaStream_t, const AtmView &, const LineHdr64 *, const double3 *, const int *, const int *, int,
+                       int, const VoigtTables &, double *);
 void fsg_launch_span(cudaStream_t, int64_t, const int32_t *, const int32_t *, const int32_t *, int *, int *);
-void fsg_launch_accum_fp64(cudaStream_t, const AtmView &, const double *, int, int, const int *, const int *,
-                           const int32_t *, const int32_t *, const int32_t *, int64_t, const double3 *,
-                           const VoigtTables &, double *, double *);
-void fsg_launch_wide_fp64(cudaStream_t, const AtmView &, const LineView &, int, const int64_t *, const int32_t *,
-                          const int32_t *, const int32_t *, double3 *, const VoigtTables &, int, int, double *,
-                          double *);
 int fsg_launch_radtran(cudaStream_t, const AtmView &, const double *, const double *, int, const double *,
                        const double *, double *, double *, double *, double *);
 void fsg_launch_hvoigt(cudaStream_t, int64_t, const double *, const double *, double *, const VoigtTables &);
@@ -231,7 +229,7 @@ struct fsg_ctx {
     DBuf l_wl, l_elo, l_gf, l_grad, l_gqst, l_gvdw, l_spc, l_ismol, l_ihe;
     DBuf d_flags, d_ileft, d_iright, d_idx, d_counts, d_offs, d_total, d_hist, d_nkeep;
     // block buffers
-    DBuf d_wing, d_core, d_hdr, d_tlo, d_thi, d_p64, d_lstart, d_lstop, d_widx, d_pw, d_evals, d_err, d_ncore, d_span, d_lswork, d_linstr, d_rflags, d_rleft, d_rright, d_gkappa, d_adjwork, d_cbuf, d_ctaps;
+    DBuf d_wing, d_core, d_hdr, d_hdr64, d_tlo, d_thi, d_p64, d_lstart, d_lstop, d_widx, d_pw, d_evals, d_err, d_ncore, d_span, d_lswork, d_linstr, d_rflags, d_rleft, d_rright, d_gkappa, d_adjwork, d_cbuf, d_ctaps;
     // spectra
     DBuf d_spl, d_spc, d_sfl, d_sfc, d_work, d_a, d_v, d_h, d_l;
     // magnetic
@@ -322,7 +320,7 @@ void fsg_destroy(fsg_ctx *ctx) {
                      &ctx->d_wmu, &ctx->d_lineopac, &ctx->d_maglineopac, &ctx->l_wl, &ctx->l_elo, &ctx->l_gf,
                      &ctx->l_grad, &ctx->l_gqst, &ctx->l_gvdw, &ctx->l_spc, &ctx->l_ismol, &ctx->l_ihe,
                      &ctx->d_flags, &ctx->d_ileft, &ctx->d_iright, &ctx->d_idx, &ctx->d_counts, &ctx->d_offs,
-                     &ctx->d_total, &ctx->d_hist, &ctx->d_nkeep, &ctx->d_wing, &ctx->d_core, &ctx->d_hdr,
+                     &ctx->d_total, &ctx->d_hist, &ctx->d_nkeep, &ctx->d_wing, &ctx->d_core, &ctx->d_hdr, &ctx->d_hdr64,
                      &ctx->d_tlo, &ctx->d_thi, &ctx->d_err, &ctx->d_ncore, &ctx->d_span, &ctx->d_lswork, &ctx->d_linstr, &ctx->d_rflags, &ctx->d_rleft, &ctx->d_rright, &ctx->d_gkappa, &ctx->d_adjwork, &ctx->d_cbuf, &ctx->d_ctaps, &ctx->d_p64, &ctx->d_lstart, &ctx->d_lstop, &ctx->d_widx,
                      &ctx->d_pw, &ctx->d_evals, &ctx->d_spl, &ctx->d_spc, &ctx->d_sfl, &ctx->d_sfc,
                      &ctx->d_work, &ctx->d_a, &ctx->d_v, &ctx->d_h, &ctx->d_l, &ctx->z_npi, &ctx->z_nsi,
@@ -698,6 +696,24 @@ static int central_pass(fsg_ctx *ctx, const LineView &LV, int64_t *nkeep) {
     return FSG_OK;
 }
 
+// FP64 rows of the lines list[0 .. nb) (list null: i0 .. i0 + nb) with their headers (d_hdr64) and the tile
+// ranges of k_accum64 (d_tlo, d_thi); lines with any flag of skip get an empty window
+static int rows64(fsg_ctx *ctx, const AtmView &A, const LineView &LV, const int64_t *list, int64_t i0, int64_t nb,
+                  int skip, const int32_t *fl, const int32_t *il, const int32_t *ir, DBuf &p64) {
+    const int ntiles = fsg_fast_tiles(ctx->nwl);
+    ALLOC(p64, sizeof(double3) * (size_t)nb * ctx->ntau);
+    ALLOC(ctx->d_hdr64, sizeof(LineHdr64) * (size_t)nb);
+    ALLOC(ctx->d_span, fsg_tile_span_scratch(nb));
+    ALLOC(ctx->d_tlo, sizeof(int) * ntiles); ALLOC(ctx->d_thi, sizeof(int) * ntiles);
+    fsg_launch_params_fp64(ctx->stream, A, LV, list, i0, nb, skip, fl, il, ir, p64.as<double3>(),
+                           ctx->d_hdr64.as<LineHdr64>());
+    if (fsg_launch_tile_span64(ctx->stream, fsg_accum64_tile(), ctx->nwl, nb, ctx->d_hdr64.as<LineHdr64>(),
+                               ctx->d_tlo.as<int>(), ctx->d_thi.as<int>(), ctx->d_span.p, ctx->d_span.cap))
+        return cuda_fail(ctx, cudaGetLastError(), "FP64 tile span");
+    ctx->launches += 7;
+    return FSG_OK;
+}
+
 // mixed-precision accumulation: classes by window width, blocks within a class
 // fl/il/ir: LinFlag, Ileft, Iright of the list (device); [i0, i1]: 1-based wavelength range to fill
 // (1..nwl for the whole grid).  Lines are classed by their full windows and evaluated over the part
@@ -800,8 +816,8 @@ static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, fsg_stats *st, cons
             nblocks++;
         }
     }
-    // He I lines with Stark-shifted profiles (hestark.f90): the FP64 per-wavelength kernel of the
-    // wide lines, which applies the per-depth shift (opacity.f90:297-346)
+    // He I lines with Stark-shifted profiles (hestark.f90): the FP64 tile kernel, which applies the
+    // per-depth shift (opacity.f90:297-346)
     if (ctx->nhe > 0) {
         int rc3 = fsg_select(s, n, sf, il, ir, -3, ctx->d_counts.as<int>(), ctx->d_offs.as<int64_t>(),
                              ctx->d_idx.as<int64_t>(), ctx->d_total.as<int64_t>());
@@ -811,11 +827,12 @@ static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, fsg_stats *st, cons
         CK(cudaStreamSynchronize(s), "He I lines");
         ctx->launches += 3;
         if (nhl > 0) {
-            ALLOC(ctx->d_pw, sizeof(double3) * nhl * nt);
-            ALLOC(ctx->d_evals, sizeof(double));
-            fsg_launch_wide_fp64(s, A, LV, (int)nhl, ctx->d_idx.as<int64_t>(), sf, wl_, wr_, ctx->d_pw.as<double3>(),
-                                 ctx->tab, i0, i1, ctx->d_lineopac.as<double>(), ctx->d_evals.as<double>());
-            ctx->launches += 2;
+            rc3 = rows64(ctx, A, LV, ctx->d_idx.as<int64_t>(), 0, nhl, FSG_F_WEAK, sf, wl_, wr_, ctx->d_pw);
+            if (rc3) return rc3;
+            if (fsg_launch_accum64(s, A, ctx->d_hdr64.as<LineHdr64>(), ctx->d_pw.as<double3>(), ctx->d_tlo.as<int>(),
+                                   ctx->d_thi.as<int>(), i0, i1, ctx->tab, ctx->d_lineopac.as<double>()))
+                return cuda_fail(ctx, cudaGetLastError(), "k_accum64");
+            ctx->launches += 1;
         }
     }
     CK(cudaGetLastError(), "fast accumulation");
@@ -886,34 +903,34 @@ static int accumulate_fp64(fsg_ctx *ctx, const LineView &LV, int64_t nkeep, fsg_
     ctx->launches += pack ? 5 : 1;
     unsigned long long nwide = 0;
     CK(cudaMemcpyAsync(&nwide, d_nw, sizeof nwide, cudaMemcpyDeviceToHost, s), "wide");
-    // Lstart/Lstop (synth.f90:955-978)
-    ALLOC(ctx->d_lstart, sizeof(int) * nwl); ALLOC(ctx->d_lstop, sizeof(int) * nwl);
-    {
-        std::vector<int> ls(nwl, (int)nw), le(nwl, 1);
-        CK(cudaMemcpyAsync(ctx->d_lstart.p, ls.data(), sizeof(int) * nwl, cudaMemcpyHostToDevice, s), "lstart");
-        CK(cudaMemcpyAsync(ctx->d_lstop.p, le.data(), sizeof(int) * nwl, cudaMemcpyHostToDevice, s), "lstop");
-        CK(cudaStreamSynchronize(s), "lstart");
-    }
-    fsg_launch_span(s, nw, pf, pl, pr, ctx->d_lstart.as<int>(), ctx->d_lstop.as<int>());
-    ctx->launches += 1;
-    ALLOC(ctx->d_evals, sizeof(double));
-    CK(cudaMemsetAsync(ctx->d_evals.p, 0, sizeof(double), s), "evals");
-    // wide lines: list, parameters, per-wavelength ordered accumulation
+    CK(cudaStreamSynchronize(s), "wide");
+    // wide lines, in line order
     if (nwide > 0) {
         ALLOC(ctx->d_widx, sizeof(int64_t) * nwide);
         fsg_select_wide(s, nw, pf, ctx->d_counts.as<int>(), ctx->d_offs.as<int64_t>(), ctx->d_widx.as<int64_t>(),
                         ctx->d_total.as<int64_t>());
-        ALLOC(ctx->d_pw, sizeof(double3) * nwide * nt);
-        fsg_launch_wide_fp64(s, A, W, (int)nwide, ctx->d_widx.as<int64_t>(), pf, pl, pr, ctx->d_pw.as<double3>(),
-                             ctx->tab, i0, i1, ctx->d_lineopac.as<double>(), ctx->d_evals.as<double>());
-        ctx->launches += 5;
+        int rc = rows64(ctx, A, W, ctx->d_widx.as<int64_t>(), 0, (int64_t)nwide, FSG_F_WEAK, pf, pl, pr, ctx->d_pw);
+        if (rc) return rc;
+        if (fsg_launch_accum64(s, A, ctx->d_hdr64.as<LineHdr64>(), ctx->d_pw.as<double3>(), ctx->d_tlo.as<int>(),
+                               ctx->d_thi.as<int>(), i0, i1, ctx->tab, ctx->d_lineopac.as<double>()))
+            return cuda_fail(ctx, cudaGetLastError(), "k_accum64");
+        ctx->launches += 4;
     }
-    // segment loop (synth.f90:1006-1088): choose segments on the host from Lstart/Lstop
-    std::vector<int> ls(nwl), le(nwl);
-    CK(cudaMemcpyAsync(ls.data(), ctx->d_lstart.p, sizeof(int) * nwl, cudaMemcpyDeviceToHost, s), "lstart");
-    CK(cudaMemcpyAsync(le.data(), ctx->d_lstop.p, sizeof(int) * nwl, cudaMemcpyDeviceToHost, s), "lstop");
-    CK(cudaStreamSynchronize(s), "lstart");
-    ALLOC(ctx->d_p64, sizeof(double3) * (size_t)std::min<int64_t>(nstep, nw) * nt);
+    // segment loop (synth.f90:1006-1088): choose segments on the host from Lstart/Lstop (synth.f90:955-978); a
+    // list that fits one block is one segment and needs neither
+    std::vector<int> ls, le;
+    if (nstep < nw) {
+        ls.assign(nwl, (int)nw); le.assign(nwl, 1);
+        ALLOC(ctx->d_lstart, sizeof(int) * nwl); ALLOC(ctx->d_lstop, sizeof(int) * nwl);
+        CK(cudaMemcpyAsync(ctx->d_lstart.p, ls.data(), sizeof(int) * nwl, cudaMemcpyHostToDevice, s), "lstart");
+        CK(cudaMemcpyAsync(ctx->d_lstop.p, le.data(), sizeof(int) * nwl, cudaMemcpyHostToDevice, s), "lstop");
+        fsg_launch_span(s, nw, pf, pl, pr, ctx->d_lstart.as<int>(), ctx->d_lstop.as<int>());
+        ctx->launches += 1;
+        CK(cudaStreamSynchronize(s), "lstart");         // the host arrays are reused below
+        CK(cudaMemcpyAsync(ls.data(), ctx->d_lstart.p, sizeof(int) * nwl, cudaMemcpyDeviceToHost, s), "lstart");
+        CK(cudaMemcpyAsync(le.data(), ctx->d_lstop.p, sizeof(int) * nwl, cudaMemcpyDeviceToHost, s), "lstop");
+        CK(cudaStreamSynchronize(s), "lstart");
+    }
     int64_t iline1 = 1, ilineb = 0;
     int iwl1 = 1;
     int64_t nblocks = 0;
@@ -942,15 +959,15 @@ static int accumulate_fp64(fsg_ctx *ctx, const LineView &LV, int64_t nkeep, fsg_
         if (ra <= rb) {
             if (iline1 != ilineb) {
                 ilineb = iline1;
-                fsg_launch_params_fp64(s, A, W, loff, iline2 - loff, pf, ctx->d_p64.as<double3>());
-                ctx->launches += 1;
+                int rc = rows64(ctx, A, W, nullptr, loff, iline2 - loff, FSG_F_WEAK | FSG_F_WIDE, pf, pl, pr, ctx->d_p64);
+                if (rc) return rc;
                 nblocks++;
             }
             cudaEvent_t ea = ctx->ev[4], eb = ctx->ev[5];
             cudaEventRecord(ea, s);
-            fsg_launch_accum_fp64(s, A, W.wl, ra, rb, ctx->d_lstart.as<int>(), ctx->d_lstop.as<int>(), pf, pl, pr,
-                                  loff, ctx->d_p64.as<double3>(), ctx->tab, ctx->d_lineopac.as<double>(),
-                                  ctx->d_evals.as<double>());
+            if (fsg_launch_accum64(s, A, ctx->d_hdr64.as<LineHdr64>(), ctx->d_p64.as<double3>(), ctx->d_tlo.as<int>(),
+                                   ctx->d_thi.as<int>(), ra, rb, ctx->tab, ctx->d_lineopac.as<double>()))
+                return cuda_fail(ctx, cudaGetLastError(), "k_accum64");
             CK(cudaGetLastError(), "fp64 accumulation");
             cudaEventRecord(eb, s);
             CK(cudaEventSynchronize(eb), "fp64 accumulation");
@@ -960,10 +977,10 @@ static int accumulate_fp64(fsg_ctx *ctx, const LineView &LV, int64_t nkeep, fsg_
         if (iwl2 == nwl) break;
         iwl1 = iwl2 + 1;
     }
-    double ev = 0;
-    CK(cudaMemcpyAsync(&ev, ctx->d_evals.p, sizeof ev, cudaMemcpyDeviceToHost, s), "evals");
-    CK(cudaStreamSynchronize(s), "fp64 accumulation");
-    if (st) { st->nwide = (int64_t)nwide; st->nblocks = nblocks; st->line_evals = ev; }
+    if (st) {
+        st->nwide = (int64_t)nwide; st->nblocks = nblocks;
+        st->line_evals = count_windows(ctx, nw, pf, pl, pr, i0, i1) * nt;
+    }
     // per-line outputs in original order: scatter the packed wide flags back
     if (pack) {
         fsg_launch_scatter_flags(s, nw, ctx->d_idx.as<int64_t>(), pf, ctx->d_flags.as<int32_t>());

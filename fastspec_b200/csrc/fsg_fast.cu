@@ -668,6 +668,30 @@ int fsg_launch_tile_span(cudaStream_t s, int cls, int nwl, int64_t nb, const Lin
                                    scratch, scratch_bytes);
 }
 
+// as k_span_extract, over the windows of FP64 headers
+__global__ void k_span_extract64(int nb, const LineHdr64 *__restrict__ hdr, int *right, int *rev_left) {
+    int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= nb) return;
+    int l = hdr[j].il, r = hdr[j].ir;
+    if (l > r) { l = 0x7fffffff; r = -1; }
+    right[j] = r;
+    rev_left[nb - 1 - j] = l;
+}
+
+// scans of the extracted spans, then one binary search per tile; scratch: fsg_tile_span_scratch(nb) bytes,
+// its first 2 nb ints the spans
+static int tile_search(cudaStream_t s, int tw, int nwl, int64_t nb, int *lo, int *hi, void *scratch,
+                       size_t scratch_bytes) {
+    const int ntiles = (nwl + tw - 1) / tw;
+    int *right = (int *)scratch, *revl = right + nb, *R = revl + nb, *V = R + nb;
+    void *tmp = (void *)(((uintptr_t)(V + nb) + 255) & ~(uintptr_t)255);
+    size_t tb = scratch_bytes - ((char *)tmp - (char *)scratch);
+    if (cub::DeviceScan::InclusiveScan(tmp, tb, right, R, cuda::maximum<>{}, (int)nb, s) != cudaSuccess) return FSG_E_CUDA;
+    if (cub::DeviceScan::InclusiveScan(tmp, tb, revl, V, cuda::minimum<>{}, (int)nb, s) != cudaSuccess) return FSG_E_CUDA;
+    k_tile_search<<<(ntiles + 255) / 256, 256, 0, s>>>((int)nb, ntiles, tw, nwl, R, V, lo, hi);
+    return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
+}
+
 // tile ranges for tiles of tw wavelengths over the windows (use_core = 0) or the core ranges
 int fsg_launch_tile_span_tw(cudaStream_t s, int tw, int use_core, int nwl, int64_t nb, const LineHdr *hdr, int *lo,
                             int *hi, void *scratch, size_t scratch_bytes) {
@@ -676,14 +700,17 @@ int fsg_launch_tile_span_tw(cudaStream_t s, int tw, int use_core, int nwl, int64
         k_tile_reset<<<(ntiles + 255) / 256, 256, 0, s>>>(ntiles, lo, hi);
         return FSG_OK;
     }
-    int *right = (int *)scratch, *revl = right + nb, *R = revl + nb, *V = R + nb;
-    void *tmp = (void *)(((uintptr_t)(V + nb) + 255) & ~(uintptr_t)255);
-    size_t tb = scratch_bytes - ((char *)tmp - (char *)scratch);
+    int *right = (int *)scratch, *revl = right + nb;
     k_span_extract<<<(unsigned)((nb + 255) / 256), 256, 0, s>>>((int)nb, use_core, hdr, right, revl);
-    if (cub::DeviceScan::InclusiveScan(tmp, tb, right, R, cuda::maximum<>{}, (int)nb, s) != cudaSuccess) return FSG_E_CUDA;
-    if (cub::DeviceScan::InclusiveScan(tmp, tb, revl, V, cuda::minimum<>{}, (int)nb, s) != cudaSuccess) return FSG_E_CUDA;
-    k_tile_search<<<(ntiles + 255) / 256, 256, 0, s>>>((int)nb, ntiles, tw, nwl, R, V, lo, hi);
-    return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
+    return tile_search(s, tw, nwl, nb, lo, hi, scratch, scratch_bytes);
+}
+
+// the same over the windows of FP64 headers (nb > 0)
+int fsg_launch_tile_span64(cudaStream_t s, int tw, int nwl, int64_t nb, const LineHdr64 *hdr, int *lo, int *hi,
+                           void *scratch, size_t scratch_bytes) {
+    int *right = (int *)scratch, *revl = right + nb;
+    k_span_extract64<<<(unsigned)((nb + 255) / 256), 256, 0, s>>>((int)nb, hdr, right, revl);
+    return tile_search(s, tw, nwl, nb, lo, hi, scratch, scratch_bytes);
 }
 
 // Restriction to the wavelength range [i0, i1]: lines whose window misses it are marked weak for the

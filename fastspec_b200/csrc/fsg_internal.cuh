@@ -91,6 +91,12 @@ static_assert(sizeof(CoreRec) == 32, "core record: 32 bytes");
 // range of a partly covered tile); the magnetic pass keeps its He I table index there.
 struct __align__(16) LineHdr { float wlh, wll; int ileft, iright; int cl, cr, pad0, pad1; };
 
+// Line header of the FP64 tile kernels: the centre offset Wlcent, the window, the core range [cl, cr]
+// (every wavelength of the window where some depth may have s < 196, He I shifts included; cl > cr:
+// none) and the He I Stark table entry (0: none).  Lines a launch leaves out have an empty window.
+struct __align__(16) LineHdr64 { double wlc; int il, ir, cl, cr, ihe, pad; };
+static_assert(sizeof(LineHdr64) == 32, "FP64 header: 32 bytes");
+
 // Zeeman components of a device line list (CSR by line)
 struct ZView {
     const int32_t *npi, *nsi;

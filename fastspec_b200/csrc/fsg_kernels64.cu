@@ -5,9 +5,8 @@
 //   k_center        LineopCalc central pass (synth.f90:833-907): XlineSetup + XlineDepth,
 //                   weak-line bound and centre tests, AnalyticWindow + WaveIdx windows
 //   k_params_fast   block refill (synth.f90:1049-1070) into FP32 wing/core records
-//   k_params_fp64   block refill into FP64 (LinCop, LinVvgt, LinAvgt) for the plain path
-//   k_span, k_accum_fp64, k_wide_fp64   plain FP64 LineOpacity1 gather (opacity.f90:297-346)
-//                   and the wide-line accumulation (synth.f90:981-1001)
+//   k_params_fp64   block refill into FP64 (LinCop, LinVvgt, LinAvgt) and headers for the plain path
+//   k_span          Lstart/Lstop of the plain path's segments (synth.f90:955-978)
 //   k_radtran       RadTranCalc (synth.f90:1825-1866) + DiskInteg quadrature (convol.f90:233-234)
 //   k_radtran_sph   RadTranCalc for spherical models (synth.f90:1868-1898): LocPrfSph along each ray
 //   k_linstr        LinStrCalc (synth.f90:1774-1822), both geometries
@@ -368,33 +367,62 @@ void fsg_launch_params_fast(cudaStream_t s, const AtmView &A, const LineView &L,
                                                                             iright, T.anode, T.aida, wing, core, hdr);
 }
 
-// FP64 parameters for the plain path: p64[j][t] = (LinCop, LinVvgt, LinAvgt)
-__global__ void k_params_fp64(AtmView A, LineView L, int64_t i0, int64_t nb,
-                              const int32_t *__restrict__ flags, double3 *p64) {
-    int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nb) return;
-    int64_t i = i0 + j;
-    int f = flags[i];
-    if (f & FSG_F_WEAK) return;
-    double wlc = L.wl[i] - A.wfirst;
+// FP64 records of the plain path: row q holds the list line list[q] (list null: i0 + q) as
+// p64[q][t] = (LinCop, LinVvgt, LinAvgt) and its header.  Lines with any flag of skip get an empty
+// window.  One warp per line, lanes over depths: XlineDepth's FP64 chain is long, and a thread per line
+// walked all depths one after another (84 + 71 us for the 19,362 lines of a 200 A solar list, narrow and wide).
+__global__ void __launch_bounds__(128)
+k_params_fp64(AtmView A, LineView L, const int64_t *__restrict__ list, int64_t i0, int64_t nb, int skip,
+              const int32_t *__restrict__ flags, const int32_t *__restrict__ ileft,
+              const int32_t *__restrict__ iright, double3 *p64, LineHdr64 *hdr) {
+    const int64_t q = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (q >= nb) return;                                // whole warps leave together
+    const int64_t i = list ? list[q] : i0 + q;
+    const int f = flags[i], nt = A.ntau;
+    LineHdr64 h;
+    h.wlc = L.wl[i] - A.wfirst;
+    h.il = 1; h.ir = 0; h.cl = 1; h.cr = 0; h.ihe = (f >> 8) & 255; h.pad = 0;
+    if (f & skip) { if (lane == 0) hdr[q] = h; return; }
     XCoef XC;
-    xline_setup(A, L, i, wlc, f, &XC);
-    for (int t = 0; t < A.ntau; t++) {
+    xline_setup(A, L, i, h.wlc, f, &XC);
+    double hcore = -1.0, shmax = 0.0;
+    for (int t = lane; t < nt; t += 32) {
         double cop, vv, av;
         xline_depth(A, t, XC, &cop, &vv, &av);
-        p64[(size_t)j * A.ntau + t] = make_double3(cop, vv, av);
+        p64[(size_t)q * nt + t] = make_double3(cop, vv, av);
+        const double r = 196.05 - av * av;
+        if (r > 0.0) hcore = fmax(hcore, sqrt(r) / vv * (1.0 + 1e-5));
+        if (h.ihe > 0) shmax = fmax(shmax, fabs(A.heshf[(size_t)(h.ihe - 1) * nt + t]));
     }
+    for (int o = 16; o > 0; o >>= 1) {
+        hcore = fmax(hcore, __shfl_xor_sync(0xffffffffu, hcore, o));
+        shmax = fmax(shmax, __shfl_xor_sync(0xffffffffu, shmax, o));
+    }
+    if (lane != 0) return;
+    h.il = ileft[i]; h.ir = iright[i];
+    if (hcore >= 0.0) {
+        // 1-based indices of the first wavelength >= wlc - half and the last <= wlc + half, widened by one
+        // and clipped to the window
+        const double half = hcore + shmax;
+        int a = lower_index(A.wave, A.nwl, h.wlc - half) + 1;
+        int b = lower_index(A.wave, A.nwl, h.wlc + half);
+        if (b < A.nwl && A.wave[b] == h.wlc + half) b++;
+        const int cl = max(a - 1, h.il), cr = min(b + 1, h.ir);
+        if (cl <= cr) { h.cl = cl; h.cr = cr; }
+    }
+    hdr[q] = h;
 }
 
-void fsg_launch_params_fp64(cudaStream_t s, const AtmView &A, const LineView &L, int64_t i0, int64_t nb,
-                            const int32_t *flags, double3 *p64) {
+void fsg_launch_params_fp64(cudaStream_t s, const AtmView &A, const LineView &L, const int64_t *list, int64_t i0,
+                            int64_t nb, int skip, const int32_t *flags, const int32_t *il, const int32_t *ir,
+                            double3 *p64, LineHdr64 *hdr) {
     if (nb <= 0) return;
-    k_params_fp64<<<(unsigned)((nb + 127) / 128), 128, 0, s>>>(A, L, i0, nb, flags, p64);
+    k_params_fp64<<<(unsigned)((nb + 3) / 4), 128, 0, s>>>(A, L, list, i0, nb, skip, flags, il, ir, p64, hdr);
 }
 
 // ================================================================================================
-// Plain FP64 path: Lstart/Lstop pointers (synth.f90:955-978), wide lines (synth.f90:981-1001)
-// and the per-wavelength gather LineOpacity1 (opacity.f90:297-346).
+// Plain FP64 path: Lstart/Lstop pointers (synth.f90:955-978); the sums are in fsg_accum64.cu.
 // ================================================================================================
 __global__ void k_span(int64_t n, const int32_t *flags, const int32_t *ileft, const int32_t *iright,
                        int *lstart, int *lstop) {
@@ -412,124 +440,6 @@ void fsg_launch_span(cudaStream_t s, int64_t n, const int32_t *flags, const int3
                      const int32_t *iright, int *lstart, int *lstop) {
     if (n <= 0) return;
     k_span<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(n, flags, ileft, iright, lstart, lstop);
-}
-
-// One warp per wavelength; lanes stride the depths.  Lines l1..l2 (1-based), block offset loff.
-#define FP64_MAXD 4   // up to 128 depths
-__global__ void k_accum_fp64(AtmView A, const double *__restrict__ wl, int iwl1, int iwl2,
-                             const int *__restrict__ lstart, const int *__restrict__ lstop,
-                             const int32_t *__restrict__ flags, const int32_t *__restrict__ ileft,
-                             const int32_t *__restrict__ iright, int64_t loff, const double3 *__restrict__ p64,
-                             const float *__restrict__ vtab, const double *__restrict__ anode,
-                             const double *__restrict__ aida, double *lineopac, double *evals) {
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    int iwl = iwl1 + warp;
-    if (iwl > iwl2) return;
-    const int nt = A.ntau;
-    double acc[FP64_MAXD];
-#pragma unroll
-    for (int k = 0; k < FP64_MAXD; k++) acc[k] = 0.0;
-    double Wl = A.wave[iwl - 1];
-    int l1 = lstart[iwl - 1], l2 = lstop[iwl - 1];
-    double cnt = 0.0;
-    for (int il = l1; il <= l2; il++) {
-        int f = flags[il - 1];
-        if ((f & FSG_F_WEAK) || (f & FSG_F_WIDE) || iwl < ileft[il - 1] || iwl > iright[il - 1]) continue;
-        int ihe = (f >> 8) & 255;
-        double dWl0 = Wl - (wl[il - 1] - A.wfirst);
-        const double3 *p = p64 + (size_t)(il - 1 - loff) * nt;
-#pragma unroll
-        for (int k = 0; k < FP64_MAXD; k++) {
-            int t = lane + 32 * k;
-            if (t < nt) {
-                double dWl = dWl0;
-                if (ihe > 0) dWl = dWl0 - A.heshf[(ihe - 1) * nt + t];
-                double3 q = p[t];
-                double V = dWl * q.y;
-                acc[k] = acc[k] + hvoigt64(vtab, anode, aida, q.z, V) * q.x;
-            }
-        }
-        cnt += 1.0;
-    }
-    double *dst = lineopac + (size_t)(iwl - 1) * nt;
-#pragma unroll
-    for (int k = 0; k < FP64_MAXD; k++) {
-        int t = lane + 32 * k;
-        if (t < nt) {
-            double v = acc[k];
-            if (A.motype == 1) v = v / A.contstd[t];
-            dst[t] = dst[t] + v;
-        }
-    }
-    if (lane == 0 && cnt > 0.0) atomicAdd(evals, cnt * nt);
-}
-
-void fsg_launch_accum_fp64(cudaStream_t s, const AtmView &A, const double *wl, int iwl1, int iwl2,
-                           const int *lstart, const int *lstop, const int32_t *flags, const int32_t *ileft,
-                           const int32_t *iright, int64_t loff, const double3 *p64, const VoigtTables &T,
-                           double *lineopac, double *evals) {
-    int nw = iwl2 - iwl1 + 1;
-    if (nw <= 0) return;
-    k_accum_fp64<<<(nw + 7) / 8, 256, 0, s>>>(A, wl, iwl1, iwl2, lstart, lstop, flags, ileft, iright, loff,
-                                              p64, T.vtab, T.anode, T.aida, lineopac, evals);
-}
-
-// Wide lines, in line order, each over its own window (LineOpacity2): one warp per wavelength,
-// looping over the wide-line list so the per-wavelength additions keep the reference's order.
-__global__ void k_wide_fp64(AtmView A, LineView L, int nwide, const int64_t *__restrict__ widx,
-                            const int32_t *__restrict__ flags, const int32_t *__restrict__ ileft,
-                            const int32_t *__restrict__ iright, const double3 *__restrict__ pw,
-                            const float *__restrict__ vtab, const double *__restrict__ anode,
-                            const double *__restrict__ aida, int wlo, int whi, double *lineopac,
-                            double *evals) {
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    int iwl = wlo + warp;
-    if (iwl > whi) return;
-    const int nt = A.ntau;
-    double Wl = A.wave[iwl - 1];
-    double *dst = lineopac + (size_t)(iwl - 1) * nt;
-    double cnt = 0.0;
-    for (int q = 0; q < nwide; q++) {
-        int64_t i = widx[q];
-        if (iwl < ileft[i] || iwl > iright[i]) continue;
-        int f = flags[i], ihe = (f >> 8) & 255;
-        double dWl0 = Wl - (L.wl[i] - A.wfirst);
-        for (int t = lane; t < nt; t += 32) {
-            double dWl = dWl0;
-            if (ihe > 0) dWl = dWl0 - A.heshf[(ihe - 1) * nt + t];
-            double3 p = pw[(size_t)q * nt + t];
-            double v = hvoigt64(vtab, anode, aida, p.z, dWl * p.y) * p.x;
-            if (A.motype == 1) v = v / A.contstd[t];
-            dst[t] = dst[t] + v;
-        }
-        cnt += 1.0;
-    }
-    if (lane == 0 && cnt > 0.0) atomicAdd(evals, cnt * nt);
-}
-
-__global__ void k_params_wide(AtmView A, LineView L, int nwide, const int64_t *widx,
-                              const int32_t *flags, double3 *pw) {
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nwide) return;
-    int64_t i = widx[q];
-    double wlc = L.wl[i] - A.wfirst;
-    XCoef XC;
-    xline_setup(A, L, i, wlc, flags[i], &XC);
-    for (int t = 0; t < A.ntau; t++) {
-        double cop, vv, av;
-        xline_depth(A, t, XC, &cop, &vv, &av);
-        pw[(size_t)q * A.ntau + t] = make_double3(cop, vv, av);
-    }
-}
-
-void fsg_launch_wide_fp64(cudaStream_t s, const AtmView &A, const LineView &L, int nwide, const int64_t *widx,
-                          const int32_t *flags, const int32_t *ileft, const int32_t *iright, double3 *pw,
-                          const VoigtTables &T, int wlo, int whi, double *lineopac, double *evals) {
-    if (nwide <= 0 || whi < wlo) return;
-    k_params_wide<<<(nwide + 63) / 64, 64, 0, s>>>(A, L, nwide, widx, flags, pw);
-    int nw = whi - wlo + 1;
-    k_wide_fp64<<<(nw + 7) / 8, 256, 0, s>>>(A, L, nwide, widx, flags, ileft, iright, pw, T.vtab, T.anode,
-                                             T.aida, wlo, whi, lineopac, evals);
 }
 
 // ================================================================================================
