@@ -1,5 +1,5 @@
-// fsg_accum64.cu -- plain FP64 line opacity: LineOpacity1 (opacity.f90:297-346) and the wide lines
-// (synth.f90:981-1001) on wavelength tiles.
+// fsg_accum64.cu -- plain FP64 line opacity on wavelength tiles: LineOpacity1 (opacity.f90:297-346) with the
+// wide lines (synth.f90:981-1001), and MagLineOpacity1/3 (opacity.f90:391-464, 526-591).
 //
 //   LineOpac(t, p) += sum over lines l with Ileft(l) <= p <= Iright(l) of HVoigt(a(l,t), v) LinCop(l,t)
 //
@@ -59,6 +59,40 @@ __device__ __forceinline__ double core64(const float *__restrict__ vtab, const C
     return FSG_SQRTPIINV * ((p + 0.5) * di - q * dr) / (dr * dr + di * di) * c.cop;
 }
 
+// Rows lo .. hi whose windows meet the wavelengths first .. last, in order: group(head, n) gets them G at a
+// time (the last call fewer) as queue[(head + i) & 63], i < n; queue holds 64 rows of the calling warp.
+template <int G, class F>
+__device__ __forceinline__ void tile_lines(const LineHdr64 *__restrict__ hdr, int lo, int hi, int first, int last,
+                                           int *queue, int lane, F group) {
+    int head = 0, cnt = 0;
+    for (int base = lo; base <= hi; base += 32) {
+        const int j = base + lane;
+        bool sel = false;
+        if (j <= hi) {
+            const int2 w = *(const int2 *)&hdr[j].il;
+            sel = w.x <= w.y && w.x <= last && w.y >= first;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, sel);
+        if (!m) continue;
+        if (sel) queue[(head + cnt + __popc(m & ((1u << lane) - 1u))) & 63] = j;
+        cnt += __popc(m);
+        __syncwarp();
+        while (cnt >= G) { group(head, G); head += G; cnt -= G; }
+    }
+    if (cnt > 0) group(head, cnt);
+}
+
+// table row and weight of a as HVoigt takes them (voigt.f90:84-92); ia = 0: a >= 8
+__device__ __forceinline__ void table_row64(const double *__restrict__ anode, const double *__restrict__ aida, double a,
+                                            int &ia, double &ua) {
+    if (!(a < 8.0)) { ia = 0; ua = 0.0; }
+    else if (a < anode[1]) { ia = 1; ua = a * aida[0]; }
+    else {
+        ia = min((int)(sqrt(a) * (1.0 / (2.8284271247461903 / 400.0))) + 1, FSG_NVA);
+        ua = (a - anode[ia - 1]) * aida[ia - 1];
+    }
+}
+
 struct Accum64Job {
     int ntau, nwl, w0, w1;              // wavelengths w0 .. w1 (1-based) are filled
     int tile0, ntiles, ngrp;            // first tile, tiles, depth groups of A64_D
@@ -83,7 +117,7 @@ __global__ void __launch_bounds__(32 * A64_W, 5) k_accum64(Accum64Job J) {
     const int ntau = J.ntau, lo = J.lo[tile], hi = J.hi[tile];
     if (lo > hi) return;
     const int first = max(tile * A64_TW + 1, J.w0), last = min(tile * A64_TW + A64_TW, J.w1);
-    int *queue = queue_s[warp];
+    const int *queue = queue_s[warp];
     double wv[A64_P], acc[A64_P][A64_D];
     int pix[A64_P];                                      // 1-based
 #pragma unroll
@@ -109,13 +143,7 @@ __global__ void __launch_bounds__(32 * A64_W, 5) k_accum64(Accum64Job J) {
                 if (h.ihe > 0 || (h.cl <= h.cr && h.cr >= first && h.cl <= last)) {
                     Core64 c;
                     c.vv = p.y; c.a = p.z; c.cop = p.x; c.pad = 0;
-                    // table row and weight as HVoigt takes them (voigt.f90:84-92); ia = 0: a >= 8
-                    if (!(p.z < 8.0)) { c.ia = 0; c.ua = 0.0; }
-                    else if (p.z < J.anode[1]) { c.ia = 1; c.ua = p.z * J.aida[0]; }
-                    else {
-                        c.ia = min((int)(sqrt(p.z) * (1.0 / (2.8284271247461903 / 400.0))) + 1, FSG_NVA);
-                        c.ua = (p.z - J.anode[c.ia - 1]) * J.aida[c.ia - 1];
-                    }
+                    table_row64(J.anode, J.aida, p.z, c.ia, c.ua);
                     core_s[warp][tq][td] = c;
                 }
             }
@@ -167,22 +195,7 @@ __global__ void __launch_bounds__(32 * A64_W, 5) k_accum64(Accum64Job J) {
         }
         __syncwarp();                                    // the group's shared records may be replaced
     };
-    int head = 0, cnt = 0;
-    for (int base = lo; base <= hi; base += 32) {
-        const int j = base + lane;
-        bool sel = false;
-        if (j <= hi) {
-            const int2 w = *(const int2 *)&J.hdr[j].il;
-            sel = w.x <= w.y && w.x <= last && w.y >= first;
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, sel);
-        if (!m) continue;
-        if (sel) queue[(head + cnt + __popc(m & ((1u << lane) - 1u))) & 63] = j;
-        cnt += __popc(m);
-        __syncwarp();
-        while (cnt >= A64_G) { group(head, A64_G); head += A64_G; cnt -= A64_G; }
-    }
-    if (cnt > 0) group(head, cnt);
+    tile_lines<A64_G>(J.hdr, lo, hi, first, last, queue_s[warp], lane, group);
 #pragma unroll
     for (int k = 0; k < A64_P; k++) {
         if (pix[k] < J.w0 || pix[k] > J.w1) continue;
@@ -193,6 +206,19 @@ __global__ void __launch_bounds__(32 * A64_W, 5) k_accum64(Accum64Job J) {
     }
 }
 
+static Accum64Job accum64_job(const AtmView &A, const LineHdr64 *hdr, const double3 *p64, const int *lo, const int *hi,
+                              int w0, int w1, int tw, int depths, const VoigtTables &T, double *out) {
+    Accum64Job J;
+    J.ntau = A.ntau; J.nwl = A.nwl; J.w0 = w0; J.w1 = w1;
+    J.tile0 = (w0 - 1) / tw;
+    J.ntiles = (w1 - 1) / tw - J.tile0 + 1;
+    J.ngrp = (A.ntau + depths - 1) / depths;
+    J.wave = A.wave; J.hdr = hdr; J.p64 = p64; J.lo = lo; J.hi = hi;
+    J.heshf = A.heshf; J.contstd = A.motype == 1 ? A.contstd : nullptr;
+    J.anode = T.anode; J.aida = T.aida; J.vtab = T.vtab; J.lineopac = out;
+    return J;
+}
+
 int fsg_accum64_tile() { return A64_TW; }
 
 // rows hdr / p64 with the tile ranges lo / hi (tiles of fsg_accum64_tile() wavelengths of the whole grid) onto
@@ -200,15 +226,191 @@ int fsg_accum64_tile() { return A64_TW; }
 int fsg_launch_accum64(cudaStream_t s, const AtmView &A, const LineHdr64 *hdr, const double3 *p64, const int *lo,
                        const int *hi, int w0, int w1, const VoigtTables &T, double *lineopac) {
     if (w1 < w0) return FSG_OK;
-    Accum64Job J;
-    J.ntau = A.ntau; J.nwl = A.nwl; J.w0 = w0; J.w1 = w1;
-    J.tile0 = (w0 - 1) / A64_TW;
-    J.ntiles = (w1 - 1) / A64_TW - J.tile0 + 1;
-    J.ngrp = (A.ntau + A64_D - 1) / A64_D;
-    J.wave = A.wave; J.hdr = hdr; J.p64 = p64; J.lo = lo; J.hi = hi;
-    J.heshf = A.heshf; J.contstd = A.motype == 1 ? A.contstd : nullptr;
-    J.anode = T.anode; J.aida = T.aida; J.vtab = T.vtab; J.lineopac = lineopac;
+    Accum64Job J = accum64_job(A, hdr, p64, lo, hi, w0, w1, A64_TW, A64_D, T, lineopac);
     const int64_t items = (int64_t)J.ntiles * J.ngrp;
     k_accum64<<<(unsigned)((items + A64_W - 1) / A64_W), 32 * A64_W, 0, s>>>(J);
+    return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
+}
+
+// ---- magnetic lines ----------------------------------------------------------------------------------
+// MagLineOpac(6, t, p) += sum over lines and Zeeman components of (H, L)(a, v_k) LinCop Str_k with
+// v_k = (lambda - lambda_c - shift_k) LinVvgt, into the pi, blue and red absorption (H) and dispersion (L)
+// profiles.  As k_accum64 with one wavelength per lane and M64_D depths per warp (six sums each).  Outside
+// the line's core range (Zeeman shifts included) a component takes FVoigt's rational pair (voigt.f90:280-289)
+//   u = v^2, D = u (u + 2 a^2 - 1) + (a^2 + 1/2)^2,  H = a/sqrt(pi) h,  L = v/sqrt(pi) (h - 1/D),
+//   h = (u + a^2 + 1/2) / D
+// in 13 FP64 instructions (the FP64 pipe bounds it); LinCop a/sqrt(pi) and LinCop/sqrt(pi) multiply the
+// line's six sums once.
+#define M64_D 2
+#define M64_G (32 / M64_D)
+
+struct MagWing64 { double vv, b1, b0, ah, ch, cv; };
+
+// FVoigt's (H, L) where s < 196 (voigt.f90:256-352), L odd in v
+__device__ __forceinline__ void fcore64(const float2 *__restrict__ ftab, const Core64 &c, double v, double &H, double &L) {
+    const double av = fabs(v);
+    if (c.ia > 0 && av < 8.0) {
+        const double fv = av * 125.0;
+        const int iv = min((int)fv, FSG_NVV - 1);
+        const double tv = fv - (double)iv;
+        const float2 *p0 = ftab + (c.ia - 1) * FSG_NV1 + iv, *p1 = p0 + FSG_NV1;
+        const float2 t00 = __ldg(p0), t01 = __ldg(p0 + 1), t10 = __ldg(p1), t11 = __ldg(p1 + 1);
+        const double h0 = (double)t00.x + tv * (double)(t01.x - t00.x), h1 = (double)t10.x + tv * (double)(t11.x - t10.x);
+        const double l0 = (double)t00.y + tv * (double)(t01.y - t00.y), l1 = (double)t10.y + tv * (double)(t11.y - t10.y);
+        H = h0 + c.ua * (h1 - h0);
+        L = l0 + c.ua * (l1 - l0);
+    } else {
+        const double a2 = c.a * c.a, v2 = av * av, p = v2 - a2 - 1.5, q = 2.0 * av * c.a;
+        const double dr = av * p - c.a * q, di = av * q + c.a * p, w = FSG_SQRTPIINV / (dr * dr + di * di);
+        H = w * ((p + 0.5) * di - q * dr);
+        L = w * ((p + 0.5) * dr + q * di);
+    }
+    L = copysign(fabs(L), v);
+}
+
+__global__ void __launch_bounds__(32 * A64_W, 5) k_mag64(Accum64Job J, ZView Z, const float2 *__restrict__ ftab) {
+    __shared__ int queue_s[A64_W][64];
+    __shared__ __align__(16) LineHdr64 hdr_s[A64_W][M64_G];
+    __shared__ MagWing64 wing_s[A64_W][M64_G][M64_D];
+    __shared__ Core64 core_s[A64_W][M64_G][M64_D];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t item = (int64_t)blockIdx.x * A64_W + warp;
+    if (item >= (int64_t)J.ntiles * J.ngrp) return;      // warps are independent: no CTA barrier below
+    const int tile = J.tile0 + (int)(item / J.ngrp), t0 = (int)(item % J.ngrp) * M64_D;
+    const int ntau = J.ntau, lo = J.lo[tile], hi = J.hi[tile];
+    if (lo > hi) return;
+    const int first = max(tile * 32 + 1, J.w0), last = min(tile * 32 + 32, J.w1);
+    const int *queue = queue_s[warp];
+    const int pix = tile * 32 + lane + 1;                // 1-based
+    const double wv = J.wave[min(pix, J.nwl) - 1];
+    double acc[M64_D][6];
+#pragma unroll
+    for (int d = 0; d < M64_D; d++)
+#pragma unroll
+        for (int r = 0; r < 6; r++) acc[d][r] = 0.0;
+    const int tq = lane / M64_D, td = lane % M64_D;      // this lane's (line, depth) of a group
+    auto group = [&](int head, int n) {
+        if (tq < n) {
+            const int row = queue[(head + tq) & 63];
+            const LineHdr64 h = J.hdr[row];
+            if (td == 0) hdr_s[warp][tq] = h;
+            MagWing64 w = { 0.0, 0.0, 1.0, 0.0, 0.0, 0.0 };
+            if (t0 + td < ntau) {
+                const double3 p = J.p64[(size_t)row * ntau + t0 + td];
+                const double a2 = p.z * p.z;
+                w.vv = p.y; w.b1 = 2.0 * a2 - 1.0; w.ah = a2 + 0.5; w.b0 = w.ah * w.ah;
+                w.cv = p.x * FSG_SQRTPIINV; w.ch = w.cv * p.z;
+                Core64 c;
+                c.vv = p.y; c.a = p.z; c.cop = p.x; c.pad = 0;
+                if (h.cl <= h.cr && h.cr >= first && h.cl <= last) table_row64(J.anode, J.aida, p.z, c.ia, c.ua);
+                core_s[warp][tq][td] = c;
+            }
+            wing_s[warp][tq][td] = w;
+        }
+        __syncwarp();
+        for (int q = 0; q < n; q++) {
+            const LineHdr64 g = hdr_s[warp][q];
+            const double dl = wv - g.wlc;
+            const bool in = pix >= g.il && pix <= g.ir;
+            const int np = Z.npi[g.zi], ns = Z.nsi[g.zi], nsh = ns / 2;
+            const float *spi = Z.splpi + Z.pi_off[g.zi], *ssi = Z.splsi + Z.si_off[g.zi];
+            const float *rpi = Z.strpi + Z.pi_off[g.zi], *rsi = Z.strsi + Z.si_off[g.zi];
+            double vv[M64_D], vb[M64_D], s[M64_D][6];
+#pragma unroll
+            for (int d = 0; d < M64_D; d++) {
+                const int t = min(t0 + d, ntau - 1);
+                const double sh = g.ihe > 0 ? J.heshf[(size_t)(g.ihe - 1) * ntau + t] : 0.0;
+                vv[d] = wing_s[warp][q][d].vv;
+                vb[d] = (dl - sh) * vv[d];
+#pragma unroll
+                for (int r = 0; r < 6; r++) s[d][r] = 0.0;
+            }
+            if (g.cl > g.cr || g.cr < first || g.cl > last) {
+                double b1[M64_D], b0[M64_D], ah[M64_D];
+#pragma unroll
+                for (int d = 0; d < M64_D; d++) {
+                    b1[d] = wing_s[warp][q][d].b1; b0[d] = wing_s[warp][q][d].b0; ah[d] = wing_s[warp][q][d].ah;
+                }
+                auto comps = [&](const float *sp_, const float *st_, int k0, int k1, int r) {
+                    for (int k = k0; k < k1; k++) {
+                        const double sp = (double)sp_[k], st = (double)st_[k];
+#pragma unroll
+                        for (int d = 0; d < M64_D; d++) {
+                            const double v = fma(-sp, vv[d], vb[d]), u = v * v;
+                            const double rr = rcp64(fma(u, u + b1[d], b0[d]));
+                            const double hq = (u + ah[d]) * rr;
+                            s[d][r] = fma(st, hq, s[d][r]);
+                            s[d][r + 3] = fma(st, (hq - rr) * v, s[d][r + 3]);
+                        }
+                    }
+                };
+                comps(spi, rpi, 0, np, 0);
+                comps(ssi, rsi, 0, nsh, 1);
+                comps(ssi, rsi, nsh, ns, 2);
+                if (in) {
+#pragma unroll
+                    for (int d = 0; d < M64_D; d++) {
+                        const double ch = wing_s[warp][q][d].ch, cv = wing_s[warp][q][d].cv;
+#pragma unroll
+                        for (int r = 0; r < 3; r++) {
+                            acc[d][r] = fma(s[d][r], ch, acc[d][r]);
+                            acc[d][r + 3] = fma(s[d][r + 3], cv, acc[d][r + 3]);
+                        }
+                    }
+                }
+            } else if (in) {
+                auto comps = [&](const float *sp_, const float *st_, int k0, int k1, int r) {
+                    for (int k = k0; k < k1; k++) {
+                        const double sp = (double)sp_[k], st = (double)st_[k];
+#pragma unroll
+                        for (int d = 0; d < M64_D; d++) {
+                            if (t0 + d >= ntau) break;
+                            const Core64 &c = core_s[warp][q][d];
+                            const double v = fma(-sp, vv[d], vb[d]), u = v * v;
+                            double H, L;
+                            if (u + c.a * c.a >= 196.0) {
+                                const MagWing64 &w = wing_s[warp][q][d];
+                                const double rr = rcp64(fma(u, u + w.b1, w.b0)), hq = (u + w.ah) * rr;
+                                H = FSG_SQRTPIINV * c.a * hq; L = FSG_SQRTPIINV * (hq - rr) * v;
+                            } else fcore64(ftab, c, v, H, L);
+                            s[d][r] = fma(st, H, s[d][r]);
+                            s[d][r + 3] = fma(st, L, s[d][r + 3]);
+                        }
+                    }
+                };
+                comps(spi, rpi, 0, np, 0);
+                comps(ssi, rsi, 0, nsh, 1);
+                comps(ssi, rsi, nsh, ns, 2);
+#pragma unroll
+                for (int d = 0; d < M64_D; d++) {
+                    if (t0 + d >= ntau) break;
+                    const double cop = core_s[warp][q][d].cop;
+#pragma unroll
+                    for (int r = 0; r < 6; r++) acc[d][r] = fma(s[d][r], cop, acc[d][r]);
+                }
+            }
+        }
+        __syncwarp();                                    // the group's shared records may be replaced
+    };
+    tile_lines<M64_G>(J.hdr, lo, hi, first, last, queue_s[warp], lane, group);
+    if (pix < J.w0 || pix > J.w1) return;
+#pragma unroll
+    for (int d = 0; d < M64_D; d++) {
+        if (t0 + d >= ntau) break;
+        double *dst = J.lineopac + ((size_t)(pix - 1) * ntau + t0 + d) * 6;
+#pragma unroll
+        for (int r = 0; r < 6; r++) dst[r] += J.contstd ? acc[d][r] / J.contstd[t0 + d] : acc[d][r];
+    }
+}
+
+int fsg_mag64_tile() { return 32; }
+
+// as fsg_launch_accum64, onto MagLineOpac (tiles of fsg_mag64_tile() wavelengths)
+int fsg_launch_mag64(cudaStream_t s, const AtmView &A, const LineHdr64 *hdr, const double3 *p64, const ZView &Z,
+                     const int *lo, const int *hi, int w0, int w1, const VoigtTables &T, double *mlo) {
+    if (w1 < w0) return FSG_OK;
+    Accum64Job J = accum64_job(A, hdr, p64, lo, hi, w0, w1, 32, M64_D, T, mlo);
+    const int64_t items = (int64_t)J.ntiles * J.ngrp;
+    k_mag64<<<(unsigned)((items + A64_W - 1) / A64_W), 32 * A64_W, 0, s>>>(J, Z, T.fvtab);
     return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }

@@ -84,7 +84,11 @@ void fsg_launch_params_fast(cudaStream_t, const AtmView &, const LineView &, con
                             int64_t, const int32_t *, const int32_t *, const int32_t *, const VoigtTables &,
                             WingRec *, CoreRec *, LineHdr *);
 void fsg_launch_params_fp64(cudaStream_t, const AtmView &, const LineView &, const int64_t *, int64_t, int64_t, int,
-                            const int32_t *, const int32_t *, const int32_t *, double3 *, LineHdr64 *);
+                            const int32_t *, const int32_t *, const int32_t *, const ZView *, const int64_t *, double3 *,
+                            LineHdr64 *);
+int fsg_mag64_tile();
+int fsg_launch_mag64(cudaStream_t, const AtmView &, const LineHdr64 *, const double3 *, const ZView &, const int *,
+                     const int *, int, int, const VoigtTables &, double *);
 int fsg_launch_tile_span64(cudaStream_t, int, int, int64_t, const LineHdr64 *, int *, int *, void *, size_t);
 int fsg_accum64_tile();
 int fsg_launch_accum64(cudaStream_t, const AtmView &, const LineHdr64 *, const double3 *, const int *, const int *, int,
@@ -157,15 +161,6 @@ size_t fsg_stokes_work(int, int, int);
 int fsg_stokes_chunk(int, int, int, size_t);
 void fsg_launch_mag_center(cudaStream_t, const AtmView &, const LineView &, const ZView &, double, const VoigtTables &,
                            int32_t *, int32_t *, int32_t *, unsigned long long *);
-void fsg_launch_mag_params(cudaStream_t, const AtmView &, const LineView &, int64_t, const int64_t *, int64_t,
-                           const int32_t *, double3 *);
-void fsg_launch_mag_accum(cudaStream_t, const AtmView &, const double *, const ZView &, const int64_t *, int, int,
-                          const int *, const int *, const int32_t *, const int32_t *, const int32_t *, int64_t,
-                          const double3 *, const VoigtTables &, double *, double *);
-void fsg_launch_mag_wide(cudaStream_t, const AtmView &, const double *, const ZView &, const int64_t *, int,
-                         const int64_t *, const int32_t *, const int32_t *, const int32_t *, const double3 *,
-                         const VoigtTables &, double *);
-
 std::string fsg_cuda_msg(cudaError_t e, const char *what) {
     char b[512];
     snprintf(b, sizeof b, "%s: CUDA error %d (%s)", what, (int)e, cudaGetErrorString(e));
@@ -229,7 +224,7 @@ struct fsg_ctx {
     DBuf l_wl, l_elo, l_gf, l_grad, l_gqst, l_gvdw, l_spc, l_ismol, l_ihe;
     DBuf d_flags, d_ileft, d_iright, d_idx, d_counts, d_offs, d_total, d_hist, d_nkeep;
     // block buffers
-    DBuf d_wing, d_core, d_hdr, d_hdr64, d_tlo, d_thi, d_p64, d_lstart, d_lstop, d_widx, d_pw, d_evals, d_err, d_ncore, d_span, d_lswork, d_linstr, d_rflags, d_rleft, d_rright, d_gkappa, d_adjwork, d_cbuf, d_ctaps;
+    DBuf d_wing, d_core, d_hdr, d_hdr64, d_tlo, d_thi, d_p64, d_lstart, d_lstop, d_widx, d_pw, d_err, d_ncore, d_span, d_lswork, d_linstr, d_rflags, d_rleft, d_rright, d_gkappa, d_adjwork, d_cbuf, d_ctaps;
     // spectra
     DBuf d_spl, d_spc, d_sfl, d_sfc, d_work, d_a, d_v, d_h, d_l;
     // magnetic
@@ -322,7 +317,7 @@ void fsg_destroy(fsg_ctx *ctx) {
                      &ctx->d_flags, &ctx->d_ileft, &ctx->d_iright, &ctx->d_idx, &ctx->d_counts, &ctx->d_offs,
                      &ctx->d_total, &ctx->d_hist, &ctx->d_nkeep, &ctx->d_wing, &ctx->d_core, &ctx->d_hdr, &ctx->d_hdr64,
                      &ctx->d_tlo, &ctx->d_thi, &ctx->d_err, &ctx->d_ncore, &ctx->d_span, &ctx->d_lswork, &ctx->d_linstr, &ctx->d_rflags, &ctx->d_rleft, &ctx->d_rright, &ctx->d_gkappa, &ctx->d_adjwork, &ctx->d_cbuf, &ctx->d_ctaps, &ctx->d_p64, &ctx->d_lstart, &ctx->d_lstop, &ctx->d_widx,
-                     &ctx->d_pw, &ctx->d_evals, &ctx->d_spl, &ctx->d_spc, &ctx->d_sfl, &ctx->d_sfc,
+                     &ctx->d_pw, &ctx->d_spl, &ctx->d_spc, &ctx->d_sfl, &ctx->d_sfc,
                      &ctx->d_work, &ctx->d_a, &ctx->d_v, &ctx->d_h, &ctx->d_l, &ctx->z_npi, &ctx->z_nsi,
                      &ctx->z_pioff, &ctx->z_sioff, &ctx->z_splpi, &ctx->z_strpi, &ctx->z_splsi, &ctx->z_strsi,
                      &ctx->d_zsc, &ctx->z_rawpi, &ctx->z_rawsi, &ctx->d_zmap, &ctx->d_geo,
@@ -697,17 +692,19 @@ static int central_pass(fsg_ctx *ctx, const LineView &LV, int64_t *nkeep) {
 }
 
 // FP64 rows of the lines list[0 .. nb) (list null: i0 .. i0 + nb) with their headers (d_hdr64) and the tile
-// ranges of k_accum64 (d_tlo, d_thi); lines with any flag of skip get an empty window
+// ranges (d_tlo, d_thi) of k_accum64, or of k_mag64 when the list's Zeeman components are given (line i's at
+// zmap[i]); lines with any flag of skip get an empty window
 static int rows64(fsg_ctx *ctx, const AtmView &A, const LineView &LV, const int64_t *list, int64_t i0, int64_t nb,
-                  int skip, const int32_t *fl, const int32_t *il, const int32_t *ir, DBuf &p64) {
+                  int skip, const int32_t *fl, const int32_t *il, const int32_t *ir, DBuf &p64,
+                  const ZView *Z = nullptr, const int64_t *zmap = nullptr) {
     const int ntiles = fsg_fast_tiles(ctx->nwl);
     ALLOC(p64, sizeof(double3) * (size_t)nb * ctx->ntau);
     ALLOC(ctx->d_hdr64, sizeof(LineHdr64) * (size_t)nb);
     ALLOC(ctx->d_span, fsg_tile_span_scratch(nb));
     ALLOC(ctx->d_tlo, sizeof(int) * ntiles); ALLOC(ctx->d_thi, sizeof(int) * ntiles);
-    fsg_launch_params_fp64(ctx->stream, A, LV, list, i0, nb, skip, fl, il, ir, p64.as<double3>(),
+    fsg_launch_params_fp64(ctx->stream, A, LV, list, i0, nb, skip, fl, il, ir, Z, zmap, p64.as<double3>(),
                            ctx->d_hdr64.as<LineHdr64>());
-    if (fsg_launch_tile_span64(ctx->stream, fsg_accum64_tile(), ctx->nwl, nb, ctx->d_hdr64.as<LineHdr64>(),
+    if (fsg_launch_tile_span64(ctx->stream, Z ? fsg_mag64_tile() : fsg_accum64_tile(), ctx->nwl, nb, ctx->d_hdr64.as<LineHdr64>(),
                                ctx->d_tlo.as<int>(), ctx->d_thi.as<int>(), ctx->d_span.p, ctx->d_span.cap))
         return cuda_fail(ctx, cudaGetLastError(), "FP64 tile span");
     ctx->launches += 7;
@@ -853,6 +850,26 @@ static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, fsg_stats *st, cons
     return FSG_OK;
 }
 
+// Lstart/Lstop of every wavelength (synth.f90:955-978) of nw lines in blocks of at most nstep; left empty
+// for a list that fits one block, which is one segment and needs neither
+static int segment_bounds(fsg_ctx *ctx, int64_t nw, int64_t nstep, const int32_t *fl, const int32_t *il,
+                          const int32_t *ir, std::vector<int> &ls, std::vector<int> &le) {
+    if (nstep >= nw) return FSG_OK;
+    const int nwl = ctx->nwl;
+    cudaStream_t s = ctx->stream;
+    ls.assign(nwl, (int)nw); le.assign(nwl, 1);
+    ALLOC(ctx->d_lstart, sizeof(int) * nwl); ALLOC(ctx->d_lstop, sizeof(int) * nwl);
+    CK(cudaMemcpyAsync(ctx->d_lstart.p, ls.data(), sizeof(int) * nwl, cudaMemcpyHostToDevice, s), "lstart");
+    CK(cudaMemcpyAsync(ctx->d_lstop.p, le.data(), sizeof(int) * nwl, cudaMemcpyHostToDevice, s), "lstop");
+    fsg_launch_span(s, nw, fl, il, ir, ctx->d_lstart.as<int>(), ctx->d_lstop.as<int>());
+    ctx->launches += 1;
+    CK(cudaStreamSynchronize(s), "lstart");             // the host arrays receive the result below
+    CK(cudaMemcpyAsync(ls.data(), ctx->d_lstart.p, sizeof(int) * nwl, cudaMemcpyDeviceToHost, s), "lstart");
+    CK(cudaMemcpyAsync(le.data(), ctx->d_lstop.p, sizeof(int) * nwl, cudaMemcpyDeviceToHost, s), "lstop");
+    CK(cudaStreamSynchronize(s), "lstart");
+    return FSG_OK;
+}
+
 // plain FP64 path mirroring LineopCalc's PACK / MarkWideLines / Lstart-Lstop / segment loop, over the
 // windows in ctx->d_flags / d_ileft / d_iright.  [i0, i1]: 1-based wavelength range to fill (1..nwl for
 // the whole grid); PACK, the wide-line marking and the segments are those of the whole grid, so every
@@ -919,18 +936,7 @@ static int accumulate_fp64(fsg_ctx *ctx, const LineView &LV, int64_t nkeep, fsg_
     // segment loop (synth.f90:1006-1088): choose segments on the host from Lstart/Lstop (synth.f90:955-978); a
     // list that fits one block is one segment and needs neither
     std::vector<int> ls, le;
-    if (nstep < nw) {
-        ls.assign(nwl, (int)nw); le.assign(nwl, 1);
-        ALLOC(ctx->d_lstart, sizeof(int) * nwl); ALLOC(ctx->d_lstop, sizeof(int) * nwl);
-        CK(cudaMemcpyAsync(ctx->d_lstart.p, ls.data(), sizeof(int) * nwl, cudaMemcpyHostToDevice, s), "lstart");
-        CK(cudaMemcpyAsync(ctx->d_lstop.p, le.data(), sizeof(int) * nwl, cudaMemcpyHostToDevice, s), "lstop");
-        fsg_launch_span(s, nw, pf, pl, pr, ctx->d_lstart.as<int>(), ctx->d_lstop.as<int>());
-        ctx->launches += 1;
-        CK(cudaStreamSynchronize(s), "lstart");         // the host arrays are reused below
-        CK(cudaMemcpyAsync(ls.data(), ctx->d_lstart.p, sizeof(int) * nwl, cudaMemcpyDeviceToHost, s), "lstart");
-        CK(cudaMemcpyAsync(le.data(), ctx->d_lstop.p, sizeof(int) * nwl, cudaMemcpyDeviceToHost, s), "lstop");
-        CK(cudaStreamSynchronize(s), "lstart");
-    }
+    int rcs = segment_bounds(ctx, nw, nstep, pf, pl, pr, ls, le); if (rcs) return rcs;
     int64_t iline1 = 1, ilineb = 0;
     int iwl1 = 1;
     int64_t nblocks = 0;
@@ -1427,33 +1433,28 @@ static int mag_lineop_calc_body(fsg_ctx *ctx, const fsg_lines *lines, int bframe
     fsg_launch_mark_wide(s, A, nw, W.wl, nstep, pf, pl, pr, d_nw);
     unsigned long long nwide = 0;
     CK(cudaMemcpyAsync(&nwide, d_nw, sizeof nwide, cudaMemcpyDeviceToHost, s), "wide");
-    ALLOC(ctx->d_lstart, sizeof(int) * nwl); ALLOC(ctx->d_lstop, sizeof(int) * nwl);
-    {
-        std::vector<int> ls(nwl, (int)nw), le(nwl, 1);
-        CK(cudaMemcpyAsync(ctx->d_lstart.p, ls.data(), sizeof(int) * nwl, cudaMemcpyHostToDevice, s), "lstart");
-        CK(cudaMemcpyAsync(ctx->d_lstop.p, le.data(), sizeof(int) * nwl, cudaMemcpyHostToDevice, s), "lstop");
-        CK(cudaStreamSynchronize(s), "lstart");
-    }
-    fsg_launch_span(s, nw, pf, pl, pr, ctx->d_lstart.as<int>(), ctx->d_lstop.as<int>());
-    ctx->launches += 2;
-    ALLOC(ctx->d_evals, sizeof(double));
-    CK(cudaMemsetAsync(ctx->d_evals.p, 0, sizeof(double), s), "evals");
+    CK(cudaStreamSynchronize(s), "wide");
+    ctx->launches += 1;
     double *mlo = ctx->d_maglineopac.as<double>();
+    auto sum64 = [&](DBuf &p64, int w0, int w1) -> int {
+        if (fsg_launch_mag64(s, A, ctx->d_hdr64.as<LineHdr64>(), p64.as<double3>(), Z, ctx->d_tlo.as<int>(),
+                             ctx->d_thi.as<int>(), w0, w1, ctx->tab, mlo))
+            return cuda_fail(ctx, cudaGetLastError(), "k_mag64");
+        ctx->launches += 1;
+        return FSG_OK;
+    };
     if (nwide > 0) {
         ALLOC(ctx->d_widx, sizeof(int64_t) * nwide);
         fsg_select_wide(s, nw, pf, ctx->d_counts.as<int>(), ctx->d_offs.as<int64_t>(), ctx->d_widx.as<int64_t>(),
                         ctx->d_total.as<int64_t>());
-        ALLOC(ctx->d_pw, sizeof(double3) * nwide * nt);
-        fsg_launch_mag_params(s, A, W, (int64_t)nwide, ctx->d_widx.as<int64_t>(), 0, pf, ctx->d_pw.as<double3>());
-        fsg_launch_mag_wide(s, A, W.wl, Z, zmap, (int)nwide, ctx->d_widx.as<int64_t>(), pf, pl, pr,
-                            ctx->d_pw.as<double3>(), ctx->tab, mlo);
-        ctx->launches += 5;
+        rc = rows64(ctx, A, W, ctx->d_widx.as<int64_t>(), 0, (int64_t)nwide, FSG_F_WEAK, pf, pl, pr, ctx->d_pw, &Z, zmap);
+        if (!rc) rc = sum64(ctx->d_pw, 1, nwl);
+        if (rc) return rc;
+        ctx->launches += 3;
     }
-    std::vector<int> ls(nwl), le(nwl);
-    CK(cudaMemcpyAsync(ls.data(), ctx->d_lstart.p, sizeof(int) * nwl, cudaMemcpyDeviceToHost, s), "lstart");
-    CK(cudaMemcpyAsync(le.data(), ctx->d_lstop.p, sizeof(int) * nwl, cudaMemcpyDeviceToHost, s), "lstop");
-    CK(cudaStreamSynchronize(s), "lstart");
-    ALLOC(ctx->d_p64, sizeof(double3) * (size_t)std::min<int64_t>(nstep, nw) * nt);
+    // a list that fits one block is one segment; others choose their segments from Lstart/Lstop
+    std::vector<int> ls, le;
+    rc = segment_bounds(ctx, nw, nstep, pf, pl, pr, ls, le); if (rc) return rc;
     int64_t iline1 = 1, ilineb = 0, nblocks = 0;
     int iwl1 = 1;
     for (;;) {
@@ -1479,13 +1480,11 @@ static int mag_lineop_calc_body(fsg_ctx *ctx, const fsg_lines *lines, int bframe
         int64_t loff = iline1 - 1;
         if (iline1 != ilineb) {
             ilineb = iline1;
-            fsg_launch_mag_params(s, A, W, iline2 - loff, nullptr, loff, pf, ctx->d_p64.as<double3>());
-            ctx->launches += 1;
+            rc = rows64(ctx, A, W, nullptr, loff, iline2 - loff, FSG_F_WEAK | FSG_F_WIDE, pf, pl, pr, ctx->d_p64, &Z, zmap);
+            if (rc) return rc;
             nblocks++;
         }
-        fsg_launch_mag_accum(s, A, W.wl, Z, zmap, iwl1, iwl2, ctx->d_lstart.as<int>(), ctx->d_lstop.as<int>(), pf, pl,
-                             pr, loff, ctx->d_p64.as<double3>(), ctx->tab, mlo, ctx->d_evals.as<double>());
-        ctx->launches += 1;
+        rc = sum64(ctx->d_p64, iwl1, iwl2); if (rc) return rc;
         CK(cudaGetLastError(), "mag accumulation");
         if (iwl2 == nwl) break;
         iwl1 = iwl2 + 1;
@@ -1494,8 +1493,6 @@ static int mag_lineop_calc_body(fsg_ctx *ctx, const fsg_lines *lines, int bframe
         fsg_launch_scatter_flags(s, nw, ctx->d_idx.as<int64_t>(), pf, ctx->d_flags.as<int32_t>());
         ctx->launches += 1;
     }
-    double ev = 0;
-    CK(cudaMemcpyAsync(&ev, ctx->d_evals.p, sizeof ev, cudaMemcpyDeviceToHost, s), "evals");
     CK(cudaEventRecord(ctx->ev[2], s), "event");
     size_t n4 = sizeof(int32_t) * n;
     if (flags) CK(cudaMemcpyAsync(flags, ctx->d_flags.p, n4, cudaMemcpyDeviceToHost, s), "flags");
@@ -1510,7 +1507,6 @@ static int mag_lineop_calc_body(fsg_ctx *ctx, const fsg_lines *lines, int bframe
         cudaEventElapsedTime(&b, ctx->ev[1], ctx->ev[2]);
         st->ms_center = a; st->ms_accum = b; st->ms_total = a + b;
         st->nwide = (int64_t)nwide; st->nblocks = nblocks;
-        (void)ev;                                          // the kernels' own count leaves components out
         st->line_evals = count_windows(ctx, n, ctx->d_flags.as<int32_t>(), ctx->d_ileft.as<int32_t>(),
                                        ctx->d_iright.as<int32_t>(), 1, nwl, Z.npi, Z.nsi) * nt;
     }

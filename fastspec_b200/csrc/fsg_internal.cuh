@@ -93,8 +93,9 @@ struct __align__(16) LineHdr { float wlh, wll; int ileft, iright; int cl, cr, pa
 
 // Line header of the FP64 tile kernels: the centre offset Wlcent, the window, the core range [cl, cr]
 // (every wavelength of the window where some depth may have s < 196, He I shifts included; cl > cr:
-// none) and the He I Stark table entry (0: none).  Lines a launch leaves out have an empty window.
-struct __align__(16) LineHdr64 { double wlc; int il, ir, cl, cr, ihe, pad; };
+// none), the He I Stark table entry (0: none) and, for magnetic lists, the line's place in ZView (Zeeman
+// shifts widen its core range).  Lines a launch leaves out have an empty window.
+struct __align__(16) LineHdr64 { double wlc; int il, ir, cl, cr, ihe, zi; };
 static_assert(sizeof(LineHdr64) == 32, "FP64 header: 32 bytes");
 
 // Zeeman components of a device line list (CSR by line)

@@ -369,12 +369,14 @@ void fsg_launch_params_fast(cudaStream_t s, const AtmView &A, const LineView &L,
 
 // FP64 records of the plain path: row q holds the list line list[q] (list null: i0 + q) as
 // p64[q][t] = (LinCop, LinVvgt, LinAvgt) and its header.  Lines with any flag of skip get an empty
-// window.  One warp per line, lanes over depths: XlineDepth's FP64 chain is long, and a thread per line
+// window.  Magnetic lists give their Zeeman components (Z, line i's at zmap[i]): the core range is widened
+// by the largest component shift, and the header keeps zmap[i].  One warp per line, lanes over depths: XlineDepth's FP64 chain is long, and a thread per line
 // walked all depths one after another (84 + 71 us for the 19,362 lines of a 200 A solar list, narrow and wide).
 __global__ void __launch_bounds__(128)
 k_params_fp64(AtmView A, LineView L, const int64_t *__restrict__ list, int64_t i0, int64_t nb, int skip,
               const int32_t *__restrict__ flags, const int32_t *__restrict__ ileft,
-              const int32_t *__restrict__ iright, double3 *p64, LineHdr64 *hdr) {
+              const int32_t *__restrict__ iright, ZView Z, const int64_t *__restrict__ zmap, double3 *p64,
+              LineHdr64 *hdr) {
     const int64_t q = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (q >= nb) return;                                // whole warps leave together
@@ -382,7 +384,7 @@ k_params_fp64(AtmView A, LineView L, const int64_t *__restrict__ list, int64_t i
     const int f = flags[i], nt = A.ntau;
     LineHdr64 h;
     h.wlc = L.wl[i] - A.wfirst;
-    h.il = 1; h.ir = 0; h.cl = 1; h.cr = 0; h.ihe = (f >> 8) & 255; h.pad = 0;
+    h.il = 1; h.ir = 0; h.cl = 1; h.cr = 0; h.ihe = (f >> 8) & 255; h.zi = zmap ? (int)zmap[i] : 0;
     if (f & skip) { if (lane == 0) hdr[q] = h; return; }
     XCoef XC;
     xline_setup(A, L, i, h.wlc, f, &XC);
@@ -394,6 +396,13 @@ k_params_fp64(AtmView A, LineView L, const int64_t *__restrict__ list, int64_t i
         const double r = 196.05 - av * av;
         if (r > 0.0) hcore = fmax(hcore, sqrt(r) / vv * (1.0 + 1e-5));
         if (h.ihe > 0) shmax = fmax(shmax, fabs(A.heshf[(size_t)(h.ihe - 1) * nt + t]));
+    }
+    if (zmap) {
+        double zmax = 0.0;
+        for (int k = lane; k < Z.npi[h.zi]; k += 32) zmax = fmax(zmax, fabs((double)Z.splpi[Z.pi_off[h.zi] + k]));
+        for (int k = lane; k < Z.nsi[h.zi]; k += 32) zmax = fmax(zmax, fabs((double)Z.splsi[Z.si_off[h.zi] + k]));
+        for (int o = 16; o > 0; o >>= 1) zmax = fmax(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
+        shmax += zmax;
     }
     for (int o = 16; o > 0; o >>= 1) {
         hcore = fmax(hcore, __shfl_xor_sync(0xffffffffu, hcore, o));
@@ -416,9 +425,10 @@ k_params_fp64(AtmView A, LineView L, const int64_t *__restrict__ list, int64_t i
 
 void fsg_launch_params_fp64(cudaStream_t s, const AtmView &A, const LineView &L, const int64_t *list, int64_t i0,
                             int64_t nb, int skip, const int32_t *flags, const int32_t *il, const int32_t *ir,
-                            double3 *p64, LineHdr64 *hdr) {
+                            const ZView *Z, const int64_t *zmap, double3 *p64, LineHdr64 *hdr) {
     if (nb <= 0) return;
-    k_params_fp64<<<(unsigned)((nb + 3) / 4), 128, 0, s>>>(A, L, list, i0, nb, skip, flags, il, ir, p64, hdr);
+    k_params_fp64<<<(unsigned)((nb + 3) / 4), 128, 0, s>>>(A, L, list, i0, nb, skip, flags, il, ir, Z ? *Z : ZView{},
+                                                          Z ? zmap : nullptr, p64, hdr);
 }
 
 // ================================================================================================

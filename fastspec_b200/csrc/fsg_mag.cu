@@ -6,8 +6,7 @@
 //                   FP32 (Kz |B| lambda^2, synth.f90:1193-1194), centre test (LineOpacity2),
 //                   doubling search with MagLineOpacity2 and RefineIdx bisection
 //                   (opacity.f90:468-520, 611-675)
-//   k_mag_accum     MagLineOpacity1 per wavelength (opacity.f90:391-464)
-//   k_mag_wide      MagLineOpacity3 for the wide lines, in line order (synth.f90:1341-1361)
+//   (the sums, MagLineOpacity1/3, are in fsg_accum64.cu and fsg_magfast.cu)
 //   k_stokes_thr    StokesPrfPP (solver.f90:265-394) + Solve4x4 (solver.f90:541-588), one thread per
 //                   (wavelength, angle); k_stokes_flux the Stokes-I flux quadrature
 //   k_stokes_sph    StokesPrfSph (solver.f90:402-538) along the rays of a spherical model, one thread per
@@ -174,89 +173,6 @@ __device__ __forceinline__ void mag_profiles_t(const AtmView &A, int t, double W
         fvoigt_line64(fvtab, FL, V, &Vg, &Fv);
         double Str = Xn * (double)rsi[k];
         m[2] = m[2] + Str * Vg; m[5] = m[5] + Str * Fv;
-    }
-}
-
-// MagLineOpacity1 (opacity.f90:391-464): one warp per wavelength, lanes stride the depths.
-__global__ void k_mag_accum(AtmView A, const double *__restrict__ wl, ZView Z, const int64_t *__restrict__ zmap,
-                            int iwl1, int iwl2, const int *__restrict__ lstart, const int *__restrict__ lstop,
-                            const int32_t *__restrict__ flags, const int32_t *__restrict__ ileft,
-                            const int32_t *__restrict__ iright, int64_t loff, const double3 *__restrict__ p64,
-                            const float2 *__restrict__ fvtab, const double *__restrict__ anode,
-                            const double *__restrict__ aida, double *mlo, double *evals) {
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    int iwl = iwl1 + warp;
-    if (iwl > iwl2) return;
-    const int nt = A.ntau;
-    double Wl = A.wave[iwl - 1];
-    double cnt = 0.0;
-    for (int t0 = 0; t0 < nt; t0 += 32) {
-        int t = t0 + lane;
-        double m[6] = { 0, 0, 0, 0, 0, 0 };
-        for (int il = lstart[iwl - 1]; il <= lstop[iwl - 1]; il++) {
-            int f = flags[il - 1];
-            if ((f & FSG_F_WEAK) || (f & FSG_F_WIDE) || iwl < ileft[il - 1] || iwl > iright[il - 1]) continue;
-            if (t < nt) {
-                double3 p = p64[(size_t)(il - 1 - loff) * nt + t];
-                mag_profiles_t(A, t, Wl, wl[il - 1] - A.wfirst, (f >> 8) & 255, Z, zmap[il - 1], p.x, p.y, p.z,
-                               fvtab, anode, aida, m);
-            }
-            if (t0 == 0) cnt += 1.0;
-        }
-        if (t < nt) {
-            double *dst = mlo + ((size_t)(iwl - 1) * nt + t) * 6;
-            for (int q = 0; q < 6; q++) {
-                double v = m[q];
-                if (A.motype == 1) v = v / A.contstd[t];
-                dst[q] = dst[q] + v;
-            }
-        }
-    }
-    if (lane == 0 && cnt > 0.0) atomicAdd(evals, cnt * nt);
-}
-
-// MagLineOpacity3 over the wide lines, in line order, one warp per wavelength
-__global__ void k_mag_wide(AtmView A, const double *__restrict__ wl, ZView Z, const int64_t *__restrict__ zmap,
-                           int nwide, const int64_t *__restrict__ widx, const int32_t *__restrict__ flags,
-                           const int32_t *__restrict__ ileft, const int32_t *__restrict__ iright,
-                           const double3 *__restrict__ pw, const float2 *__restrict__ fvtab,
-                           const double *__restrict__ anode, const double *__restrict__ aida, double *mlo) {
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    int iwl = 1 + warp;
-    if (iwl > A.nwl) return;
-    const int nt = A.ntau;
-    double Wl = A.wave[iwl - 1];
-    for (int q = 0; q < nwide; q++) {
-        int64_t il = widx[q];
-        if (iwl < ileft[il] || iwl > iright[il]) continue;
-        int ihe = (flags[il] >> 8) & 255;
-        for (int t = lane; t < nt; t += 32) {
-            double m[6] = { 0, 0, 0, 0, 0, 0 };
-            double3 p = pw[(size_t)q * nt + t];
-            mag_profiles_t(A, t, Wl, wl[il] - A.wfirst, ihe, Z, zmap[il], p.x, p.y, p.z, fvtab, anode, aida, m);
-            double *dst = mlo + ((size_t)(iwl - 1) * nt + t) * 6;
-            for (int r = 0; r < 6; r++) {
-                double v = m[r];
-                if (A.motype == 1) v = v / A.contstd[t];
-                dst[r] = dst[r] + v;
-            }
-        }
-    }
-}
-
-__global__ void k_mag_params(AtmView A, LineView L, int64_t n, const int64_t *__restrict__ list, int64_t off,
-                             const int32_t *__restrict__ flags, double3 *p) {
-    int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n) return;
-    int64_t i = list ? list[q] : off + q;
-    int f = flags[i];
-    if (f & FSG_F_WEAK) return;
-    XCoef XC;
-    xline_setup(A, L, i, L.wl[i] - A.wfirst, f, &XC);
-    for (int t = 0; t < A.ntau; t++) {
-        double cop, vv, av;
-        xline_depth(A, t, XC, &cop, &vv, &av);
-        p[(size_t)q * A.ntau + t] = make_double3(cop, vv, av);
     }
 }
 
@@ -608,30 +524,6 @@ void fsg_launch_mag_center(cudaStream_t s, const AtmView &A, const LineView &L, 
         k_mag_center<<<(unsigned)((L.n + 3) / 4), 128, 0, s>>>(A, L, Z, Bsplit, T.vtab, T.anode, T.aida, flags, ileft,
                                                                 iright, nkeep);
 }
-
-void fsg_launch_mag_params(cudaStream_t s, const AtmView &A, const LineView &L, int64_t n, const int64_t *list,
-                           int64_t off, const int32_t *flags, double3 *p) {
-    if (n > 0) k_mag_params<<<(unsigned)((n + 63) / 64), 64, 0, s>>>(A, L, n, list, off, flags, p);
-}
-
-void fsg_launch_mag_accum(cudaStream_t s, const AtmView &A, const double *wl, const ZView &Z, const int64_t *zmap,
-                          int iwl1, int iwl2, const int *lstart, const int *lstop, const int32_t *flags,
-                          const int32_t *ileft, const int32_t *iright, int64_t loff, const double3 *p64,
-                          const VoigtTables &T, double *mlo, double *evals) {
-    int nw = iwl2 - iwl1 + 1;
-    if (nw > 0)
-        k_mag_accum<<<(nw + 7) / 8, 256, 0, s>>>(A, wl, Z, zmap, iwl1, iwl2, lstart, lstop, flags, ileft, iright, loff,
-                                                 p64, T.fvtab, T.anode, T.aida, mlo, evals);
-}
-
-void fsg_launch_mag_wide(cudaStream_t s, const AtmView &A, const double *wl, const ZView &Z, const int64_t *zmap,
-                         int nwide, const int64_t *widx, const int32_t *flags, const int32_t *ileft,
-                         const int32_t *iright, const double3 *pw, const VoigtTables &T, double *mlo) {
-    if (nwide > 0)
-        k_mag_wide<<<(A.nwl + 7) / 8, 256, 0, s>>>(A, wl, Z, zmap, nwide, widx, flags, ileft, iright, pw, T.fvtab,
-                                                   T.anode, T.aida, mlo);
-}
-
 
 // ================================================================================================
 // MagLineOpacity1 and StokesPrfPP on their own, batched (kernel-level entry points)

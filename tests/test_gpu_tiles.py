@@ -44,3 +44,30 @@ def test_tile_edges(fsg, oracle_mod, prec, ntau, nwl, n):
     err = np.max(np.abs(g["lineopac"] - r["lineopac"]) / (r["lineopac"] + co))
     assert err < (1e-12 if prec == "fp64" else 2e-6)
     C.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("ntau,nwl,n", [(3, 2, 1), (4, 31, 5), (9, 33, 17), (33, 64, 20), (65, 300, 33), (128, 97, 12)])
+def test_magnetic_tile_edges(fsg, oracle_mod, prec, ntau, nwl, n):
+    """The same for Zeeman lines; errors on the scale of the depth's peak absorption profile (FP64: the
+    offset of a component carries the rounding of lambda - lambda_c and of the shift, 2 v dv < 1e-13)."""
+    from fastspec_b200 import workloads as W
+    grid, st, co, _ = case(ntau, nwl, 1, 0)
+    L = W.zeeman_lines(n, grid["wstart"], grid["wend"], 19 * ntau + nwl)
+    z = W.zeeman_components(L, oracle_mod.zeeman_pattern)
+    C = fsg.Context(precision=fsg.PREC_FP64 if prec == "fp64" else fsg.PREC_MIXED, vmicro=1.0)
+    C.set_grid(grid["wmode"], grid["wstart"], grid["wend"], grid["dstep"])
+    C.set_atmosphere(st)
+    C.set_contopac(co)
+    b = np.array([3000.0, 50.0, 20.0])
+    g = C.mag_lineop_calc(fsg.LineList.from_arrays(L.arrays(), zeeman=z), 1, b)
+    S = oracle_mod.State(grid, st, contopac=co, vmicro=1.0)
+    r = oracle_mod.mag_lineop_calc(S, oracle_mod.Lines(**L.arrays(), kind=2, zeeman=z), 1, b)
+    keep = (r["flags"] & 1) == 0
+    np.testing.assert_array_equal((g["flags"] & 1) == 0, keep)
+    np.testing.assert_array_equal(g["ileft"][keep], r["ileft"][keep])
+    np.testing.assert_array_equal(g["iright"][keep], r["iright"][keep])
+    om = r["maglineopac"]
+    scale = np.maximum(om[..., :3].max(axis=(0, 2)), 1e-300)[None, :, None]
+    assert np.max(np.abs(g["maglineopac"] - om) / scale) < (1e-12 if prec == "fp64" else 2e-6)
+    C.close()
