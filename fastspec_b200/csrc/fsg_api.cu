@@ -82,7 +82,7 @@ void fsg_launch_center(cudaStream_t, const AtmView &, const LineView &, const Vo
                        int32_t *, int32_t *, unsigned long long *);
 void fsg_launch_params_fast(cudaStream_t, const AtmView &, const LineView &, const int64_t *, int64_t, int64_t,
                             int64_t, const int32_t *, const int32_t *, const int32_t *, const VoigtTables &,
-                            WingRec *, CoreRec *, LineHdr *);
+                            WingPair *, CoreRec *, LineHdr *);
 void fsg_launch_params_fp64(cudaStream_t, const AtmView &, const LineView &, const int64_t *, int64_t, int64_t, int,
                             const int32_t *, const int32_t *, const int32_t *, const ZView *, const int64_t *, double3 *,
                             LineHdr64 *);
@@ -101,12 +101,13 @@ void fsg_launch_fvoigt(cudaStream_t, int64_t, const double *, const double *, do
                        const VoigtTables &);
 void fsg_launch_locprf(cudaStream_t, int, int, const double *, int, const double *, const double *, const double *,
                        double *, double *);
-int fsg_launch_accum_fast(cudaStream_t, int, int, int, const double *, const LineHdr *, const WingRec *,
-                          const int *, const int *, double *, int *, unsigned, unsigned long long);
-int fsg_launch_core_fast(cudaStream_t, int, int, const double *, const LineHdr *, const WingRec *, const CoreRec *,
-                         const int *, const int *, const float4 *, double *, unsigned long long *, int *, unsigned,
+int fsg_launch_accum_fast(cudaStream_t, int, int, int, const double *, const LineHdr *, const WingPair *, const int *,
+                          const int *, double *);
+int fsg_launch_core_fast(cudaStream_t, int, int, const double *, const LineHdr *, const CoreRec *, const int *,
+                         const int *, const float4 *, double *, unsigned long long *, int *, unsigned,
                          unsigned long long);
-int fsg_launch_accum_batch(cudaStream_t, int, int, const WingJob *, const int *, int, int, unsigned *, int *);
+int fsg_wing_groups(int, int);
+int fsg_launch_accum_batch(cudaStream_t, int, const WingJob *, const int *, int, int, unsigned *);
 int fsg_launch_core_batch(cudaStream_t, int, const CoreJob *, const int *, int, int, const float4 *, unsigned *,
                           int *);
 int fsg_class_pix(int);
@@ -761,7 +762,8 @@ static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, fsg_stats *st, cons
     CK(cudaMemsetAsync(ctx->d_err.p, 0, sizeof(int), s), "err reset");
     ALLOC(ctx->d_ncore, sizeof(unsigned long long));
     CK(cudaMemsetAsync(ctx->d_ncore.p, 0, sizeof(unsigned long long), s), "core count reset");
-    size_t per_line = (size_t)nt * (sizeof(WingRec) + sizeof(CoreRec)) + sizeof(LineHdr);
+    const size_t npair = wing_pairs(nt);
+    size_t per_line = npair * sizeof(WingPair) + (size_t)nt * sizeof(CoreRec) + sizeof(LineHdr);
     int64_t cap = block_capacity(ctx, per_line);
     int64_t nblocks = 0;
     for (int c = 0; c < 32; c++) {
@@ -777,23 +779,22 @@ static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, fsg_stats *st, cons
         // launch has work, however small the blocks
         const int64_t nblk = (nc + cap - 1) / cap;
         const int64_t bcap = (nc + nblk - 1) / nblk;
-        ALLOC(ctx->d_wing, sizeof(WingRec) * (size_t)bcap * nt);
+        ALLOC(ctx->d_wing, sizeof(WingPair) * (size_t)bcap * npair);
         ALLOC(ctx->d_core, sizeof(CoreRec) * (size_t)bcap * nt);
         ALLOC(ctx->d_hdr, sizeof(LineHdr) * (size_t)bcap);
         ALLOC(ctx->d_span, fsg_tile_span_scratch(bcap));
         for (int64_t b = 0; b < nblk; b++) {
             const int64_t nb = (nc - b + nblk - 1) / nblk;
             fsg_launch_params_fast(s, A, LV, ctx->d_idx.as<int64_t>(), b, nblk, nb, fl, wl_, wr_, ctx->tab,
-                                   ctx->d_wing.as<WingRec>(), ctx->d_core.as<CoreRec>(), ctx->d_hdr.as<LineHdr>());
+                                   ctx->d_wing.as<WingPair>(), ctx->d_core.as<CoreRec>(), ctx->d_hdr.as<LineHdr>());
             if (fsg_launch_tile_span(s, c, ctx->nwl, nb, ctx->d_hdr.as<LineHdr>(), ctx->d_tlo.as<int>(),
                                      ctx->d_thi.as<int>(), ctx->d_span.p, ctx->d_span.cap))
                 return cuda_fail(ctx, cudaGetLastError(), "tile span");
             cudaEvent_t ea = kevent(), em = kevent(), eb = kevent();
             cudaEventRecord(ea, s);
             int rc2 = fsg_launch_accum_fast(s, c, nt, ctx->nwl, ctx->d_wave.as<double>(), ctx->d_hdr.as<LineHdr>(),
-                                            ctx->d_wing.as<WingRec>(), ctx->d_tlo.as<int>(), ctx->d_thi.as<int>(),
-                                            ctx->d_lineopac.as<double>(), ctx->d_err.as<int>(), ctx->fault_extra_tx,
-                                            ctx->fault_wait_ns);
+                                            ctx->d_wing.as<WingPair>(), ctx->d_tlo.as<int>(), ctx->d_thi.as<int>(),
+                                            ctx->d_lineopac.as<double>());
             if (rc2) return cuda_fail(ctx, cudaGetLastError(), "k_accum_fast");
             cudaEventRecord(em, s);
             // core ranges of the same lines, 32-wavelength tiles
@@ -801,8 +802,8 @@ static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, fsg_stats *st, cons
                                      ctx->d_thi.as<int>(), ctx->d_span.p, ctx->d_span.cap))
                 return cuda_fail(ctx, cudaGetLastError(), "core tile span");
             rc2 = fsg_launch_core_fast(s, nt, ctx->nwl, ctx->d_wave.as<double>(), ctx->d_hdr.as<LineHdr>(),
-                                       ctx->d_wing.as<WingRec>(), ctx->d_core.as<CoreRec>(), ctx->d_tlo.as<int>(),
-                                       ctx->d_thi.as<int>(), ctx->tab.vtab4, ctx->d_lineopac.as<double>(),
+                                       ctx->d_core.as<CoreRec>(), ctx->d_tlo.as<int>(), ctx->d_thi.as<int>(),
+                                       ctx->tab.vtab4, ctx->d_lineopac.as<double>(),
                                        ctx->d_ncore.as<unsigned long long>(), ctx->d_err.as<int>(),
                                        ctx->fault_extra_tx, ctx->fault_wait_ns);
             if (rc2) return cuda_fail(ctx, cudaGetLastError(), "k_core_fast");
@@ -2377,7 +2378,7 @@ static int batch_prepare(fsg_batch *b, int P) {
             return cuda_fail(ctx, e, "batch class order");
         }
         fsg_launch_params_fast(s, A, LV, a.order.as<int64_t>(), 0, 1, a.cn, a.flags.as<int32_t>(), a.il.as<int32_t>(),
-                               a.ir.as<int32_t>(), c->tab, a.wing.as<WingRec>(), a.core.as<CoreRec>(),
+                               a.ir.as<int32_t>(), c->tab, a.wing.as<WingPair>(), a.core.as<CoreRec>(),
                                a.hdr.as<LineHdr>());
         if (fsg_launch_btile_span(s, 0, a.cn, a.hdr.as<LineHdr>(), a.coff.as<int64_t>(), a.ncls, BATCH_NARROW, 64,
                                   32 * P, c->nwl, batch_wing_stride(c), a.wtlo.as<int>(), a.wthi.as<int>(), a.span.p,
@@ -2426,13 +2427,12 @@ static int batch_jobs(fsg_batch *b, int P) {
                 const int ws = batch_wing_stride(c), cs = batch_core_stride(c);
                 if (kind < 2) {
                     jw.push_back(WingJob{ c->ntau, c->nwl, c->d_wave.as<double>(), a.hdr.as<LineHdr>(),
-                                          a.wing.as<WingRec>(), a.wtlo.as<int>() + (size_t)c0 * ws,
-                                          a.wthi.as<int>() + (size_t)c0 * ws, c->d_lineopac.as<double>(), 0u, WAIT_NS,
-                                          nseg, ws });
-                    t0.push_back(t0.back() + (c->nwl + 32 * Pk - 1) / (32 * Pk));
+                                          a.wing.as<WingPair>(), a.wtlo.as<int>() + (size_t)c0 * ws,
+                                          a.wthi.as<int>() + (size_t)c0 * ws, c->d_lineopac.as<double>(), nseg, ws });
+                    t0.push_back(t0.back() + (c->nwl + 32 * Pk - 1) / (32 * Pk) * fsg_wing_groups(Pk, c->ntau));
                 } else {
                     jc.push_back(CoreJob{ c->ntau, c->nwl, c->d_wave.as<double>(), a.hdr.as<LineHdr>(),
-                                          a.wing.as<WingRec>(), a.core.as<CoreRec>(), a.ctlo.as<int>(), a.cthi.as<int>(),
+                                          a.core.as<CoreRec>(), a.ctlo.as<int>(), a.cthi.as<int>(),
                                           c->d_lineopac.as<double>(), b->evals.as<unsigned long long>(), 0u, WAIT_NS,
                                           nseg, cs });
                     t0.push_back(t0.back() + (c->nwl + 31) / 32);
@@ -2485,8 +2485,8 @@ static int batch_accumulate_solve(fsg_batch *b, const fsg_batch_tuning &t, cudaE
     if (ev) batch_mark(ev[0], s);
     for (size_t i = 0; i < nw; i++) {
         const fsg_batch::Launch &L = b->lw[i];
-        if (fsg_launch_accum_batch(s, L.P, L.ntau_max, b->jobs_w.as<WingJob>() + L.j0, b->tile0_w.as<int>() + L.t0,
-                                   L.nj, t.wing_ctas, q + i, b->err.as<int>()))
+        if (fsg_launch_accum_batch(s, L.P, b->jobs_w.as<WingJob>() + L.j0, b->tile0_w.as<int>() + L.t0, L.nj,
+                                   t.wing_ctas, q + i))
             return cuda_fail(ctx, cudaGetLastError(), "k_accum_batch");
     }
     if (ev) batch_mark(ev[1], s);
@@ -2586,7 +2586,7 @@ int fsg_batch_create(fsg_ctx *const *atms, int natm, const fsg_lines *lines, dou
         const size_t nsb = (cn + 1023) / 1024 * (ncl + 1);          // class counts per CTA of the order
         const size_t ws = batch_wing_stride(c) * ncl, cs = batch_core_stride(c) * ncl;
         if (a.flags.ensure(4 * cn) || a.il.ensure(4 * cn) || a.ir.ensure(4 * cn) ||
-            a.wing.ensure(sizeof(WingRec) * cn * nt) || a.core.ensure(sizeof(CoreRec) * cn * nt) ||
+            a.wing.ensure(sizeof(WingPair) * cn * wing_pairs(c->ntau)) || a.core.ensure(sizeof(CoreRec) * cn * nt) ||
             a.hdr.ensure(sizeof(LineHdr) * cn) || a.wtlo.ensure(4 * ws) || a.wthi.ensure(4 * ws) ||
             a.ctlo.ensure(4 * cs) || a.cthi.ensure(4 * cs) || a.span.ensure(fsg_bspan_scratch(cn)) ||
             a.order.ensure(8 * cn) || a.ccnt.ensure(4 * nsb) || a.coff.ensure(8 * nsb) || a.ctot.ensure(8) ||

@@ -7,13 +7,13 @@
 // window where some depth may have s = v^2 + a^2 < 196); outside it every depth takes the
 // reference's rational wing form (voigt.f90:100-101).
 //
-// Wing pass (k_accum_fast): a CTA owns a tile of TW = 32 P wavelengths x all depths; warp w owns
-// depths [w*D, w*D + D), lane l the wavelengths tile0 + l + 32k (k < P).  Line headers and wing
-// records arrive in shared memory by bulk copies; each thread keeps P x D FP32 partials over FOLD
-// lines, folded into Kahan (sum, compensation) pairs in shared memory.  Lines are binned by window
-// width (class c holds windows of up to 256 * 2^c wavelengths) and processed class by class, so a
-// tile's candidate range stays close to the lines that touch it; narrow classes use 64-wavelength
-// tiles, wide ones 128.
+// Wing pass (k_accum_fast): a warp owns a tile of TW = 32 P wavelengths x D depths, lane l the
+// wavelengths tile0 + l + 32k (k < P).  It picks the tile's lines from the candidate range and brings their
+// headers and records to shared memory a group at a time, the next group's loads in flight while it works
+// through the present one; each thread keeps P x D FP32 partials over FOLD lines, folded into Kahan (sum,
+// compensation) pairs in shared memory.  Lines are binned by window width (class c holds windows of up to
+// 256 * 2^c wavelengths) and processed class by class, so a tile's candidate range stays close to the lines
+// that touch it; narrow classes use 64-wavelength tiles, wide ones 128.
 //
 // Core pass (k_core_fast): over the core ranges, 32-wavelength tiles, the points where s < 196: the
 // table lerp (|v| < 8, a < 8) or the two-term continued fraction (voigt.f90:103-107), exactly as
@@ -45,22 +45,8 @@ __device__ __forceinline__ float hv_cf32(float av, float a, float cop) {
 // memory.  The partials carry at most FOLD terms, so their rounding stays at the FP32 unit
 // roundoff of a few terms; the Kahan pairs carry the long sums.
 #define FOLD 32
-// Candidate lines staged per TMA bulk copy, and the wing pass's staging buffers (copies in flight)
-#define CH 32
-#define WNB 2
 // cp.async.bulk moves multiples of 16 bytes between 16-byte aligned addresses
-static_assert(sizeof(WingRec) % 16 == 0 && sizeof(LineHdr) % 16 == 0 && sizeof(CoreRec) % 16 == 0, "bulk-copied records: multiples of 16 bytes");
-
-// Issue the bulk copies of chunk c (lines lo + c*CH ...) into buffer b; one thread calls this.
-__device__ __forceinline__ void stage_chunk(int c, int lo, int hi, int ntau, const LineHdr *hdr, const WingRec *wing,
-                                            LineHdr *shdr, WingRec *swing, uint64_t *bar, unsigned extra_tx) {
-    int j0 = lo + c * CH;
-    int n = min(CH, hi - j0 + 1);
-    unsigned brec = (unsigned)(n * ntau * (int)sizeof(WingRec)), bhdr = (unsigned)(n * (int)sizeof(LineHdr));
-    mbar_expect_tx(bar, brec + bhdr + extra_tx);
-    tma_bulk_g2s(swing, wing + (size_t)j0 * ntau, brec, bar);
-    tma_bulk_g2s(shdr, hdr + j0, bhdr, bar);
-}
+static_assert(sizeof(LineHdr) % 16 == 0 && sizeof(CoreRec) % 16 == 0, "bulk-copied records: multiples of 16 bytes");
 
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
@@ -79,279 +65,253 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // exactly 0 too: the two passes split the points by the same FP32 test, so each point is evaluated
 // once.
 
-// shared memory of the wing pass for at most ntau_max depths:
-// wing records [WNB][CH][ntau_max] | headers [WNB][CH] | mbarriers [WNB] | Kahan pairs [D * P][blockDim.x]
-// (a warp reads up to D - 1 <= 7 records past its line's last depth: at most 112 bytes past the
-// last record buffer, inside the headers that follow it)
-__host__ __device__ inline size_t wing_smem_recs(int ntau_max) {
-    return sizeof(WingRec) * WNB * CH * (size_t)ntau_max + sizeof(LineHdr) * WNB * CH;
-}
+// A line as the warp's group holds it: {wlh, wll, code, xm}.  code: first and last wavelength of the window
+// inside the tile (bits 0-7, 8-15), WING_FULL (the window covers the tile and no core range meets it),
+// WING_CORE (a core range meets it); xm: the x that silences a point.
+#define WING_FULL (1 << 16)
+#define WING_CORE (1 << 17)
+#define WING_G 8                      // lines per group
 
-// One tile of one job.  Called by every thread of the CTA with the mbarriers initialised; kk counts
-// the chunks the CTA has consumed so far (their buffer and phase parity), across tiles.  Returns
-// false after a copy did not complete within its bound (error reported in *err).
+// shared memory of one warp
 template <int D, int P>
-__device__ __forceinline__ bool wing_tile(const WingJob &J, int tile, unsigned char *smem_raw, int ntau_max,
-                                          unsigned &kk, int *err) {
-    const int ntau = J.ntau, nwl = J.nwl;
-    const double *__restrict__ wave = J.wave;
-    const LineHdr *__restrict__ hdr = J.hdr;
-    const WingRec *__restrict__ wing = J.wing;
-    WingRec *swing = (WingRec *)smem_raw;
-    LineHdr *shdr = (LineHdr *)(swing + WNB * CH * ntau_max);
-    uint64_t *bars = (uint64_t *)(shdr + WNB * CH);
-    float2 *ksum = (float2 *)(bars + WNB);               // [D * P][blockDim.x]
-    constexpr int TW = 32 * P;
+struct __align__(16) WingWarp {
+    float4 rec[WING_G][D];            // D / 2 depth pairs of two float4
+    float4 hdr[WING_G];
+    float2 ksum[D * P][32];           // Kahan (sum, compensation)
+    int queue[64];
+};
+
+// One tile and depth group (depths t0 .. t0 + D - 1, t0 a multiple of D) of one job, by one warp; warps
+// share nothing.  Per evaluation two packed FMAs on the depth pair's halves (t, t^2 + 2a^2, c1 (t + 1), the
+// sum: four for two), and one reciprocal.
+template <int D, int P>
+__device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, WingWarp<D, P> &S, int lane) {
+    constexpr int TW = 32 * P, NP = D / 2, U = WING_G * D / 32;      // U: record loads per lane and group
+    const int ntau = J.ntau, nwl = J.nwl, units = 2 * wing_pairs(ntau);
     bool any = false;                                   // some segment has lines touching the tile
     for (int sg = 0; sg < J.nseg; sg++)
         any = any || J.tile_lo[sg * J.seg_stride + tile] <= J.tile_hi[sg * J.seg_stride + tile];
-    if (!any) return true;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t0 = warp * D;
-    const int nd = max(0, min(D, ntau - t0));            // warps past the last depth only help staging
+    if (!any) return;
+    const float4 *__restrict__ wing = (const float4 *)J.wing;
     const int p0 = tile * TW;
-    const int nth = blockDim.x;
     // wavelength offsets as FP32 hi + lo: dl = (wvh - wlh) + (wvl - wll) keeps dl to FP32 relative
     // accuracy next to the line centre
     float wvh[P], wvl[P];
-    int pix[P];
 #pragma unroll
     for (int k = 0; k < P; k++) {
-        pix[k] = p0 + lane + 32 * k;
-        double w = wave[min(pix[k], nwl - 1)];
+        double w = J.wave[min(p0 + lane + 32 * k, nwl - 1)];
         wvh[k] = (float)w;
         wvl[k] = (float)(w - (double)wvh[k]);
     }
-    float part[D][P];
+    float2 part[NP][P];
 #pragma unroll
-    for (int d = 0; d < D; d++)
+    for (int j = 0; j < NP; j++)
 #pragma unroll
         for (int k = 0; k < P; k++) {
-            part[d][k] = 0.0f;
-            ksum[(d * P + k) * nth + threadIdx.x] = make_float2(0.0f, 0.0f);
+            part[j][k] = make_float2(0.0f, 0.0f);
+            S.ksum[2 * (j * P + k)][lane] = make_float2(0.0f, 0.0f);
+            S.ksum[2 * (j * P + k) + 1][lane] = make_float2(0.0f, 0.0f);
         }
     int nfold = 0;
     const int tile_first = p0 + 1, tile_last = min(p0 + TW, nwl);
-    for (int sg = 0; sg < J.nseg; sg++) {               // the job's segments of lines, in turn
-        const int lo = J.tile_lo[sg * J.seg_stride + tile], hi = J.tile_hi[sg * J.seg_stride + tile];
-        if (lo > hi) continue;
-        const int nchunks = (hi - lo + CH) / CH;
-        // chunk c of this tile is the CTA's chunk g = kk + c: buffer g % WNB, phase parity (g / WNB) & 1
-        if (threadIdx.x == 0) {
-            for (int c = 0; c < WNB && c < nchunks; c++) {
-                const int b = (kk + c) % WNB;
-                stage_chunk(c, lo, hi, ntau, hdr, wing, shdr + b * CH, swing + b * CH * ntau_max, &bars[b],
-                            J.extra_tx);
-            }
+    float4 rnext[U], hnext;                             // the next group's records and (lanes < n) header
+    int nnext = 0;
+    auto fetch = [&](int head, int n) {
+        nnext = n;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int e = lane + 32 * u, q = e / D, i = t0 + e % D;
+            rnext[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);          // past the last depth: never stored
+            if (q < n && i < units) rnext[u] = __ldg(wing + (size_t)S.queue[(head + q) & 63] * units + i);
         }
-        int failed = -1;                                     // chunk whose copy did not complete
-        for (int c = 0; c < nchunks; c++) {
-            const unsigned g = kk + c;
-            const int b = g % WNB;
-            const bool ok = mbar_wait(&bars[b], (g / WNB) & 1, J.wait_ns);
-            if (__syncthreads_or(!ok)) { failed = c; break; }
-            const LineHdr *ch = shdr + b * CH;
-            const WingRec *cw = swing + b * CH * ntau_max;
-            const int n = min(CH, hi - (lo + c * CH) + 1);
-            if (nd > 0) {
-                for (int q = 0; q < n; q++) {
-                    const LineHdr h = ch[q];
-                    if (h.iright < tile_first || h.ileft > tile_last) continue;   // window misses the tile
-                    float x[P];
+        if (lane < n) {
+            const LineHdr h = J.hdr[S.queue[(head + lane) & 63]];
+            const bool core_hit = h.cl <= h.cr && h.cr >= tile_first && h.cl <= tile_last;
+            const bool full = h.ileft <= tile_first && h.iright >= tile_last && !core_hit;
+            const int l = max(h.ileft - tile_first, 0), r = min(h.iright - tile_first, TW - 1);
+            hnext = make_float4(h.wlh, h.wll, __int_as_float(l | r << 8 | (full ? WING_FULL : 0) | (core_hit ? WING_CORE : 0)),
+                                __int_as_float(h.pad0));
+        }
+    };
+    auto stage = [&]() -> int {                         // the fetched group into shared memory; its line count
+        __syncwarp();                                   // every lane is done with the group before
+#pragma unroll
+        for (int u = 0; u < U; u++) (&S.rec[0][0])[lane + 32 * u] = rnext[u];
+        if (lane < nnext) S.hdr[lane] = hnext;
+        __syncwarp();
+        const int n = nnext;
+        nnext = 0;
+        return n;
+    };
+    auto work = [&](int n) {
+        for (int q = 0; q < n; q++) {
+            const float4 h = S.hdr[q];
+            const int code = __float_as_int(h.z);
+            float x[P];
+#pragma unroll
+            for (int k = 0; k < P; k++) {
+                float dl = (wvh[k] - h.x) + (wvl[k] - h.y);
+                x[k] = dl * dl;
+            }
+            if (!(code & WING_FULL)) {
+                // points outside the window take the header's offset x, for which the wing term is exactly 0
+                const int l = code & 255, r = code >> 8 & 255;
+#pragma unroll
+                for (int k = 0; k < P; k++) {
+                    const int p = lane + 32 * k;
+                    x[k] = (p >= l && p <= r) ? x[k] : h.w;
+                }
+            }
+            const bool core_hit = code & WING_CORE;
+#pragma unroll
+            for (int j = 0; j < NP; j++) {
+                const float4 a = S.rec[q][2 * j], b = S.rec[q][2 * j + 1];
+                const float2 vv2 = make_float2(a.x, a.y), c2m1 = make_float2(a.z, a.w);
+                const float2 twoA = make_float2(b.x, b.y), c1 = make_float2(b.z, b.w);
+                if (!core_hit) {
 #pragma unroll
                     for (int k = 0; k < P; k++) {
-                        float dl = (wvh[k] - h.wlh) + (wvl[k] - h.wll);
-                        x[k] = dl * dl;
+                        const float2 t = __ffma2_rn(make_float2(x[k], x[k]), vv2, c2m1);
+                        const float2 den = __ffma2_rn(t, t, twoA), num = __ffma2_rn(c1, t, c1);
+                        part[j][k] = __ffma2_rn(num, make_float2(rcp_approx(den.x), rcp_approx(den.y)), part[j][k]);
                     }
-                    // depths past the job's last (last warp only) read the next records of the buffer, or
-                    // the headers after it: their partials are never stored
-                    const WingRec *wq = cw + q * ntau + t0;
-                    WingRec w[D];
+                } else {
 #pragma unroll
-                    for (int d = 0; d < D; d++) w[d] = wq[d];
-                    const bool core_hit = h.cl <= h.cr && h.cr >= tile_first && h.cl <= tile_last;
-                    const bool full = h.ileft <= tile_first && h.iright >= tile_last && !core_hit;
-                    if (!full) {
-                        // points outside the window take the header's offset x, for which the wing term is
-                        // exactly 0
-                        const float xm = __int_as_float(h.pad0);
-#pragma unroll
-                        for (int k = 0; k < P; k++) {
-                            const int p1 = pix[k] + 1;
-                            const bool in = p1 >= h.ileft && p1 <= h.iright;
-                            x[k] = in ? x[k] : xm;
-                        }
-                    }
-                    if (!core_hit) {
-#pragma unroll
-                        for (int d = 0; d < D; d++)
-#pragma unroll
-                            for (int k = 0; k < P; k++) {
-                                float t = fmaf(x[k], w[d].vv2, w[d].c2m1);
-                                float den = fmaf(t, t, w[d].twoA);
-                                float num = fmaf(w[d].c1, t, w[d].c1);
-                                part[d][k] = fmaf(num, rcp_approx(den), part[d][k]);
-                            }
-                    } else {
-#pragma unroll
-                        for (int d = 0; d < D; d++)
-#pragma unroll
-                            for (int k = 0; k < P; k++) {
-                                float t = fmaf(x[k], w[d].vv2, w[d].c2m1);
-                                t = t < 195.5f ? 1.0e19f : t;        // the core pass's point
-                                float den = fmaf(t, t, w[d].twoA);
-                                float num = fmaf(w[d].c1, t, w[d].c1);
-                                part[d][k] = fmaf(num, rcp_approx(den), part[d][k]);
-                            }
-                    }
-                    if (++nfold == FOLD) {
-                        nfold = 0;
-#pragma unroll
-                        for (int d = 0; d < D; d++)
-#pragma unroll
-                            for (int k = 0; k < P; k++) {
-                                float2 &qq = ksum[(d * P + k) * nth + threadIdx.x];
-                                float2 sc = qq;
-                                KAHAN(sc.x, sc.y, part[d][k]);
-                                qq = sc;
-                                part[d][k] = 0.0f;
-                            }
+                    for (int k = 0; k < P; k++) {
+                        float2 t = __ffma2_rn(make_float2(x[k], x[k]), vv2, c2m1);
+                        t.x = t.x < 195.5f ? 1.0e19f : t.x;          // the core pass's points
+                        t.y = t.y < 195.5f ? 1.0e19f : t.y;
+                        const float2 den = __ffma2_rn(t, t, twoA), num = __ffma2_rn(c1, t, c1);
+                        part[j][k] = __ffma2_rn(num, make_float2(rcp_approx(den.x), rcp_approx(den.y)), part[j][k]);
                     }
                 }
             }
-            __syncthreads();                                   // every warp is done with buffer b
-            if (threadIdx.x == 0 && c + WNB < nchunks)
-                stage_chunk(c + WNB, lo, hi, ntau, hdr, wing, shdr + b * CH, swing + b * CH * ntau_max, &bars[b],
-                            J.extra_tx);
-        }
-        if (failed >= 0) {
-            // a copy never completed: report, then wait (bounded) for the copies still in flight,
-            // chunks failed .. failed + WNB - 1, before the CTA's shared memory is released
-            if (threadIdx.x == 0) {
-                atomicExch(err, FSG_E_TIMEOUT);
-                for (int c = failed; c < nchunks && c < failed + WNB; c++) {
-                    const unsigned g = kk + c;
-                    mbar_wait(&bars[g % WNB], (g / WNB) & 1, J.wait_ns);
-                }
+            if (++nfold == FOLD) {
+                nfold = 0;
+#pragma unroll
+                for (int j = 0; j < NP; j++)
+#pragma unroll
+                    for (int k = 0; k < P; k++) {
+                        float2 s0 = S.ksum[2 * (j * P + k)][lane], s1 = S.ksum[2 * (j * P + k) + 1][lane];
+                        KAHAN(s0.x, s0.y, part[j][k].x);
+                        KAHAN(s1.x, s1.y, part[j][k].y);
+                        S.ksum[2 * (j * P + k)][lane] = s0;
+                        S.ksum[2 * (j * P + k) + 1][lane] = s1;
+                        part[j][k] = make_float2(0.0f, 0.0f);
+                    }
             }
-            __syncthreads();
-            return false;
         }
-        kk += nchunks;
+    };
+    int head = 0, cnt = 0;
+    auto advance = [&](int n) {                         // n queued lines into flight, the group before worked through
+        if (nnext) {
+            const int m = stage();
+            fetch(head, n);
+            head += n; cnt -= n;
+            work(m);
+        } else {
+            fetch(head, n);
+            head += n; cnt -= n;
+        }
+    };
+    for (int sg = 0; sg < J.nseg; sg++) {               // the job's segments of lines, in turn
+        const int lo = J.tile_lo[sg * J.seg_stride + tile], hi = J.tile_hi[sg * J.seg_stride + tile];
+        for (int base = lo; base <= hi; base += 32) {
+            const int i = base + lane;
+            bool sel = false;
+            if (i <= hi) {
+                const int2 w = *(const int2 *)&J.hdr[i].ileft;
+                sel = w.y >= tile_first && w.x <= tile_last;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, sel);
+            if (!m) continue;
+            if (sel) S.queue[(head + cnt + __popc(m & ((1u << lane) - 1u))) & 63] = i;
+            cnt += __popc(m);
+            __syncwarp();
+            while (cnt >= WING_G) advance(WING_G);
+        }
     }
-    if (nd <= 0) return true;
+    if (cnt) advance(cnt);
+    if (nnext) work(stage());
 #pragma unroll
     for (int k = 0; k < P; k++) {
-        if (pix[k] >= nwl) continue;
-        double *dst = J.lineopac + (size_t)pix[k] * ntau + t0;
+        const int pix = p0 + lane + 32 * k;
+        if (pix >= nwl) continue;
+        double *dst = J.lineopac + (size_t)pix * ntau + t0;
 #pragma unroll
-        for (int d = 0; d < D; d++) {
-            float2 sc = ksum[(d * P + k) * nth + threadIdx.x];
-            KAHAN(sc.x, sc.y, part[d][k]);
-            if (d < nd) dst[d] = dst[d] + ((double)sc.x - (double)sc.y);
+        for (int j = 0; j < NP; j++) {
+            float2 s0 = S.ksum[2 * (j * P + k)][lane], s1 = S.ksum[2 * (j * P + k) + 1][lane];
+            KAHAN(s0.x, s0.y, part[j][k].x);
+            KAHAN(s1.x, s1.y, part[j][k].y);
+            if (t0 + 2 * j < ntau) dst[2 * j] += (double)s0.x - (double)s0.y;
+            if (t0 + 2 * j + 1 < ntau) dst[2 * j + 1] += (double)s1.x - (double)s1.y;
         }
     }
-    return true;
 }
 
-__device__ __forceinline__ void wing_bars_init(unsigned char *smem_raw, int ntau_max) {
-    uint64_t *bars = (uint64_t *)(smem_raw + wing_smem_recs(ntau_max));
-    if (threadIdx.x == 0) {
-        for (int b = 0; b < WNB; b++) mbar_init(&bars[b], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-}
+// depths per warp for P wavelengths per lane: P x D = 16 evaluations per thread and line
+#define WING_D(P) (16 / (P))
+#define WING_W 4                      // warps per CTA
+#define WING_BW 8                     // warps per CTA of the persistent form
 
-// one tile per CTA (blockIdx.x)
+// one (tile, depth group) per warp, the groups of a tile in turn
 template <int D, int P>
-__global__ void __launch_bounds__(32 * 18, 1)
-k_accum_fast(WingJob J, int *__restrict__ err) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    if (J.tile_lo[blockIdx.x] > J.tile_hi[blockIdx.x]) return;
-    wing_bars_init(smem_raw, J.ntau);
-    unsigned kk = 0;
-    wing_tile<D, P>(J, blockIdx.x, smem_raw, J.ntau, kk, err);
+__global__ void __launch_bounds__(32 * WING_W)
+k_accum_fast(WingJob J, int ntiles) {
+    __shared__ WingWarp<D, P> S[WING_W];
+    const int warp = threadIdx.x >> 5, ng = (J.ntau + D - 1) / D;
+    const int64_t item = (int64_t)blockIdx.x * WING_W + warp;
+    if (item >= (int64_t)ntiles * ng) return;           // warps are independent: no CTA barrier
+    wing_tile<D, P>(J, (int)(item / ng), (int)(item % ng) * D, S[warp], threadIdx.x & 31);
 }
 
-// Persistent form for many jobs (batched atmospheres): CTAs take (job, tile) items from a device
-// work queue (*queue, zero at launch) until jobs[njobs - 1] is done; tile0[j] is the first item of
-// job j (prefix sums of the jobs' tile counts, tile0[njobs] = total).
+// Persistent form for many jobs (batched atmospheres): warps take (job, tile, depth group) items from a
+// device work queue (*queue, zero at launch) until all are done; item0[j] is the first item of job j
+// (prefix sums of the jobs' tiles x groups, item0[njobs] = total).
 template <int D, int P>
-__global__ void __launch_bounds__(32 * 18, 1)
-k_accum_batch(const WingJob *__restrict__ jobs, const int *__restrict__ tile0, int njobs, int ntau_max,
-              unsigned *queue, int *__restrict__ err) {
+__global__ void __launch_bounds__(32 * WING_BW)
+k_accum_batch(const WingJob *__restrict__ jobs, const int *__restrict__ item0, int njobs, unsigned *queue) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ int s_item;
-    wing_bars_init(smem_raw, ntau_max);
-    unsigned kk = 0;
-    const int total = tile0[njobs];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    WingWarp<D, P> &S = ((WingWarp<D, P> *)smem_raw)[warp];
+    const int total = item0[njobs];
     for (;;) {
-        if (threadIdx.x == 0) s_item = (int)atomicAdd(queue, 1u);
-        __syncthreads();
-        const int item = s_item;
-        __syncthreads();
+        int item = 0;
+        if (lane == 0) item = (int)atomicAdd(queue, 1u);
+        item = __shfl_sync(0xffffffffu, item, 0);
         if (item >= total) break;
-        int a = 0, b = njobs - 1;                          // job with tile0[a] <= item < tile0[a + 1]
-        while (a < b) { int m = (a + b + 1) >> 1; if (tile0[m] <= item) a = m; else b = m - 1; }
+        int a = 0, b = njobs - 1;                          // job with item0[a] <= item < item0[a + 1]
+        while (a < b) { int m = (a + b + 1) >> 1; if (item0[m] <= item) a = m; else b = m - 1; }
         const WingJob J = jobs[a];
-        if (!wing_tile<D, P>(J, item - tile0[a], smem_raw, ntau_max, kk, err)) break;
+        const int ng = (J.ntau + D - 1) / D, r = item - item0[a];
+        wing_tile<D, P>(J, r / ng, (r % ng) * D, S, lane);
     }
 }
 
 // Tile width per window-width class: narrow windows get narrower tiles so fewer lanes idle.
 int fsg_class_pix(int cls) { return cls <= 1 ? 2 : 4; }
 
-// depths per warp for P wavelengths per lane: P x D = 16 evaluations per thread and line, at most
-// 18 warps per CTA
-static int wing_depths(int P, int ntau) {
-    int D = 16 / P;
-    if ((ntau + D - 1) / D > 18) D = (ntau + 17) / 18;
-    return D;
-}
-
-size_t fsg_wing_smem(int P, int ntau_max) {
-    const int D = wing_depths(P, ntau_max), nwarps = (ntau_max + D - 1) / D;
-    return wing_smem_recs(ntau_max) + WNB * sizeof(uint64_t) + sizeof(float2) * (size_t)D * P * 32 * nwarps;
-}
-
-#define WING_DISPATCH(P, D, LAUNCH) do { \
-        if (P == 2) { if (D == 8) LAUNCH(8, 2); else return FSG_E_ARG; } \
-        else switch (D) { case 4: LAUNCH(4, 4); break; case 5: LAUNCH(5, 4); break; case 6: LAUNCH(6, 4); break; \
-                          case 7: LAUNCH(7, 4); break; case 8: LAUNCH(8, 4); break; default: return FSG_E_ARG; } \
-    } while (0)
+// depth groups of the wing pass
+int fsg_wing_groups(int P, int ntau) { return (ntau + WING_D(P) - 1) / WING_D(P); }
 
 int fsg_launch_accum_fast(cudaStream_t st, int cls, int ntau, int nwl, const double *wave, const LineHdr *hdr,
-                          const WingRec *wing, const int *tile_lo, const int *tile_hi, double *lineopac, int *err,
-                          unsigned extra_tx, unsigned long long wait_ns) {
-    const int P = fsg_class_pix(cls);
-    const int TW = 32 * P;
-    const int ntiles = (nwl + TW - 1) / TW;
-    const int D = wing_depths(P, ntau);
-    const int nwarps = (ntau + D - 1) / D;
-    const size_t smem = fsg_wing_smem(P, ntau);
-    if (smem > 200 * 1024) return FSG_E_ARG;
-    WingJob J{ ntau, nwl, wave, hdr, wing, tile_lo, tile_hi, lineopac, extra_tx, wait_ns, 1, 0 };
-#define LAUNCH(DD, PP) do { \
-        cudaFuncSetAttribute(k_accum_fast<DD, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        k_accum_fast<DD, PP><<<ntiles, 32 * nwarps, smem, st>>>(J, err); } while (0)
-    WING_DISPATCH(P, D, LAUNCH);
-#undef LAUNCH
+                          const WingPair *wing, const int *tile_lo, const int *tile_hi, double *lineopac) {
+    const int P = fsg_class_pix(cls), TW = 32 * P, ntiles = (nwl + TW - 1) / TW;
+    const unsigned grid = (unsigned)(((int64_t)ntiles * fsg_wing_groups(P, ntau) + WING_W - 1) / WING_W);
+    WingJob J{ ntau, nwl, wave, hdr, wing, tile_lo, tile_hi, lineopac, 1, 0 };
+    if (P == 2) k_accum_fast<WING_D(2), 2><<<grid, 32 * WING_W, 0, st>>>(J, ntiles);
+    else k_accum_fast<WING_D(4), 4><<<grid, 32 * WING_W, 0, st>>>(J, ntiles);
     return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }
 
-// the persistent wing pass over njobs jobs (device array), P wavelengths per lane, ctas CTAs
-int fsg_launch_accum_batch(cudaStream_t st, int P, int ntau_max, const WingJob *jobs, const int *tile0, int njobs,
-                           int ctas, unsigned *queue, int *err) {
-    const int D = wing_depths(P, ntau_max);
-    const int nwarps = (ntau_max + D - 1) / D;
-    const size_t smem = fsg_wing_smem(P, ntau_max);
-    if (smem > 200 * 1024) return FSG_E_ARG;
-#define LAUNCH(DD, PP) do { \
-        cudaFuncSetAttribute(k_accum_batch<DD, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        k_accum_batch<DD, PP><<<ctas, 32 * nwarps, smem, st>>>(jobs, tile0, njobs, ntau_max, queue, err); } while (0)
-    WING_DISPATCH(P, D, LAUNCH);
-#undef LAUNCH
+// the persistent wing pass over njobs jobs (device array), P wavelengths per lane; ctas counts CTAs of 16
+// warps (two of the kernel's)
+int fsg_launch_accum_batch(cudaStream_t st, int P, const WingJob *jobs, const int *item0, int njobs, int ctas,
+                           unsigned *queue) {
+    const size_t smem = WING_BW * (P == 2 ? sizeof(WingWarp<WING_D(2), 2>) : sizeof(WingWarp<WING_D(4), 4>));
+    const unsigned grid = (unsigned)ctas * (16 / WING_BW);
+    if (P == 2) k_accum_batch<WING_D(2), 2><<<grid, 32 * WING_BW, smem, st>>>(jobs, item0, njobs, queue);
+    else k_accum_batch<WING_D(4), 4><<<grid, 32 * WING_BW, smem, st>>>(jobs, item0, njobs, queue);
     return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }
 
@@ -359,7 +319,7 @@ int fsg_launch_accum_batch(cudaStream_t st, int P, int ntau_max, const WingJob *
 // table lerp or the continued fraction, as HVoigt branches (voigt.f90:81-107); the wing pass takes the
 // others (the same FP32 test splits the points, so each is evaluated once).  A CTA owns 32 wavelengths
 // x all depths: warp w depths [w*D, w*D + D), lane l wavelength tile0 + l, Kahan sums in
-// registers.  Headers, wing records and core records of the tile's candidate lines arrive in shared
+// registers.  Headers and core records of the tile's candidate lines arrive in shared
 // memory CHC lines at a time by double-buffered bulk copies completing on mbarriers (waits bounded;
 // on expiry the kernel reports FSG_E_TIMEOUT and drains its copies), so the loop over lines reads
 // shared memory; per line a thread forms its depths' branch predicates first and issues their table
@@ -368,20 +328,19 @@ int fsg_launch_accum_batch(cudaStream_t st, int P, int ntau_max, const WingJob *
 
 
 // shared memory of the core pass for at most ntau_max depths and chc lines per chunk:
-// wing records [2][chc][ntau_max] | core records [2][chc][ntau_max] | headers [2][chc] | mbarriers [2]
+// core records [2][chc][ntau_max] | headers [2][chc] | mbarriers [2]
 __host__ __device__ inline size_t core_smem(int ntau_max, int chc) {
-    return (sizeof(WingRec) + sizeof(CoreRec)) * 2 * (size_t)chc * ntau_max + sizeof(LineHdr) * 2 * (size_t)chc +
+    return sizeof(CoreRec) * 2 * (size_t)chc * ntau_max + sizeof(LineHdr) * 2 * (size_t)chc +
            2 * sizeof(uint64_t);
 }
 
 __device__ __forceinline__ void core_stage(int c, int lo, int hi, int ntau, int chc, const CoreJob &J,
-                                           WingRec *sw, CoreRec *sc, LineHdr *sh, uint64_t *bar) {
+                                           CoreRec *sc, LineHdr *sh, uint64_t *bar) {
     const int j0 = lo + c * chc;
     const int n = min(chc, hi - j0 + 1);
-    const unsigned bw = (unsigned)(n * ntau * (int)sizeof(WingRec)), bc = (unsigned)(n * ntau * (int)sizeof(CoreRec));
+    const unsigned bc = (unsigned)(n * ntau * (int)sizeof(CoreRec));
     const unsigned bh = (unsigned)(n * (int)sizeof(LineHdr));
-    mbar_expect_tx(bar, bw + bc + bh + J.extra_tx);
-    tma_bulk_g2s(sw, J.wing + (size_t)j0 * ntau, bw, bar);
+    mbar_expect_tx(bar, bc + bh + J.extra_tx);
     tma_bulk_g2s(sc, J.core + (size_t)j0 * ntau, bc, bar);
     tma_bulk_g2s(sh, J.hdr + j0, bh, bar);
 }
@@ -397,8 +356,7 @@ __device__ bool core_tile(const CoreJob &J, int tile, const float4 *__restrict__
     for (int sg = 0; sg < J.nseg; sg++)
         any = any || J.tile_lo[sg * J.seg_stride + tile] <= J.tile_hi[sg * J.seg_stride + tile];
     if (!any) return true;
-    WingRec *sw = (WingRec *)smem_raw;
-    CoreRec *sc = (CoreRec *)(sw + 2 * (size_t)chc * ntau_max);
+    CoreRec *sc = (CoreRec *)smem_raw;
     LineHdr *sh = (LineHdr *)(sc + 2 * (size_t)chc * ntau_max);
     uint64_t *bars = (uint64_t *)(sh + 2 * chc);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -419,8 +377,7 @@ __device__ bool core_tile(const CoreJob &J, int tile, const float4 *__restrict__
         if (threadIdx.x == 0)
             for (int c = 0; c < 2 && c < nchunks; c++) {
                 const int b = (kk + c) & 1;
-                core_stage(c, lo, hi, ntau, chc, J, sw + (size_t)b * chc * ntau_max, sc + (size_t)b * chc * ntau_max,
-                           sh + b * chc, &bars[b]);
+                core_stage(c, lo, hi, ntau, chc, J, sc + (size_t)b * chc * ntau_max, sh + b * chc, &bars[b]);
             }
         int failed = -1;
         for (int c = 0; c < nchunks; c++) {
@@ -429,7 +386,6 @@ __device__ bool core_tile(const CoreJob &J, int tile, const float4 *__restrict__
             const bool ok = mbar_wait(&bars[b], (g >> 1) & 1, J.wait_ns);
             if (__syncthreads_or(!ok)) { failed = c; break; }
             const LineHdr *ch = sh + b * chc;
-            const WingRec *cw = sw + (size_t)b * chc * ntau_max;
             const CoreRec *cc = sc + (size_t)b * chc * ntau_max;
             const int n = min(chc, hi - (lo + c * chc) + 1);
             if (nd > 0) {
@@ -450,9 +406,8 @@ __device__ bool core_tile(const CoreJob &J, int tile, const float4 *__restrict__
                         for (int e = 0; e < 4; e++) {
                             const int d = g0 + e;
                             const int td = t0 + min(d, nd - 1);
-                            const WingRec w = cw[q * ntau + td];
                             const CoreRec cr = cc[q * ntau + td];
-                            const float t = fmaf(x, w.vv2, w.c2m1);
+                            const float t = fmaf(x, cr.vv2, cr.c2m1);
                             core[e] = in && d < nd && t < 195.5f;
                             const double av = adl * cr.vv;
                             tab[e] = core[e] && cr.ia > 0 && av < 8.0;
@@ -486,8 +441,7 @@ __device__ bool core_tile(const CoreJob &J, int tile, const float4 *__restrict__
             }
             __syncthreads();                                   // every warp is done with buffer b
             if (threadIdx.x == 0 && c + 2 < nchunks)
-                core_stage(c + 2, lo, hi, ntau, chc, J, sw + (size_t)b * chc * ntau_max,
-                           sc + (size_t)b * chc * ntau_max, sh + b * chc, &bars[b]);
+                core_stage(c + 2, lo, hi, ntau, chc, J, sc + (size_t)b * chc * ntau_max, sh + b * chc, &bars[b]);
         }
         if (failed >= 0) {
             if (threadIdx.x == 0) {
@@ -562,7 +516,7 @@ k_core_batch(const CoreJob *__restrict__ jobs, const int *__restrict__ tile0, in
 // SM's L1 with the table gathers: per 1e8-line step the core pass took 1.82 / 1.71 / 1.75 / 1.85 s
 // with 48 / 32 / 24 / 16 KB.
 static int core_chunk(int ntau_max) {
-    const int per_line = ntau_max * (int)(sizeof(WingRec) + sizeof(CoreRec)) + (int)sizeof(LineHdr);
+    const int per_line = ntau_max * (int)sizeof(CoreRec) + (int)sizeof(LineHdr);
     return std::max(4, std::min(16, (32 * 1024) / per_line));
 }
 
@@ -571,15 +525,14 @@ static int core_chunk(int ntau_max) {
 static int core_depths(int) { return 8; }
 
 int fsg_launch_core_fast(cudaStream_t st, int ntau, int nwl, const double *wave, const LineHdr *hdr,
-                         const WingRec *wing, const CoreRec *core, const int *tile_lo, const int *tile_hi,
-                         const float4 *vtab4, double *lineopac, unsigned long long *nevals, int *err,
+                         const CoreRec *core, const int *tile_lo, const int *tile_hi, const float4 *vtab4, double *lineopac, unsigned long long *nevals, int *err,
                          unsigned extra_tx, unsigned long long wait_ns) {
     const int ntiles = (nwl + 31) / 32;
     const int D = core_depths(ntau), nwarps = (ntau + D - 1) / D;
     if (nwarps > 18) return FSG_E_ARG;
     const int chc = core_chunk(ntau);
     const size_t smem = core_smem(ntau, chc);
-    CoreJob J{ ntau, nwl, wave, hdr, wing, core, tile_lo, tile_hi, lineopac, nevals, extra_tx, wait_ns, 1, 0 };
+    CoreJob J{ ntau, nwl, wave, hdr, core, tile_lo, tile_hi, lineopac, nevals, extra_tx, wait_ns, 1, 0 };
     if (D == 4) {
         cudaFuncSetAttribute(k_core_fast<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_core_fast<4><<<ntiles, 32 * nwarps, smem, st>>>(J, vtab4, chc, err);

@@ -74,13 +74,18 @@ struct XCoef {
 // With y = s + 1/2 the denominator is exactly (y - 1)^2 + 2 a^2, so with t = y - 1
 //   H * LinCop = c1 (t + 1) / (t^2 + twoA),  t = dl^2 vv2 + c2m1,
 // with vv2 = LinVvgt^2, c2m1 = a^2 - 1/2, twoA = 2 a^2, c1 = LinCop a / sqrt(pi).
-struct __align__(16) WingRec { float vv2, c2m1, twoA, c1; };
+// The records of two neighbouring depths (t even, t + 1) lie side by side: the wing pass evaluates depth
+// pairs in packed FP32.  A line has wing_pairs(ntau) of them; the last half of an odd count is 0.
+struct __align__(16) WingPair { float vv2[2], c2m1[2], twoA[2], c1[2]; };
+static_assert(sizeof(WingPair) == 32, "wing pair: two 16-byte loads");
+__host__ __device__ inline int wing_pairs(int ntau) { return (ntau + 1) >> 1; }
 // Table / continued-fraction region (s < 196): LinVvgt in FP64, LinCop, a, and the table row ia
 // (1-based) with its interpolation weight ua as HVoigt derives them from a in FP64
 // (voigt.f90:84-92); ia = 0 when a >= 8 (no table).  v = |dl| LinVvgt and the table column and
 // fraction are formed in FP64 as the reference forms them: on the Gaussian flanks of a line core
-// H falls as exp(-v^2), so an FP32 v (relative error ~1e-7) would move H by 2 v^2 * 1e-7.
-struct __align__(16) CoreRec { double vv; float cop, ua, a; int ia; int pad0, pad1; };
+// H falls as exp(-v^2), so an FP32 v (relative error ~1e-7) would move H by 2 v^2 * 1e-7.  vv2 and c2m1
+// are the wing record's: both passes split the points by the same FP32 t.
+struct __align__(16) CoreRec { double vv; float cop, ua, a; int ia; float vv2, c2m1; };
 static_assert(sizeof(CoreRec) == 32, "core record: 32 bytes");
 
 // Line header of a retained line inside a block (fast path).  The centre offset Wlcent is split
@@ -119,27 +124,24 @@ static_assert(sizeof(XCoef) == sizeof(fsg_xcoef), "fsg_xcoef mirrors XCoef");
 // One wing-pass job: the line records and tiles of one LineOpac (one atmosphere and grid).  Its
 // tile ranges come in nseg segments (window-width classes of one record array), segment s at
 // tile_lo / tile_hi + s * seg_stride; a tile takes the segments' lines in turn into one sum.
-// extra_tx / wait_ns: 0 and WAIT_NS in use; a test of the error path (fsg_set_fault) makes every
-// chunk expect extra_tx bytes more than its copies deliver and bounds the waits by wait_ns.
 struct WingJob {
     int ntau, nwl;
     const double *wave;
     const LineHdr *hdr;
-    const WingRec *wing;
+    const WingPair *wing;
     const int *tile_lo, *tile_hi;
     double *lineopac;
-    unsigned extra_tx;
-    unsigned long long wait_ns;
     int nseg, seg_stride;
 };
 
-// One core-pass job: as WingJob plus the core records; tiles of 32 wavelengths.  nevals (may be
-// null) counts the evaluations.
+// One core-pass job: as WingJob with the core records; tiles of 32 wavelengths.  nevals (may be
+// null) counts the evaluations.  extra_tx / wait_ns: 0 and WAIT_NS in use; a test of the error path
+// (fsg_set_fault) makes every chunk expect extra_tx bytes more than its copies deliver and bounds the waits
+// by wait_ns.
 struct CoreJob {
     int ntau, nwl;
     const double *wave;
     const LineHdr *hdr;
-    const WingRec *wing;
     const CoreRec *core;
     const int *tile_lo, *tile_hi;
     double *lineopac;
