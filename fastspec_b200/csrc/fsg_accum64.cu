@@ -19,6 +19,7 @@
 // evaluations/s).  P = 2 and D = 4 keep the per-line work (offsets, window test, 8 shared loads) under a
 // tenth of the evaluations' and leave registers for five 4-warp CTAs per SM.
 #include "fsg_fp64.cuh"
+#include "fsg_tile.cuh"
 
 #define A64_P 2
 #define A64_D 4
@@ -57,29 +58,6 @@ __device__ __forceinline__ double core64(const float *__restrict__ vtab, const C
     const double a2 = c.a * c.a, v2 = av * av, p = v2 - a2 - 1.5, q = 2.0 * av * c.a;
     const double dr = av * p - c.a * q, di = av * q + c.a * p;
     return FSG_SQRTPIINV * ((p + 0.5) * di - q * dr) / (dr * dr + di * di) * c.cop;
-}
-
-// Rows lo .. hi whose windows meet the wavelengths first .. last, in order: group(head, n) gets them G at a
-// time (the last call fewer) as queue[(head + i) & 63], i < n; queue holds 64 rows of the calling warp.
-template <int G, class F>
-__device__ __forceinline__ void tile_lines(const LineHdr64 *__restrict__ hdr, int lo, int hi, int first, int last,
-                                           int *queue, int lane, F group) {
-    int head = 0, cnt = 0;
-    for (int base = lo; base <= hi; base += 32) {
-        const int j = base + lane;
-        bool sel = false;
-        if (j <= hi) {
-            const int2 w = *(const int2 *)&hdr[j].il;
-            sel = w.x <= w.y && w.x <= last && w.y >= first;
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, sel);
-        if (!m) continue;
-        if (sel) queue[(head + cnt + __popc(m & ((1u << lane) - 1u))) & 63] = j;
-        cnt += __popc(m);
-        __syncwarp();
-        while (cnt >= G) { group(head, G); head += G; cnt -= G; }
-    }
-    if (cnt > 0) group(head, cnt);
 }
 
 // table row and weight of a as HVoigt takes them (voigt.f90:84-92); ia = 0: a >= 8

@@ -122,10 +122,10 @@ size_t fsg_tile_span_scratch(int64_t);
 int fsg_launch_tile_span_tw(cudaStream_t, int, int, int, int64_t, const LineHdr *, int *, int *, void *, size_t);
 void fsg_launch_mag_params_fast(cudaStream_t, const AtmView &, const LineView &, const ZView &, const int64_t *, int64_t,
                                 int64_t, const int32_t *, const int32_t *, const int32_t *, const VoigtTables &, void *,
-                                LineHdr *, int64_t *);
-size_t fsg_mag_rec_bytes();
-int fsg_launch_mag_fast(cudaStream_t, const AtmView &, const LineHdr *, const void *, const int64_t *, const ZView &,
-                        const int *, const int *, const VoigtTables &, double *);
+                                LineHdr *);
+size_t fsg_mag_rec_bytes(int);
+int fsg_launch_mag_fast(cudaStream_t, const AtmView &, const LineHdr *, void *, int64_t, const ZView &, const int *,
+                        const int *, const VoigtTables &, double *);
 void fsg_launch_conv(cudaStream_t, int, const double *, int, const double *, int, double *, const double *, double);
 size_t fsg_adjoint_work(int, int, int64_t, int);
 int fsg_launch_adjoint(cudaStream_t, const AtmView &, const LineView &, const VoigtTables &, const double *,
@@ -1351,11 +1351,10 @@ static int mag_lineop_calc_body(fsg_ctx *ctx, const fsg_lines *lines, int bframe
                        ctx->d_idx.as<int64_t>(), ctx->d_total.as<int64_t>()))
             return cuda_fail(ctx, cudaGetLastError(), "select");
         ctx->launches += 3;
-        const size_t per_line = fsg_mag_rec_bytes() * nt + sizeof(LineHdr) + sizeof(int64_t);
+        const size_t per_line = fsg_mag_rec_bytes(nt) + sizeof(LineHdr);
         const int64_t bcap = std::min<int64_t>(std::max<int64_t>(nkeep, 1), block_capacity(ctx, per_line));
-        ALLOC(ctx->d_wing, fsg_mag_rec_bytes() * (size_t)bcap * nt);
+        ALLOC(ctx->d_wing, fsg_mag_rec_bytes(nt) * (size_t)bcap);
         ALLOC(ctx->d_hdr, sizeof(LineHdr) * (size_t)bcap);
-        ALLOC(ctx->d_zmap, sizeof(int64_t) * (size_t)bcap);
         ALLOC(ctx->d_span, fsg_tile_span_scratch(bcap));
         ALLOC(ctx->d_tlo, sizeof(int) * (size_t)fsg_fast_tiles(nwl)); ALLOC(ctx->d_thi, sizeof(int) * (size_t)fsg_fast_tiles(nwl));
         double *mlo = ctx->d_maglineopac.as<double>();
@@ -1363,10 +1362,10 @@ static int mag_lineop_calc_body(fsg_ctx *ctx, const fsg_lines *lines, int bframe
         for (int64_t j0 = 0; j0 < nkeep; j0 += bcap) {
             const int64_t nb = std::min(bcap, nkeep - j0);
             fsg_launch_mag_params_fast(s, A, LV, Z, ctx->d_idx.as<int64_t>(), j0, nb, pf, pl, pr, ctx->tab, ctx->d_wing.p,
-                                       ctx->d_hdr.as<LineHdr>(), ctx->d_zmap.as<int64_t>());
+                                       ctx->d_hdr.as<LineHdr>());
             if (fsg_launch_tile_span_tw(s, 32, 0, nwl, nb, ctx->d_hdr.as<LineHdr>(), ctx->d_tlo.as<int>(),
                                         ctx->d_thi.as<int>(), ctx->d_span.p, ctx->d_span.cap) ||
-                fsg_launch_mag_fast(s, A, ctx->d_hdr.as<LineHdr>(), ctx->d_wing.p, ctx->d_zmap.as<int64_t>(), Z,
+                fsg_launch_mag_fast(s, A, ctx->d_hdr.as<LineHdr>(), ctx->d_wing.p, nb, Z,
                                     ctx->d_tlo.as<int>(), ctx->d_thi.as<int>(), ctx->tab, mlo))
                 return cuda_fail(ctx, cudaGetLastError(), "k_mag_fast");
             ctx->launches += 8;
