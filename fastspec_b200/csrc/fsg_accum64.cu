@@ -27,16 +27,6 @@
 #define A64_TW (32 * A64_P)
 #define A64_W 4                     // warps per CTA
 
-// 1 / d for normal d in FP64: the hardware's approximate reciprocal r (relative error e, |e| < 2^-19)
-// and one third-order step r (1 + e + e^2), e = 1 - d r, which leaves e^3
-__device__ __forceinline__ double rcp64(double d) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    double e = fma(-d, r, 1.0);
-    e = fma(e, e, e);
-    return fma(r, e, r);
-}
-
 struct Wing64 { double vv2, c2m1, twoA, c1; };
 struct Core64 { double vv, a, ua, cop; int ia, pad; };
 

@@ -132,9 +132,8 @@ int fsg_launch_adjoint(cudaStream_t, const AtmView &, const LineView &, const Vo
                        const double *, int, const double *, const double *, const RayView &, const int32_t *,
                        const int32_t *, const int32_t *, const double *, double *, double *, double, double *,
                        double *, int, int);
-size_t fsg_linstr_work(int64_t, int, int);
-void fsg_launch_linstr(cudaStream_t, const AtmView &, const LineView &, const VoigtTables &, const int32_t *, int64_t,
-                       int64_t, int, const double *, const double *, const double *, const RayView &, double *, float *);
+void fsg_launch_linstr(cudaStream_t, const AtmView &, const LineView &, const VoigtTables &, const int32_t *, int,
+                       const double *, const double *, const double *, const RayView &, float *);
 int fsg_launch_radtran_sph(cudaStream_t, const AtmView &, const double *, const RayView &, const double *, double *,
                            double *, double *, double *);
 int fsg_launch_stokes_sph(cudaStream_t, const AtmView &, const double *, const double *, const RayView &,
@@ -225,7 +224,7 @@ struct fsg_ctx {
     DBuf l_wl, l_elo, l_gf, l_grad, l_gqst, l_gvdw, l_spc, l_ismol, l_ihe;
     DBuf d_flags, d_ileft, d_iright, d_idx, d_counts, d_offs, d_total, d_hist, d_nkeep;
     // block buffers
-    DBuf d_wing, d_core, d_hdr, d_hdr64, d_tlo, d_thi, d_p64, d_lstart, d_lstop, d_widx, d_pw, d_err, d_ncore, d_span, d_lswork, d_linstr, d_rflags, d_rleft, d_rright, d_gkappa, d_adjwork, d_cbuf, d_ctaps;
+    DBuf d_wing, d_core, d_hdr, d_hdr64, d_tlo, d_thi, d_p64, d_lstart, d_lstop, d_widx, d_pw, d_err, d_ncore, d_span, d_linstr, d_rflags, d_rleft, d_rright, d_gkappa, d_adjwork, d_cbuf, d_ctaps;
     // spectra
     DBuf d_spl, d_spc, d_sfl, d_sfc, d_work, d_a, d_v, d_h, d_l;
     // magnetic
@@ -317,7 +316,7 @@ void fsg_destroy(fsg_ctx *ctx) {
                      &ctx->l_grad, &ctx->l_gqst, &ctx->l_gvdw, &ctx->l_spc, &ctx->l_ismol, &ctx->l_ihe,
                      &ctx->d_flags, &ctx->d_ileft, &ctx->d_iright, &ctx->d_idx, &ctx->d_counts, &ctx->d_offs,
                      &ctx->d_total, &ctx->d_hist, &ctx->d_nkeep, &ctx->d_wing, &ctx->d_core, &ctx->d_hdr, &ctx->d_hdr64,
-                     &ctx->d_tlo, &ctx->d_thi, &ctx->d_err, &ctx->d_ncore, &ctx->d_span, &ctx->d_lswork, &ctx->d_linstr, &ctx->d_rflags, &ctx->d_rleft, &ctx->d_rright, &ctx->d_gkappa, &ctx->d_adjwork, &ctx->d_cbuf, &ctx->d_ctaps, &ctx->d_p64, &ctx->d_lstart, &ctx->d_lstop, &ctx->d_widx,
+                     &ctx->d_tlo, &ctx->d_thi, &ctx->d_err, &ctx->d_ncore, &ctx->d_span, &ctx->d_linstr, &ctx->d_rflags, &ctx->d_rleft, &ctx->d_rright, &ctx->d_gkappa, &ctx->d_adjwork, &ctx->d_cbuf, &ctx->d_ctaps, &ctx->d_p64, &ctx->d_lstart, &ctx->d_lstop, &ctx->d_widx,
                      &ctx->d_pw, &ctx->d_spl, &ctx->d_spc, &ctx->d_sfl, &ctx->d_sfc,
                      &ctx->d_work, &ctx->d_a, &ctx->d_v, &ctx->d_h, &ctx->d_l, &ctx->z_npi, &ctx->z_nsi,
                      &ctx->z_pioff, &ctx->z_sioff, &ctx->z_splpi, &ctx->z_strpi, &ctx->z_splsi, &ctx->z_strsi,
@@ -500,7 +499,7 @@ static int rays_prepare(fsg_ctx *ctx, RayView *R) {
     const int nt = ctx->ntau, nmu = ctx->nmu, M = 2 * nt;
     R->nmu = nmu; R->stride = M;
     if (!ctx->rays_ok) {
-        std::vector<double> rk(nt), rm((size_t)nmu * M, 0.0), ml((size_t)nmu * M, 0.0);
+        std::vector<double> rk(nt), rm((size_t)4 * nmu * M, 0.0), ml((size_t)nmu * M, 0.0);   // rm: m | dm | idm | lam
         std::vector<int> n(nmu), gz(nmu), mp((size_t)nmu * M, 0);
         for (int k = 0; k < nt; k++) rk[k] = ctx->radius + ctx->h_height[k];
         const double *rhox = ctx->h_rhox.data();
@@ -512,7 +511,7 @@ static int rays_prepare(fsg_ctx *ctx, RayView *R) {
             const double P = rk[0] * sqrt((1.0 - mu) * (1.0 + mu));
             const int g = P > rk[nt - 1];
             int deep = nt;
-            if (g) {
+            if (g) {                                        // turn below the deepest layer
                 int kt = 2;
                 while (kt <= nt && !(P >= rk[kt - 1])) kt++;
                 deep = kt - 1;
@@ -530,17 +529,25 @@ static int rays_prepare(fsg_ctx *ctx, RayView *R) {
             }
             gz[im] = g;
             n[im] = nt;
-            if (!g) continue;
-            double chord = 2.0 * sqrt((rk[deep - 1] - P) * (rk[deep - 1] + P));
-            m[deep] = m[deep - 1] + chord * (rhox[deep] - rhox[deep - 1]) / (rk[deep - 1] - rk[deep]);
-            q[deep] = deep - 1;
-            c[deep] = -c[deep - 1];
-            for (int k = deep + 1; k < 2 * deep; k++) {          // the far half mirrors the near one
-                m[k] = m[k - 1] + (m[2 * deep - k] - m[2 * deep - k - 1]);
-                q[k] = 2 * deep - 1 - k;
-                c[k] = -c[2 * deep - 1 - k];
+            if (g) {                                        // turn below the deepest layer
+                double chord = 2.0 * sqrt((rk[deep - 1] - P) * (rk[deep - 1] + P));
+                m[deep] = m[deep - 1] + chord * (rhox[deep] - rhox[deep - 1]) / (rk[deep - 1] - rk[deep]);
+                q[deep] = deep - 1;
+                c[deep] = -c[deep - 1];
+                for (int k = deep + 1; k < 2 * deep; k++) {          // the far half mirrors the near one
+                    m[k] = m[k - 1] + (m[2 * deep - k] - m[2 * deep - k - 1]);
+                    q[k] = 2 * deep - 1 - k;
+                    c[k] = -c[2 * deep - 1 - k];
+                }
+                n[im] = 2 * deep;
             }
-            n[im] = 2 * deep;
+            // steps, their reciprocals and TauStep's Lambda (solver.f90:605) for the sweeps
+            double *dm = m + (size_t)nmu * M, *idm = dm + (size_t)nmu * M, *lam = idm + (size_t)nmu * M;
+            for (int k = 0; k < n[im] - 1; k++) {
+                dm[k] = m[k + 1] - m[k];
+                idm[k] = 1.0 / dm[k];
+                if (k > 0) lam[k] = (1.0 + dm[k] / (dm[k - 1] + dm[k])) / 3.0;
+            }
         }
         ALLOC(ctx->d_ray_n, sizeof(int) * nmu); ALLOC(ctx->d_ray_graz, sizeof(int) * nmu);
         ALLOC(ctx->d_ray_map, sizeof(int) * mp.size()); ALLOC(ctx->d_ray_m, sizeof(double) * rm.size());
@@ -555,6 +562,7 @@ static int rays_prepare(fsg_ctx *ctx, RayView *R) {
     }
     R->n = ctx->d_ray_n.as<int>(); R->graz = ctx->d_ray_graz.as<int>();
     R->map = ctx->d_ray_map.as<int>(); R->m = ctx->d_ray_m.as<double>();
+    R->dm = R->m + (size_t)nmu * M; R->idm = R->dm + (size_t)nmu * M; R->lam = R->idm + (size_t)nmu * M;
     return FSG_OK;
 }
 
@@ -1143,23 +1151,18 @@ static int lineop_calc_dev_body(fsg_ctx *ctx, const fsg_lines *d_lines, fsg_stat
 }
 
 // LinStrCalc (synth.f90:1774-1822) for the retained lines of the list whose central pass set
-// ctx->d_flags (original order); host output, 0 for rejected lines.  Chunks of at most 2^18 lines.
+// ctx->d_flags (original order); host output, 0 for rejected lines.
 static int linstr_calc(fsg_ctx *ctx, const fsg_lines *D, float *linstr) {
     cudaStream_t s = ctx->stream;
     const int64_t n = D->n;
-    const int64_t chunk = std::min<int64_t>(n, 1 << 18);
-    ALLOC(ctx->d_lswork, fsg_linstr_work(chunk, ctx->ntau, ctx->nmu));
     ALLOC(ctx->d_linstr, sizeof(float) * (size_t)n);
     LineView LV = make_view(D);
     AtmView A = fsg_view(ctx);
     RayView R;
     int rc = rays_prepare(ctx, &R); if (rc) return rc;
-    for (int64_t i0 = 0; i0 < n; i0 += chunk) {
-        fsg_launch_linstr(s, A, LV, ctx->tab, ctx->d_flags.as<int32_t>(), i0, std::min(chunk, n - i0), ctx->nmu,
-                          ctx->d_xmu.as<double>(), ctx->d_wmu.as<double>(), ctx->d_rhox.as<double>(), R,
-                          ctx->d_lswork.as<double>(), ctx->d_linstr.as<float>());
-        ctx->launches += 1;
-    }
+    fsg_launch_linstr(s, A, LV, ctx->tab, ctx->d_flags.as<int32_t>(), ctx->nmu, ctx->d_xmu.as<double>(),
+                      ctx->d_wmu.as<double>(), ctx->d_rhox.as<double>(), R, ctx->d_linstr.as<float>());
+    ctx->launches += 1;
     CK(cudaGetLastError(), "k_linstr");
     CK(cudaMemcpyAsync(linstr, ctx->d_linstr.p, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, s), "linstr");
     CK(cudaStreamSynchronize(s), "linstr");

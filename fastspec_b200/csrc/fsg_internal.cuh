@@ -153,11 +153,12 @@ struct CoreJob {
 
 // Rays of a spherical model (SphereInit, solver.f90:45-120), device arrays [nmu][stride], stride =
 // 2 ntau.  Ray im has n[im] points (ntau, or 2 n for a grazing ray that turns below layer n); point k
-// samples layer map[im][k] (0-based) at column mass m[im][k] along the ray.  nmu = 0: plane-parallel.
+// samples layer map[im][k] (0-based) at column mass m[im][k] along the ray; dm, idm the step to point k + 1 and
+// its reciprocal, lam TauStep's Lambda at k (0 < k < n - 1).  nmu = 0: plane-parallel.
 struct RayView {
     int nmu, stride;
     const int *n, *graz, *map;
-    const double *m;
+    const double *m, *dm, *idm, *lam;
 };
 
 // Error reporting

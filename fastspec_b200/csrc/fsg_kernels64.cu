@@ -7,9 +7,8 @@
 //   k_params_fast   block refill (synth.f90:1049-1070) into FP32 wing/core records
 //   k_params_fp64   block refill into FP64 (LinCop, LinVvgt, LinAvgt) and headers for the plain path
 //   k_span          Lstart/Lstop of the plain path's segments (synth.f90:955-978)
-//   k_radtran       RadTranCalc (synth.f90:1825-1866) + DiskInteg quadrature (convol.f90:233-234)
-//   k_radtran_sph   RadTranCalc for spherical models (synth.f90:1868-1898): LocPrfSph along each ray
-//   k_linstr        LinStrCalc (synth.f90:1774-1822), both geometries
+//   k_locprf        LocPrfPP over independent profiles (kernel-level entry point; the drivers' solver is in
+//                   fsg_solve.cu)
 #include "fsg_fp64.cuh"
 
 #include <algorithm>
@@ -465,181 +464,6 @@ void fsg_launch_span(cudaStream_t s, int64_t n, const int32_t *flags, const int3
 }
 
 // ================================================================================================
-// RadTranCalc + disk integration.  A CTA takes RT_LW wavelengths; the two opacity columns
-// (continuum, continuum + line) of each wavelength are staged in shared memory with coalesced
-// loads, TauStep / CentDer / U run over depths in parallel, then one thread per
-// (wavelength, kind, mu) sweeps the depths (LocPrfPP, solver.f90:123-179).
-// ================================================================================================
-#define RT_LW 8
-#define RT_MAXT 128
-#define RT_MAXMU 16
-
-__global__ void k_radtran(AtmView A, const double *__restrict__ lineopac, const double *__restrict__ rhox,
-                          int nmu, const double *__restrict__ xmu, const double *__restrict__ wmu,
-                          double *spl, double *spc, double *sfl, double *sfc) {
-    extern __shared__ double sm[];
-    const int nt = A.ntau;
-    const int w0 = blockIdx.x * RT_LW;
-    const int nw = min(RT_LW, A.nwl - w0);
-    // layout: X[kind][w][t], S[w][t], D[kind][w][t], R[kind][w][t] (derivative), U[kind][w][t]
-    double *X = sm, *S = X + 2 * RT_LW * nt, *D = S + RT_LW * nt, *R = D + 2 * RT_LW * nt,
-           *U = R + 2 * RT_LW * nt, *I = U + 2 * RT_LW * nt;      // I[kind][w][mu]
-    const double PlkC1 = FSG_HC * FSG_VC * 1e13 / FSG_KBOLT;
-    for (int e = threadIdx.x; e < nw * nt; e += blockDim.x) {
-        int w = e / nt, t = e - w * nt;
-        size_t g = (size_t)(w0 + w) * nt + t;
-        double c = A.contopac[g];
-        X[(0 * RT_LW + w) * nt + t] = c;
-        X[(1 * RT_LW + w) * nt + t] = c + lineopac[g];
-        double wl = A.wave[w0 + w] + A.wfirst;
-        double C1 = PlkC1 / wl, C2 = exp(50.7649141 - 5.0 * log(wl));
-        S[w * nt + t] = C2 / (exp(C1 / A.xi[XI_T * nt + t]) - 1.0);
-    }
-    __syncthreads();
-    // TauStep at mu = 1 (solver.f90:591-615)
-    for (int e = threadIdx.x; e < 2 * nw * nt; e += blockDim.x) {
-        int kw = e / nt, t = e - kw * nt;            // kw = kind * nw + w
-        int kind = kw / nw, w = kw - kind * nw;
-        const double *x = X + (kind * RT_LW + w) * nt;
-        double *d = D + (kind * RT_LW + w) * nt;
-        if (t == 0) {
-            double Dx1 = (rhox[1] - rhox[0]) / 1.0;
-            double Yp = (x[1] - x[0]) / Dx1;
-            d[0] = Dx1 * (x[1] + 2.0 * x[0] + Dx1 / 2.0 * Yp) / 3.0;
-        } else if (t < nt - 1) {
-            int k = t + 1;
-            double Dx = (rhox[k - 1] - rhox[k - 2]) / 1.0, Dx1 = (rhox[k] - rhox[k - 1]) / 1.0;
-            double Der = (x[k - 1] - x[k - 2]) / Dx, Der1 = (x[k] - x[k - 1]) / Dx1, Yp;
-            if (Der * Der1 > 0.0) {
-                double Lambda = (1.0 + Dx1 / (Dx + Dx1)) / 3.0;
-                Yp = (Der / (Lambda * Der1 + (1.0 - Lambda) * Der)) * Der1;
-            } else Yp = 0.0;
-            d[k - 1] = Dx1 * (x[k] + 2.0 * x[k - 1] + Dx1 / 2.0 * Yp) / 3.0;
-        } else d[nt - 1] = 0.0;
-    }
-    __syncthreads();
-    // CentDer of the source function on each Deltau scale (solver.f90:618-647)
-    for (int e = threadIdx.x; e < 2 * nw * nt; e += blockDim.x) {
-        int kw = e / nt, t = e - kw * nt;
-        int kind = kw / nw, w = kw - kind * nw;
-        const double *d = D + (kind * RT_LW + w) * nt, *y = S + w * nt;
-        double *r = R + (kind * RT_LW + w) * nt;
-        if (t == 0) r[0] = (y[1] - y[0]) / d[0];
-        else if (t == nt - 1) r[nt - 1] = (y[nt - 1] - y[nt - 2]) / d[nt - 2];
-        else {
-            int k = t + 1;
-            double Dx = d[k - 2], Dx1 = d[k - 1];
-            double InvDx = 1.0 / Dx, InvDx1 = 1.0 / Dx1;
-            double Lambda = (1.0 + Dx1 / (Dx + Dx1)) / 3.0, Lambda1 = 1.0 - Lambda;
-            double Der = (y[k - 1] - y[k - 2]) * InvDx, Der1 = (y[k] - y[k - 1]) * InvDx1;
-            r[k - 1] = (Der * Der1 > 0.0) ? (Der / (Lambda * Der1 + Lambda1 * Der)) * Der1 : 0.0;
-        }
-    }
-    __syncthreads();
-    // Bezier control term U (solver.f90:136-138)
-    for (int e = threadIdx.x; e < 2 * nw * nt; e += blockDim.x) {
-        int kw = e / nt, t = e - kw * nt;
-        int kind = kw / nw, w = kw - kind * nw;
-        if (t >= nt - 1) continue;
-        const double *d = D + (kind * RT_LW + w) * nt, *r = R + (kind * RT_LW + w) * nt, *y = S + w * nt;
-        U[(kind * RT_LW + w) * nt + t] = 0.5 * (y[t] + 0.5 * d[t] * r[t] + y[t + 1] - 0.5 * d[t] * r[t + 1]);
-    }
-    __syncthreads();
-    // sweeps: one thread per (kind, w, mu)
-    for (int e = threadIdx.x; e < 2 * nw * nmu; e += blockDim.x) {
-        int kw = e / nmu, im = e - kw * nmu;
-        int kind = kw / nw, w = kw - kind * nw;
-        const double *d = D + (kind * RT_LW + w) * nt, *u = U + (kind * RT_LW + w) * nt, *y = S + w * nt;
-        double Imu = 1.0 / xmu[im], Y = y[nt - 1];
-        for (int k = nt - 2; k >= 0; k--) {
-            double Eps, Alpha, Beta, Gamma;
-            delo_coef(d[k] * Imu, Eps, Alpha, Beta, Gamma);
-            Y = Y * Eps + Alpha * y[k] + Beta * y[k + 1] + Gamma * u[k];
-        }
-        I[(kind * RT_LW + w) * nmu + im] = Y;
-        double *out = (kind == 0) ? spc : spl;
-        if (out) out[(size_t)(w0 + w) * nmu + im] = Y;
-    }
-    __syncthreads();
-    // disk integration without broadening: Sf = sum over mu of Sp * Wmu (convol.f90:233-234)
-    for (int e = threadIdx.x; e < 2 * nw; e += blockDim.x) {
-        int kind = e / nw, w = e - kind * nw;
-        double a = 0.0;
-        for (int im = 0; im < nmu; im++) a = a + I[(kind * RT_LW + w) * nmu + im] * wmu[im];
-        double *out = (kind == 0) ? sfc : sfl;
-        if (out) out[w0 + w] = a;
-    }
-}
-
-size_t fsg_radtran_smem(int nt, int nmu) {
-    return sizeof(double) * ((size_t)(2 + 1 + 2 + 2 + 2) * RT_LW * nt + 2 * RT_LW * nmu);
-}
-
-int fsg_launch_radtran(cudaStream_t s, const AtmView &A, const double *lineopac, const double *rhox,
-                       int nmu, const double *xmu, const double *wmu, double *spl, double *spc,
-                       double *sfl, double *sfc) {
-    size_t sm = fsg_radtran_smem(A.ntau, nmu);
-    static int attr_set = 0;
-    if (!attr_set) {
-        cudaFuncSetAttribute(k_radtran, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        attr_set = 1;
-    }
-    int nb = (A.nwl + RT_LW - 1) / RT_LW;
-    k_radtran<<<nb, 128, sm, s>>>(A, lineopac, rhox, nmu, xmu, wmu, spl, spc, sfl, sfc);
-    return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
-}
-
-// RadTranCalc for spherical models (synth.f90:1868-1898): LocPrfSph along each ray.  A CTA stages
-// RT_LW wavelengths' opacity columns and Planck source as k_radtran does; then one thread per
-// (wavelength, kind, ray) runs delo_ray, whose steps come from that ray's own column-mass scale.
-// With spl and sfl null only the continuum is solved (as MagRadTranCalc needs).
-__global__ void k_radtran_sph(AtmView A, const double *__restrict__ lineopac, RayView R,
-                              const double *__restrict__ wmu, double *spl, double *spc, double *sfl, double *sfc) {
-    extern __shared__ double sm[];
-    const int nt = A.ntau, nmu = R.nmu;
-    const int w0 = blockIdx.x * RT_LW;
-    const int nw = min(RT_LW, A.nwl - w0);
-    const int nk = (spl || sfl) ? 2 : 1;                    // kinds computed: 0 continuum, 1 line
-    double *X = sm, *S = X + 2 * RT_LW * nt, *I = S + RT_LW * nt;   // X[kind][w][t], S[w][t], I[kind][w][mu]
-    const double PlkC1 = FSG_HC * FSG_VC * 1e13 / FSG_KBOLT;
-    for (int e = threadIdx.x; e < nw * nt; e += blockDim.x) {
-        int w = e / nt, t = e - w * nt;
-        size_t g = (size_t)(w0 + w) * nt + t;
-        double c = A.contopac[g];
-        X[(0 * RT_LW + w) * nt + t] = c;
-        if (nk == 2) X[(1 * RT_LW + w) * nt + t] = c + lineopac[g];
-        double wl = A.wave[w0 + w] + A.wfirst;
-        double C1 = PlkC1 / wl, C2 = exp(50.7649141 - 5.0 * log(wl));
-        S[w * nt + t] = C2 / (exp(C1 / A.xi[XI_T * nt + t]) - 1.0);
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < nk * nw * nmu; e += blockDim.x) {
-        int kw = e / nmu, im = e - kw * nmu;
-        int kind = kw / nw, w = kw % nw;
-        double Y = delo_ray(R, im, X + (kind * RT_LW + w) * nt, S + w * nt);
-        I[(kind * RT_LW + w) * nmu + im] = Y;
-        double *out = (kind == 0) ? spc : spl;
-        if (out) out[(size_t)(w0 + w) * nmu + im] = Y;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < nk * nw; e += blockDim.x) {
-        int kind = e / nw, w = e % nw;
-        double a = 0.0;
-        for (int im = 0; im < nmu; im++) a = a + I[(kind * RT_LW + w) * nmu + im] * wmu[im];
-        double *out = (kind == 0) ? sfc : sfl;
-        if (out) out[w0 + w] = a;
-    }
-}
-
-int fsg_launch_radtran_sph(cudaStream_t s, const AtmView &A, const double *lineopac, const RayView &R,
-                           const double *wmu, double *spl, double *spc, double *sfl, double *sfc) {
-    size_t sm = sizeof(double) * ((size_t)3 * RT_LW * A.ntau + 2 * RT_LW * R.nmu);
-    int nb = (A.nwl + RT_LW - 1) / RT_LW;
-    k_radtran_sph<<<nb, 128, sm, s>>>(A, lineopac, R, wmu, spl, spc, sfl, sfc);
-    return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
-}
-
-// ================================================================================================
 // Elemental HVoigt / FVoigt over arrays (kernel-level entry points)
 // ================================================================================================
 __global__ void k_hvoigt(int64_t n, const double *a, const double *v, double *h, const float *vtab,
@@ -720,65 +544,6 @@ __global__ void k_locprf(int nprof, int nmu, const double *xmu, int nt, const do
     double *d = work + (size_t)p * 3 * nt;
     locprf_one(nmu, xmu, nt, xki + (size_t)p * nt, src + (size_t)p * nt, rhox, d, d + nt, d + 2 * nt,
                ploc + (size_t)p * nmu);
-}
-
-// LinStrCalc (synth.f90:1774-1822): central depth of each retained line from the
-// continuum and continuum + line intensities at its centre (the centre opacities of the central
-// pass: ContOpac at Wlcent, LineOpacity2 at Wlcent), disk-integrated with Wmu when nmu > 1.
-// One thread per line of [i0, i0 + nl); work holds 6 nt + 2 nmu doubles per thread.
-__global__ void k_linstr(AtmView A, LineView L, const float *__restrict__ vtab, const double *__restrict__ anode,
-                         const double *__restrict__ aida, const int32_t *__restrict__ flags, int64_t i0, int64_t nl,
-                         int nmu, const double *__restrict__ xmu, const double *__restrict__ wmu,
-                         const double *__restrict__ rhox, RayView R, double *work, float *linstr) {
-    const double PlkC1 = FSG_HC * FSG_VC * 1e13 / FSG_KBOLT;
-    int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nl) return;
-    const int64_t i = i0 + k;
-    const int f = flags[i];
-    if (f & FSG_F_WEAK) { linstr[i] = 0.0f; return; }
-    const int nt = A.ntau;
-    double *xc = work + (size_t)k * (6 * nt + 2 * nmu), *xl = xc + nt, *y = xl + nt, *d = y + nt;
-    double *ic = d + 3 * nt, *il = ic + nmu;
-    double wlc = L.wl[i] - A.wfirst;
-    XCoef XC;
-    xline_setup(A, L, i, wlc, line_input_flags(L, i, 0), &XC);
-    const int ihe = XC.IxHe;
-    int iwl = waveidx(A, wlc);
-    double dW = (wlc - A.wave[iwl - 1]) / (A.wave[iwl] - A.wave[iwl - 1]);
-    const double wl = wlc + A.wfirst;
-    const double C1 = PlkC1 / wl, C2 = exp(50.7649141 - 5.0 * log(wl));
-    for (int t = 0; t < nt; t++) {
-        double cop, vv, av;
-        xline_depth(A, t, XC, &cop, &vv, &av);
-        double dWl = 0.0;
-        if (ihe > 0) dWl = 0.0 - center_shift(A, ihe, t);
-        double lo = hvoigt64(vtab, anode, aida, av, dWl * vv) * cop;
-        if (A.motype == 1) lo = lo / A.contstd[t];
-        double co = cont_center(A, iwl, dW, t);
-        xc[t] = co;
-        xl[t] = co + lo;
-        y[t] = C2 / (exp(C1 / A.xi[XI_T * nt + t]) - 1.0);
-    }
-    if (R.nmu > 0) {                       // spherical: LocPrfSph (synth.f90:1801-1803)
-        for (int m = 0; m < nmu; m++) { ic[m] = delo_ray(R, m, xc, y); il[m] = delo_ray(R, m, xl, y); }
-    } else {
-        locprf_one(nmu, xmu, nt, xc, y, rhox, d, d + nt, d + 2 * nt, ic);
-        locprf_one(nmu, xmu, nt, xl, y, rhox, d, d + nt, d + 2 * nt, il);
-    }
-    if (nmu == 1) { linstr[i] = (float)(1.0 - il[0] / ic[0]); return; }
-    double FlxL = 0.0, FlxC = 0.0;
-    for (int m = 0; m < nmu; m++) { FlxL = FlxL + wmu[m] * il[m]; FlxC = FlxC + wmu[m] * ic[m]; }
-    linstr[i] = (float)(1.0 - FlxL / FlxC);
-}
-
-size_t fsg_linstr_work(int64_t nl, int nt, int nmu) { return sizeof(double) * (size_t)nl * (6 * nt + 2 * nmu); }
-
-void fsg_launch_linstr(cudaStream_t s, const AtmView &A, const LineView &L, const VoigtTables &T,
-                       const int32_t *flags, int64_t i0, int64_t nl, int nmu, const double *xmu, const double *wmu,
-                       const double *rhox, const RayView &R, double *work, float *linstr) {
-    if (nl > 0)
-        k_linstr<<<(unsigned)((nl + 127) / 128), 128, 0, s>>>(A, L, T.vtab, T.anode, T.aida, flags, i0, nl, nmu,
-                                                              xmu, wmu, rhox, R, work, linstr);
 }
 
 void fsg_launch_locprf(cudaStream_t s, int nprof, int nmu, const double *xmu, int nt, const double *xki,

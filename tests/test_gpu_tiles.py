@@ -71,3 +71,26 @@ def test_magnetic_tile_edges(fsg, oracle_mod, prec, ntau, nwl, n):
     scale = np.maximum(om[..., :3].max(axis=(0, 2)), 1e-300)[None, :, None]
     assert np.max(np.abs(g["maglineopac"] - om) / scale) < (1e-12 if prec == "fp64" else 2e-6)
     C.close()
+
+
+@pytest.mark.parametrize("ntau,nwl,nmu", [(3, 2, 1), (4, 7, 2), (64, 9, 9), (65, 17, 16), (128, 8, 5)])
+def test_solver_edges(fsg, oracle_mod, ntau, nwl, nmu):
+    """The formal solver around its CTA's eight wavelengths and its thread counts, on a line opacity spread over
+    nine decades of the continuum's.  Bar: 1e-10 relative, as for the drivers (the DELO differences amplify a
+    rounding of the exponential 1e7 times just above the Taylor branch)."""
+    grid, st, co, _ = case(ntau, nwl, 1, 0)
+    lo = co * 10.0 ** np.random.default_rng(ntau + nwl).uniform(-4.0, 5.0, co.shape)
+    x, w, _ = fsg.mu_quadrature(1, nmu)
+    C = fsg.Context(vmicro=1.0)
+    C.set_grid(grid["wmode"], grid["wstart"], grid["wend"], grid["dstep"])
+    C.set_atmosphere(st)
+    C.set_contopac(co)
+    C.set_mu(x, w)
+    C.lineop_set(lo)
+    spl, spc, sfl, sfc = C.radtran()
+    S = oracle_mod.State(grid, st, contopac=co, vmicro=1.0)
+    ospl, ospc = oracle_mod.radtran(S, x, lo)
+    osfl, osfc = oracle_mod.disk_integ(w, ospl, ospc)
+    for a, b in ((spl, ospl), (spc, ospc), (sfl, osfl), (sfc, osfc)):
+        assert np.max(np.abs(a / b - 1)) < 1e-10
+    C.close()
