@@ -17,6 +17,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-ccbin", "/u
 UNITS = [
     ("fsg_kernels64.cu", ["-fmad=false"]),
     ("fsg_solve.cu", ["-fmad=false"]),
+    ("fsg_conv.cu", ["-fmad=true"]),
     ("fsg_mag.cu", ["-fmad=false"]),
     ("fsg_fast.cu", ["-fmad=true"]),
     ("fsg_accum64.cu", ["-fmad=true"]),

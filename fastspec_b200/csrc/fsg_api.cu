@@ -127,6 +127,9 @@ size_t fsg_mag_rec_bytes(int);
 int fsg_launch_mag_fast(cudaStream_t, const AtmView &, const LineHdr *, void *, int64_t, const ZView &, const int *,
                         const int *, const VoigtTables &, double *);
 void fsg_launch_conv(cudaStream_t, int, const double *, int, const double *, int, double *, const double *, double);
+int fsg_launch_disk_conv(cudaStream_t, int, int, const double *, const double *, const double *, const int *,
+                         const int *, const int *, const int *, const double *, int, int, double *, double *, double *,
+                         double *);
 size_t fsg_adjoint_work(int, int, int64_t, int);
 int fsg_launch_adjoint(cudaStream_t, const AtmView &, const LineView &, const VoigtTables &, const double *,
                        const double *, int, const double *, const double *, const RayView &, const int32_t *,
@@ -210,7 +213,7 @@ struct fsg_ctx {
     // mu
     int nmu = 0;
     DBuf d_xmu, d_wmu;
-    std::vector<double> h_xmu;
+    std::vector<double> h_xmu, h_wmu;
     // geometry: radius <= 0 plane-parallel; spherical rays (SphereInit) rebuilt when mu, the
     // atmosphere or the geometry change
     double radius = -1.0;
@@ -482,6 +485,7 @@ int fsg_set_mu(fsg_ctx *ctx, int nmu, const double *xmu, const double *wmu) {
     CK(cudaStreamSynchronize(ctx->stream), "mu upload");
     ctx->nmu = nmu;
     ctx->h_xmu.assign(xmu, xmu + nmu);
+    ctx->h_wmu.assign(wmu, wmu + nmu);
     ctx->rays_ok = 0;
     return FSG_OK;
 }
@@ -1600,8 +1604,8 @@ static int mag_radtran_body(fsg_ctx *ctx, int bframe, const double *bfield, int 
         CK(cudaStreamSynchronize(s), "mag radtran");
         return FSG_OK;
     }
-    std::vector<double> xmu(nmu), geo(5 * nmu);
-    CK(cudaMemcpy(xmu.data(), ctx->d_xmu.p, sizeof(double) * nmu, cudaMemcpyDeviceToHost), "mu");
+    const std::vector<double> &xmu = ctx->h_xmu;
+    std::vector<double> geo(5 * nmu);
     const double d2r = FSG_PI / 180.0;
     for (int im = 0; im < nmu; im++) {
         double Sphi, Spsi, Cpsi, CPhi;
@@ -2095,9 +2099,7 @@ int fsg_disk_integ_conv_dev(fsg_ctx *ctx, const double *radii, double vsini, dou
     if (!ctx->have_grid || ctx->nmu < 1) return fail(ctx, FSG_E_STATE, "fsg_disk_integ_conv_dev: set grid and mu first");
     cudaSetDevice(ctx->device);
     const int nwl = ctx->nwl, nmu = ctx->nmu;
-    std::vector<double> xmu(nmu), wmu(nmu);
-    CK(cudaMemcpy(xmu.data(), ctx->d_xmu.p, sizeof(double) * nmu, cudaMemcpyDeviceToHost), "mu");
-    CK(cudaMemcpy(wmu.data(), ctx->d_wmu.p, sizeof(double) * nmu, cudaMemcpyDeviceToHost), "mu");
+    const std::vector<double> &xmu = ctx->h_xmu, &wmu = ctx->h_wmu;
     const double dv = ctx->wmode == 0 ? 2.0 * ctx->dstep / (ctx->wfirst + ctx->wlast) * FSG_VC : ctx->dstep;
     const double sigma = vmacro / dv / std::sqrt(2.0);
     const int nmk = std::max(3, std::min((int)(10.0 * sigma), (int)((nwl - 3) / 2)));
@@ -2106,8 +2108,6 @@ int fsg_disk_integ_conv_dev(fsg_ctx *ctx, const double *radii, double vsini, dou
     ALLOC(ctx->d_ctaps, sizeof(double) * (size_t)(nmu * (nrk_max + nm) + 2 * nm + 8));
     double *tL = ctx->d_cbuf.as<double>(), *tC = tL + nwl, *uL = tC + nwl, *uC = uL + nwl;
     cudaStream_t s = ctx->stream;
-    CK(cudaMemsetAsync(d_sfl, 0, sizeof(double) * nwl, s), "flux reset");
-    CK(cudaMemsetAsync(d_sfc, 0, sizeof(double) * nwl, s), "flux reset");
     // all taps of all annuli in one upload: [rotation | macroturbulence] per annulus
     std::vector<double> taps;
     std::vector<int> roff(nmu), rn(nmu, 0), moff(nmu), mn(nmu, 0);
@@ -2152,6 +2152,17 @@ int fsg_disk_integ_conv_dev(fsg_ctx *ctx, const double *radii, double vsini, dou
     ALLOC(ctx->d_ctaps, sizeof(double) * taps.size());
     CK(cudaMemcpyAsync(ctx->d_ctaps.p, taps.data(), sizeof(double) * taps.size(), cudaMemcpyHostToDevice, s), "taps");
     const double *dk = ctx->d_ctaps.as<double>();
+    const int rf = fsg_launch_disk_conv(s, nwl, nmu, d_spl, d_spc, dk, roff.data(), rn.data(), moff.data(), mn.data(),
+                                        wmu.data(), goff, gn, tL, tC, d_sfl, d_sfc);
+    if (rf >= 0) {
+        if (rf) return cuda_fail(ctx, cudaGetLastError(), "k_disk_conv");
+        ctx->launches += gn ? 2 : 1;
+        CK(cudaStreamSynchronize(s), "disk integration");
+        return FSG_OK;
+    }
+    // kernels too wide for shared memory: annulus by annulus
+    CK(cudaMemsetAsync(d_sfl, 0, sizeof(double) * nwl, s), "flux reset");
+    CK(cudaMemsetAsync(d_sfc, 0, sizeof(double) * nwl, s), "flux reset");
     for (int im = 0; im < nmu; im++) {
         // SiL, SiC: the annulus intensities (stride nmu), rotation, macroturbulence, then the flux sum
         const double *iL = d_spl + im, *iC = d_spc + im;

@@ -94,3 +94,33 @@ def test_solver_edges(fsg, oracle_mod, ntau, nwl, nmu):
     for a, b in ((spl, ospl), (spc, ospc), (sfl, osfl), (sfc, osfc)):
         assert np.max(np.abs(a / b - 1)) < 1e-10
     C.close()
+
+
+@pytest.mark.parametrize("nwl,nmu,vsini,vmacro,vgau", [(9, 2, 0.0, 0.0, 0.0), (9, 3, 30.0, 5.0, 2.0e4), (640, 7, 12.0, 0.0, 0.0),
+                                                       (641, 16, 0.0, 3.0, 9.0e4), (1283, 5, 40.0, 6.0, 5.0),
+                                                       (3000, 1, 7.0, 2.0, 0.0), (14001, 3, 900.0, 90.0, 3.0e3)])
+def test_broadening_edges(fsg, oracle_mod, nwl, nmu, vsini, vmacro, vgau):
+    """The broadened flux around the tile of 640 wavelengths, with kernels wider than the spectrum and (the last
+    case: 6,000 points either side) wider than the staged halo allows.  Sums of positive products: 1e-16 each,
+    12,000 of them at most, below 1e-12."""
+    import torch
+    R = 2.0e6 if vsini > 100.0 else 3.0e5
+    dstep = 2.99792458e5 / R
+    grid = dict(wmode=1, wstart=5000.0, wend=5000.0 * np.exp((nwl - 0.5) / R), dstep=dstep)
+    x, w, r = fsg.mu_quadrature(1, nmu)
+    C = fsg.Context()
+    wave = C.set_grid(1, grid["wstart"], grid["wend"], dstep) + grid["wstart"]
+    assert len(wave) == nwl
+    C.set_mu(x, w)
+    rng = np.random.default_rng(nwl)
+    spc = rng.uniform(0.9, 1.1, (nwl, nmu))
+    spl = spc * rng.uniform(0.05, 1.0, (nwl, nmu))
+    d = [torch.from_numpy(a).cuda() for a in (spl, spc)] + [torch.empty(nwl, dtype=torch.float64, device="cuda")
+                                                            for _ in range(2)]
+    torch.cuda.synchronize()
+    C.disk_integ_conv_dev(r, vsini, vmacro, vgau, *[t.data_ptr() for t in d])
+    osfl, osfc = oracle_mod.disk_integ_conv(x, w, r, spl, spc, oracle_mod.grid_dv(grid, wave), vsini, vmacro,
+                                            oracle_mod.gauss_sigma_pix(grid, wave, vgau) if vgau > 0 else 0.0)
+    assert np.max(np.abs(d[2].cpu().numpy() / osfl - 1)) < 1e-12
+    assert np.max(np.abs(d[3].cpu().numpy() / osfc - 1)) < 1e-12
+    C.close()
