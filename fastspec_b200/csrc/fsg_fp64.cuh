@@ -250,19 +250,34 @@ __device__ __forceinline__ double cont_center(const AtmView &A, int iwl, double 
 }
 
 // ---- DELO-Bezier (solver.f90) -----------------------------------------------------------------
+// (constants multiplied, one reciprocal; the differences in the reference's order: just above Dtau = 5e-3 they
+// amplify a rounding of Eps 1e7 times)
 __device__ __forceinline__ void delo_coef(double Dtau, double &Eps, double &Alpha, double &Beta, double &Gamma) {
-    double Dtau2 = Dtau * Dtau, Idtau2 = 1.0 / Dtau2;
+    const double Dtau2 = Dtau * Dtau;
     if (Dtau < 5e-3) {
-        Eps = 1.0 - Dtau + 0.5 * Dtau2 - Dtau2 * Dtau / 6.0 + Dtau2 * Dtau2 / 24.0;
-        Alpha = Dtau / 3.0 - Dtau2 / 12.0 + Dtau2 * Dtau / 60.0;
-        Beta = Dtau / 3.0 - Dtau2 * 0.25 + Dtau2 * Dtau * 0.1;
-        Gamma = Dtau / 3.0 - Dtau2 / 6.0 + Dtau2 * Dtau * 0.05;
+        const double Dtau3 = Dtau2 * Dtau;
+        Eps = 1.0 - Dtau + 0.5 * Dtau2 - Dtau3 * (1.0 / 6.0) + Dtau2 * Dtau2 * (1.0 / 24.0);
+        Alpha = Dtau * (1.0 / 3.0) - Dtau2 * (1.0 / 12.0) + Dtau3 * (1.0 / 60.0);
+        Beta = Dtau * (1.0 / 3.0) - Dtau2 * 0.25 + Dtau3 * 0.1;
+        Gamma = Dtau * (1.0 / 3.0) - Dtau2 * (1.0 / 6.0) + Dtau3 * 0.05;
     } else {
+        const double Idtau2 = rcp64(Dtau2), D2 = 2.0 * Dtau;
         Eps = (Dtau < 100.0) ? exp(-Dtau) : 0.0;
-        Alpha = (Dtau2 - 2.0 * Dtau + 2.0 - 2.0 * Eps) * Idtau2;
-        Beta = (2.0 - (2.0 + 2.0 * Dtau + Dtau2) * Eps) * Idtau2;
-        Gamma = (2.0 * Dtau - 4.0 + (2.0 * Dtau + 4.0) * Eps) * Idtau2;
+        Alpha = (Dtau2 - D2 + 2.0 - 2.0 * Eps) * Idtau2;
+        Beta = (2.0 - (2.0 + D2 + Dtau2) * Eps) * Idtau2;
+        Gamma = (D2 - 4.0 + (D2 + 4.0) * Eps) * Idtau2;
     }
+}
+
+// harmonic mean Der Der1 / (Lambda Der1 + (1 - Lambda) Der) of two slopes of one sign, else 0
+// (solver.f90:604-610, 637-643)
+__device__ __forceinline__ double hmean(double der, double der1, double lam) {
+    return der * der1 > 0.0 ? der * rcp64(fma(lam, der1, (1.0 - lam) * der)) * der1 : 0.0;
+}
+
+// CentDer's Lambda from the steps on either side (solver.f90:632)
+__device__ __forceinline__ double lambda_of(double dx, double dx1) {
+    return (1.0 + dx1 * rcp64(dx + dx1)) * (1.0 / 3.0);
 }
 
 // ---- spherical rays ---------------------------------------------------------------------------

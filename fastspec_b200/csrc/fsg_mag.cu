@@ -197,91 +197,126 @@ __device__ __forceinline__ void centder_pt(const double *D, const double *Y, int
     *out = (Der * Der1 > 0.0) ? (Der / (Lambda * Der1 + Lambda1 * Der)) * Der1 : 0.0;
 }
 
-// full 4x4 propagation matrix from its 6 distinct elements (solver.f90:311-326), column-major
-__device__ __forceinline__ void build_k(const double *e, double *K) {
-    double PhiQ = e[0], PhiU = e[1], PhiV = e[2], PsiQ = e[3], PsiU = e[4], PsiV = e[5];
-    K[0] = 0.0;   K[4] = PhiQ;  K[8] = PhiU;   K[12] = PhiV;
-    K[1] = PhiQ;  K[5] = 0.0;   K[9] = PsiV;   K[13] = -PsiU;
-    K[2] = PhiU;  K[6] = -PsiV; K[10] = 0.0;   K[14] = PsiQ;
-    K[3] = PhiV;  K[7] = PsiU;  K[11] = -PsiQ; K[15] = 0.0;
-}
-
-__device__ void solve4x4(const double *A, const double *B, double *X) {
-    double M[16], R[4];
-    for (int q = 0; q < 16; q++) M[q] = A[q];
-    for (int q = 0; q < 4; q++) R[q] = B[q];
-#define MM(i, j) M[((i) - 1) + 4 * ((j) - 1)]
-    for (int k = 1; k <= 3; k++) {
-        int ip = k; double p = fabs(MM(k, k));
-        for (int i = k + 1; i <= 4; i++) if (fabs(MM(i, k)) > p) { p = fabs(MM(i, k)); ip = i; }
-        if (ip != k) {
-            for (int j = k; j <= 4; j++) { double sw = MM(k, j); MM(k, j) = MM(ip, j); MM(ip, j) = sw; }
-            double sw = R[k - 1]; R[k - 1] = R[ip - 1]; R[ip - 1] = sw;
+// Gaussian elimination with row pivoting (Solve4x4, solver.f90:541-588)
+__device__ __forceinline__ void solve4x4(double (&M)[4][4], double (&R)[4], double (&X)[4]) {
+    double ip[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (k < 3) {
+            int piv = k;
+            double p = fabs(M[k][k]);
+#pragma unroll
+            for (int i = k + 1; i < 4; i++) if (fabs(M[i][k]) > p) { p = fabs(M[i][k]); piv = i; }
+#pragma unroll
+            for (int i = k + 1; i < 4; i++)
+                if (piv == i) {
+#pragma unroll
+                    for (int j = k; j < 4; j++) { const double sw = M[k][j]; M[k][j] = M[i][j]; M[i][j] = sw; }
+                    const double sw = R[k]; R[k] = R[i]; R[i] = sw;
+                }
         }
-        p = 1.0 / MM(k, k);
-        for (int i = k + 1; i <= 4; i++) {
-            double f = MM(i, k) * p;
-            for (int j = k + 1; j <= 4; j++) MM(i, j) = MM(i, j) - f * MM(k, j);
-            R[i - 1] = R[i - 1] - f * R[k - 1];
+        ip[k] = rcp64(M[k][k]);
+#pragma unroll
+        for (int i = k + 1; i < 4; i++) {
+            const double f = M[i][k] * ip[k];
+#pragma unroll
+            for (int j = k + 1; j < 4; j++) M[i][j] = fma(-f, M[k][j], M[i][j]);
+            R[i] = fma(-f, R[k], R[i]);
         }
     }
-    X[3] = R[3] / MM(4, 4);
-    X[2] = (R[2] - MM(3, 4) * X[3]) / MM(3, 3);
-    X[1] = (R[1] - MM(2, 3) * X[2] - MM(2, 4) * X[3]) / MM(2, 2);
-    X[0] = (R[0] - MM(1, 2) * X[1] - MM(1, 3) * X[2] - MM(1, 4) * X[3]) / MM(1, 1);
-#undef MM
+#pragma unroll
+    for (int k = 3; k >= 0; k--) {
+        double r = R[k];
+#pragma unroll
+        for (int j = k + 1; j < 4; j++) r = fma(-M[k][j], X[j], r);
+        X[k] = r * ip[k];
+    }
+}
+
+// The propagation matrix of one point (solver.f90:311-326) by its 6 distinct elements: symmetric in the first
+// row and column (Q, U, V absorption), antisymmetric below (dispersion), zero diagonal.
+struct PropK {
+    double a, b, c, q, u, v;             // PhiQ, PhiU, PhiV, PsiQ, PsiU, PsiV
+    // K x
+    __device__ __forceinline__ void mul(const double (&x)[4], double (&y)[4]) const {
+        y[0] = fma(a, x[1], fma(b, x[2], c * x[3]));
+        y[1] = fma(a, x[0], fma(v, x[2], -(u * x[3])));
+        y[2] = fma(b, x[0], fma(-v, x[1], q * x[3]));
+        y[3] = fma(c, x[0], fma(u, x[1], -(q * x[2])));
+    }
+    // element (i, j)
+    __device__ __forceinline__ double at(int i, int j) const {
+        const double t[4][4] = { { 0.0, a, b, c }, { a, 0.0, v, -u }, { b, -v, 0.0, q }, { c, u, -q, 0.0 } };
+        return t[i][j];
+    }
+};
+
+// K K + K' of a point: ten distinct values of K K, K' of K's own form
+__device__ __forceinline__ void prop_square(const PropK &k, const PropK &d, double (&X)[4][4]) {
+    const double aa = k.a * k.a, bb = k.b * k.b, cc = k.c * k.c, qq = k.q * k.q, uu = k.u * k.u, vv = k.v * k.v;
+    const double s12 = fma(k.a, k.b, k.u * k.q), s13 = fma(k.a, k.c, k.v * k.q), s23 = fma(k.b, k.c, k.v * k.u);
+    const double n01 = fma(k.c, k.u, -(k.b * k.v)), n02 = fma(k.a, k.v, -(k.c * k.q)), n03 = fma(k.b, k.q, -(k.a * k.u));
+    X[0][0] = aa + bb + cc; X[1][1] = aa - vv - uu; X[2][2] = bb - vv - qq; X[3][3] = cc - uu - qq;
+    X[0][1] = d.a + n01; X[1][0] = d.a - n01;
+    X[0][2] = d.b + n02; X[2][0] = d.b - n02;
+    X[0][3] = d.c + n03; X[3][0] = d.c - n03;
+    X[1][2] = s12 + d.v; X[2][1] = s12 - d.v;
+    X[1][3] = s13 - d.u; X[3][1] = s13 + d.u;
+    X[2][3] = s23 + d.q; X[3][2] = s23 - d.q;
 }
 
 // The DELO-Bezier sweep of StokesPrfPP / StokesPrfSph (solver.f90:341-390, 486-534) over the N points of
-// one ray, run by one thread from the per-point fields in shared memory (field-major, leading dimension
-// ld): Kv / KD the 6 distinct propagation elements and their derivatives, SRC4 / SRD the source vector
-// and its derivative, Dt the optical-depth steps.  XINT2 holds the boundary Stokes vector on entry and
-// the emergent one on return.
-__device__ void stokes_sweep(int N, int ld, const double *Kv, const double *KD, const double *SRC4,
-                             const double *SRD, const double *Dt, double *XINT2, size_t es = 1) {
-    double K1[16], K0[16], KD0[16], XKA[16], XKB[16], QA[16], QB[16], AA[16], e6[6], d6[6], XINT1[4];
-    for (int q = 0; q < 6; q++) { e6[q] = Kv[(q * ld + N - 1) * es]; d6[q] = KD[(q * ld + N - 1) * es]; }
-    build_k(e6, K0); build_k(d6, KD0);
-    for (int j = 0; j < 4; j++) for (int i = 0; i < 4; i++) {
-        double acc = 0.0;
-        for (int q = 0; q < 4; q++) acc = acc + K0[i + 4 * q] * K0[q + 4 * j];
-        XKB[i + 4 * j] = acc + KD0[i + 4 * j];
-    }
-    for (int q = 0; q < 16; q++) K1[q] = K0[q];         // XK at k1
+// one ray, run by one thread from per-point fields (field-major, leading dimension ld, element stride es):
+// Kv / KD the 6 distinct propagation elements and their derivatives, SRC4 / SRD the source vector and its
+// derivative, Dt the optical-depth steps.  XINT2 holds the boundary Stokes vector on entry and the emergent one
+// on return.  With G = Gamma Dtau/2 and Q = K K + K' the step (solver.f90:360-388) is
+//   [1 + (Alpha + Gamma (Dtau/2 + 1)) K0 + G Q0] I0 = Eps I1 + G Q1 I1 + K1 [(Gamma (Dtau/2 - 1) - Beta) I1 - G S1]
+//                    + (Beta + Gamma) S1 + (Alpha + Gamma) S0 + G (K0 S0 + S0' - S1')
+// in which K's form leaves 12 products of each K x and 18 of K K.
+__device__ __forceinline__ void stokes_sweep(int N, int ld, const double *Kv, const double *KD, const double *SRC4,
+                                             const double *SRD, const double *Dt, double (&XINT2)[4], size_t es = 1) {
+    auto prop = [&](const double *f, int k) {
+        return PropK{ f[k * es], f[(ld + k) * es], f[((size_t)2 * ld + k) * es], f[((size_t)3 * ld + k) * es],
+                      f[((size_t)4 * ld + k) * es], f[((size_t)5 * ld + k) * es] };
+    };
+    PropK K1 = prop(Kv, N - 1);
+    double Q1[4][4], S1[4], D1[4];
+    prop_square(K1, prop(KD, N - 1), Q1);
+#pragma unroll
+    for (int i = 0; i < 4; i++) { S1[i] = SRC4[((size_t)i * ld + N - 1) * es]; D1[i] = SRD[((size_t)i * ld + N - 1) * es]; }
     for (int k = N - 2; k >= 0; k--) {
-        int k1 = k + 1;
-        double Dtau = Dt[k * es], Dtau05 = 0.5 * Dtau, Eps, Alpha, Beta, Gamma;
+        const PropK K0 = prop(Kv, k), KD0 = prop(KD, k);
+        const double Dtau = Dt[k * es], h = 0.5 * Dtau;
+        double Eps, Alpha, Beta, Gamma, S0[4], D0[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) { S0[i] = SRC4[((size_t)i * ld + k) * es]; D0[i] = SRD[((size_t)i * ld + k) * es]; }
         delo_coef(Dtau, Eps, Alpha, Beta, Gamma);
         Gamma = Gamma * 0.5;
-        for (int q = 0; q < 6; q++) { e6[q] = Kv[(q * ld + k) * es]; d6[q] = KD[(q * ld + k) * es]; }
-        build_k(e6, K0); build_k(d6, KD0);
-        for (int q = 0; q < 16; q++) XKA[q] = XKB[q];
-        for (int j = 0; j < 4; j++) for (int i = 0; i < 4; i++) {
-            double acc = 0.0;
-            for (int q = 0; q < 4; q++) acc = acc + K0[i + 4 * q] * K0[q + 4 * j];
-            XKB[i + 4 * j] = acc + KD0[i + 4 * j];
-        }
-        for (int j = 0; j < 4; j++) for (int i = 0; i < 4; i++) {
-            int e = i + 4 * j;
-            QA[e] = Dtau05 * XKA[e] + (Dtau05 - 1.0) * K1[e];
-            QB[e] = -(Dtau05 * XKB[e]) - (Dtau05 + 1.0) * K0[e];
-            AA[e] = ((i == j) ? 1.0 : 0.0) + Alpha * K0[e] - Gamma * QB[e];
-        }
-        double GD = Gamma * Dtau05;
+        const double G = Gamma * h, c1 = fma(Gamma, h - 1.0, -Beta), c0 = fma(Gamma, h + 1.0, Alpha);
+        double w[4], y[4], z[4], R[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) w[i] = fma(c1, XINT2[i], -(G * S1[i]));
+        K1.mul(w, y);
+        K0.mul(S0, z);
+#pragma unroll
         for (int i = 0; i < 4; i++) {
-            double m1 = 0.0, m2 = 0.0, m3 = 0.0, m4 = 0.0;
-            for (int q = 0; q < 4; q++) {
-                m1 = m1 + K1[i + 4 * q] * XINT2[q];
-                m2 = m2 + QA[i + 4 * q] * XINT2[q];
-                m3 = m3 + K1[i + 4 * q] * SRC4[(q * ld + k1) * es];
-                m4 = m4 + K0[i + 4 * q] * SRC4[(q * ld + k) * es];
-            }
-            XINT1[i] = Eps * XINT2[i] - Beta * m1 + Gamma * m2 + (Beta + Gamma) * SRC4[(i * ld + k1) * es]
-                     - GD * m3 + (Alpha + Gamma) * SRC4[(i * ld + k) * es] + GD * m4
-                     + GD * (SRD[(i * ld + k) * es] - SRD[(i * ld + k1) * es]);
+            double m = 0.0;
+#pragma unroll
+            for (int j = 0; j < 4; j++) m = fma(Q1[i][j], XINT2[j], m);
+            R[i] = fma(Eps, XINT2[i], y[i]) + fma(Beta + Gamma, S1[i], (Alpha + Gamma) * S0[i]) +
+                   G * (m + z[i] + (D0[i] - D1[i]));
         }
-        solve4x4(AA, XINT1, XINT2);
-        for (int q = 0; q < 16; q++) K1[q] = K0[q];
+        double M[4][4];
+        prop_square(K0, KD0, Q1);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                M[i][j] = i == j ? fma(G, Q1[i][j], 1.0) : fma(c0, K0.at(i, j), G * Q1[i][j]);
+        solve4x4(M, R, XINT2);
+        K1 = K0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) { S1[i] = S0[i]; D1[i] = D0[i]; }
     }
 }
 
@@ -307,9 +342,11 @@ __device__ __forceinline__ double stokes_point(const double *m, double lop, doub
 // StokesPrfPP, one thread per (wavelength, angle) from the first wavelength iwl0 on, in two launches
 // over per-thread global work arrays (STK_FIELDS x ntau doubles, element stride = the launch's thread
 // count T, so that the threads of a warp touch consecutive addresses).  k_stokes_prep builds the
-// propagation data, TauStep and CentDer over depth; it needs few registers, so many warps hide the
-// latency of its array traffic.  k_stokes_thr runs the sequential 4x4 sweep (about 200 registers);
-// every lane of every warp sweeps.  The reference's operations, in its order.
+// propagation data, TauStep and CentDer over depth: a thread takes a run of depths (blockIdx.y) with the
+// points, steps and slopes around the present one in registers, so each field is written once and nothing is
+// read back; k_stokes_thr runs the sequential 4x4 sweep, every lane of every warp.  Bound by the traffic of
+// the 21 fields (8.5 GB of 50,001 wavelengths x 9 angles x 56 depths, there and back).
+#define STK_RUNS 4
 __global__ void __launch_bounds__(128)
 k_stokes_prep(AtmView A, const double *__restrict__ lineopac, const double *__restrict__ mlo,
               const double *__restrict__ rhox, int nmu, const double *__restrict__ xmu,
@@ -318,7 +355,8 @@ k_stokes_prep(AtmView A, const double *__restrict__ lineopac, const double *__re
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= nwl_chunk * nmu) return;
     const int iwl = iwl0 + g / nmu, im = g - (g / nmu) * nmu;
-    const int N = A.ntau;
+    const int N = A.ntau, run = (N + STK_RUNS - 1) / STK_RUNS, ta = blockIdx.y * run, tb = min(ta + run, N);
+    if (ta >= tb) return;
     double *W = work + g;
 #define F(f, t) W[((size_t)(f) * N + (t)) * T]
     const double PlkC1 = FSG_HC * FSG_VC * 1e13 / FSG_KBOLT;
@@ -326,48 +364,67 @@ k_stokes_prep(AtmView A, const double *__restrict__ lineopac, const double *__re
     const double C1 = PlkC1 / wl, C2 = exp(50.7649141 - 5.0 * log(wl));
     const double gm[5] = { geo[0 * nmu + im], geo[1 * nmu + im], geo[2 * nmu + im], geo[3 * nmu + im],
                            geo[4 * nmu + im] };
-    for (int t = 0; t < N; t++) {
+    const double imu = 1.0 / xmu[im];
+    // the point at depth t: PhiI, then y = the 6 elements and the source vector
+    auto point = [&](int t, double (&y)[10]) {
         const size_t o = (size_t)iwl * N + t;
         const double sr = C2 / (exp(C1 / A.xi[XI_T * N + t]) - 1.0);
         double e6[6], s4[4];
-        F(0, t) = stokes_point(mlo + o * 6, lineopac[o], A.contopac[o], sr, gm, e6, s4);
-        for (int q = 0; q < 6; q++) F(1 + q, t) = e6[q];
-        for (int q = 0; q < 4; q++) F(13 + q, t) = s4[q];
+        const double p = stokes_point(mlo + o * 6, lineopac[o], A.contopac[o], sr, gm, e6, s4);
+#pragma unroll
+        for (int q = 0; q < 6; q++) y[q] = e6[q];
+#pragma unroll
+        for (int q = 0; q < 4; q++) y[6 + q] = s4[q];
+        return p;
+    };
+    // TauStep (solver.f90:591-615) from depth t to t + 1 with Xmu(im), given the slopes of PhiI behind and before
+    auto step = [&](int t) { return (rhox[t + 1] - rhox[t]) * imu; };
+    auto tau = [&](int t, double p0, double p1, double sa, double sb) {
+        const double dx = step(t), yp = t == 0 ? sb : hmean(sa, sb, lambda_of(step(t - 1), dx));
+        return dx * (p1 + 2.0 * p0 + dx * 0.5 * yp) * (1.0 / 3.0);
+    };
+    double y0[10], y1[10], gp[10];        // point t, point t + 1, slopes over the step before t
+    double p0, p1, sa = 0.0, dprev = 0.0;
+    if (ta > 0) {
+        double ym[10], yq[10];
+        const double pm = point(ta - 1, ym);
+        p0 = point(ta, y0);
+        sa = (p0 - pm) * rcp64(step(ta - 1));
+        const double sq = ta > 1 ? (pm - point(ta - 2, yq)) * rcp64(step(ta - 2)) : 0.0;
+        dprev = tau(ta - 1, pm, p0, sq, sa);
+        const double id = rcp64(dprev);
+#pragma unroll
+        for (int q = 0; q < 10; q++) gp[q] = (y0[q] - ym[q]) * id;
+    } else {
+        p0 = point(0, y0);
     }
-    // TauStep (solver.f90:591-615) with Xmu(im)
-    const double Xmu = xmu[im];
-    for (int t = 0; t < N - 1; t++) {
-        if (t == 0) {
-            double Dx1 = (rhox[1] - rhox[0]) / Xmu;
-            double Yp = (F(0, 1) - F(0, 0)) / Dx1;
-            F(21, 0) = Dx1 * (F(0, 1) + 2.0 * F(0, 0) + Dx1 / 2.0 * Yp) / 3.0;
-        } else {
-            const int k = t + 1;
-            double Dx = (rhox[k - 1] - rhox[k - 2]) / Xmu, Dx1 = (rhox[k] - rhox[k - 1]) / Xmu;
-            double Der = (F(0, k - 1) - F(0, k - 2)) / Dx, Der1 = (F(0, k) - F(0, k - 1)) / Dx1, Yp;
-            if (Der * Der1 > 0.0) {
-                double Lambda = (1.0 + Dx1 / (Dx + Dx1)) / 3.0;
-                Yp = (Der / (Lambda * Der1 + (1.0 - Lambda) * Der)) * Der1;
-            } else Yp = 0.0;
-            F(21, k - 1) = Dx1 * (F(0, k) + 2.0 * F(0, k - 1) + Dx1 / 2.0 * Yp) / 3.0;
-        }
-    }
-    // CentDer (solver.f90:618-647) of SRC4 (fields 13-16 -> 17-20) and of the 6 elements (1-6 -> 7-12)
-    for (int row = 0; row < 10; row++) {
-        const int fi = row < 4 ? 13 + row : 1 + (row - 4), fo = row < 4 ? 17 + row : 7 + (row - 4);
-        for (int k = 0; k < N; k++) {
-            double out;
-            if (k == 0) out = (F(fi, 1) - F(fi, 0)) / F(21, 0);
-            else if (k == N - 1) out = (F(fi, N - 1) - F(fi, N - 2)) / F(21, N - 2);
-            else {
-                double Dx = F(21, k - 1), Dx1 = F(21, k);
-                double InvDx = 1.0 / Dx, InvDx1 = 1.0 / Dx1;
-                double Lambda = (1.0 + Dx1 / (Dx + Dx1)) / 3.0, Lambda1 = 1.0 - Lambda;
-                double Der = (F(fi, k) - F(fi, k - 1)) * InvDx, Der1 = (F(fi, k + 1) - F(fi, k)) * InvDx1;
-                out = (Der * Der1 > 0.0) ? (Der / (Lambda * Der1 + Lambda1 * Der)) * Der1 : 0.0;
+    for (int t = ta; t < tb; t++) {
+        // CentDer (solver.f90:618-647) of every component at t from the slopes on either side
+        double out[10], d = 0.0;
+        if (t < N - 1) {
+            p1 = point(t + 1, y1);
+            const double sb = (p1 - p0) * rcp64(step(t));
+            d = tau(t, p0, p1, sa, sb);
+            F(21, t) = d;
+            const double id = rcp64(d), lam = t > 0 ? lambda_of(dprev, d) : 0.0;
+#pragma unroll
+            for (int q = 0; q < 10; q++) {
+                const double gn = (y1[q] - y0[q]) * id;
+                out[q] = t > 0 ? hmean(gp[q], gn, lam) : gn;
+                gp[q] = gn;
             }
-            F(fo, k) = out;
+            sa = sb;
+        } else {
+#pragma unroll
+            for (int q = 0; q < 10; q++) out[q] = gp[q];
         }
+#pragma unroll
+        for (int q = 0; q < 6; q++) { F(1 + q, t) = y0[q]; F(7 + q, t) = out[q]; }
+#pragma unroll
+        for (int q = 0; q < 4; q++) { F(13 + q, t) = y0[6 + q]; F(17 + q, t) = out[6 + q]; }
+        p0 = p1; dprev = d;
+#pragma unroll
+        for (int q = 0; q < 10; q++) y0[q] = y1[q];
     }
 #undef F
 }
@@ -497,7 +554,7 @@ int fsg_launch_stokes(cudaStream_t s, const AtmView &A, const double *lineopac, 
     for (int w0 = 0; w0 < A.nwl; w0 += nwl_chunk) {
         const int nw = std::min(nwl_chunk, A.nwl - w0);
         const int nb = (nwl_chunk * nmu + 127) / 128;      // the grid of a full chunk: fixed element stride
-        k_stokes_prep<<<nb, 128, 0, s>>>(A, lineopac, mlo, rhox, nmu, xmu, geo, w0, nw, work);
+        k_stokes_prep<<<dim3(nb, STK_RUNS), 128, 0, s>>>(A, lineopac, mlo, rhox, nmu, xmu, geo, w0, nw, work);
         k_stokes_thr<<<nb, 128, 0, s>>>(A, nmu, w0, nw, work, spz);
     }
     if (sfl) k_stokes_flux<<<(A.nwl + 127) / 128, 128, 0, s>>>(A.nwl, nmu, spz, wmu, sfl);

@@ -18,36 +18,11 @@
 
 #define SOLVE_C 8
 
-// DELO coefficients (solver.f90:357-370) as delo_coef, in its order of operations where the differences
-// cancel (just above Dtau = 5e-3 they amplify a rounding of Eps 1e7 times)
+// one step of the sweep (solver.f90:139-142): Y Eps + Alpha y0 + Beta y1 + Gamma u
 __device__ __forceinline__ double delo_step(double d, double Y, double y0, double y1, double u) {
-    const double d2 = d * d;
     double Eps, Al, Be, Ga;
-    if (d < 5e-3) {
-        const double d3 = d2 * d;
-        Eps = 1.0 - d + 0.5 * d2 - d3 * (1.0 / 6.0) + d2 * d2 * (1.0 / 24.0);
-        Al = d * (1.0 / 3.0) - d2 * (1.0 / 12.0) + d3 * (1.0 / 60.0);
-        Be = d * (1.0 / 3.0) - d2 * 0.25 + d3 * 0.1;
-        Ga = d * (1.0 / 3.0) - d2 * (1.0 / 6.0) + d3 * 0.05;
-    } else {
-        Eps = d < 100.0 ? exp(-d) : 0.0;
-        const double i2 = rcp64(d2), dd = 2.0 * d;
-        Al = (d2 - dd + 2.0 - 2.0 * Eps) * i2;
-        Be = (2.0 - (2.0 + dd + d2) * Eps) * i2;
-        Ga = (dd - 4.0 + (dd + 4.0) * Eps) * i2;
-    }
+    delo_coef(d, Eps, Al, Be, Ga);
     return fma(Y, Eps, fma(Al, y0, fma(Be, y1, Ga * u)));
-}
-
-// harmonic mean Der Der1 / (Lambda Der1 + (1 - Lambda) Der) of two slopes of one sign, else 0
-// (solver.f90:604-610, 637-643)
-__device__ __forceinline__ double hmean(double der, double der1, double lam) {
-    return der * der1 > 0.0 ? der * rcp64(fma(lam, der1, (1.0 - lam) * der)) * der1 : 0.0;
-}
-
-// CentDer's Lambda from the steps on either side (solver.f90:632)
-__device__ __forceinline__ double lambda_of(double dx, double dx1) {
-    return (1.0 + dx1 * rcp64(dx + dx1)) * (1.0 / 3.0);
 }
 
 // CentDer (solver.f90:618-647) of y on the scale of the steps d, at point t of nt
