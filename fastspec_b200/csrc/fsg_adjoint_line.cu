@@ -9,11 +9,9 @@
 // window-edge term (below).  Helium lines with a per-depth Stark shift (few) are reduced there
 // over their whole window in FP64 and left out of pass 2.
 //
-// Pass 2, k_adj_tiles: the accumulation's tiling turned around.  A CTA owns a tile of 64
-// wavelengths x all depths: consumer warp w keeps dL/dkappa of depths [w KD, w KD + KD) at the
-// lane's two wavelengths in registers; one producer warp picks the lines whose windows meet the
-// tile, 16 at a time, and brings their records into a double-buffered shared-memory stage by bulk
-// copies (mbarrier-tracked, released by the consumers through a second mbarrier pair).  Outside a
+// Pass 2, k_adj_tiles: the accumulation's tiling turned around.  A warp owns a tile of 128 wavelengths x KD
+// depths and keeps dL/dkappa there in registers (four wavelengths per lane); it queues the lines whose windows
+// meet the tile and takes them ADJ_G at a time, their headers and records in its shared memory.  Outside a
 // line's core range the wing form is two polynomials in X = dl^2 and one reciprocal per point,
 // with depth pairs in packed FP32 (FFMA2):
 //   D = y^2 + B1 y + B0,  y = vv^2 X,  B1 = 2a^2 - 1,  B0 = a^4 + a^2 + 1/4
@@ -21,9 +19,13 @@
 //   LinCop q Hd = K2 (1 + 2 (y^2 - B0) / D) / D                           K2 = LinCop q a / sqrt(pi)
 // i.e. per point D = (c4 X + c2) X + B0, h = e1 X + e0, p = f2 X^2 + f0, and the sums take
 // g/D * h and g/D * (p/D + K2).  Lines whose core range meets the tile take the point-by-point
-// path (FvTab or the complex rational inside, the same wing form outside).  Partial sums are
-// reduced over lanes by shuffles, over warps by the producer (FP64, fixed order), and each
-// tile's part is added to the line's FP64 sums with one atomic.
+// path (FvTab or the complex rational inside, the same wing form outside).  A line's partial sums are
+// reduced over the lanes in FP64, in a fixed order, and added to its FP64 sums with one atomic each per warp.
+// A pair of depths at a point costs eight packed FMAs and two reciprocals (the reciprocal pipe bounds it), and the
+// 16-byte record loads, which four wavelengths per lane share, come next.  1e5 lines, 100,001 wavelengths, 56
+// depths (3.2e10 evaluations): 21.1 ms; CTAs of one producer and seven consumer warps that met at two
+// mbarriers per 16 lines, with 64-wavelength tiles, took 34.9 ms.  Of the 21.1 ms the point-by-point lines take 5
+// (table gathers), picking the lines 2.5.
 //
 // Profile and derivative forms (FVoigt / FVoigtLine, voigt.f90:256-352):
 //  * wing, s >= 196: the rational H = a (s + 1/2) / (sqrt(pi) D), D = s^2 - (v^2 - a^2) + 1/4, the
@@ -39,18 +41,20 @@
 // its free edges move by dW, adding the edge profile over dW / (wavelength step) at each edge
 // (d ln W from the depth giving the maximum).
 #include "fsg_fp64.cuh"
-#include "fsg_mbar.cuh"
+#include "fsg_tile.cuh"
 
 size_t fsg_tile_span_scratch(int64_t);
 int fsg_launch_tile_span_tw(cudaStream_t, int, int, int, int64_t, const LineHdr *, int *, int *, void *, size_t);
 
 #define ADJ_SETUP_WARPS 8
-#define ADJ_P 2                        // wavelengths per lane
+#define ADJ_P 4                        // wavelengths per lane
 #define ADJ_TW (32 * ADJ_P)            // wavelengths per tile
-#define ADJ_CL 16                      // lines per stage
+#define ADJ_G 8                        // lines per group
+#define ADJ_W 4                        // warps per CTA
 
-// depths per consumer warp, and the depth count padded to a multiple of it
-static int adj_kd(int nt) { return nt >= 32 ? 8 : (nt >= 8 ? 4 : 2); }
+// depths per warp, and the depth count padded to a multiple of it.  Four: the weights of eight take 128 registers
+// (16 warps per SM instead of 20: 22.8 ms)
+static int adj_kd(int nt) { return nt >= 8 ? 4 : 2; }
 static int adj_ntp(int nt) { const int k = adj_kd(nt); return (nt + k - 1) / k * k; }
 
 // Pass-2 records of line i: ntp/2 depth pairs x 4 float4, pair (t, t+1) as
@@ -215,7 +219,7 @@ k_adj_setup(AtmView A, LineView L, const float *__restrict__ vtab, const float2 
 }
 
 struct AdjTileJob {
-    int nwl, nt, ntp, nw;              // wavelengths, depths, padded depths, consumer warps
+    int nwl, nt, ntp, ntiles, ngrp;    // wavelengths, depths, padded depths, tiles, depth groups
     const float *gk32;                 // dL/dkappa, FP32, [nt][nwl]
     const float *wvh, *wvl;            // wavelength offsets as FP32 hi + lo, [nwl]
     const float4 *prec;                // [n][ntp / 2][4]
@@ -223,9 +227,8 @@ struct AdjTileJob {
     const float2 *tabi;                // [n][nt]
     const LineHdr *hdr;                // [n]
     const int *tlo, *thi;              // line range of each tile (inclusive)
-    const float2 *fvtab;
+    const float4 *fvtab2;
     double *glin, *gvmic;
-    int *err;
 };
 
 __device__ __forceinline__ float rcp_approx(float x) {
@@ -235,7 +238,7 @@ __device__ __forceinline__ float rcp_approx(float x) {
 }
 
 // H and Hd at (v, a) for s = v^2 + a^2 < 196: FvTab interpolation or the complex rational
-__device__ __forceinline__ void core_h_hd(const float2 *__restrict__ ftab, float2 ti, float v, float a,
+__device__ __forceinline__ void core_h_hd(const float4 *__restrict__ ftab2, float2 ti, float v, float a,
                                           float *H, float *Hd) {
     const float av = fabsf(v);
     const int ia = (int)ti.y;
@@ -244,10 +247,10 @@ __device__ __forceinline__ void core_h_hd(const float2 *__restrict__ ftab, float
         const float fv = av * 125.0f;                     // 1 / (8 / 1000)
         const int iv = (int)fv;
         const float tv = fv - (float)iv;
-        const float2 *c0p = ftab + (ia - 1) * FSG_NV1 + iv, *c1p = c0p + FSG_NV1;
-        const float2 t00 = __ldg(c0p), t01 = __ldg(c0p + 1), t10 = __ldg(c1p), t11 = __ldg(c1p + 1);
-        const float h0 = fmaf(tv, t01.x - t00.x, t00.x), h1 = fmaf(tv, t11.x - t10.x, t10.x);
-        const float l0 = fmaf(tv, t01.y - t00.y, t00.y), l1 = fmaf(tv, t11.y - t10.y, t10.y);
+        const float4 *p0 = ftab2 + (ia - 1) * FSG_NV1 + iv;
+        const float4 g0 = __ldg(p0), g1 = __ldg(p0 + FSG_NV1);      // (H_i, L_i, H_i+1, L_i+1) of rows ia, ia+1
+        const float h0 = fmaf(tv, g0.z - g0.x, g0.x), h1 = fmaf(tv, g1.z - g1.x, g1.x);
+        const float l0 = fmaf(tv, g0.w - g0.y, g0.y), l1 = fmaf(tv, g1.w - g1.y, g1.y);
         h = fmaf(ti.x, h1 - h0, h0);
         l = fmaf(ti.x, l1 - l0, l0);
     } else {
@@ -291,22 +294,21 @@ __device__ __forceinline__ void wing_line(const float4 *__restrict__ rp, const f
     }
 }
 
-// point by point: lines whose core range meets the tile
-template <int KD>
-__device__ __forceinline__ void core_line(const AdjTileJob &J, int line, int t0, const float2 (&g)[ADJ_P][KD / 2],
+// point by point: lines whose core range meets the tile.  A loop over depths that reads its weights from memory
+// again: unrolled over the warp's depths the three profile forms outgrew the instruction cache.
+__device__ __forceinline__ void core_line(const AdjTileJob &J, int line, int t0, int t1, const int (&pix)[ADJ_P],
                                           const float (&dl)[ADJ_P], const bool (&in)[ADJ_P], float2 &s1,
                                           float2 &s2) {
-    const int nt = J.nt;
+#pragma unroll 1
+    for (int t = t0; t < t1; t++) {
+        const float4 cr = __ldg(&J.crec[(size_t)line * J.nt + t]);
+        const float2 ti = __ldg(&J.tabi[(size_t)line * J.nt + t]);
+        const float a = cr.y, a2 = a * a;
+        float h1 = 0.0f, h2 = 0.0f;
 #pragma unroll
-    for (int k = 0; k < ADJ_P; k++) {
-        if (!in[k]) continue;
-#pragma unroll
-        for (int d = 0; d < KD; d++) {
-            const int t = t0 + d;
-            if (t >= nt) break;
-            const float4 cr = __ldg(&J.crec[(size_t)line * nt + t]);
-            const float v = dl[k] * cr.x, a = cr.y, a2 = a * a;
-            const float s = fmaf(v, v, a2);
+        for (int k = 0; k < ADJ_P; k++) {
+            if (!in[k]) continue;
+            const float v = dl[k] * cr.x, s = fmaf(v, v, a2);
             float H, Hd;
             if (s >= 196.0f) {
                 const float u = s - 2.0f * a2;
@@ -315,106 +317,34 @@ __device__ __forceinline__ void core_line(const AdjTileJob &J, int line, int t0,
                 H = aw * (s + 0.5f);
                 Hd = aw * rD * (fmaf(s, s + 2.0f * u, -s) - 0.25f);
             } else {
-                core_h_hd(J.fvtab, __ldg(&J.tabi[(size_t)line * nt + t]), v, a, &H, &Hd);
+                core_h_hd(J.fvtab2, ti, v, a, &H, &Hd);
             }
-            const float gv = (d & 1) ? g[k][d >> 1].y : g[k][d >> 1].x;
-            s1.x = fmaf(gv * cr.z, H, s1.x);
-            s2.x = fmaf(gv * cr.w, Hd, s2.x);
+            const float gv = __ldg(&J.gk32[(size_t)t * J.nwl + pix[k]]);
+            h1 = fmaf(gv, H, h1);
+            h2 = fmaf(gv, Hd, h2);
         }
+        s1.x = fmaf(h1, cr.z, s1.x);
+        s2.x = fmaf(h2, cr.w, s2.x);
     }
 }
 
-// shared memory: mbarriers full[2], empty[2] | nsel[2] (+pad) | records [2][CL][2 ntp] float4 |
-// headers [2][CL] | partials [2][CL][nw][8] float2 | line indices [2][CL]
-static size_t adj_tile_smem(int nt) {
-    const int ntp = adj_ntp(nt), nw = ntp / adj_kd(nt);
-    return 4 * sizeof(uint64_t) + 4 * sizeof(int) + sizeof(float4) * 2 * ADJ_CL * 2 * (size_t)ntp +
-           sizeof(LineHdr) * 2 * ADJ_CL + sizeof(float2) * 2 * ADJ_CL * (size_t)nw * 8 + sizeof(int) * 2 * ADJ_CL;
-}
-
-// grid: one CTA per tile; block: nw consumer warps + 1 producer warp
+// one (tile, depth group) per warp, the groups of a tile in turn
 template <int KD>
-__global__ void __launch_bounds__(32 * 17) k_adj_tiles(AdjTileJob J) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int nt = J.nt, ntp = J.ntp, nw = J.nw, nwl = J.nwl;
+__global__ void __launch_bounds__(32 * ADJ_W) k_adj_tiles(AdjTileJob J) {
+    constexpr int R = 2 * KD;                             // 16-byte record parts of a line at the warp's depths
+    __shared__ int queue_s[ADJ_W][64];
+    __shared__ LineHdr hdr_s[ADJ_W][ADJ_G];
+    __shared__ float4 rec_s[ADJ_W][ADJ_G][R];
+    __shared__ float2 part_s[ADJ_W][ADJ_G][33];
+    const int nt = J.nt, nwl = J.nwl;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint64_t *full = (uint64_t *)smem_raw, *empty = full + 2;
-    int *snsel = (int *)(empty + 2);
-    float4 *srec = (float4 *)(snsel + 4);
-    LineHdr *shdr = (LineHdr *)(srec + 2 * ADJ_CL * 2 * ntp);
-    float2 *spart = (float2 *)(shdr + 2 * ADJ_CL);
-    int *sidx = (int *)(spart + 2 * ADJ_CL * nw * 8);
-    const int tile = blockIdx.x;
+    const int64_t item = (int64_t)blockIdx.x * ADJ_W + warp;
+    if (item >= (int64_t)J.ntiles * J.ngrp) return;      // warps are independent: no CTA barrier below
+    const int tile = (int)(item / J.ngrp), t0 = (int)(item % J.ngrp) * KD;
     const int lo = J.tlo[tile], hi = J.thi[tile];
     if (lo > hi) return;
-    if (threadIdx.x == 0) {
-        mbar_init(&full[0], 1); mbar_init(&full[1], 1);
-        mbar_init(&empty[0], nw); mbar_init(&empty[1], nw);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
     const int f1 = tile * ADJ_TW + 1, l1 = min(tile * ADJ_TW + ADJ_TW, nwl);     // 1-based wavelengths
-    if (warp == nw) {
-        // producer: select, stage, and reduce what the consumers leave in the partials
-        const unsigned recb = (unsigned)(ntp * 32);
-        auto reduce = [&](int b) {
-            const int n = snsel[b];
-            if (lane < n) {
-                const float2 *pp = spart + (size_t)(b * ADJ_CL + lane) * nw * 8;
-                double a1 = 0.0, a2 = 0.0;
-                for (int w = 0; w < nw * 8; w++) { const float2 v = pp[w]; a1 += (double)v.x; a2 += (double)v.y; }
-                const int j = sidx[b * ADJ_CL + lane];
-                atomicAdd(&J.glin[j], a1);
-                atomicAdd(&J.gvmic[j], a2);
-            }
-            __syncwarp();
-        };
-        int c = 0, cand = lo;
-        bool ok = true;
-        for (;;) {
-            unsigned m = 0;
-            bool sel = false;
-            int j = 0;
-            LineHdr h = {};
-            while (cand <= hi && m == 0) {
-                j = cand + lane;
-                sel = false;
-                if (lane < ADJ_CL && j <= hi) {
-                    h = J.hdr[j];
-                    sel = h.ileft <= h.iright && h.iright >= f1 && h.ileft <= l1;
-                }
-                m = __ballot_sync(0xffffffffu, sel);
-                cand += ADJ_CL;
-            }
-            const int b = c & 1, u = c >> 1;
-            if (c >= 2) {
-                if (!mbar_wait(&empty[b], (u - 1) & 1)) { ok = false; break; }
-                reduce(b);
-            }
-            if (m == 0) {                                 // no more lines: tell the consumers
-                if (lane == 0) { snsel[b] = 0; mbar_arrive(&full[b]); }
-                break;
-            }
-            const int pos = __popc(m & ((1u << lane) - 1u));
-            if (sel) { sidx[b * ADJ_CL + pos] = j; shdr[b * ADJ_CL + pos] = h; }
-            if (lane == 0) snsel[b] = __popc(m);
-            __syncwarp();
-            if (lane == 0) mbar_expect_tx(&full[b], (unsigned)__popc(m) * recb);
-            __syncwarp();
-            if (sel)
-                tma_bulk_g2s(srec + (size_t)(b * ADJ_CL + pos) * 2 * ntp, J.prec + (size_t)j * 2 * ntp, recb, &full[b]);
-            c++;
-        }
-        if (ok && c >= 1) {                               // the last stage
-            const int b = (c - 1) & 1, u = (c - 1) >> 1;
-            if (mbar_wait(&empty[b], u & 1)) reduce(b);
-            else ok = false;
-        }
-        if (!ok && lane == 0) atomicExch(J.err, 1);
-        return;
-    }
-    // consumers
-    const int t0 = warp * KD;
+    const int *queue = queue_s[warp];
     float2 g[ADJ_P][KD / 2];
     float wh[ADJ_P], wl[ADJ_P];
     int pix[ADJ_P];
@@ -432,13 +362,15 @@ __global__ void __launch_bounds__(32 * 17) k_adj_tiles(AdjTileJob J) {
             g[k][j].y = (pin && t + 1 < nt) ? J.gk32[(size_t)(t + 1) * nwl + pix[k]] : 0.0f;
         }
     }
-    for (int c = 0;; c++) {
-        const int b = c & 1, u = c >> 1;
-        if (!mbar_wait(&full[b], u & 1)) { if (lane == 0) atomicExch(J.err, 1); break; }
-        const int n = snsel[b];
-        if (n == 0) break;
+    auto group = [&](int head, int n) {
+        if (lane < n) hdr_s[warp][lane] = J.hdr[queue[(head + lane) & 63]];
+        for (int e = lane; e < n * R; e += 32) {
+            const int q = e / R, u = e % R;
+            rec_s[warp][q][u] = __ldg(J.prec + (size_t)queue[(head + q) & 63] * 2 * J.ntp + 2 * t0 + u);
+        }
+        __syncwarp();
         for (int m = 0; m < n; m++) {
-            const LineHdr h = shdr[b * ADJ_CL + m];
+            const LineHdr h = hdr_s[warp][m];
             float dl[ADJ_P], X[ADJ_P], XX[ADJ_P];
             bool in[ADJ_P];
 #pragma unroll
@@ -449,20 +381,35 @@ __global__ void __launch_bounds__(32 * 17) k_adj_tiles(AdjTileJob J) {
                 in[k] = pix[k] + 1 >= h.ileft && pix[k] + 1 <= h.iright;
             }
             float2 s1 = make_float2(0.0f, 0.0f), s2 = make_float2(0.0f, 0.0f);
-            const float4 *rp = srec + (size_t)(b * ADJ_CL + m) * 2 * ntp + (t0 >> 1) * 4;
-            if (!(h.cr < f1 || h.cl > l1)) core_line<KD>(J, sidx[b * ADJ_CL + m], t0, g, dl, in, s1, s2);
+            const float4 *rp = rec_s[warp][m];
+            if (!(h.cr < f1 || h.cl > l1)) core_line(J, queue[(head + m) & 63], t0, min(t0 + KD, nt), pix, dl, in, s1, s2);
             else if (h.ileft <= f1 && h.iright >= l1) wing_line<KD, false>(rp, g, X, XX, in, s1, s2);
             else wing_line<KD, true>(rp, g, X, XX, in, s1, s2);
-            float v1 = s1.x + s1.y, v2 = s2.x + s2.y;
-            v1 += __shfl_xor_sync(0xffffffffu, v1, 16);
-            v2 += __shfl_xor_sync(0xffffffffu, v2, 16);
-            v1 += __shfl_xor_sync(0xffffffffu, v1, 8);
-            v2 += __shfl_xor_sync(0xffffffffu, v2, 8);
-            if (lane < 8) spart[((size_t)(b * ADJ_CL + m) * nw + warp) * 8 + lane] = make_float2(v1, v2);
+            part_s[warp][m][lane] = make_float2(s1.x + s1.y, s2.x + s2.y);
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[b]);
-    }
+        // four lanes per line sum its 32 partials in FP64
+        const int m = lane >> 2, c = lane & 3;
+        double a1 = 0.0, a2 = 0.0;
+        if (m < n) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float2 v = part_s[warp][m][c + 4 * i];
+                a1 += (double)v.x; a2 += (double)v.y;
+            }
+        }
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+            a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+        }
+        if (m < n && c < 2) {
+            const int j = queue[(head + m) & 63];
+            atomicAdd(c == 0 ? &J.glin[j] : &J.gvmic[j], c == 0 ? a1 : a2);
+        }
+        __syncwarp();                                    // the group's shared records may be replaced
+    };
+    tile_lines<ADJ_G>(J.hdr, lo, hi, f1, l1, queue_s[warp], lane, group);
 }
 
 static size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -472,14 +419,14 @@ size_t fsg_line_adjoint_work(int nwl, int nt, int64_t n) {
     const int ntiles = (nwl + ADJ_TW - 1) / ADJ_TW;
     return al256(sizeof(float) * 8 * (size_t)n * adj_ntp(nt)) + al256(sizeof(float4) * (size_t)n * nt) +
            al256(sizeof(float2) * (size_t)n * nt) + al256(sizeof(LineHdr) * (size_t)n) +
-           2 * al256(sizeof(int) * (size_t)ntiles) + al256(sizeof(int)) + al256(fsg_tile_span_scratch(n)) + 256;
+           2 * al256(sizeof(int) * (size_t)ntiles) + al256(fsg_tile_span_scratch(n)) + 256;
 }
 
 int fsg_launch_line_adjoint(cudaStream_t s, const AtmView &A, const LineView &L, const VoigtTables &T,
                             const int32_t *flags, const int32_t *ileft, const int32_t *iright, const double *gkappa,
                             const float *gk32, const float *wvh, const float *wvl, double vmic, double *glin,
                             double *gvmic, void *work, int i0, int i1) {
-    const int nt = A.ntau, nwl = A.nwl, ntp = adj_ntp(nt), kd = adj_kd(nt), nw = ntp / kd;
+    const int nt = A.ntau, nwl = A.nwl, ntp = adj_ntp(nt), kd = adj_kd(nt);
     const int64_t n = L.n;
     const int ntiles = (nwl + ADJ_TW - 1) / ADJ_TW;
     char *w = (char *)(((uintptr_t)work + 255) & ~(uintptr_t)255);
@@ -489,10 +436,8 @@ int fsg_launch_line_adjoint(cudaStream_t s, const AtmView &A, const LineView &L,
     LineHdr *hdr = (LineHdr *)w; w += al256(sizeof(LineHdr) * (size_t)n);
     int *tlo = (int *)w; w += al256(sizeof(int) * (size_t)ntiles);
     int *thi = (int *)w; w += al256(sizeof(int) * (size_t)ntiles);
-    int *err = (int *)w; w += al256(sizeof(int));
     const size_t span_bytes = fsg_tile_span_scratch(n);
     void *span = (void *)w;
-    if (cudaMemsetAsync(err, 0, sizeof(int), s) != cudaSuccess) return FSG_E_CUDA;
     size_t smem = sizeof(double) * 6 * nt * ADJ_SETUP_WARPS;
     k_adj_setup<<<(unsigned)((n + ADJ_SETUP_WARPS - 1) / ADJ_SETUP_WARPS), 32 * ADJ_SETUP_WARPS, smem, s>>>(
         A, L, T.vtab, T.fvtab, T.anode, T.aida, flags, ileft, iright, gkappa, vmic, ntp, prec, crec, tabi, hdr, glin,
@@ -500,25 +445,11 @@ int fsg_launch_line_adjoint(cudaStream_t s, const AtmView &A, const LineView &L,
     int rc = fsg_launch_tile_span_tw(s, ADJ_TW, 0, nwl, n, hdr, tlo, thi, span, span_bytes);
     if (rc) return rc;
     AdjTileJob J;
-    J.nwl = nwl; J.nt = nt; J.ntp = ntp; J.nw = nw; J.gk32 = gk32; J.wvh = wvh; J.wvl = wvl;
+    J.nwl = nwl; J.nt = nt; J.ntp = ntp; J.ntiles = ntiles; J.ngrp = ntp / kd; J.gk32 = gk32; J.wvh = wvh; J.wvl = wvl;
     J.prec = (const float4 *)prec; J.crec = crec; J.tabi = tabi; J.hdr = hdr; J.tlo = tlo; J.thi = thi;
-    J.fvtab = T.fvtab; J.glin = glin; J.gvmic = gvmic; J.err = err;
-    const size_t tsm = adj_tile_smem(nt);
-#define ADJ_LAUNCH(K)                                                                                     \
-    do {                                                                                                  \
-        if (cudaFuncSetAttribute(k_adj_tiles<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm) != \
-            cudaSuccess)                                                                                  \
-            return FSG_E_CUDA;                                                                            \
-        k_adj_tiles<K><<<ntiles, 32 * (nw + 1), tsm, s>>>(J);                                             \
-    } while (0)
-    if (kd == 8) ADJ_LAUNCH(8);
-    else if (kd == 4) ADJ_LAUNCH(4);
-    else ADJ_LAUNCH(2);
-#undef ADJ_LAUNCH
-    if (cudaGetLastError() != cudaSuccess) return FSG_E_CUDA;
-    int herr = 0;
-    if (cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
-        return FSG_E_CUDA;
-    return herr ? FSG_E_CUDA : FSG_OK;
+    J.fvtab2 = T.fvtab2; J.glin = glin; J.gvmic = gvmic;
+    const unsigned grid = (unsigned)(((int64_t)J.ntiles * J.ngrp + ADJ_W - 1) / ADJ_W);
+    if (kd == 4) k_adj_tiles<4><<<grid, 32 * ADJ_W, 0, s>>>(J);
+    else k_adj_tiles<2><<<grid, 32 * ADJ_W, 0, s>>>(J);
+    return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }

@@ -11,13 +11,13 @@ template <int G, class H, class F>
 __device__ __forceinline__ void tile_lines(const H *__restrict__ hdr, int lo, int hi, int first, int last, int *queue,
                                            int lane, F group) {
     int head = 0, cnt = 0;
+    const int2 none = make_int2(1, 0);
+    int2 next = lo + lane <= hi ? window_of(hdr[lo + lane]) : none;
     for (int base = lo; base <= hi; base += 32) {
         const int j = base + lane;
-        bool sel = false;
-        if (j <= hi) {
-            const int2 w = window_of(hdr[j]);
-            sel = w.x <= w.y && w.x <= last && w.y >= first;
-        }
+        const int2 w = next;                            // the next 32 windows are on their way meanwhile
+        next = j + 32 <= hi ? window_of(hdr[j + 32]) : none;
+        const bool sel = w.x <= w.y && w.x <= last && w.y >= first;
         const unsigned m = __ballot_sync(0xffffffffu, sel);
         if (!m) continue;
         if (sel) queue[(head + cnt + __popc(m & ((1u << lane) - 1u))) & 63] = j;

@@ -124,3 +124,47 @@ def test_broadening_edges(fsg, oracle_mod, nwl, nmu, vsini, vmacro, vgau):
     assert np.max(np.abs(d[2].cpu().numpy() / osfl - 1)) < 1e-12
     assert np.max(np.abs(d[3].cpu().numpy() / osfc - 1)) < 1e-12
     C.close()
+
+
+@pytest.mark.parametrize("ntau,nwl,n", [(3, 2, 1), (7, 127, 8), (9, 129, 9), (33, 300, 33), (65, 640, 70)])
+def test_adjoint_tile_edges(fsg, ntau, nwl, n):
+    """The line pass of the adjoint around its tiles and depth groups: the whole-grid gradients against the sum of
+    those of two ranges (split inside a tile), and, where every window covers the grid, dL/d ln gf of the whole
+    list, which then is the sum of dL/dkappa * LineOpac, against that sum on the FP64 opacity.  The profiles are FP32 (6e-8 per
+    operation, some ten of them, summed with both signs): 2e-6 of the sum of magnitudes."""
+    import ctypes
+    import torch
+    from fastspec_b200.shard import GpuBackend
+    grid, st, co, a = case(ntau, nwl, n, 5 * ntau + nwl)
+    C = fsg.Context(precision=fsg.PREC_FP64, vmicro=1.0, epsopac=1e-12)
+    C.set_grid(grid["wmode"], grid["wstart"], grid["wend"], grid["dstep"])
+    C.set_atmosphere(st)
+    C.set_contopac(co)
+    x, w, _ = fsg.mu_quadrature(1, 3)
+    C.set_mu(x, w)
+    dt = {k: torch.from_numpy(np.ascontiguousarray(v)).cuda() for k, v in a.items()}
+    B = GpuBackend(fsg, C, dt)
+    e = lambda *s: torch.zeros(*s, dtype=torch.float64, device="cuda")      # noqa: E731
+    sfl, sfc, gk = e(nwl), e(nwl), e(nwl, ntau)
+    win = torch.zeros((3, n), dtype=torch.int32, device="cuda")
+    C.lineop_reset()
+    C.lineop_calc_dev(B.full)
+    C.radtran_dev(None, None, sfl.data_ptr(), sfc.data_ptr())
+    C.central_dev(B.full, win[0].data_ptr(), win[1].data_ptr(), win[2].data_ptr())
+    keep = (win[0] & 1) == 0
+    covered = bool(((win[1] == 1) & (win[2] == nwl))[keep].all())            # no window edge moves with gf
+    gf = torch.from_numpy(np.random.default_rng(n).normal(0.0, 1.0, nwl)).cuda() / sfc
+    out = [(e(n), e(n)) for _ in range(3)]
+    torch.cuda.synchronize()
+    C.adjoint_dev(B.full, gf.data_ptr(), out[0][0].data_ptr(), out[0][1].data_ptr(), gk.data_ptr())
+    cut = nwl // 2
+    for (i0, i1), o in zip(((1, cut), (cut + 1, nwl)), out[1:]):
+        C.adjoint_range_dev(B.full, win[0].data_ptr(), win[1].data_ptr(), win[2].data_ptr(), i0, i1, gf.data_ptr(),
+                            o[0].data_ptr(), o[1].data_ptr())
+    lo = torch.from_numpy(C.lineop_get()).cuda()
+    scale = float((gk * lo).abs().sum())
+    if covered:
+        assert abs(float(out[0][0].sum()) - float((gk * lo).sum())) < 2e-6 * scale
+    for q in range(2):
+        assert float((out[0][q] - out[1][q] - out[2][q]).abs().max()) < 2e-6 * max(scale, float(out[0][q].abs().sum()))
+    C.close()
