@@ -101,11 +101,8 @@ void fsg_launch_fvoigt(cudaStream_t, int64_t, const double *, const double *, do
                        const VoigtTables &);
 void fsg_launch_locprf(cudaStream_t, int, int, const double *, int, const double *, const double *, const double *,
                        double *, double *);
-int fsg_launch_accum_fast(cudaStream_t, int, int, int, const double *, const LineHdr *, const WingPair *, const int *,
-                          const int *, double *);
-int fsg_launch_core_fast(cudaStream_t, int, int, const double *, const LineHdr *, const CoreRec *, const int *,
-                         const int *, const float4 *, double *, unsigned long long *, int *, unsigned,
-                         unsigned long long);
+int fsg_launch_accum_fast(cudaStream_t, int, const WingJob &);
+int fsg_launch_core_fast(cudaStream_t, const CoreJob &, const float4 *, int *);
 int fsg_wing_groups(int, int);
 int fsg_launch_accum_batch(cudaStream_t, int, const WingJob *, const int *, int, int, unsigned *);
 int fsg_launch_core_batch(cudaStream_t, int, const CoreJob *, const int *, int, int, const float4 *, unsigned *,
@@ -116,8 +113,8 @@ int fsg_bclass_count(int);
 int fsg_launch_bclass_order(cudaStream_t, int64_t, const int32_t *, const int32_t *, const int32_t *, int, int *,
                             int64_t *, int64_t *, int64_t *);
 size_t fsg_bspan_scratch(int64_t);
-int fsg_launch_btile_span(cudaStream_t, int, int64_t, const LineHdr *, const int64_t *, int, int, int, int, int, int,
-                          int *, int *, void *, size_t);
+int fsg_launch_btile_span(cudaStream_t, int64_t, const LineHdr *, const int64_t *, int, int, int, int, int, int, int,
+                          int *, int *, int, int *, int *, void *, size_t);
 size_t fsg_tile_span_scratch(int64_t);
 int fsg_launch_tile_span_tw(cudaStream_t, int, int, int, int64_t, const LineHdr *, int *, int *, void *, size_t);
 void fsg_launch_mag_params_fast(cudaStream_t, const AtmView &, const LineView &, const ZView &, const int64_t *, int64_t,
@@ -153,7 +150,8 @@ void fsg_launch_gather_lines(cudaStream_t, const LineView &, const int64_t *, in
                              const int32_t *, const int32_t *, LineView *, int32_t **, int32_t **, int32_t **);
 int fsg_select_wide(cudaStream_t, int64_t, const int32_t *, int *, int64_t *, int64_t *, int64_t *);
 void fsg_launch_scatter_flags(cudaStream_t, int64_t, const int64_t *, const int32_t *, int32_t *);
-double fsg_count_evals(fsg_ctx *, int64_t, const int32_t *, const int32_t *, const int32_t *, int, int);
+static void launch_count_windows(cudaStream_t, int64_t, const int32_t *, const int32_t *, const int32_t *, int, int,
+                                 unsigned long long *, const int32_t *npi = nullptr, const int32_t *nsi = nullptr);
 static double count_windows(fsg_ctx *, int64_t, const int32_t *, const int32_t *, const int32_t *, int, int,
                             const int32_t *npi = nullptr, const int32_t *nsi = nullptr);
 void fsg_launch_range_clip(cudaStream_t, int64_t, const int32_t *, const int32_t *, const int32_t *, int, int,
@@ -169,6 +167,9 @@ std::string fsg_cuda_msg(cudaError_t e, const char *what) {
     snprintf(b, sizeof b, "%s: CUDA error %d (%s)", what, (int)e, cudaGetErrorString(e));
     return b;
 }
+
+// window-width classes 0 .. WING_NARROW take wing tiles of 64 wavelengths, the others 128 (or, in a batch, as tuned)
+static const int WING_NARROW = 1;
 
 // ---- device buffer that only grows ---------------------------------------------------------------
 struct DBuf {
@@ -227,7 +228,8 @@ struct fsg_ctx {
     DBuf l_wl, l_elo, l_gf, l_grad, l_gqst, l_gvdw, l_spc, l_ismol, l_ihe;
     DBuf d_flags, d_ileft, d_iright, d_idx, d_counts, d_offs, d_total, d_hist, d_nkeep;
     // block buffers
-    DBuf d_wing, d_core, d_hdr, d_hdr64, d_tlo, d_thi, d_p64, d_lstart, d_lstop, d_widx, d_pw, d_err, d_ncore, d_span, d_linstr, d_rflags, d_rleft, d_rright, d_gkappa, d_adjwork, d_cbuf, d_ctaps;
+    DBuf d_block;                              // order, records and tile ranges of a list that fits one block
+    DBuf d_wing, d_core, d_hdr, d_hdr64, d_tlo, d_thi, d_p64, d_lstart, d_lstop, d_widx, d_pw, d_res, d_span, d_linstr, d_rflags, d_rleft, d_rright, d_gkappa, d_adjwork, d_cbuf, d_ctaps;
     // spectra
     DBuf d_spl, d_spc, d_sfl, d_sfc, d_work, d_a, d_v, d_h, d_l;
     // magnetic
@@ -318,8 +320,8 @@ void fsg_destroy(fsg_ctx *ctx) {
                      &ctx->d_wmu, &ctx->d_lineopac, &ctx->d_maglineopac, &ctx->l_wl, &ctx->l_elo, &ctx->l_gf,
                      &ctx->l_grad, &ctx->l_gqst, &ctx->l_gvdw, &ctx->l_spc, &ctx->l_ismol, &ctx->l_ihe,
                      &ctx->d_flags, &ctx->d_ileft, &ctx->d_iright, &ctx->d_idx, &ctx->d_counts, &ctx->d_offs,
-                     &ctx->d_total, &ctx->d_hist, &ctx->d_nkeep, &ctx->d_wing, &ctx->d_core, &ctx->d_hdr, &ctx->d_hdr64,
-                     &ctx->d_tlo, &ctx->d_thi, &ctx->d_err, &ctx->d_ncore, &ctx->d_span, &ctx->d_linstr, &ctx->d_rflags, &ctx->d_rleft, &ctx->d_rright, &ctx->d_gkappa, &ctx->d_adjwork, &ctx->d_cbuf, &ctx->d_ctaps, &ctx->d_p64, &ctx->d_lstart, &ctx->d_lstop, &ctx->d_widx,
+                     &ctx->d_total, &ctx->d_hist, &ctx->d_nkeep, &ctx->d_block, &ctx->d_wing, &ctx->d_core, &ctx->d_hdr, &ctx->d_hdr64,
+                     &ctx->d_tlo, &ctx->d_thi, &ctx->d_res, &ctx->d_span, &ctx->d_linstr, &ctx->d_rflags, &ctx->d_rleft, &ctx->d_rright, &ctx->d_gkappa, &ctx->d_adjwork, &ctx->d_cbuf, &ctx->d_ctaps, &ctx->d_p64, &ctx->d_lstart, &ctx->d_lstop, &ctx->d_widx,
                      &ctx->d_pw, &ctx->d_spl, &ctx->d_spc, &ctx->d_sfl, &ctx->d_sfc,
                      &ctx->d_work, &ctx->d_a, &ctx->d_v, &ctx->d_h, &ctx->d_l, &ctx->z_npi, &ctx->z_nsi,
                      &ctx->z_pioff, &ctx->z_sioff, &ctx->z_splpi, &ctx->z_strpi, &ctx->z_splsi, &ctx->z_strsi,
@@ -729,8 +731,9 @@ static int rows64(fsg_ctx *ctx, const AtmView &A, const LineView &LV, const int6
 // (1..nwl for the whole grid).  Lines are classed by their full windows and evaluated over the part
 // of the window inside the range, so each wavelength of the range sums the same lines in the same
 // order as in a whole-grid run.
-static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, fsg_stats *st, const int32_t *fl, const int32_t *il,
-                           const int32_t *ir, int i0, int i1) {
+// nmax: no more lines than these are retained (the retained count where it is known, else n).
+static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, int64_t nmax, fsg_stats *st, const int32_t *fl,
+                           const int32_t *il, const int32_t *ir, int i0, int i1) {
     int64_t n = LV.n;
     const int nt = ctx->ntau;
     AtmView A = fsg_view(ctx);
@@ -745,90 +748,150 @@ static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, fsg_stats *st, cons
         ctx->launches += 1;
         sf = ctx->d_rflags.as<int32_t>(); wl_ = ctx->d_rleft.as<int32_t>(); wr_ = ctx->d_rright.as<int32_t>();
     }
-    ALLOC(ctx->d_hist, sizeof(unsigned long long) * 32);
-    CK(cudaMemsetAsync(ctx->d_hist.p, 0, sizeof(unsigned long long) * 32, s), "hist");
-    fsg_launch_class_hist(s, n, sf, il, ir, ctx->d_hist.as<unsigned long long>());
-    ctx->launches += 1;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> kt, kc;   // wing pass, core pass
     size_t kev_used = 0;
     auto kevent = [&]() -> cudaEvent_t {
         if (kev_used == ctx->kev.size()) { cudaEvent_t e; cudaEventCreate(&e); ctx->kev.push_back(e); }
         return ctx->kev[kev_used++];
     };
-    unsigned long long hist[32];
-    CK(cudaMemcpyAsync(hist, ctx->d_hist.p, sizeof hist, cudaMemcpyDeviceToHost, s), "hist");
-    CK(cudaStreamSynchronize(s), "hist");
-    if (st) {                                          // lines evaluated (those meeting the range)
-        int64_t nsel = 0;
-        for (int c = 0; c < 32; c++) nsel += (int64_t)hist[c];
-        st->nlines_used = nsel;
-    }
-    int64_t nblkscan = (n + 1023) / 1024;
-    ALLOC(ctx->d_counts, sizeof(int) * std::max<int64_t>(nblkscan, 1));
-    ALLOC(ctx->d_offs, sizeof(int64_t) * std::max<int64_t>(nblkscan, 1));
-    ALLOC(ctx->d_total, sizeof(int64_t));
-    ALLOC(ctx->d_idx, sizeof(int64_t) * std::max<int64_t>(n, 1));
-    int ntiles = fsg_fast_tiles(ctx->nwl);
-    ALLOC(ctx->d_tlo, sizeof(int) * ntiles); ALLOC(ctx->d_thi, sizeof(int) * ntiles);
-    ALLOC(ctx->d_err, sizeof(int));
-    CK(cudaMemsetAsync(ctx->d_err.p, 0, sizeof(int), s), "err reset");
-    ALLOC(ctx->d_ncore, sizeof(unsigned long long));
-    CK(cudaMemsetAsync(ctx->d_ncore.p, 0, sizeof(unsigned long long), s), "core count reset");
+    const int64_t nblkscan = std::max<int64_t>((n + 1023) / 1024, 1);
     const size_t npair = wing_pairs(nt);
-    size_t per_line = npair * sizeof(WingPair) + (size_t)nt * sizeof(CoreRec) + sizeof(LineHdr);
-    int64_t cap = block_capacity(ctx, per_line);
-    int64_t nblocks = 0;
-    for (int c = 0; c < 32; c++) {
-        if (!hist[c]) continue;
-        int rc = fsg_select(s, n, sf, il, ir, c,
-                            ctx->d_counts.as<int>(), ctx->d_offs.as<int64_t>(), ctx->d_idx.as<int64_t>(),
-                            ctx->d_total.as<int64_t>());
-        if (rc) return cuda_fail(ctx, cudaGetLastError(), "select");
-        ctx->launches += 3;
-        int64_t nc = (int64_t)hist[c];
-        // blocks of at most cap lines (LIMITRAM); block b takes every nblk-th line of the class from
-        // its b-th, so each block is sorted by wavelength and spans the whole grid: every tile of a
-        // launch has work, however small the blocks
-        const int64_t nblk = (nc + cap - 1) / cap;
-        const int64_t bcap = (nc + nblk - 1) / nblk;
-        ALLOC(ctx->d_wing, sizeof(WingPair) * (size_t)bcap * npair);
-        ALLOC(ctx->d_core, sizeof(CoreRec) * (size_t)bcap * nt);
-        ALLOC(ctx->d_hdr, sizeof(LineHdr) * (size_t)bcap);
-        ALLOC(ctx->d_span, fsg_tile_span_scratch(bcap));
-        for (int64_t b = 0; b < nblk; b++) {
-            const int64_t nb = (nc - b + nblk - 1) / nblk;
-            fsg_launch_params_fast(s, A, LV, ctx->d_idx.as<int64_t>(), b, nblk, nb, fl, wl_, wr_, ctx->tab,
-                                   ctx->d_wing.as<WingPair>(), ctx->d_core.as<CoreRec>(), ctx->d_hdr.as<LineHdr>());
-            if (fsg_launch_tile_span(s, c, ctx->nwl, nb, ctx->d_hdr.as<LineHdr>(), ctx->d_tlo.as<int>(),
-                                     ctx->d_thi.as<int>(), ctx->d_span.p, ctx->d_span.cap))
-                return cuda_fail(ctx, cudaGetLastError(), "tile span");
-            cudaEvent_t ea = kevent(), em = kevent(), eb = kevent();
-            cudaEventRecord(ea, s);
-            int rc2 = fsg_launch_accum_fast(s, c, nt, ctx->nwl, ctx->d_wave.as<double>(), ctx->d_hdr.as<LineHdr>(),
-                                            ctx->d_wing.as<WingPair>(), ctx->d_tlo.as<int>(), ctx->d_thi.as<int>(),
-                                            ctx->d_lineopac.as<double>());
-            if (rc2) return cuda_fail(ctx, cudaGetLastError(), "k_accum_fast");
-            cudaEventRecord(em, s);
-            // core ranges of the same lines, 32-wavelength tiles
-            if (fsg_launch_tile_span(s, -1, ctx->nwl, nb, ctx->d_hdr.as<LineHdr>(), ctx->d_tlo.as<int>(),
-                                     ctx->d_thi.as<int>(), ctx->d_span.p, ctx->d_span.cap))
-                return cuda_fail(ctx, cudaGetLastError(), "core tile span");
-            rc2 = fsg_launch_core_fast(s, nt, ctx->nwl, ctx->d_wave.as<double>(), ctx->d_hdr.as<LineHdr>(),
-                                       ctx->d_core.as<CoreRec>(), ctx->d_tlo.as<int>(), ctx->d_thi.as<int>(),
-                                       ctx->tab.vtab4, ctx->d_lineopac.as<double>(),
-                                       ctx->d_ncore.as<unsigned long long>(), ctx->d_err.as<int>(),
-                                       ctx->fault_extra_tx, ctx->fault_wait_ns);
-            if (rc2) return cuda_fail(ctx, cudaGetLastError(), "k_core_fast");
-            cudaEventRecord(eb, s);
-            kt.push_back({ ea, em });
-            kc.push_back({ em, eb });
-            ctx->launches += 16;   // params, 2 x (extract, 2 scans of 2 kernels, search), count, wing, core
-            nblocks++;
+    const size_t per_line = npair * sizeof(WingPair) + (size_t)nt * sizeof(CoreRec) + sizeof(LineHdr);
+    const int64_t cap = block_capacity(ctx, per_line);
+    // the counts read back at the end: error word, core evaluations, selected lines, window wavelengths
+    struct Result { unsigned long long err, ncore, nsel, npix; } res{};
+    ALLOC(ctx->d_res, sizeof(Result));
+    Result *dres = ctx->d_res.as<Result>();
+    CK(cudaMemsetAsync(dres, 0, sizeof(Result), s), "result reset");
+    int64_t nblocks = 0, nsel = 0;
+    LineHdr *hdr = nullptr; WingPair *wing = nullptr; CoreRec *core = nullptr;      // the block's records
+    auto wing_job = [&](const int *tlo, const int *thi, int nseg, int stride) {
+        return WingJob{ nt, ctx->nwl, ctx->d_wave.as<double>(), hdr, wing, tlo, thi, ctx->d_lineopac.as<double>(), nseg,
+                        stride, 1 };
+    };
+    auto core_job = [&](const int *tlo, const int *thi, int nseg, int stride) {
+        return CoreJob{ nt, ctx->nwl, ctx->d_wave.as<double>(), hdr, core, tlo, thi, ctx->d_lineopac.as<double>(),
+                        &dres->ncore, ctx->fault_extra_tx, ctx->fault_wait_ns, nseg, stride };
+    };
+    // A list whose records fit one block (LIMITRAM) is one record array in window-width-class order: one launch
+    // per step for all classes, each tile adding its classes in turn, and no count needed on the host.  Lists that
+    // do not fit take the classes one by one, in blocks.
+    const int ncls = fsg_bclass_count(ctx->nwl);
+    const int ws = (ctx->nwl + 63) / 64, cs = (ctx->nwl + 31) / 32;
+    bool one = nmax <= cap && nmax > 0;
+    int *counts = nullptr, *wlo = nullptr, *whi = nullptr, *clo = nullptr, *chi = nullptr;
+    int64_t *offs = nullptr, *total = nullptr, *order = nullptr;
+    char *span = nullptr;
+    const size_t span_bytes = one ? fsg_bspan_scratch(nmax) : 0;
+    if (one) {
+        // one allocation, its parts on 256-byte boundaries
+        size_t bytes = 0;
+        auto part = [&](size_t nb) { const size_t o = bytes; bytes += (nb + 255) & ~(size_t)255; return o; };
+        const size_t nsc = (size_t)(ncls + 1) * nblkscan;
+        const size_t o_wing = part(sizeof(WingPair) * (size_t)nmax * npair), o_core = part(sizeof(CoreRec) * (size_t)nmax * nt);
+        const size_t o_hdr = part(sizeof(LineHdr) * (size_t)nmax), o_order = part(sizeof(int64_t) * (size_t)n);
+        const size_t o_counts = part(sizeof(int) * nsc), o_offs = part(sizeof(int64_t) * nsc), o_total = part(sizeof(int64_t));
+        const size_t o_w = part(sizeof(int) * 2 * (size_t)ncls * ws), o_c = part(sizeof(int) * 2 * (size_t)ncls * cs);
+        const size_t o_span = part(span_bytes);
+        one = !(ctx->fault_alloc && bytes > ctx->fault_alloc && ctx->d_block.cap < bytes) && ctx->d_block.ensure(bytes) == FSG_OK;
+        char *p = ctx->d_block.as<char>();
+        wing = (WingPair *)(p + o_wing); core = (CoreRec *)(p + o_core); hdr = (LineHdr *)(p + o_hdr);
+        order = (int64_t *)(p + o_order); counts = (int *)(p + o_counts); offs = (int64_t *)(p + o_offs);
+        total = (int64_t *)(p + o_total);
+        wlo = (int *)(p + o_w); whi = wlo + (size_t)ncls * ws;
+        clo = (int *)(p + o_c); chi = clo + (size_t)ncls * cs;
+        span = p + o_span;
+    }
+    if (one) {
+        if (fsg_launch_bclass_order(s, n, sf, il, ir, ncls, counts, offs, total, order))
+            return cuda_fail(ctx, cudaGetLastError(), "class order");
+        CK(cudaMemcpyAsync(&dres->nsel, offs + (size_t)ncls * nblkscan, sizeof(int64_t), cudaMemcpyDeviceToDevice, s),
+           "selected lines");
+        fsg_launch_params_fast(s, A, LV, order, 0, 1, nmax, fl, wl_, wr_, ctx->tab, wing, core, hdr);
+        if (fsg_launch_btile_span(s, nmax, hdr, offs, (int)nblkscan, ncls, WING_NARROW, 64, 128, ctx->nwl, ws, wlo, whi, cs,
+                                  clo, chi, span, span_bytes))
+            return cuda_fail(ctx, cudaGetLastError(), "tile span");
+        cudaEvent_t ea = kevent(), em = kevent(), eb = kevent();
+        cudaEventRecord(ea, s);
+        const int nn = std::min(ncls, WING_NARROW + 1);
+        if (fsg_launch_accum_fast(s, 2, wing_job(wlo, whi, nn, ws)) ||
+            (ncls > nn && fsg_launch_accum_fast(s, 4, wing_job(wlo + (size_t)nn * ws, whi + (size_t)nn * ws, ncls - nn, ws))))
+            return cuda_fail(ctx, cudaGetLastError(), "k_accum_fast");
+        cudaEventRecord(em, s);
+        if (fsg_launch_core_fast(s, core_job(clo, chi, ncls, cs), ctx->tab.vtab4, (int *)&dres->err))
+            return cuda_fail(ctx, cudaGetLastError(), "k_core_fast");
+        cudaEventRecord(eb, s);
+        kt.push_back({ ea, em });
+        kc.push_back({ em, eb });
+        ctx->launches += ncls > nn ? 13 : 12;            // order 3, params, spans 6, wing 1 or 2, core
+        nblocks = 1;
+    } else if (nmax > 0) {
+        ALLOC(ctx->d_hist, sizeof(unsigned long long) * 32);
+        CK(cudaMemsetAsync(ctx->d_hist.p, 0, sizeof(unsigned long long) * 32, s), "hist");
+        fsg_launch_class_hist(s, n, sf, il, ir, ctx->d_hist.as<unsigned long long>());
+        ctx->launches += 1;
+        unsigned long long hist[32];
+        CK(cudaMemcpyAsync(hist, ctx->d_hist.p, sizeof hist, cudaMemcpyDeviceToHost, s), "hist");
+        CK(cudaStreamSynchronize(s), "hist");
+        for (int c = 0; c < 32; c++) nsel += (int64_t)hist[c];
+        ALLOC(ctx->d_counts, sizeof(int) * nblkscan);
+        ALLOC(ctx->d_offs, sizeof(int64_t) * nblkscan);
+        ALLOC(ctx->d_total, sizeof(int64_t));
+        ALLOC(ctx->d_idx, sizeof(int64_t) * std::max<int64_t>(n, 1));
+        const int ntiles = fsg_fast_tiles(ctx->nwl);
+        ALLOC(ctx->d_tlo, sizeof(int) * ntiles); ALLOC(ctx->d_thi, sizeof(int) * ntiles);
+        for (int c = 0; c < 32; c++) {
+            if (!hist[c]) continue;
+            int rc = fsg_select(s, n, sf, il, ir, c,
+                                ctx->d_counts.as<int>(), ctx->d_offs.as<int64_t>(), ctx->d_idx.as<int64_t>(),
+                                ctx->d_total.as<int64_t>());
+            if (rc) return cuda_fail(ctx, cudaGetLastError(), "select");
+            ctx->launches += 3;
+            int64_t nc = (int64_t)hist[c];
+            // blocks of at most cap lines (LIMITRAM); block b takes every nblk-th line of the class from
+            // its b-th, so each block is sorted by wavelength and spans the whole grid: every tile of a
+            // launch has work, however small the blocks
+            const int64_t nblk = (nc + cap - 1) / cap;
+            const int64_t bcap = (nc + nblk - 1) / nblk;
+            ALLOC(ctx->d_wing, sizeof(WingPair) * (size_t)bcap * npair);
+            ALLOC(ctx->d_core, sizeof(CoreRec) * (size_t)bcap * nt);
+            ALLOC(ctx->d_hdr, sizeof(LineHdr) * (size_t)bcap);
+            ALLOC(ctx->d_span, fsg_tile_span_scratch(bcap));
+            wing = ctx->d_wing.as<WingPair>(); core = ctx->d_core.as<CoreRec>(); hdr = ctx->d_hdr.as<LineHdr>();
+            for (int64_t b = 0; b < nblk; b++) {
+                const int64_t nb = (nc - b + nblk - 1) / nblk;
+                fsg_launch_params_fast(s, A, LV, ctx->d_idx.as<int64_t>(), b, nblk, nb, fl, wl_, wr_, ctx->tab, wing, core,
+                                       hdr);
+                if (fsg_launch_tile_span(s, c, ctx->nwl, nb, hdr, ctx->d_tlo.as<int>(),
+                                         ctx->d_thi.as<int>(), ctx->d_span.p, ctx->d_span.cap))
+                    return cuda_fail(ctx, cudaGetLastError(), "tile span");
+                cudaEvent_t ea = kevent(), em = kevent(), eb = kevent();
+                cudaEventRecord(ea, s);
+                if (fsg_launch_accum_fast(s, fsg_class_pix(c), wing_job(ctx->d_tlo.as<int>(), ctx->d_thi.as<int>(), 1, 0)))
+                    return cuda_fail(ctx, cudaGetLastError(), "k_accum_fast");
+                cudaEventRecord(em, s);
+                // core ranges of the same lines, 32-wavelength tiles
+                if (fsg_launch_tile_span(s, -1, ctx->nwl, nb, hdr, ctx->d_tlo.as<int>(),
+                                         ctx->d_thi.as<int>(), ctx->d_span.p, ctx->d_span.cap))
+                    return cuda_fail(ctx, cudaGetLastError(), "core tile span");
+                if (fsg_launch_core_fast(s, core_job(ctx->d_tlo.as<int>(), ctx->d_thi.as<int>(), 1, 0), ctx->tab.vtab4,
+                                         (int *)&dres->err))
+                    return cuda_fail(ctx, cudaGetLastError(), "k_core_fast");
+                cudaEventRecord(eb, s);
+                kt.push_back({ ea, em });
+                kc.push_back({ em, eb });
+                ctx->launches += 15;   // params, 2 x (extract, 2 scans of 2 kernels, search), wing, core
+                nblocks++;
+            }
         }
     }
     // He I lines with Stark-shifted profiles (hestark.f90): the FP64 tile kernel, which applies the
     // per-depth shift (opacity.f90:297-346)
     if (ctx->nhe > 0) {
+        ALLOC(ctx->d_counts, sizeof(int) * nblkscan);
+        ALLOC(ctx->d_offs, sizeof(int64_t) * nblkscan);
+        ALLOC(ctx->d_total, sizeof(int64_t));
+        ALLOC(ctx->d_idx, sizeof(int64_t) * std::max<int64_t>(n, 1));
         int rc3 = fsg_select(s, n, sf, il, ir, -3, ctx->d_counts.as<int>(), ctx->d_offs.as<int64_t>(),
                              ctx->d_idx.as<int64_t>(), ctx->d_total.as<int64_t>());
         if (rc3) return cuda_fail(ctx, cudaGetLastError(), "select He I lines");
@@ -845,20 +908,24 @@ static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, fsg_stats *st, cons
             ctx->launches += 1;
         }
     }
+    if (st) {
+        launch_count_windows(s, n, fl, il, ir, i0, i1, &dres->npix);
+        ctx->launches += 1;
+    }
     CK(cudaGetLastError(), "fast accumulation");
+    CK(cudaMemcpyAsync(&res, dres, sizeof res, cudaMemcpyDeviceToHost, s), "counts");
     CK(cudaStreamSynchronize(s), "fast accumulation");
-    int kerr = 0;
-    CK(cudaMemcpy(&kerr, ctx->d_err.p, sizeof(int), cudaMemcpyDeviceToHost), "err read");
-    if (kerr) return fail(ctx, FSG_E_TIMEOUT, "k_accum_fast: a line-record copy did not complete within its bound");
-    unsigned long long ncore = 0;
-    CK(cudaMemcpy(&ncore, ctx->d_ncore.p, sizeof ncore, cudaMemcpyDeviceToHost), "core count read");
+    if ((int)res.err) return fail(ctx, FSG_E_TIMEOUT, "k_core_fast: a line-record copy did not complete within its bound");
+    if (nblocks == 1 && one) nsel = (int64_t)res.nsel;
     double msw = 0.0, msc = 0.0;
     for (auto &p : kt) { float x = 0; cudaEventElapsedTime(&x, p.first, p.second); msw += x; }
     for (auto &p : kc) { float x = 0; cudaEventElapsedTime(&x, p.first, p.second); msc += x; }
     if (st) {
         st->nblocks = nblocks; st->accum_launches = (int64_t)kt.size(); st->ms_accum_kernels = msw + msc;
         st->ms_wing_kernels = msw; st->ms_core_kernels = msc;
-        st->core_evals = (double)ncore;
+        st->core_evals = (double)res.ncore;
+        st->nlines_used = nsel;                        // lines evaluated (those meeting the range)
+        st->line_evals = (double)res.npix * nt;
     }
     return FSG_OK;
 }
@@ -1072,7 +1139,7 @@ static int lineop_dev(fsg_ctx *ctx, const fsg_lines *D, fsg_stats *st, const fsg
     CK(cudaEventRecord(ctx->ev[1], s), "event");
     if (st) { st->nlines_used = nkeep; st->nweak = D->n - nkeep; }
     if (ctx->cfg.precision == FSG_PREC_FP64) rc = accumulate_fp64(ctx, LV, nkeep, st, 1, ctx->nwl);
-    else rc = accumulate_fast(ctx, LV, st, ctx->d_flags.as<int32_t>(), ctx->d_ileft.as<int32_t>(),
+    else rc = accumulate_fast(ctx, LV, nkeep, st, ctx->d_flags.as<int32_t>(), ctx->d_ileft.as<int32_t>(),
                               ctx->d_iright.as<int32_t>(), 1, ctx->nwl);
     if (rc) return rc;
     CK(cudaEventRecord(ctx->ev[2], s), "event");
@@ -1082,9 +1149,6 @@ static int lineop_dev(fsg_ctx *ctx, const fsg_lines *D, fsg_stats *st, const fsg
         cudaEventElapsedTime(&a, ctx->ev[0], ctx->ev[1]);
         cudaEventElapsedTime(&b, ctx->ev[1], ctx->ev[2]);
         st->ms_center = a; st->ms_accum = b; st->ms_total = a + b;
-        if (ctx->cfg.precision != FSG_PREC_FP64)
-            st->line_evals = fsg_count_evals(ctx, D->n, ctx->d_flags.as<int32_t>(), ctx->d_ileft.as<int32_t>(),
-                                             ctx->d_iright.as<int32_t>(), 1, ctx->nwl);
     }
     return FSG_OK;
 }
@@ -1133,7 +1197,7 @@ int fsg_accumulate_dev(fsg_ctx *ctx, const fsg_lines *d_lines, const int32_t *d_
         CK(cudaMemcpyAsync(ctx->d_iright.p, d_iright, nb, cudaMemcpyDeviceToDevice, s), "windows");
         rc = accumulate_fp64(ctx, make_view(d_lines), -1, st, i0, i1);
     } else {
-        rc = accumulate_fast(ctx, make_view(d_lines), st, d_flags, d_ileft, d_iright, i0, i1);
+        rc = accumulate_fast(ctx, make_view(d_lines), d_lines->n, st, d_flags, d_ileft, d_iright, i0, i1);
     }
     if (rc) return rc;
     CK(cudaEventRecord(ctx->ev[2], s), "event");
@@ -1142,8 +1206,6 @@ int fsg_accumulate_dev(fsg_ctx *ctx, const fsg_lines *d_lines, const int32_t *d_
         float b = 0;
         cudaEventElapsedTime(&b, ctx->ev[1], ctx->ev[2]);
         st->ms_accum = b; st->ms_total = b;
-        if (ctx->cfg.precision != FSG_PREC_FP64)
-            st->line_evals = fsg_count_evals(ctx, d_lines->n, d_flags, d_ileft, d_iright, i0, i1);
     }
     return FSG_OK;
 }
@@ -2353,7 +2415,6 @@ static LineView batch_view(const fsg_batch *b, const BAtm &a) {
 
 // Wing tiles: 64 wavelengths for the two narrowest window classes (windows up to 512), 32 * P for
 // the others; core tiles: 32 wavelengths.  Tile arrays hold ncls rows of tstride entries.
-static const int BATCH_NARROW = 1;             // classes 0 .. BATCH_NARROW take the narrow tiles
 static int batch_wing_stride(const fsg_ctx *c) { return (c->nwl + 63) / 64; }
 static int batch_core_stride(const fsg_ctx *c) { return (c->nwl + 31) / 32; }
 
@@ -2393,11 +2454,9 @@ static int batch_prepare(fsg_batch *b, int P) {
         fsg_launch_params_fast(s, A, LV, a.order.as<int64_t>(), 0, 1, a.cn, a.flags.as<int32_t>(), a.il.as<int32_t>(),
                                a.ir.as<int32_t>(), c->tab, a.wing.as<WingPair>(), a.core.as<CoreRec>(),
                                a.hdr.as<LineHdr>());
-        if (fsg_launch_btile_span(s, 0, a.cn, a.hdr.as<LineHdr>(), a.coff.as<int64_t>(), a.ncls, BATCH_NARROW, 64,
-                                  32 * P, c->nwl, batch_wing_stride(c), a.wtlo.as<int>(), a.wthi.as<int>(), a.span.p,
-                                  a.span.cap) ||
-            fsg_launch_btile_span(s, 1, a.cn, a.hdr.as<LineHdr>(), a.coff.as<int64_t>(), a.ncls, a.ncls, 32, 32,
-                                  c->nwl, batch_core_stride(c), a.ctlo.as<int>(), a.cthi.as<int>(), a.span.p,
+        if (fsg_launch_btile_span(s, a.cn, a.hdr.as<LineHdr>(), a.coff.as<int64_t>(), (int)((a.cn + 1023) / 1024), a.ncls,
+                                  WING_NARROW, 64, 32 * P, c->nwl, batch_wing_stride(c), a.wtlo.as<int>(),
+                                  a.wthi.as<int>(), batch_core_stride(c), a.ctlo.as<int>(), a.cthi.as<int>(), a.span.p,
                                   a.span.cap))
         {
             const cudaError_t e = cudaGetLastError();
@@ -2434,14 +2493,14 @@ static int batch_jobs(fsg_batch *b, int P) {
             for (auto &a : b->atm) {
                 fsg_ctx *c = a.ctx;
                 if (a.cn == 0 || (c->ntau - 1) / 8 != bucket) continue;
-                const int c0 = kind == 1 ? BATCH_NARROW + 1 : 0;
-                const int nseg = kind == 0 ? std::min(a.ncls, BATCH_NARROW + 1) : kind == 1 ? a.ncls - c0 : a.ncls;
+                const int c0 = kind == 1 ? WING_NARROW + 1 : 0;
+                const int nseg = kind == 0 ? std::min(a.ncls, WING_NARROW + 1) : kind == 1 ? a.ncls - c0 : a.ncls;
                 if (nseg <= 0) continue;
                 const int ws = batch_wing_stride(c), cs = batch_core_stride(c);
                 if (kind < 2) {
                     jw.push_back(WingJob{ c->ntau, c->nwl, c->d_wave.as<double>(), a.hdr.as<LineHdr>(),
                                           a.wing.as<WingPair>(), a.wtlo.as<int>() + (size_t)c0 * ws,
-                                          a.wthi.as<int>() + (size_t)c0 * ws, c->d_lineopac.as<double>(), nseg, ws });
+                                          a.wthi.as<int>() + (size_t)c0 * ws, c->d_lineopac.as<double>(), nseg, ws, 0 });
                     t0.push_back(t0.back() + (c->nwl + 32 * Pk - 1) / (32 * Pk) * fsg_wing_groups(Pk, c->ntau));
                 } else {
                     jc.push_back(CoreJob{ c->ntau, c->nwl, c->d_wave.as<double>(), a.hdr.as<LineHdr>(),
@@ -2899,19 +2958,21 @@ __global__ void k_count_evals(int64_t n, const int32_t *flags, const int32_t *il
     if ((threadIdx.x & 31) == 0 && v) atomicAdd(acc, v);
 }
 
-double fsg_count_evals(fsg_ctx *ctx, int64_t n, const int32_t *fl, const int32_t *il, const int32_t *ir, int i0,
-                       int i1) {
-    return count_windows(ctx, n, fl, il, ir, i0, i1) * ctx->ntau;
+// adds to *acc (device) the retained-window wavelengths (inside [i0, i1]) of n lines, times their Zeeman
+// components when given
+static void launch_count_windows(cudaStream_t s, int64_t n, const int32_t *fl, const int32_t *il, const int32_t *ir,
+                                 int i0, int i1, unsigned long long *acc, const int32_t *npi, const int32_t *nsi) {
+    k_count_evals<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, fl, il, ir, i0, i1, npi, nsi, acc);
 }
 
-// retained-window wavelengths (inside [i0, i1]) of n lines, times their Zeeman components when given
+// the same, read back
 static double count_windows(fsg_ctx *ctx, int64_t n, const int32_t *fl, const int32_t *il, const int32_t *ir, int i0,
                             int i1, const int32_t *npi, const int32_t *nsi) {
     if (ctx->d_nkeep.ensure(sizeof(unsigned long long)) != FSG_OK) return 0.0;
     ctx->launches += 1;
     unsigned long long *d = ctx->d_nkeep.as<unsigned long long>();
     cudaMemsetAsync(d, 0, sizeof(unsigned long long), ctx->stream);
-    k_count_evals<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(n, fl, il, ir, i0, i1, npi, nsi, d);
+    launch_count_windows(ctx->stream, n, fl, il, ir, i0, i1, d, npi, nsi);
     unsigned long long h = 0;
     cudaMemcpyAsync(&h, d, sizeof h, cudaMemcpyDeviceToHost, ctx->stream);
     cudaStreamSynchronize(ctx->stream);

@@ -143,6 +143,20 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
         nnext = 0;
         return n;
     };
+    auto fold = [&]() {                                 // the partials into the Kahan pairs
+        nfold = 0;
+#pragma unroll
+        for (int j = 0; j < NP; j++)
+#pragma unroll
+            for (int k = 0; k < P; k++) {
+                float2 s0 = S.ksum[2 * (j * P + k)][lane], s1 = S.ksum[2 * (j * P + k) + 1][lane];
+                KAHAN(s0.x, s0.y, part[j][k].x);
+                KAHAN(s1.x, s1.y, part[j][k].y);
+                S.ksum[2 * (j * P + k)][lane] = s0;
+                S.ksum[2 * (j * P + k) + 1][lane] = s1;
+                part[j][k] = make_float2(0.0f, 0.0f);
+            }
+    };
     auto work = [&](int n) {
         for (int q = 0; q < n; q++) {
             const float4 h = S.hdr[q];
@@ -186,20 +200,7 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
                     }
                 }
             }
-            if (++nfold == FOLD) {
-                nfold = 0;
-#pragma unroll
-                for (int j = 0; j < NP; j++)
-#pragma unroll
-                    for (int k = 0; k < P; k++) {
-                        float2 s0 = S.ksum[2 * (j * P + k)][lane], s1 = S.ksum[2 * (j * P + k) + 1][lane];
-                        KAHAN(s0.x, s0.y, part[j][k].x);
-                        KAHAN(s1.x, s1.y, part[j][k].y);
-                        S.ksum[2 * (j * P + k)][lane] = s0;
-                        S.ksum[2 * (j * P + k) + 1][lane] = s1;
-                        part[j][k] = make_float2(0.0f, 0.0f);
-                    }
-            }
+            if (++nfold == FOLD) fold();
         }
     };
     int head = 0, cnt = 0;
@@ -229,6 +230,11 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
             cnt += __popc(m);
             __syncwarp();
             while (cnt >= WING_G) advance(WING_G);
+        }
+        if (J.fold_seg) {                               // this segment's lines end here
+            if (cnt) advance(cnt);
+            if (nnext) work(stage());
+            if (nfold) fold();
         }
     }
     if (cnt) advance(cnt);
@@ -294,11 +300,10 @@ int fsg_class_pix(int cls) { return cls <= 1 ? 2 : 4; }
 // depth groups of the wing pass
 int fsg_wing_groups(int P, int ntau) { return (ntau + WING_D(P) - 1) / WING_D(P); }
 
-int fsg_launch_accum_fast(cudaStream_t st, int cls, int ntau, int nwl, const double *wave, const LineHdr *hdr,
-                          const WingPair *wing, const int *tile_lo, const int *tile_hi, double *lineopac) {
-    const int P = fsg_class_pix(cls), TW = 32 * P, ntiles = (nwl + TW - 1) / TW;
-    const unsigned grid = (unsigned)(((int64_t)ntiles * fsg_wing_groups(P, ntau) + WING_W - 1) / WING_W);
-    WingJob J{ ntau, nwl, wave, hdr, wing, tile_lo, tile_hi, lineopac, 1, 0 };
+// the wing pass of one job on tiles of 32 P wavelengths
+int fsg_launch_accum_fast(cudaStream_t st, int P, const WingJob &J) {
+    const int TW = 32 * P, ntiles = (J.nwl + TW - 1) / TW;
+    const unsigned grid = (unsigned)(((int64_t)ntiles * fsg_wing_groups(P, J.ntau) + WING_W - 1) / WING_W);
     if (P == 2) k_accum_fast<WING_D(2), 2><<<grid, 32 * WING_W, 0, st>>>(J, ntiles);
     else k_accum_fast<WING_D(4), 4><<<grid, 32 * WING_W, 0, st>>>(J, ntiles);
     return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
@@ -483,7 +488,6 @@ template <int D>
 __global__ void __launch_bounds__(32 * 18, D == 4 ? 2 : 1)
 k_core_fast(CoreJob J, const float4 *__restrict__ vtab4, int chc, int *__restrict__ err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    if (J.tile_lo[blockIdx.x] > J.tile_hi[blockIdx.x]) return;
     core_bars_init(smem_raw, J.ntau, chc);
     unsigned kk = 0;
     core_tile<D>(J, blockIdx.x, vtab4, smem_raw, J.ntau, chc, kk, err);
@@ -524,15 +528,12 @@ static int core_chunk(int ntau_max) {
 // longer on the 1e8-line step)
 static int core_depths(int) { return 8; }
 
-int fsg_launch_core_fast(cudaStream_t st, int ntau, int nwl, const double *wave, const LineHdr *hdr,
-                         const CoreRec *core, const int *tile_lo, const int *tile_hi, const float4 *vtab4, double *lineopac, unsigned long long *nevals, int *err,
-                         unsigned extra_tx, unsigned long long wait_ns) {
-    const int ntiles = (nwl + 31) / 32;
-    const int D = core_depths(ntau), nwarps = (ntau + D - 1) / D;
+int fsg_launch_core_fast(cudaStream_t st, const CoreJob &J, const float4 *vtab4, int *err) {
+    const int ntiles = (J.nwl + 31) / 32;
+    const int D = core_depths(J.ntau), nwarps = (J.ntau + D - 1) / D;
     if (nwarps > 18) return FSG_E_ARG;
-    const int chc = core_chunk(ntau);
-    const size_t smem = core_smem(ntau, chc);
-    CoreJob J{ ntau, nwl, wave, hdr, core, tile_lo, tile_hi, lineopac, nevals, extra_tx, wait_ns, 1, 0 };
+    const int chc = core_chunk(J.ntau);
+    const size_t smem = core_smem(J.ntau, chc);
     if (D == 4) {
         cudaFuncSetAttribute(k_core_fast<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_core_fast<4><<<ntiles, 32 * nwarps, smem, st>>>(J, vtab4, chc, err);
@@ -796,17 +797,18 @@ int fsg_select_wide(cudaStream_t s, int64_t n, const int32_t *flags, int *counts
     return fsg_select(s, n, flags, flags, flags, -2, counts, offs, out, d_total);
 }
 
-// ---- batched lists: records in window-width-class order --------------------------------------
-// An atmosphere of a batch keeps its candidate lines in one record array, grouped by window-width
+// ---- records in window-width-class order -------------------------------------------------------
+// A list that fits one block (an atmosphere of a batch, or a single synthesis) is one record array, grouped by window-width
 // class (retained lines of class 0, 1, ..., ncls - 1, then the rejected ones), in list (wavelength)
 // order inside each class.  A tile's candidate range is then searched inside one class, so it spans
 // lines of like width only: the prefix-max / suffix-min spans of a single list with a few very wide
 // windows would stage every line between such a window's centre and the tile.
 #define BCLS_MAX 24
 
-// class of a line for the record order: ncls for rejected lines (and empty windows)
+// class of a line for the record order: ncls for rejected lines, empty windows and He I lines with a Stark shift
+// per depth (which the FP32 classes leave out)
 __device__ __forceinline__ int bclass_of(int f, int il, int ir, int ncls) {
-    if ((f & FSG_F_WEAK) || il > ir) return ncls;
+    if ((f & FSG_F_WEAK) || il > ir || ((f >> 8) & 255)) return ncls;
     return min(width_class(il, ir), ncls - 1);
 }
 
@@ -864,70 +866,83 @@ int fsg_bclass_count(int nwl) {
     return std::min(c + 1, BCLS_MAX);
 }
 
-// Segmented spans: key = class << 32 | value, so one prefix max (of right + 1) and one suffix min
-// (of left) over the whole record array stay inside each class, and both key arrays are sorted.
-__global__ void k_bspan_extract(int nb, int use_core, const LineHdr *__restrict__ hdr,
-                                const int64_t *__restrict__ offs, int nblk, int ncls, unsigned long long *right,
-                                unsigned long long *rev_left) {
+// Segmented spans of the wing pass (windows) and of the core pass (core ranges) in one array of 2 nb keys,
+// the core's after the wing's: key = (pass * BCLS_PASS + class) << 32 | value, so one prefix max (of right + 1)
+// and one suffix min (of left) over the whole array stay inside each pass and class, and both key arrays are
+// sorted.
+#define BCLS_PASS 32
+__global__ void k_bspan_extract(int nb, const LineHdr *__restrict__ hdr, const int64_t *__restrict__ offs, int nblk,
+                                int ncls, unsigned long long *right, unsigned long long *rev_left) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nb) return;
     int seg = 0;
-    while (seg < ncls && offs[(seg + 1) * nblk] <= j) seg++;
-    int l, r;
-    span_of(hdr[j], use_core, &l, &r);
-    if (seg == ncls) { l = 0x7fffffff; r = -1; }
-    right[j] = ((unsigned long long)seg << 32) | (unsigned)(r + 1);
-    rev_left[nb - 1 - j] = ((unsigned long long)seg << 32) | (unsigned)l;
+    while (seg < ncls && offs[(size_t)(seg + 1) * nblk] <= j) seg++;
+    const LineHdr h = hdr[j];
+    for (int pass = 0; pass < 2; pass++) {
+        int l, r;
+        span_of(h, pass, &l, &r);
+        if (seg == ncls) { l = 0x7fffffff; r = -1; }
+        const unsigned long long key = (unsigned long long)(pass * BCLS_PASS + seg) << 32;
+        right[pass * nb + j] = key | (unsigned)(r + 1);
+        rev_left[2 * nb - 1 - (pass * nb + j)] = key | (unsigned)l;
+    }
 }
 
-// Tile t of class c (blockIdx.y): tiles of tw_n wavelengths for classes <= cnarrow, tw_w for the
-// others; lo/hi at c * tstride + t are record indices of class c (lo > hi: no line touches it).
-__global__ void k_btile_search(int nb, int cnarrow, int tw_n, int tw_w, int nwl, int tstride,
+// Tile t of class c (blockIdx.y) of the wing pass (blockIdx.z = 0: tiles of tw_n wavelengths for classes <=
+// cnarrow, tw_w for the others) or the core pass (1: tiles of 32); lo/hi at c * stride + t are record indices of
+// class c (lo > hi: no line touches it).
+struct SpanOut { int *lo, *hi, stride; };
+__global__ void k_btile_search(int nb, int cnarrow, int tw_n, int tw_w, int nwl,
                                const unsigned long long *__restrict__ R, const unsigned long long *__restrict__ V,
-                               int *lo, int *hi) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
-    const int tw = c <= cnarrow ? tw_n : tw_w;
+                               SpanOut wing, SpanOut core) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y, pass = blockIdx.z;
+    const int tw = pass ? 32 : c <= cnarrow ? tw_n : tw_w;
     if (t >= (nwl + tw - 1) / tw) return;
-    const int f = t * tw + 1, l = min(t * tw + tw, nwl);
-    const unsigned long long kf = ((unsigned long long)c << 32) | (unsigned)(f + 1);
-    const unsigned long long kl = ((unsigned long long)c << 32) | (unsigned)l;
-    int a = 0, b = nb;                                   // first j with R_j >= kf
+    const SpanOut out = pass ? core : wing;
+    const int f = t * tw + 1, l = min(t * tw + tw, nwl), n = 2 * nb;
+    const unsigned long long key = (unsigned long long)(pass * BCLS_PASS + c) << 32;
+    const unsigned long long kf = key | (unsigned)(f + 1), kl = key | (unsigned)l;
+    int a = 0, b = n;                                    // first j with R_j >= kf
     while (a < b) { const int m = (a + b) >> 1; if (R[m] >= kf) b = m; else a = m + 1; }
     const int jlo = a;
-    a = 0; b = nb;                                       // first j with S_j > kl, S_j = V[nb - 1 - j]
-    while (a < b) { const int m = (a + b) >> 1; if (V[nb - 1 - m] > kl) b = m; else a = m + 1; }
-    lo[c * tstride + t] = jlo;
-    hi[c * tstride + t] = a - 1;
+    a = 0; b = n;                                        // first j with S_j > kl, S_j = V[n - 1 - j]
+    while (a < b) { const int m = (a + b) >> 1; if (V[n - 1 - m] > kl) b = m; else a = m + 1; }
+    out.lo[c * out.stride + t] = jlo - pass * nb;
+    out.hi[c * out.stride + t] = a - 1 - pass * nb;
 }
 
 size_t fsg_bspan_scratch(int64_t nb) {
     size_t t1 = 0, t2 = 0;
     typedef unsigned long long u64;
-    cub::DeviceScan::InclusiveScan(nullptr, t1, (const u64 *)nullptr, (u64 *)nullptr, cuda::maximum<>{}, (int)nb);
-    cub::DeviceScan::InclusiveScan(nullptr, t2, (const u64 *)nullptr, (u64 *)nullptr, cuda::minimum<>{}, (int)nb);
-    return 4 * sizeof(u64) * (size_t)nb + std::max(t1, t2) + 256;
+    const int n = (int)(2 * nb);
+    cub::DeviceScan::InclusiveScan(nullptr, t1, (const u64 *)nullptr, (u64 *)nullptr, cuda::maximum<>{}, n);
+    cub::DeviceScan::InclusiveScan(nullptr, t2, (const u64 *)nullptr, (u64 *)nullptr, cuda::minimum<>{}, n);
+    return 4 * sizeof(u64) * (size_t)n + std::max(t1, t2) + 256;
 }
 
-// tile ranges of every class of a class-ordered record array (offs from fsg_launch_bclass_order)
-int fsg_launch_btile_span(cudaStream_t s, int use_core, int64_t nb, const LineHdr *hdr, const int64_t *offs,
-                          int ncls, int cnarrow, int tw_n, int tw_w, int nwl, int tstride, int *lo, int *hi,
-                          void *scratch, size_t scratch_bytes) {
+// tile ranges of every class of a class-ordered record array, both passes (offs: class c starts at record
+// offs[c * nblk], as fsg_launch_bclass_order leaves them); wing and core arrays hold ncls rows of wstride /
+// cstride entries
+int fsg_launch_btile_span(cudaStream_t s, int64_t nb, const LineHdr *hdr, const int64_t *offs, int nblk, int ncls,
+                          int cnarrow, int tw_n, int tw_w, int nwl, int wstride, int *wlo, int *whi, int cstride, int *clo,
+                          int *chi, void *scratch, size_t scratch_bytes) {
     typedef unsigned long long u64;
     if (nb <= 0) {
-        for (int c = 0; c < ncls; c++) k_tile_reset<<<(tstride + 255) / 256, 256, 0, s>>>(tstride, lo + c * tstride,
-                                                                                          hi + c * tstride);
+        k_tile_reset<<<(wstride * ncls + 255) / 256, 256, 0, s>>>(wstride * ncls, wlo, whi);
+        k_tile_reset<<<(cstride * ncls + 255) / 256, 256, 0, s>>>(cstride * ncls, clo, chi);
         return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
     }
-    const int nblk = (int)((nb + SCAN_BS - 1) / SCAN_BS);
-    u64 *right = (u64 *)scratch, *revl = right + nb, *R = revl + nb, *V = R + nb;
-    void *tmp = (void *)(((uintptr_t)(V + nb) + 255) & ~(uintptr_t)255);
+    const int n = (int)(2 * nb);
+    u64 *right = (u64 *)scratch, *revl = right + n, *R = revl + n, *V = R + n;
+    void *tmp = (void *)(((uintptr_t)(V + n) + 255) & ~(uintptr_t)255);
     size_t tb = scratch_bytes - ((char *)tmp - (char *)scratch);
-    k_bspan_extract<<<(unsigned)((nb + 255) / 256), 256, 0, s>>>((int)nb, use_core, hdr, offs, nblk, ncls, right, revl);
-    if (cub::DeviceScan::InclusiveScan(tmp, tb, right, R, cuda::maximum<>{}, (int)nb, s) != cudaSuccess) return FSG_E_CUDA;
-    if (cub::DeviceScan::InclusiveScan(tmp, tb, revl, V, cuda::minimum<>{}, (int)nb, s) != cudaSuccess) return FSG_E_CUDA;
-    const int tmax = (nwl + std::min(tw_n, tw_w) - 1) / std::min(tw_n, tw_w);
-    k_btile_search<<<dim3((tmax + 255) / 256, ncls), 256, 0, s>>>((int)nb, cnarrow, tw_n, tw_w, nwl, tstride, R, V,
-                                                                  lo, hi);
+    k_bspan_extract<<<(unsigned)((nb + 255) / 256), 256, 0, s>>>((int)nb, hdr, offs, nblk, ncls, right, revl);
+    if (cub::DeviceScan::InclusiveScan(tmp, tb, right, R, cuda::maximum<>{}, n, s) != cudaSuccess) return FSG_E_CUDA;
+    if (cub::DeviceScan::InclusiveScan(tmp, tb, revl, V, cuda::minimum<>{}, n, s) != cudaSuccess) return FSG_E_CUDA;
+    const int tmax = (nwl + 31) / 32;
+    k_btile_search<<<dim3((tmax + 255) / 256, ncls, 2), 256, 0, s>>>((int)nb, cnarrow, tw_n, tw_w, nwl, R, V,
+                                                                     SpanOut{ wlo, whi, wstride },
+                                                                     SpanOut{ clo, chi, cstride });
     return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }
 

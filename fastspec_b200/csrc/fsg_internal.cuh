@@ -132,6 +132,8 @@ struct WingJob {
     const int *tile_lo, *tile_hi;
     double *lineopac;
     int nseg, seg_stride;
+    int fold_seg;                        // the FP32 partials end with each segment (a class's sum does not depend on
+                                         // the others')
 };
 
 // One core-pass job: as WingJob with the core records; tiles of 32 wavelengths.  nevals (may be

@@ -168,7 +168,7 @@ void fsg_launch_xline_init(cudaStream_t s, int nt, const double *T, const double
 }
 
 // ================================================================================================
-// Central pass (synth.f90:833-907).  One thread per line and one sweep over depth: XlineDepth once per
+// Central pass (synth.f90:833-907).  One sweep over depth: XlineDepth once per
 // depth feeds the LinCop bound test against the continuum, the single-line opacity at the line centre
 // (LineOpacity2) and AnalyticWindow; no Ntau-long arrays are held.
 // ================================================================================================
@@ -176,66 +176,103 @@ __device__ __forceinline__ double center_shift(const AtmView &A, int ihe, int t)
     return (ihe > 0) ? A.heshf[(ihe - 1) * A.ntau + t] : 0.0;
 }
 
-// Eight 128-thread CTAs per SM (64 registers, a few spilled): the sweep is bound by the FP64 pipe,
-// and the extra resident warps hide more of its latency (177 -> 150 ms on the 1e8-line list).
+// The per-line part before the sweep and one depth of the three maxima the reference takes in turn
+// (synth.f90:876-907): (1) the upper bound LinCop / ContOpac (H(a, v) <= 1), (2) the single-line opacity at
+// the line centre (LineOpacity2 at Wl = Wlcent) and (3) the AnalyticWindow half-width (opacity.f90:678-710).
+// Each is a maximum over depths of per-depth values that do not depend on the others, so computing
+// XlineDepth once per depth for all three gives the reference's tests and windows exactly; the
+// later maxima are used only when the earlier tests keep the line.
+struct CenterLine { XCoef XC; double wlc, dW; int f, iwl; };
+__device__ __forceinline__ CenterLine center_line(const AtmView &A, const LineView &L, int64_t i) {
+    CenterLine c;
+    c.f = line_input_flags(L, i, 0);
+    c.wlc = L.wl[i] - A.wfirst;
+    xline_setup(A, L, i, c.wlc, c.f, &c.XC);
+    if (c.XC.IxHe > 0) c.f |= (c.XC.IxHe << 8);
+    c.iwl = waveidx(A, c.wlc);
+    c.dW = (c.wlc - A.wave[c.iwl - 1]) / (A.wave[c.iwl] - A.wave[c.iwl - 1]);
+    return c;
+}
+__device__ __forceinline__ void center_depth(const AtmView &A, const CenterLine &c, int t, const float *__restrict__ vtab,
+                                             const double *__restrict__ anode, const double *__restrict__ aida,
+                                             double &mx1, double &mx2, double &dWwin) {
+    const double iSqrtPi = 0.5641895835477563;
+    const int ihe = c.XC.IxHe;
+    double cop, vv, av;
+    xline_depth(A, t, c.XC, &cop, &vv, &av);
+    const double co = cont_center(A, c.iwl, c.dW, t);
+    mx1 = fmax(mx1, (A.motype == 1) ? cop / (co * A.contstd[t]) : cop / co);
+    double dWl = 0.0;
+    if (ihe > 0) dWl = 0.0 - center_shift(A, ihe, t);
+    double lo = hvoigt64(vtab, anode, aida, av, dWl * vv) * cop;
+    if (A.motype == 1) lo = lo / A.contstd[t];
+    mx2 = fmax(mx2, lo / co);
+    double r = cop / (A.epsopac * co);
+    if (A.motype == 1) r = r / A.contstd[t];
+    if (r <= 1.0) return;
+    double w = sqrt(log(r) + fmax(0.0, av * (r * iSqrtPi - av))) / vv;
+    if (ihe > 0) w = w + fabs(center_shift(A, ihe, t));
+    dWwin = fmax(dWwin, w);
+}
+// flags and window of the line from the maxima; whether it is kept
+__device__ __forceinline__ bool center_result(const AtmView &A, const CenterLine &c, double mx1, double mx2, double dWwin,
+                                              int64_t i, int32_t *flags, int32_t *ileft, int32_t *iright) {
+    int f = c.f, il = 1, ir = A.nwl;
+    if (mx1 < A.epsopac || mx2 < A.epsopac) {
+        f |= FSG_F_WEAK;
+    } else {
+        il = waveidx(A, c.wlc - dWwin);                    // WaveIdx (synth.f90:904-906)
+        ir = waveidx(A, c.wlc + dWwin) + 1;
+        if (ir > A.nwl) ir = A.nwl;
+    }
+    flags[i] = f; ileft[i] = il; iright[i] = ir;
+    return !(f & FSG_F_WEAK);
+}
+
+// One thread per line.  Eight 128-thread CTAs per SM (64 registers, a few spilled): the sweep is bound by the
+// FP64 pipe, and the extra resident warps hide more of its latency (177 -> 150 ms on the 1e8-line list).
 __global__ void __launch_bounds__(128, 8) k_center(AtmView A, LineView L, const float *__restrict__ vtab,
                          const double *__restrict__ anode, const double *__restrict__ aida,
                          int32_t *flags, int32_t *ileft, int32_t *iright, unsigned long long *nkeep) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= L.n) return;
-    const int nt = A.ntau;
-    int f = line_input_flags(L, i, 0);
-    double wlc = L.wl[i] - A.wfirst;
-    XCoef XC;
-    xline_setup(A, L, i, wlc, f, &XC);
-    if (XC.IxHe > 0) f |= (XC.IxHe << 8);
-    int ihe = XC.IxHe;
-    int iwl = waveidx(A, wlc);
-    double dW = (wlc - A.wave[iwl - 1]) / (A.wave[iwl] - A.wave[iwl - 1]);
-    // One sweep over depth gives the three maxima the reference takes in turn (synth.f90:876-907):
-    // (1) the upper bound LinCop / ContOpac (H(a, v) <= 1), (2) the single-line opacity at the line
-    // centre (LineOpacity2 at Wl = Wlcent) and (3) the AnalyticWindow half-width (opacity.f90:678-710).
-    // Each is a maximum over depths of per-depth values that do not depend on the others, so computing
-    // XlineDepth once per depth for all three gives the reference's tests and windows exactly; the
-    // later maxima are used only when the earlier tests keep the line.
-    const double iSqrtPi = 0.5641895835477563;
+    const CenterLine c = center_line(A, L, i);
     double mx1 = -1.0e308, mx2 = -1.0e308, dWwin = 0.0;
-    for (int t = 0; t < nt; t++) {
-        double cop, vv, av;
-        xline_depth(A, t, XC, &cop, &vv, &av);
-        const double co = cont_center(A, iwl, dW, t);
-        mx1 = fmax(mx1, (A.motype == 1) ? cop / (co * A.contstd[t]) : cop / co);
-        double dWl = 0.0;
-        if (ihe > 0) dWl = 0.0 - center_shift(A, ihe, t);
-        double lo = hvoigt64(vtab, anode, aida, av, dWl * vv) * cop;
-        if (A.motype == 1) lo = lo / A.contstd[t];
-        mx2 = fmax(mx2, lo / co);
-        double r = cop / (A.epsopac * co);
-        if (A.motype == 1) r = r / A.contstd[t];
-        if (r <= 1.0) continue;
-        double w = sqrt(log(r) + fmax(0.0, av * (r * iSqrtPi - av))) / vv;
-        if (ihe > 0) w = w + fabs(center_shift(A, ihe, t));
-        dWwin = fmax(dWwin, w);
-    }
-    int il = 1, ir = A.nwl;
-    if (mx1 < A.epsopac || mx2 < A.epsopac) {
-        f |= FSG_F_WEAK;
-    } else {
-        il = waveidx(A, wlc - dWwin);                      // WaveIdx (synth.f90:904-906)
-        ir = waveidx(A, wlc + dWwin) + 1;
-        if (ir > A.nwl) ir = A.nwl;
-    }
-    flags[i] = f; ileft[i] = il; iright[i] = ir;
+    for (int t = 0; t < A.ntau; t++) center_depth(A, c, t, vtab, anode, aida, mx1, mx2, dWwin);
+    const bool keep = center_result(A, c, mx1, mx2, dWwin, i, flags, ileft, iright);
     // warp-aggregated count of retained lines
-    unsigned m = __ballot_sync(__activemask(), !(f & FSG_F_WEAK));
+    unsigned m = __ballot_sync(__activemask(), keep);
     if ((threadIdx.x & 31) == (__ffs(__activemask()) - 1) && m) atomicAdd(nkeep, (unsigned long long)__popc(m));
 }
 
+// One warp per line, lanes over depths: the same values, and maxima are exact in any order.
+__global__ void __launch_bounds__(128) k_center_warp(AtmView A, LineView L, const float *__restrict__ vtab,
+                         const double *__restrict__ anode, const double *__restrict__ aida,
+                         int32_t *flags, int32_t *ileft, int32_t *iright, unsigned long long *nkeep) {
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= L.n) return;                                // whole warps leave together
+    const CenterLine c = center_line(A, L, i);
+    double mx1 = -1.0e308, mx2 = -1.0e308, dWwin = 0.0;
+    for (int t = lane; t < A.ntau; t += 32) center_depth(A, c, t, vtab, anode, aida, mx1, mx2, dWwin);
+    for (int o = 16; o > 0; o >>= 1) {
+        mx1 = fmax(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+        mx2 = fmax(mx2, __shfl_xor_sync(0xffffffffu, mx2, o));
+        dWwin = fmax(dWwin, __shfl_xor_sync(0xffffffffu, dWwin, o));
+    }
+    if (lane == 0 && center_result(A, c, mx1, mx2, dWwin, i, flags, ileft, iright)) atomicAdd(nkeep, 1ull);
+}
+
+// A thread's sweep over the depths takes 125 us whatever the number of lines (the latency of an FP64 chain), and
+// a list fills the GPU with threads from 150,000 lines on; a warp per line repeats the line's set-up in every
+// lane.  CENTER_RULE
 void fsg_launch_center(cudaStream_t s, const AtmView &A, const LineView &L, const VoigtTables &T,
                        int32_t *flags, int32_t *ileft, int32_t *iright, unsigned long long *nkeep) {
     if (L.n <= 0) return;
-    unsigned nb = (unsigned)((L.n + 127) / 128);
-    k_center<<<nb, 128, 0, s>>>(A, L, T.vtab, T.anode, T.aida, flags, ileft, iright, nkeep);
+    if (L.n <= 65536)
+        k_center_warp<<<(unsigned)((L.n + 3) / 4), 128, 0, s>>>(A, L, T.vtab, T.anode, T.aida, flags, ileft, iright, nkeep);
+    else
+        k_center<<<(unsigned)((L.n + 127) / 128), 128, 0, s>>>(A, L, T.vtab, T.anode, T.aida, flags, ileft, iright, nkeep);
 }
 
 // ================================================================================================
