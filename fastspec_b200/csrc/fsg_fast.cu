@@ -25,6 +25,7 @@
 #include <cub/device/device_scan.cuh>
 #include <cuda/functional>
 #include <algorithm>
+#include <type_traits>
 
 #define CLASS_W0 128      // class c: windows of at most CLASS_W0 * 2^(c+1) wavelengths
 
@@ -59,18 +60,28 @@ __device__ __forceinline__ float rcp_approx(float x) {
 //   val = c1 (t + 1) / (t^2 + twoA),  t = dl^2 vv2 + c2m1
 // (three FMAs, one reciprocal, one FMA into the partial sum).  Outside the line's core range [cl, cr]
 // that is every depth.  Lines whose window covers the whole tile outside their core range (the common
-// case for wide windows) skip the mask; for the others the points outside the window get an x for
-// which the term is exactly 0.  On tiles that meet the core range, each point whose t is below 195.5
-// (table or continued fraction, the core pass's share) has its t replaced by 1e19, whose term is
-// exactly 0 too: the two passes split the points by the same FP32 test, so each point is evaluated
-// once.
+// case for wide windows) need no mask, and two of them share a reciprocal:
+//   n0 / d0 + n1 / d1 = (n0 d1 + n1 d0) / (d0 d1).
+// For the others the points outside the window get an x for which the term is exactly 0.  On tiles that meet
+// the core range, each point whose t is below 195.5 (table or continued fraction, the core pass's share) has
+// its t replaced by 1e19, whose term is exactly 0 too: the two passes split the points by the same FP32 test,
+// so each point is evaluated once.
+//
+// What bounds it: the reciprocal unit takes 8 cycles a warp and evaluation, the four FMAs 4; paired, 4 and 5 (a
+// loop of nothing else reaches 8.5 and 6.9).  Eight depths x 4 wavelengths a lane halve the record loads per
+// evaluation against 4 x 4, sixteen lines a group the staging against 8: a million lines, 483,000 wavelengths, 56 depths
+// 44.9 -> 40.3 ms (single, 4 x 4) -> 33.0 ms (pairs, 8 x 4, 16 lines).
+//
+// A pair rounds in other places than two single terms (the error against 64 bits is the same: 20,000 lines over
+// 200 A 7e-11 of the flux either way).  Where few lines make up a pixel the difference shows, 4e-9 of the flux at
+// 150 lines per pixel against 2e-10 at 1,000, and there the pass is short; tiles with fewer than WING_PAIR_MIN
+// candidate lines take them one at a time.
 
 // A line as the warp's group holds it: {wlh, wll, code, xm}.  code: first and last wavelength of the window
-// inside the tile (bits 0-7, 8-15), WING_FULL (the window covers the tile and no core range meets it),
-// WING_CORE (a core range meets it); xm: the x that silences a point.
-#define WING_FULL (1 << 16)
-#define WING_CORE (1 << 17)
-#define WING_G 8                      // lines per group
+// inside the tile (bits 0-7, 8-15), WING_CORE (a core range meets it); xm: the x that silences a point.
+#define WING_CORE (1 << 16)
+#define WING_G 16                     // lines per group
+#define WING_PAIR_MIN 2048
 
 // shared memory of one warp
 template <int D, int P>
@@ -82,16 +93,16 @@ struct __align__(16) WingWarp {
 };
 
 // One tile and depth group (depths t0 .. t0 + D - 1, t0 a multiple of D) of one job, by one warp; warps
-// share nothing.  Per evaluation two packed FMAs on the depth pair's halves (t, t^2 + 2a^2, c1 (t + 1), the
-// sum: four for two), and one reciprocal.
+// share nothing.  The arithmetic is packed FP32 on depth pairs.
 template <int D, int P>
 __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, WingWarp<D, P> &S, int lane) {
     constexpr int TW = 32 * P, NP = D / 2, U = WING_G * D / 32;      // U: record loads per lane and group
     const int ntau = J.ntau, nwl = J.nwl, units = 2 * wing_pairs(ntau);
-    bool any = false;                                   // some segment has lines touching the tile
+    int64_t ncand = 0;                                  // lines that may touch the tile
     for (int sg = 0; sg < J.nseg; sg++)
-        any = any || J.tile_lo[sg * J.seg_stride + tile] <= J.tile_hi[sg * J.seg_stride + tile];
-    if (!any) return;
+        ncand += max(J.tile_hi[sg * J.seg_stride + tile] - J.tile_lo[sg * J.seg_stride + tile] + 1, 0);
+    if (!ncand) return;
+    const bool pairs = ncand >= WING_PAIR_MIN;
     const float4 *__restrict__ wing = (const float4 *)J.wing;
     const int p0 = tile * TW;
     // wavelength offsets as FP32 hi + lo: dl = (wvh - wlh) + (wvl - wll) keeps dl to FP32 relative
@@ -115,9 +126,10 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
     int nfold = 0;
     const int tile_first = p0 + 1, tile_last = min(p0 + TW, nwl);
     float4 rnext[U], hnext;                             // the next group's records and (lanes < n) header
-    int nnext = 0;
+    int nnext = 0, npair = 0, slot = 0;                            // lines; lane q's line's place in the group
     auto fetch = [&](int head, int n) {
         nnext = n;
+        bool pair = false;
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int e = lane + 32 * u, q = e / D, i = t0 + e % D;
@@ -129,19 +141,24 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
             const bool core_hit = h.cl <= h.cr && h.cr >= tile_first && h.cl <= tile_last;
             const bool full = h.ileft <= tile_first && h.iright >= tile_last && !core_hit;
             const int l = max(h.ileft - tile_first, 0), r = min(h.iright - tile_first, TW - 1);
-            hnext = make_float4(h.wlh, h.wll, __int_as_float(l | r << 8 | (full ? WING_FULL : 0) | (core_hit ? WING_CORE : 0)),
+            hnext = make_float4(h.wlh, h.wll, __int_as_float(l | r << 8 | (core_hit ? WING_CORE : 0)),
                                 __int_as_float(h.pad0));
+            pair = pairs && full && h.pad1;
         }
+        // the lines to be paired first
+        const unsigned pm = __ballot_sync(0xffffffffu, pair), before = __popc(pm & ((1u << lane) - 1u));
+        npair = __popc(pm);
+        slot = pair ? before : npair + lane - before;
     };
-    auto stage = [&]() -> int {                         // the fetched group into shared memory; its line count
+    auto stage = [&](int m) {                              // the fetched group into shared memory
         __syncwarp();                                   // every lane is done with the group before
 #pragma unroll
-        for (int u = 0; u < U; u++) (&S.rec[0][0])[lane + 32 * u] = rnext[u];
-        if (lane < nnext) S.hdr[lane] = hnext;
+        for (int u = 0; u < U; u++) {
+            const int e = lane + 32 * u;
+            S.rec[__shfl_sync(0xffffffffu, slot, e / D)][e % D] = rnext[u];
+        }
+        if (lane < m) S.hdr[slot] = hnext;
         __syncwarp();
-        const int n = nnext;
-        nnext = 0;
-        return n;
     };
     auto fold = [&]() {                                 // the partials into the Kahan pairs
         nfold = 0;
@@ -157,24 +174,46 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
                 part[j][k] = make_float2(0.0f, 0.0f);
             }
     };
-    auto work = [&](int n) {
-        for (int q = 0; q < n; q++) {
+    auto offsets = [&](float4 h, float (&x)[P]) {       // x = dl^2 of the lane's wavelengths
+#pragma unroll
+        for (int k = 0; k < P; k++) {
+            const float dl = (wvh[k] - h.x) + (wvl[k] - h.y);
+            x[k] = dl * dl;
+        }
+    };
+    auto work = [&](int n, int np) {
+        int q = 0;
+        for (; q + 1 < np; q += 2) {                    // full lines, two at a time
+            float x0[P], x1[P];
+            offsets(S.hdr[q], x0);
+            offsets(S.hdr[q + 1], x1);
+#pragma unroll
+            for (int j = 0; j < NP; j++) {
+                const float4 a0 = S.rec[q][2 * j], b0 = S.rec[q][2 * j + 1];
+                const float4 a1 = S.rec[q + 1][2 * j], b1 = S.rec[q + 1][2 * j + 1];
+                const float2 c0 = make_float2(b0.z, b0.w), c1 = make_float2(b1.z, b1.w);
+#pragma unroll
+                for (int k = 0; k < P; k++) {
+                    const float2 t0 = __ffma2_rn(make_float2(x0[k], x0[k]), make_float2(a0.x, a0.y), make_float2(a0.z, a0.w));
+                    const float2 t1 = __ffma2_rn(make_float2(x1[k], x1[k]), make_float2(a1.x, a1.y), make_float2(a1.z, a1.w));
+                    const float2 d0 = __ffma2_rn(t0, t0, make_float2(b0.x, b0.y)), d1 = __ffma2_rn(t1, t1, make_float2(b1.x, b1.y));
+                    const float2 n0 = __ffma2_rn(c0, t0, c0), n1 = __ffma2_rn(c1, t1, c1);
+                    const float2 den = __fmul2_rn(d0, d1), num = __ffma2_rn(n0, d1, __fmul2_rn(n1, d0));
+                    part[j][k] = __ffma2_rn(num, make_float2(rcp_approx(den.x), rcp_approx(den.y)), part[j][k]);
+                }
+            }
+        }
+        for (; q < n; q++) {
             const float4 h = S.hdr[q];
             const int code = __float_as_int(h.z);
             float x[P];
+            offsets(h, x);
+            // points outside the window take the header's offset x, for which the wing term is exactly 0
+            const int l = code & 255, r = code >> 8 & 255;
 #pragma unroll
             for (int k = 0; k < P; k++) {
-                float dl = (wvh[k] - h.x) + (wvl[k] - h.y);
-                x[k] = dl * dl;
-            }
-            if (!(code & WING_FULL)) {
-                // points outside the window take the header's offset x, for which the wing term is exactly 0
-                const int l = code & 255, r = code >> 8 & 255;
-#pragma unroll
-                for (int k = 0; k < P; k++) {
-                    const int p = lane + 32 * k;
-                    x[k] = (p >= l && p <= r) ? x[k] : h.w;
-                }
+                const int p = lane + 32 * k;
+                x[k] = (p >= l && p <= r) ? x[k] : h.w;
             }
             const bool core_hit = code & WING_CORE;
 #pragma unroll
@@ -182,63 +221,61 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
                 const float4 a = S.rec[q][2 * j], b = S.rec[q][2 * j + 1];
                 const float2 vv2 = make_float2(a.x, a.y), c2m1 = make_float2(a.z, a.w);
                 const float2 twoA = make_float2(b.x, b.y), c1 = make_float2(b.z, b.w);
-                if (!core_hit) {
 #pragma unroll
-                    for (int k = 0; k < P; k++) {
-                        const float2 t = __ffma2_rn(make_float2(x[k], x[k]), vv2, c2m1);
-                        const float2 den = __ffma2_rn(t, t, twoA), num = __ffma2_rn(c1, t, c1);
-                        part[j][k] = __ffma2_rn(num, make_float2(rcp_approx(den.x), rcp_approx(den.y)), part[j][k]);
-                    }
-                } else {
-#pragma unroll
-                    for (int k = 0; k < P; k++) {
-                        float2 t = __ffma2_rn(make_float2(x[k], x[k]), vv2, c2m1);
-                        t.x = t.x < 195.5f ? 1.0e19f : t.x;          // the core pass's points
+                for (int k = 0; k < P; k++) {
+                    float2 t = __ffma2_rn(make_float2(x[k], x[k]), vv2, c2m1);
+                    if (core_hit) {                     // the core pass's points
+                        t.x = t.x < 195.5f ? 1.0e19f : t.x;
                         t.y = t.y < 195.5f ? 1.0e19f : t.y;
-                        const float2 den = __ffma2_rn(t, t, twoA), num = __ffma2_rn(c1, t, c1);
-                        part[j][k] = __ffma2_rn(num, make_float2(rcp_approx(den.x), rcp_approx(den.y)), part[j][k]);
                     }
+                    const float2 den = __ffma2_rn(t, t, twoA), num = __ffma2_rn(c1, t, c1);
+                    part[j][k] = __ffma2_rn(num, make_float2(rcp_approx(den.x), rcp_approx(den.y)), part[j][k]);
                 }
             }
-            if (++nfold == FOLD) fold();
         }
+        nfold += n;
+        if (nfold > FOLD - WING_G) fold();
     };
-    int head = 0, cnt = 0;
-    auto advance = [&](int n) {                         // n queued lines into flight, the group before worked through
-        if (nnext) {
-            const int m = stage();
-            fetch(head, n);
-            head += n; cnt -= n;
-            work(m);
-        } else {
-            fetch(head, n);
-            head += n; cnt -= n;
-        }
-    };
-    for (int sg = 0; sg < J.nseg; sg++) {               // the job's segments of lines, in turn
-        const int lo = J.tile_lo[sg * J.seg_stride + tile], hi = J.tile_hi[sg * J.seg_stride + tile];
-        for (int base = lo; base <= hi; base += 32) {
+    // One loop, so that each of the forms above stands in the code once: lines into the queue, a group of them
+    // into flight, the group before through the arithmetic.
+    int head = 0, cnt = 0, sg = 0, base = 0, hi = -1;
+    bool open = false;                                  // lines of segment sg are left to look at
+    for (;;) {
+        while (cnt < WING_G) {
+            if (!open) {
+                if (sg == J.nseg || (J.fold_seg && (cnt || nnext || nfold))) break;
+                base = J.tile_lo[sg * J.seg_stride + tile];
+                hi = J.tile_hi[sg * J.seg_stride + tile];
+                sg++;
+                open = base <= hi;
+                continue;
+            }
             const int i = base + lane;
             bool sel = false;
             if (i <= hi) {
                 const int2 w = *(const int2 *)&J.hdr[i].ileft;
                 sel = w.y >= tile_first && w.x <= tile_last;
             }
+            base += 32;
+            open = base <= hi;
             const unsigned m = __ballot_sync(0xffffffffu, sel);
-            if (!m) continue;
             if (sel) S.queue[(head + cnt + __popc(m & ((1u << lane) - 1u))) & 63] = i;
             cnt += __popc(m);
-            __syncwarp();
-            while (cnt >= WING_G) advance(WING_G);
         }
-        if (J.fold_seg) {                               // this segment's lines end here
-            if (cnt) advance(cnt);
-            if (nnext) work(stage());
+        __syncwarp();
+        const int n = min(cnt, WING_G);
+        const int m = nnext, mp = npair;
+        nnext = 0;
+        if (m) stage(m);
+        if (n) fetch(head, n);
+        head += n;
+        cnt -= n;
+        if (m) work(m, mp);
+        if (!n && !m) {                               // nothing in flight: the tile's lines, or this segment's, end here
             if (nfold) fold();
+            if (sg == J.nseg && !open) break;
         }
     }
-    if (cnt) advance(cnt);
-    if (nnext) work(stage());
 #pragma unroll
     for (int k = 0; k < P; k++) {
         const int pix = p0 + lane + 32 * k;
@@ -246,23 +283,20 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
         double *dst = J.lineopac + (size_t)pix * ntau + t0;
 #pragma unroll
         for (int j = 0; j < NP; j++) {
-            float2 s0 = S.ksum[2 * (j * P + k)][lane], s1 = S.ksum[2 * (j * P + k) + 1][lane];
-            KAHAN(s0.x, s0.y, part[j][k].x);
-            KAHAN(s1.x, s1.y, part[j][k].y);
+            const float2 s0 = S.ksum[2 * (j * P + k)][lane], s1 = S.ksum[2 * (j * P + k) + 1][lane];
             if (t0 + 2 * j < ntau) dst[2 * j] += (double)s0.x - (double)s0.y;
             if (t0 + 2 * j + 1 < ntau) dst[2 * j + 1] += (double)s1.x - (double)s1.y;
         }
     }
 }
 
-// depths per warp for P wavelengths per lane: P x D = 16 evaluations per thread and line
-#define WING_D(P) (16 / (P))
+#define WING_D 8                      // depths per warp
 #define WING_W 4                      // warps per CTA
 #define WING_BW 8                     // warps per CTA of the persistent form
 
 // one (tile, depth group) per warp, the groups of a tile in turn
 template <int D, int P>
-__global__ void __launch_bounds__(32 * WING_W)
+__global__ void __launch_bounds__(32 * WING_W, P == 2 ? 5 : 4)
 k_accum_fast(WingJob J, int ntiles) {
     __shared__ WingWarp<D, P> S[WING_W];
     const int warp = threadIdx.x >> 5, ng = (J.ntau + D - 1) / D;
@@ -275,7 +309,7 @@ k_accum_fast(WingJob J, int ntiles) {
 // device work queue (*queue, zero at launch) until all are done; item0[j] is the first item of job j
 // (prefix sums of the jobs' tiles x groups, item0[njobs] = total).
 template <int D, int P>
-__global__ void __launch_bounds__(32 * WING_BW)
+__global__ void __launch_bounds__(32 * WING_BW, 2)
 k_accum_batch(const WingJob *__restrict__ jobs, const int *__restrict__ item0, int njobs, unsigned *queue) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -298,14 +332,14 @@ k_accum_batch(const WingJob *__restrict__ jobs, const int *__restrict__ item0, i
 int fsg_class_pix(int cls) { return cls <= 1 ? 2 : 4; }
 
 // depth groups of the wing pass
-int fsg_wing_groups(int P, int ntau) { return (ntau + WING_D(P) - 1) / WING_D(P); }
+int fsg_wing_groups(int P, int ntau) { return (ntau + WING_D - 1) / WING_D; }
 
 // the wing pass of one job on tiles of 32 P wavelengths
 int fsg_launch_accum_fast(cudaStream_t st, int P, const WingJob &J) {
     const int TW = 32 * P, ntiles = (J.nwl + TW - 1) / TW;
     const unsigned grid = (unsigned)(((int64_t)ntiles * fsg_wing_groups(P, J.ntau) + WING_W - 1) / WING_W);
-    if (P == 2) k_accum_fast<WING_D(2), 2><<<grid, 32 * WING_W, 0, st>>>(J, ntiles);
-    else k_accum_fast<WING_D(4), 4><<<grid, 32 * WING_W, 0, st>>>(J, ntiles);
+    if (P == 2) k_accum_fast<WING_D, 2><<<grid, 32 * WING_W, 0, st>>>(J, ntiles);
+    else k_accum_fast<WING_D, 4><<<grid, 32 * WING_W, 0, st>>>(J, ntiles);
     return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }
 
@@ -313,10 +347,12 @@ int fsg_launch_accum_fast(cudaStream_t st, int P, const WingJob &J) {
 // warps (two of the kernel's)
 int fsg_launch_accum_batch(cudaStream_t st, int P, const WingJob *jobs, const int *item0, int njobs, int ctas,
                            unsigned *queue) {
-    const size_t smem = WING_BW * (P == 2 ? sizeof(WingWarp<WING_D(2), 2>) : sizeof(WingWarp<WING_D(4), 4>));
+    const size_t smem = WING_BW * (P == 2 ? sizeof(WingWarp<WING_D, 2>) : sizeof(WingWarp<WING_D, 4>));
     const unsigned grid = (unsigned)ctas * (16 / WING_BW);
-    if (P == 2) k_accum_batch<WING_D(2), 2><<<grid, 32 * WING_BW, smem, st>>>(jobs, item0, njobs, queue);
-    else k_accum_batch<WING_D(4), 4><<<grid, 32 * WING_BW, smem, st>>>(jobs, item0, njobs, queue);
+    const void *fn = P == 2 ? (const void *)k_accum_batch<WING_D, 2> : (const void *)k_accum_batch<WING_D, 4>;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return FSG_E_CUDA;
+    if (P == 2) k_accum_batch<WING_D, 2><<<grid, 32 * WING_BW, smem, st>>>(jobs, item0, njobs, queue);
+    else k_accum_batch<WING_D, 4><<<grid, 32 * WING_BW, smem, st>>>(jobs, item0, njobs, queue);
     return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }
 

@@ -93,7 +93,8 @@ static_assert(sizeof(CoreRec) == 32, "core record: 32 bytes");
 // every wavelength index of the window where some depth may have s < 196 lies inside it
 // (cl > cr when no depth has a core).  pad0 holds, in the wing pass's headers, the FP32 bits of the
 // x = dl^2 that makes every depth's wing term exactly 0 (points outside the window or inside the core
-// range of a partly covered tile); the magnetic pass keeps its He I table index there.
+// range of a partly covered tile), pad1 whether the line may share a reciprocal with another; the magnetic pass
+// keeps its He I table index in pad0.
 struct __align__(16) LineHdr { float wlh, wll; int ileft, iright; int cl, cr, pad0, pad1; };
 
 // Line header of the FP64 tile kernels: the centre offset Wlcent, the window, the core range [cl, cr]

@@ -265,11 +265,12 @@ __global__ void __launch_bounds__(128) k_center_warp(AtmView A, LineView L, cons
 
 // A thread's sweep over the depths takes 125 us whatever the number of lines (the latency of an FP64 chain), and
 // a list fills the GPU with threads from 150,000 lines on; a warp per line repeats the line's set-up in every
-// lane.  CENTER_RULE
+// lane.  300 lines: 126 us by threads, 11 us by warps; 20,000: 133 and 66 us, 3.3 us more per thousand, so the two
+// meet near 40,000.
 void fsg_launch_center(cudaStream_t s, const AtmView &A, const LineView &L, const VoigtTables &T,
                        int32_t *flags, int32_t *ileft, int32_t *iright, unsigned long long *nkeep) {
     if (L.n <= 0) return;
-    if (L.n <= 65536)
+    if (L.n <= 32768)
         k_center_warp<<<(unsigned)((L.n + 3) / 4), 128, 0, s>>>(A, L, T.vtab, T.anode, T.aida, flags, ileft, iright, nkeep);
     else
         k_center<<<(unsigned)((L.n + 127) / 128), 128, 0, s>>>(A, L, T.vtab, T.anode, T.aida, flags, ileft, iright, nkeep);
@@ -298,6 +299,8 @@ k_params_fast(AtmView A, LineView L, const int64_t *__restrict__ idx, int64_t j0
     __shared__ XCoef xs[PF_WARPS][32];
     __shared__ unsigned long long hcs[PF_WARPS][32];   // bits of hcore + 1 (0: no depth has a core)
     __shared__ unsigned vms[PF_WARPS][32];             // bits of the smallest vv2 (non-negative floats)
+    __shared__ double xms[PF_WARPS][32];               // largest dl^2 in the window
+    __shared__ int big[PF_WARPS][32];                  // some depth leaves the range of paired denominators
     const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t jb = ((int64_t)blockIdx.x * PF_WARPS + wp) * lpw;
     if (jb >= nb) return;                               // whole warps only: no block barrier below
@@ -309,7 +312,15 @@ k_params_fast(AtmView A, LineView L, const int64_t *__restrict__ idx, int64_t j0
         f = flags[i];
         wlc = L.wl[i] - A.wfirst;
         xline_setup(A, L, i, wlc, f, &xs[wp][lane]);
+        const int il = ileft[i], ir = iright[i];
+        double xm = 0.0;
+        if (il >= 1 && il <= ir && ir <= A.nwl) {
+            const double dl = wlc - A.wave[il - 1], dr = wlc - A.wave[ir - 1];
+            xm = fmax(dl * dl, dr * dr);
+        }
+        xms[wp][lane] = xm;
     }
+    big[wp][lane] = 0;
     hcs[wp][lane] = 0ull;
     vms[wp][lane] = __float_as_uint(3.0e38f);
     __syncwarp();
@@ -335,6 +346,7 @@ k_params_fast(AtmView A, LineView L, const int64_t *__restrict__ idx, int64_t j0
             twoA = (float)(2.0 * a2);
             c1 = (float)(cop * av * FSG_SQRTPIINV);
             vv2 = wv2;
+            if (!(xms[wp][ln] * wv2 + a2 < 2147483648.0 && fabsf(c1) < 1073741824.0f)) big[wp][ln] = 1;
             CoreRec c;
             c.vv = vv; c.cop = (float)cop; c.a = (float)av; c.vv2 = wv2; c.c2m1 = c2m1;
             // table row and weight of a in FP64 (sqrt(a) nodes, voigt.f90:84-92); ia = 0: a >= 8
@@ -394,11 +406,13 @@ k_params_fast(AtmView A, LineView L, const int64_t *__restrict__ idx, int64_t j0
         int cl = max(a - 1, h.ileft), cr = min(b + 1, h.iright);
         if (cl <= cr) { h.cl = cl; h.cr = cr; }
     }
+    // pad1: the line may share a reciprocal in the wing pass (no depth's denominator above 2^62, no coefficient
+    // above 2^30: the product of two stays below 2^126, its numerator finite)
     // x offset that silences a point in the wing pass: with dl^2 replaced by 1e19 / min vv2, every
     // depth has t >= 1e19, so t^2 >= 1e38 and the FP32 reciprocal (flush-to-zero) is exactly 0 while
     // c1 (t + 1) stays finite; the point then adds exactly 0
     h.pad0 = __float_as_int(1.0e19f / vv2min);
-    h.pad1 = 0;
+    h.pad1 = !big[wp][lane];
     hdr[jb + lane] = h;
 }
 

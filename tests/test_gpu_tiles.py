@@ -46,6 +46,55 @@ def test_tile_edges(fsg, oracle_mod, prec, ntau, nwl, n):
     C.close()
 
 
+@pytest.mark.parametrize("step,nwl,n,eps", [(0.011, 300, 2500, 1e-10), (0.011, 4000, 9000, 1e-6), (9.0, 501, 4001, 1e-14)])
+def test_paired_lines(fsg, step, nwl, n, eps):
+    """Tiles with enough lines for the wing pass to take them two to a reciprocal: windows that cover all tiles,
+    windows that end inside them, and (the last case) lines whose t^2 + 2a^2 leaves the range of a product, which
+    stay single.  Mixed against FP64, the path's bar."""
+    from fastspec_b200 import workloads as W
+    ntau = 33
+    _, st, _, _ = case(ntau, 2, 1, 0)
+    w0 = 4000.0
+    wave = fsg.make_grid(0, w0, w0 + (nwl - 0.5) * step, step) + w0
+    co = np.tile(1e-2 * (1.0 + np.arange(ntau)), (len(wave), 1))
+    L = fsg.LineList.from_arrays(W.atomic_lines(n, wave[0], wave[-1], nwl, exact=False).arrays())
+    out = {}
+    for prec in (fsg.PREC_FP64, fsg.PREC_MIXED):
+        C = fsg.Context(precision=prec, vmicro=1.0, epsopac=eps)
+        C.set_grid(0, w0, w0 + (nwl - 0.5) * step, step)
+        C.set_atmosphere(st)
+        C.set_contopac(co)
+        out[prec] = C.lineop_calc(L)
+        C.close()
+    f, m = out[fsg.PREC_FP64], out[fsg.PREC_MIXED]
+    keep = (f["flags"] & 1) == 0
+    assert (f["iright"] - f["ileft"])[keep].astype(np.int64).sum() > 2048 * nwl     # lines to pair on a tile
+    np.testing.assert_array_equal(f["ileft"][keep], m["ileft"][keep])
+    assert np.max(np.abs(m["lineopac"] - f["lineopac"]) / (f["lineopac"] + co)) < 2e-6
+
+
+@pytest.mark.parametrize("n", [32769, 45001])
+def test_central_pass_forms(fsg, n):
+    """Flags and windows do not depend on how the central pass spreads its lines: a list above 32,768 lines takes
+    a thread per line, the parts of it a warp."""
+    from fastspec_b200 import workloads as W
+    grid, st, co, _ = case(31, 64, 1, 0)
+    a = W.atomic_lines(n, grid["wstart"] - 40.0, grid["wend"] + 40.0, n, exact=False).arrays()
+
+    def windows(a):
+        C = fsg.Context(vmicro=1.0)
+        C.set_grid(grid["wmode"], grid["wstart"], grid["wend"], grid["dstep"])
+        C.set_atmosphere(st)
+        C.set_contopac(co)
+        g = C.lineop_calc(fsg.LineList.from_arrays(a))
+        C.close()
+        return np.stack([g["flags"], g["ileft"], g["iright"]])
+
+    cut = [0, 300, 16000, n]
+    parts = [windows({k: v[i:j] for k, v in a.items()}) for i, j in zip(cut, cut[1:])]
+    np.testing.assert_array_equal(windows(a), np.concatenate(parts, axis=1))
+
+
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
 @pytest.mark.parametrize("ntau,nwl,n", [(3, 2, 1), (4, 31, 5), (9, 33, 17), (33, 64, 20), (65, 300, 33), (128, 97, 12)])
 def test_magnetic_tile_edges(fsg, oracle_mod, prec, ntau, nwl, n):
