@@ -2507,7 +2507,7 @@ static int batch_jobs(fsg_batch *b, int P) {
                                           a.core.as<CoreRec>(), a.ctlo.as<int>(), a.cthi.as<int>(),
                                           c->d_lineopac.as<double>(), b->evals.as<unsigned long long>(), 0u, WAIT_NS,
                                           nseg, cs });
-                    t0.push_back(t0.back() + (c->nwl + 31) / 32);
+                    t0.push_back(t0.back() + (c->nwl + 31) / 32 * fsg_core_groups(c->ntau));
                 }
                 L.nj++;
             }

@@ -15,7 +15,7 @@
 // 256 * 2^c wavelengths) and processed class by class, so a tile's candidate range stays close to the lines
 // that touch it; narrow classes use 64-wavelength tiles, wide ones 128.
 //
-// Core pass (k_core_fast): over the core ranges, 32-wavelength tiles, the points where s < 196: the
+// Core pass (k_core_fast): over the core ranges, 32-wavelength tiles x 8 depths per warp, the points where s < 196: the
 // table lerp (|v| < 8, a < 8) or the two-term continued fraction (voigt.f90:103-107), exactly as
 // HVoigt branches.  No atomics; one read-modify-write of the FP64 LineOpac per tile and launch;
 // deterministic order.
@@ -35,7 +35,9 @@ __device__ __forceinline__ float hv_cf32(float av, float a, float cop) {
     float a2 = a * a, v2 = av * av;
     float p = v2 - a2 - 1.5f, q = 2.0f * av * a;
     float dr = av * p - a * q, di = av * q + a * p;
-    return 0.56418958354775628f * __fdividef((p + 0.5f) * di - q * dr, dr * dr + di * di) * cop;
+    float r;                                            // the denominator is of the order of v^6: no subnormals
+    asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"((p + 0.5f) * di - q * dr), "f"(dr * dr + di * di));
+    return 0.56418958354775628f * r * cop;
 }
 
 // Kahan-compensated accumulation of one value
@@ -358,241 +360,226 @@ int fsg_launch_accum_batch(cudaStream_t st, int P, const WingJob *jobs, const in
 
 // Core pass.  Over each line's core range [cl, cr], the points where fl32(t) < 195.5 (s < 196): the
 // table lerp or the continued fraction, as HVoigt branches (voigt.f90:81-107); the wing pass takes the
-// others (the same FP32 test splits the points, so each is evaluated once).  A CTA owns 32 wavelengths
-// x all depths: warp w depths [w*D, w*D + D), lane l wavelength tile0 + l, Kahan sums in
-// registers.  Headers and core records of the tile's candidate lines arrive in shared
-// memory CHC lines at a time by double-buffered bulk copies completing on mbarriers (waits bounded;
-// on expiry the kernel reports FSG_E_TIMEOUT and drains its copies), so the loop over lines reads
-// shared memory; per line a thread forms its depths' branch predicates first and issues their table
-// gathers (one 16-byte load of the cell-major VgtTab copy each) together.  D = 4 depths per warp up to
-// 72 depths, 8 beyond (18 warps at most).
+// others (the same FP32 test splits the points, so each is evaluated once).  A warp owns 32 wavelengths x
+// CORE_D depths, Kahan sums in registers; warps share nothing.  It queues the lines whose core range meets
+// the tile and stages them CORE_G at a time, double-buffered: the headers by plain loads, each line's records of the
+// warp's depths by one bulk copy, a group's copies completing on the buffer's mbarrier (waits bounded; on
+// expiry the kernel reports FSG_E_TIMEOUT, waits for its copies in flight, bounded again, and leaves).  Per
+// line a lane forms its depths' branch predicates four at a time and issues their table gathers (one 16-byte
+// load of the cell-major VgtTab copy each) together.
+//
+// What bounds it: instruction issue (60 to 70 % of the cycles) and the gathers, one 128-byte line of L1 a lane.  Hence
+// floor() by an addition and not by conversions (the conversion unit takes 8 cycles a warp, the FP64 one 2), the
+// continued fraction and whole depth groups left out where no lane needs them, and no barrier between depth groups.
+// Against a CTA per tile that staged all depths of a chunk: 1e6 lines, 483,000 wavelengths, 56 depths 15.4 -> 10.9 ms; a
+// batch of 24 atmospheres 19.7 -> 12.9 ms; 20,000 lines, 40,001 wavelengths 736 -> 480 us.  5 CTAs a SM (96
+// registers): 4 take 7 % longer, 6 spill; the persistent form spills at 5.
+#define CORE_D 8                      // depths per warp (two groups of four gathers)
+#define CORE_G 16                     // lines per group
+#define CORE_W 4                      // warps per CTA
 
+struct __align__(16) CoreWarp {
+    CoreRec rec[2][CORE_G][CORE_D];
+    LineHdr hdr[2][CORE_G];
+    uint64_t bar[2];
+    int queue[64];
+};
 
-// shared memory of the core pass for at most ntau_max depths and chc lines per chunk:
-// core records [2][chc][ntau_max] | headers [2][chc] | mbarriers [2]
-__host__ __device__ inline size_t core_smem(int ntau_max, int chc) {
-    return sizeof(CoreRec) * 2 * (size_t)chc * ntau_max + sizeof(LineHdr) * 2 * (size_t)chc +
-           2 * sizeof(uint64_t);
+__device__ __forceinline__ void core_bars_init(CoreWarp &S, int lane) {
+    if (lane == 0) {
+        mbar_init(&S.bar[0], 1);
+        mbar_init(&S.bar[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
 }
 
-__device__ __forceinline__ void core_stage(int c, int lo, int hi, int ntau, int chc, const CoreJob &J,
-                                           CoreRec *sc, LineHdr *sh, uint64_t *bar) {
-    const int j0 = lo + c * chc;
-    const int n = min(chc, hi - j0 + 1);
-    const unsigned bc = (unsigned)(n * ntau * (int)sizeof(CoreRec));
-    const unsigned bh = (unsigned)(n * (int)sizeof(LineHdr));
-    mbar_expect_tx(bar, bc + bh + J.extra_tx);
-    tma_bulk_g2s(sc, J.core + (size_t)j0 * ntau, bc, bar);
-    tma_bulk_g2s(sh, J.hdr + j0, bh, bar);
-}
-
-// One tile of one job, called by every thread of the CTA with the mbarriers initialised; kk counts
-// the chunks the CTA has consumed (their buffer and phase parity) across tiles.  Returns false after a
-// copy did not complete within its bound (error in *err).
-template <int D>
-__device__ bool core_tile(const CoreJob &J, int tile, const float4 *__restrict__ vtab4, unsigned char *smem_raw,
-                          int ntau_max, int chc, unsigned &kk, int *err) {
-    const int ntau = J.ntau, nwl = J.nwl;
+// One tile and depth group (depths t0 .. t0 + CORE_D - 1) of one job, by one warp with its mbarriers
+// initialised; kk counts the groups of lines the warp has staged (their buffer and phase parity) across calls.
+// Returns false after a copy did not complete within its bound (error in *err).
+__device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, const float4 *__restrict__ vtab4, CoreWarp &S,
+                                          int lane, unsigned &kk, int *err) {
+    const int ntau = J.ntau, nwl = J.nwl, nd = min(CORE_D, ntau - t0);
     bool any = false;                              // some segment has core ranges touching the tile
     for (int sg = 0; sg < J.nseg; sg++)
         any = any || J.tile_lo[sg * J.seg_stride + tile] <= J.tile_hi[sg * J.seg_stride + tile];
     if (!any) return true;
-    CoreRec *sc = (CoreRec *)smem_raw;
-    LineHdr *sh = (LineHdr *)(sc + 2 * (size_t)chc * ntau_max);
-    uint64_t *bars = (uint64_t *)(sh + 2 * chc);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t0 = warp * D;
-    const int nd = max(0, min(D, ntau - t0));      // warps past the last depth only wait with the others
     const int p = tile * 32 + lane, p1 = p + 1;
     const int tile_first = tile * 32 + 1, tile_last = min(tile * 32 + 32, nwl);
     const double wd = J.wave[min(p, nwl - 1)];
     const float wvh = (float)wd, wvl = (float)(wd - (double)wvh);
-    float sum[D], cmp[D];
+    float sum[CORE_D], cmp[CORE_D];
 #pragma unroll
-    for (int d = 0; d < D; d++) { sum[d] = 0.0f; cmp[d] = 0.0f; }
+    for (int d = 0; d < CORE_D; d++) { sum[d] = 0.0f; cmp[d] = 0.0f; }
     unsigned cnt = 0;
-    for (int sg = 0; sg < J.nseg; sg++) {         // the job's segments of lines, in turn
-        const int lo = J.tile_lo[sg * J.seg_stride + tile], hi = J.tile_hi[sg * J.seg_stride + tile];
-        if (lo > hi) continue;
-        const int nchunks = (hi - lo + chc) / chc;
-        if (threadIdx.x == 0)
-            for (int c = 0; c < 2 && c < nchunks; c++) {
-                const int b = (kk + c) & 1;
-                core_stage(c, lo, hi, ntau, chc, J, sc + (size_t)b * chc * ntau_max, sh + b * chc, &bars[b]);
-            }
-        int failed = -1;
-        for (int c = 0; c < nchunks; c++) {
-            const unsigned g = kk + c;
-            const int b = g & 1;
-            const bool ok = mbar_wait(&bars[b], (g >> 1) & 1, J.wait_ns);
-            if (__syncthreads_or(!ok)) { failed = c; break; }
-            const LineHdr *ch = sh + b * chc;
-            const CoreRec *cc = sc + (size_t)b * chc * ntau_max;
-            const int n = min(chc, hi - (lo + c * chc) + 1);
-            if (nd > 0) {
-                for (int q = 0; q < n; q++) {
-                    const LineHdr h = ch[q];
-                    if (h.cr < tile_first || h.cl > tile_last) continue;          // core range misses the tile
-                    const bool in = p1 >= h.cl && p1 <= h.cr;
-                    if (!__any_sync(0xffffffffu, in)) continue;
-                    const float dl = (wvh - h.wlh) + (wvl - h.wll);
-                    const float x = dl * dl;                  // the wing pass's x: the same branch split
-                    const double adl = fabs(wd - ((double)h.wlh + (double)h.wll));
+    // records past the last depth: none of their points is a core point (the copies leave them as they are)
+    if (lane < CORE_G * 2)
+        for (int d = nd; d < CORE_D; d++) {
+            CoreRec z{};
+            z.c2m1 = 3.0e38f;
+            (&S.rec[0][0][0])[lane * CORE_D + d] = z;
+        }
+    auto work = [&](int b, int n) {
+        for (int q = 0; q < n; q++) {
+            const LineHdr h = S.hdr[b][q];
+            const float dl = (wvh - h.wlh) + (wvl - h.wll);
+            // the wing pass's x: the same branch split; outside the core range nothing is below 195.5
+            const float x = p1 >= h.cl && p1 <= h.cr ? dl * dl : 3.0e38f;
+            const double adl = fabs(wd - ((double)h.wlh + (double)h.wll)), adl125 = adl * 125.0;
+            const CoreRec *__restrict__ rec = S.rec[b][q];
 #pragma unroll
-                    for (int g0 = 0; g0 < D; g0 += 4) {               // depths in groups of four
-                        bool core[4], tab[4];
-                        float tv[4];
-                        int cell[4];
+            for (int g0 = 0; g0 < CORE_D; g0 += 4) {               // depths in groups of four
+                bool core[4], tab[4], some = false, cf = false;
 #pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const int d = g0 + e;
-                            const int td = t0 + min(d, nd - 1);
-                            const CoreRec cr = cc[q * ntau + td];
-                            const float t = fmaf(x, cr.vv2, cr.c2m1);
-                            core[e] = in && d < nd && t < 195.5f;
-                            const double av = adl * cr.vv;
-                            tab[e] = core[e] && cr.ia > 0 && av < 8.0;
-                            const double fv = av * 125.0;
-                            const int iv = tab[e] ? min((int)fv, FSG_NVV - 1) : 0;
-                            tv[e] = tab[e] ? (float)(fv - (double)iv) : (float)av;   // CF: |v| in FP32
-                            cell[e] = tab[e] ? (cr.ia - 1) * FSG_NV1 + iv : 0;
-                        }
-                        float4 gv[4];
+                for (int e = 0; e < 4; e++) {
+                    core[e] = fmaf(x, rec[g0 + e].vv2, rec[g0 + e].c2m1) < 195.5f;
+                    some = some || core[e];
+                }
+                if (!__any_sync(0xffffffffu, some)) continue;
+                float tv[4];
+                float4 gv[4];
 #pragma unroll
-                        for (int e = 0; e < 4; e++)
-                            if (tab[e]) gv[e] = __ldg(vtab4 + cell[e]);
+                for (int e = 0; e < 4; e++) {
+                    // column and fraction: 2^52 added towards minus infinity leaves floor(v / 0.008) in the low word
+                    const double fv = adl125 * rec[g0 + e].vv, m = __dadd_rd(fv, 4503599627370496.0);
+                    const int iv = __double2loint(m), ia = rec[g0 + e].ia;
+                    tab[e] = core[e] && iv < FSG_NVV - 1 && ia > 0;
+                    cf = cf || (core[e] && !tab[e]);
+                    tv[e] = (float)(fv - (m - 4503599627370496.0));
+                    if (tab[e]) gv[e] = __ldg(vtab4 + ((ia - 1) * FSG_NV1 + iv));
+                }
+                cf = __any_sync(0xffffffffu, cf);
 #pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            if (!core[e]) continue;
-                            const int d = g0 + e;
-                            const CoreRec &cr = cc[q * ntau + t0 + d];
-                            float v;
-                            if (tab[e]) {
-                                const float4 gg = gv[e];
-                                const float c0 = gg.x + tv[e] * (gg.y - gg.x), c1 = gg.z + tv[e] * (gg.w - gg.z);
-                                v = (c0 + cr.ua * (c1 - c0)) * cr.cop;
-                            } else {
-                                v = hv_cf32(tv[e], cr.a, cr.cop);
-                            }
-                            KAHAN(sum[d], cmp[d], v);
-                            cnt++;
-                        }
+                for (int e = 0; e < 4; e++) {
+                    const CoreRec &cr = rec[g0 + e];
+                    const float c0 = gv[e].x + tv[e] * (gv[e].y - gv[e].x), c1 = gv[e].z + tv[e] * (gv[e].w - gv[e].z);
+                    float v = (c0 + cr.ua * (c1 - c0)) * cr.cop;
+                    if (cf) {
+                        const float w = hv_cf32((float)(adl * cr.vv), cr.a, cr.cop);
+                        v = tab[e] ? v : w;
+                    }
+                    if (core[e]) {
+                        KAHAN(sum[g0 + e], cmp[g0 + e], v);
+                        cnt++;
                     }
                 }
             }
-            __syncthreads();                                   // every warp is done with buffer b
-            if (threadIdx.x == 0 && c + 2 < nchunks)
-                core_stage(c + 2, lo, hi, ntau, chc, J, sc + (size_t)b * chc * ntau_max, sh + b * chc, &bars[b]);
         }
-        if (failed >= 0) {
-            if (threadIdx.x == 0) {
-                atomicExch(err, FSG_E_TIMEOUT);
-                for (int c = failed; c < nchunks && c < failed + 2; c++) {
-                    const unsigned g = kk + c;
-                    mbar_wait(&bars[g & 1], (g >> 1) & 1, J.wait_ns);
-                }
+    };
+    const unsigned bytes = (unsigned)(nd * (int)sizeof(CoreRec));
+    int head = 0, ncand = 0, sg = 0, base = 0, hi = -1, nprev = 0;
+    bool ok = true;
+    for (;;) {
+        while (ncand < CORE_G) {                       // lines into the queue
+            if (base > hi) {
+                if (sg == J.nseg) break;
+                base = J.tile_lo[sg * J.seg_stride + tile];
+                hi = J.tile_hi[sg * J.seg_stride + tile];
+                sg++;
+                continue;
             }
-            __syncthreads();
-            return false;
+            const int i = base + lane;
+            bool sel = false;
+            if (i <= hi) {
+                const int2 c = *(const int2 *)&J.hdr[i].cl;
+                sel = c.x <= c.y && c.y >= tile_first && c.x <= tile_last;
+            }
+            base += 32;
+            const unsigned m = __ballot_sync(0xffffffffu, sel);
+            if (sel) S.queue[(head + ncand + __popc(m & ((1u << lane) - 1u))) & 63] = i;
+            ncand += __popc(m);
         }
-        kk += nchunks;
+        __syncwarp();                                   // the queue is written, and the buffer's last group done with
+        const int n = min(ncand, CORE_G), b = kk & 1;
+        if (n) {                                        // a group into flight
+            if (lane == 0) mbar_expect_tx(&S.bar[b], n * bytes + J.extra_tx);
+            __syncwarp();
+            if (lane < n) {
+                const int i = S.queue[(head + lane) & 63];
+                tma_bulk_g2s(S.rec[b][lane], J.core + (size_t)i * ntau + t0, bytes, &S.bar[b]);
+                S.hdr[b][lane] = J.hdr[i];
+            }
+            head += n;
+            ncand -= n;
+            kk++;
+        }
+        if (nprev) {                                    // the group before: staged as number g
+            const unsigned g = kk - (n ? 2 : 1);
+            ok = __all_sync(0xffffffffu, mbar_wait(&S.bar[g & 1], (g >> 1) & 1, J.wait_ns));
+            if (!ok) break;
+            work(g & 1, nprev);
+        }
+        nprev = n;
+        if (!n) break;
+    }
+    if (!ok) {
+        if (lane == 0) {
+            atomicExch(err, FSG_E_TIMEOUT);
+            for (unsigned g = kk - 2; g != kk; g++) mbar_wait(&S.bar[g & 1], (g >> 1) & 1, J.wait_ns);
+        }
+        __syncwarp();
+        return false;
     }
     if (J.nevals) {
         unsigned long long v = cnt;
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if (lane == 0 && v) atomicAdd(J.nevals, v);
     }
-    if (nd <= 0 || p >= nwl) return true;
+    if (p >= nwl) return true;
     double *dst = J.lineopac + (size_t)p * ntau + t0;
 #pragma unroll
-    for (int d = 0; d < D; d++)
+    for (int d = 0; d < CORE_D; d++)
         if (d < nd) dst[d] = dst[d] + ((double)sum[d] - (double)cmp[d]);
     return true;
 }
 
-__device__ __forceinline__ void core_bars_init(unsigned char *smem_raw, int ntau_max, int chc) {
-    uint64_t *bars = (uint64_t *)(smem_raw + core_smem(ntau_max, chc) - 2 * sizeof(uint64_t));
-    if (threadIdx.x == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-}
-
-template <int D>
-__global__ void __launch_bounds__(32 * 18, D == 4 ? 2 : 1)
-k_core_fast(CoreJob J, const float4 *__restrict__ vtab4, int chc, int *__restrict__ err) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    core_bars_init(smem_raw, J.ntau, chc);
+// one (tile, depth group) per warp, the groups of a tile in turn
+__global__ void __launch_bounds__(32 * CORE_W, 5)
+k_core_fast(CoreJob J, int ntiles, const float4 *__restrict__ vtab4, int *__restrict__ err) {
+    __shared__ CoreWarp S[CORE_W];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ng = fsg_core_groups(J.ntau);
+    const int64_t item = (int64_t)blockIdx.x * CORE_W + warp;
+    if (item >= (int64_t)ntiles * ng) return;           // warps are independent: no CTA barrier
+    core_bars_init(S[warp], lane);
     unsigned kk = 0;
-    core_tile<D>(J, blockIdx.x, vtab4, smem_raw, J.ntau, chc, kk, err);
+    core_tile(J, (int)(item / ng), (int)(item % ng) * CORE_D, vtab4, S[warp], lane, kk, err);
 }
 
-// persistent form: CTAs take (job, tile) items from the queue; a CTA of nwarps warps covers
-// nwarps * D depths, so every item is taken by whole CTAs
-template <int D>
-__global__ void __launch_bounds__(32 * 18, D == 4 ? 2 : 1)
-k_core_batch(const CoreJob *__restrict__ jobs, const int *__restrict__ tile0, int njobs, int ntau_max, int chc,
+// persistent form: warps take (job, tile, depth group) items from the queue
+__global__ void __launch_bounds__(32 * CORE_W, 4)
+k_core_batch(const CoreJob *__restrict__ jobs, const int *__restrict__ item0, int njobs,
              const float4 *__restrict__ vtab4, unsigned *queue, int *__restrict__ err) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ int s_item;
-    core_bars_init(smem_raw, ntau_max, chc);
+    __shared__ CoreWarp S[CORE_W];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    core_bars_init(S[warp], lane);
     unsigned kk = 0;
-    const int total = tile0[njobs];
+    const int total = item0[njobs];
     for (;;) {
-        if (threadIdx.x == 0) s_item = (int)atomicAdd(queue, 1u);
-        __syncthreads();
-        const int item = s_item;
-        __syncthreads();
+        int item = 0;
+        if (lane == 0) item = (int)atomicAdd(queue, 1u);
+        item = __shfl_sync(0xffffffffu, item, 0);
         if (item >= total) break;
-        int a = 0, b = njobs - 1;
-        while (a < b) { int m = (a + b + 1) >> 1; if (tile0[m] <= item) a = m; else b = m - 1; }
-        if (!core_tile<D>(jobs[a], item - tile0[a], vtab4, smem_raw, ntau_max, chc, kk, err)) break;
+        int a = 0, b = njobs - 1;                          // job with item0[a] <= item < item0[a + 1]
+        while (a < b) { int m = (a + b + 1) >> 1; if (item0[m] <= item) a = m; else b = m - 1; }
+        const CoreJob J = jobs[a];
+        const int ng = fsg_core_groups(J.ntau), r = item - item0[a];
+        if (!core_tile(J, r / ng, (r % ng) * CORE_D, vtab4, S[warp], lane, kk, err)) break;
     }
 }
-
-// lines per staged chunk: about 32 KB of records per buffer, 4 to 16 lines.  The buffers share the
-// SM's L1 with the table gathers: per 1e8-line step the core pass took 1.82 / 1.71 / 1.75 / 1.85 s
-// with 48 / 32 / 24 / 16 KB.
-static int core_chunk(int ntau_max) {
-    const int per_line = ntau_max * (int)sizeof(CoreRec) + (int)sizeof(LineHdr);
-    return std::max(4, std::min(16, (32 * 1024) / per_line));
-}
-
-// depths per warp: 8 (two groups of four gathers; 4 depths per warp, for up to 72 depths, took 3 %
-// longer on the 1e8-line step)
-static int core_depths(int) { return 8; }
 
 int fsg_launch_core_fast(cudaStream_t st, const CoreJob &J, const float4 *vtab4, int *err) {
     const int ntiles = (J.nwl + 31) / 32;
-    const int D = core_depths(J.ntau), nwarps = (J.ntau + D - 1) / D;
-    if (nwarps > 18) return FSG_E_ARG;
-    const int chc = core_chunk(J.ntau);
-    const size_t smem = core_smem(J.ntau, chc);
-    if (D == 4) {
-        cudaFuncSetAttribute(k_core_fast<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_core_fast<4><<<ntiles, 32 * nwarps, smem, st>>>(J, vtab4, chc, err);
-    } else {
-        cudaFuncSetAttribute(k_core_fast<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_core_fast<8><<<ntiles, 32 * nwarps, smem, st>>>(J, vtab4, chc, err);
-    }
+    const unsigned grid = (unsigned)(((int64_t)ntiles * fsg_core_groups(J.ntau) + CORE_W - 1) / CORE_W);
+    k_core_fast<<<grid, 32 * CORE_W, 0, st>>>(J, ntiles, vtab4, err);
     return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }
 
-int fsg_launch_core_batch(cudaStream_t st, int ntau_max, const CoreJob *jobs, const int *tile0, int njobs,
+// the persistent core pass over njobs jobs (device array) of at most ntau_max depths; ctas counts CTAs of one
+// warp per depth group
+int fsg_launch_core_batch(cudaStream_t st, int ntau_max, const CoreJob *jobs, const int *item0, int njobs,
                           int ctas, const float4 *vtab4, unsigned *queue, int *err) {
-    const int D = core_depths(ntau_max), nwarps = (ntau_max + D - 1) / D;
-    if (nwarps > 18) return FSG_E_ARG;
-    const int chc = core_chunk(ntau_max);
-    const size_t smem = core_smem(ntau_max, chc);
-    if (D == 4) {
-        cudaFuncSetAttribute(k_core_batch<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_core_batch<4><<<ctas, 32 * nwarps, smem, st>>>(jobs, tile0, njobs, ntau_max, chc, vtab4, queue, err);
-    } else {
-        cudaFuncSetAttribute(k_core_batch<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_core_batch<8><<<ctas, 32 * nwarps, smem, st>>>(jobs, tile0, njobs, ntau_max, chc, vtab4, queue, err);
-    }
+    const int64_t warps = (int64_t)ctas * fsg_core_groups(ntau_max);
+    k_core_batch<<<(unsigned)((warps + CORE_W - 1) / CORE_W), 32 * CORE_W, 0, st>>>(jobs, item0, njobs, vtab4, queue, err);
     return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }
 

@@ -139,7 +139,7 @@ struct WingJob {
 
 // One core-pass job: as WingJob with the core records; tiles of 32 wavelengths.  nevals (may be
 // null) counts the evaluations.  extra_tx / wait_ns: 0 and WAIT_NS in use; a test of the error path
-// (fsg_set_fault) makes every chunk expect extra_tx bytes more than its copies deliver and bounds the waits
+// (fsg_set_fault) makes every group of lines expect extra_tx bytes more than its copies deliver and bounds the waits
 // by wait_ns.
 struct CoreJob {
     int ntau, nwl;
@@ -153,6 +153,8 @@ struct CoreJob {
     unsigned long long wait_ns;
     int nseg, seg_stride;
 };
+// depth groups of the core pass (8 depths per warp)
+__host__ __device__ inline int fsg_core_groups(int ntau) { return (ntau + 7) >> 3; }
 
 // Rays of a spherical model (SphereInit, solver.f90:45-120), device arrays [nmu][stride], stride =
 // 2 ntau.  Ray im has n[im] points (ntau, or 2 n for a grazing ray that turns below layer n); point k

@@ -337,7 +337,7 @@ int fsg_adjoint_range_dev(fsg_ctx *ctx, const fsg_lines *d_lines, const int32_t 
 /* ---- failure injection, for tests of the error paths (no counterpart in the reference) -------
  * FSG_FAULT_ALLOC_LIMIT: the context's device allocations larger than value bytes fail as on an
  * exhausted device (FSG_E_NOMEM with the buffer's name; the context stays usable).
- * FSG_FAULT_COPY_TIMEOUT: every chunk of line records the accumulation kernels stage expects 16 bytes
+ * FSG_FAULT_COPY_TIMEOUT: every group of line records the core pass stages expects 16 bytes
  * more than its bulk copies deliver, so its mbarrier phase never completes and the bounded wait gives
  * up after value milliseconds (0.01-1000); the copies themselves complete, the kernel drains and
  * returns, and the call reports FSG_E_TIMEOUT.  FSG_FAULT_NONE restores normal operation. */
@@ -366,7 +366,8 @@ typedef struct fsg_batch fsg_batch;
 typedef struct {
     int32_t tile_pix;       /* wing-pass tile width of the wide classes (windows over 512
                              * wavelengths): 64 or 128; the narrower ones take 64 */
-    int32_t wing_ctas, core_ctas;   /* CTAs of the persistent wing / core launches */
+    int32_t wing_ctas, core_ctas;   /* size of the persistent launches: 16 warps each (wing), a warp per
+                             * 8 depths of the deepest atmosphere each (core) */
     double  ms_wing, ms_core;       /* their times in the tuning run [ms] */
 } fsg_batch_tuning;
 typedef struct {

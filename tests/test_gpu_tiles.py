@@ -27,7 +27,7 @@ def case(ntau, nwl, n, seed):
 
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
 @pytest.mark.parametrize("ntau,nwl,n", [(3, 2, 1), (4, 63, 7), (5, 64, 9), (9, 65, 33), (31, 127, 40), (64, 129, 200),
-                                        (65, 1000, 31), (127, 257, 65), (96, 513, 100)])
+                                        (65, 1000, 31), (127, 257, 65), (96, 513, 100), (8, 32, 16), (17, 33, 17)])
 def test_tile_edges(fsg, oracle_mod, prec, ntau, nwl, n):
     grid, st, co, a = case(ntau, nwl, n, 17 * ntau + nwl)
     C = fsg.Context(precision=fsg.PREC_FP64 if prec == "fp64" else fsg.PREC_MIXED, vmicro=1.0)
