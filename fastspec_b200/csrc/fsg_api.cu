@@ -2363,9 +2363,9 @@ static int adjoint_common(fsg_ctx *ctx, const fsg_lines *d_lines, const int32_t 
 // Batched synthesis: many atmospheres (each an fsg_ctx with grid, atmosphere, continuum and mu
 // set), one shared line list.  Per atmosphere: central pass of the lines in its span (plus a
 // margin), their records in window-width-class order (block refill), tile ranges per class; then
-// per group of atmospheres of like depth count and per class, a persistent wing-pass launch and a
-// persistent core-pass launch take (atmosphere, tile) items from device work queues; then the formal
-// solver and flux of each atmosphere.  The whole sequence has no host synchronisation and is captured
+// two persistent wing-pass launches (narrow and wide classes) and a persistent core-pass launch take
+// (atmosphere, tile, depth group) items from device work queues; then the formal solver and flux of
+// each atmosphere.  The whole sequence has no host synchronisation and is captured
 // once as a CUDA graph; later runs replay it.  The wide classes' tile width and the CTA counts of
 // the persistent launches are chosen by timing the candidates on the first run (fsg_batch_tune).
 // ================================================================================================
@@ -2469,10 +2469,9 @@ static int batch_prepare(fsg_batch *b, int P) {
     return FSG_OK;
 }
 
-// Job tables and queue prefix sums (host, then uploaded).  Atmospheres are grouped by depth count
-// (buckets of 8 depths), so a persistent launch is shaped for its own group's deepest member and few
-// warps idle.  Per group three launches, each with one job per atmosphere (so no two CTAs of a launch
-// update the same LineOpac tile): the wing pass over the narrow classes (64-wavelength tiles), the
+// Job tables and queue prefix sums (host, then uploaded).  Three persistent launches, each with one job per
+// atmosphere (so no two warps of a launch update the same LineOpac tile; the items are depth groups of a tile, so
+// atmospheres of all depth counts share a launch and only its own end leaves warps idle): the wing pass over the narrow classes (64-wavelength tiles), the
 // wing pass over the wide ones (32 P), the core pass over all; a job's tile takes its classes' lines
 // in turn into one sum.
 static int batch_jobs(fsg_batch *b, int P) {
@@ -2480,39 +2479,36 @@ static int batch_jobs(fsg_batch *b, int P) {
     std::vector<WingJob> jw; std::vector<CoreJob> jc;
     std::vector<int> tw, tc;
     b->lw.clear(); b->lc.clear();
-    for (int bucket = 0; bucket * 8 < 128; bucket++) {
-        int ntmax = 0;
-        for (auto &a : b->atm)
-            if (a.cn && (a.ctx->ntau - 1) / 8 == bucket) ntmax = std::max(ntmax, a.ctx->ntau);
-        if (!ntmax) continue;
-        for (int kind = 0; kind < 3; kind++) {             // narrow wing, wide wing, core
-            const int Pk = kind == 0 ? 2 : P;
-            std::vector<int> &t0 = kind < 2 ? tw : tc;
-            fsg_batch::Launch L{ ntmax, Pk, (int)(kind < 2 ? jw.size() : jc.size()), 0, (int)t0.size() };
-            t0.push_back(0);
-            for (auto &a : b->atm) {
-                fsg_ctx *c = a.ctx;
-                if (a.cn == 0 || (c->ntau - 1) / 8 != bucket) continue;
-                const int c0 = kind == 1 ? WING_NARROW + 1 : 0;
-                const int nseg = kind == 0 ? std::min(a.ncls, WING_NARROW + 1) : kind == 1 ? a.ncls - c0 : a.ncls;
-                if (nseg <= 0) continue;
-                const int ws = batch_wing_stride(c), cs = batch_core_stride(c);
-                if (kind < 2) {
-                    jw.push_back(WingJob{ c->ntau, c->nwl, c->d_wave.as<double>(), a.hdr.as<LineHdr>(),
-                                          a.wing.as<WingPair>(), a.wtlo.as<int>() + (size_t)c0 * ws,
-                                          a.wthi.as<int>() + (size_t)c0 * ws, c->d_lineopac.as<double>(), nseg, ws, 0 });
-                    t0.push_back(t0.back() + (c->nwl + 32 * Pk - 1) / (32 * Pk) * fsg_wing_groups(Pk, c->ntau));
-                } else {
-                    jc.push_back(CoreJob{ c->ntau, c->nwl, c->d_wave.as<double>(), a.hdr.as<LineHdr>(),
-                                          a.core.as<CoreRec>(), a.ctlo.as<int>(), a.cthi.as<int>(),
-                                          c->d_lineopac.as<double>(), b->evals.as<unsigned long long>(), 0u, WAIT_NS,
-                                          nseg, cs });
-                    t0.push_back(t0.back() + (c->nwl + 31) / 32 * fsg_core_groups(c->ntau));
-                }
-                L.nj++;
+    int ntmax = 0;
+    for (auto &a : b->atm)
+        if (a.cn) ntmax = std::max(ntmax, a.ctx->ntau);
+    for (int kind = 0; kind < 3 && ntmax; kind++) {        // narrow wing, wide wing, core
+        const int Pk = kind == 0 ? 2 : P;
+        std::vector<int> &t0 = kind < 2 ? tw : tc;
+        fsg_batch::Launch L{ ntmax, Pk, (int)(kind < 2 ? jw.size() : jc.size()), 0, (int)t0.size() };
+        t0.push_back(0);
+        for (auto &a : b->atm) {
+            fsg_ctx *c = a.ctx;
+            if (a.cn == 0) continue;
+            const int c0 = kind == 1 ? WING_NARROW + 1 : 0;
+            const int nseg = kind == 0 ? std::min(a.ncls, WING_NARROW + 1) : kind == 1 ? a.ncls - c0 : a.ncls;
+            if (nseg <= 0) continue;
+            const int ws = batch_wing_stride(c), cs = batch_core_stride(c);
+            if (kind < 2) {
+                jw.push_back(WingJob{ c->ntau, c->nwl, c->d_wave.as<double>(), a.hdr.as<LineHdr>(),
+                                      a.wing.as<WingPair>(), a.wtlo.as<int>() + (size_t)c0 * ws,
+                                      a.wthi.as<int>() + (size_t)c0 * ws, c->d_lineopac.as<double>(), nseg, ws, 0 });
+                t0.push_back(t0.back() + (c->nwl + 32 * Pk - 1) / (32 * Pk) * fsg_wing_groups(Pk, c->ntau));
+            } else {
+                jc.push_back(CoreJob{ c->ntau, c->nwl, c->d_wave.as<double>(), a.hdr.as<LineHdr>(),
+                                      a.core.as<CoreRec>(), a.ctlo.as<int>(), a.cthi.as<int>(),
+                                      c->d_lineopac.as<double>(), b->evals.as<unsigned long long>(), 0u, WAIT_NS,
+                                      nseg, cs });
+                t0.push_back(t0.back() + (c->nwl + 31) / 32 * fsg_core_groups(c->ntau));
             }
-            if (L.nj) (kind < 2 ? b->lw : b->lc).push_back(L);
+            L.nj++;
         }
+        if (L.nj) (kind < 2 ? b->lw : b->lc).push_back(L);
     }
     ALLOC(b->jobs_w, sizeof(WingJob) * std::max<size_t>(jw.size(), 1));
     ALLOC(b->jobs_c, sizeof(CoreJob) * std::max<size_t>(jc.size(), 1));
