@@ -609,8 +609,8 @@ class Context:
 
     def radtran(self):
         """RadTranCalc + disk integration: (spl [nwl][nmu], spc, sfl [nwl], sfc)."""
-        spl = np.zeros((self.nwl, self.nmu)); spc = np.zeros((self.nwl, self.nmu))
-        sfl = np.zeros(self.nwl); sfc = np.zeros(self.nwl)
+        spl = np.empty((self.nwl, self.nmu)); spc = np.empty((self.nwl, self.nmu))
+        sfl = np.empty(self.nwl); sfc = np.empty(self.nwl)
         self._ck(self._lib.fsg_radtran(self.h, _p(spl, C.c_double), _p(spc, C.c_double), _p(sfl, C.c_double),
                                        _p(sfc, C.c_double)), "fsg_radtran")
         return spl, spc, sfl, sfc
@@ -644,8 +644,8 @@ class Context:
 
     def mag_radtran(self, bframe, bfield):
         bf = _f64(bfield)
-        spz = np.zeros((self.nwl, 4, self.nmu)); spc = np.zeros((self.nwl, self.nmu))
-        sfl = np.zeros(self.nwl); sfc = np.zeros(self.nwl)
+        spz = np.empty((self.nwl, 4, self.nmu)); spc = np.empty((self.nwl, self.nmu))
+        sfl = np.empty(self.nwl); sfc = np.empty(self.nwl)
         self._ck(self._lib.fsg_mag_radtran(self.h, int(bframe), _p(bf, C.c_double), len(bf), _p(spz, C.c_double),
                                            _p(spc, C.c_double), _p(sfl, C.c_double), _p(sfc, C.c_double)),
                  "fsg_mag_radtran")
