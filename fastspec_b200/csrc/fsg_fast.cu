@@ -12,7 +12,7 @@
 // headers and records to shared memory a group at a time, the next group's loads in flight while it works
 // through the present one; each thread keeps P x D FP32 partials over FOLD lines, folded into Kahan (sum,
 // compensation) pairs in shared memory.  Lines are binned by window width (class c holds windows of up to
-// 256 * 2^c wavelengths) and processed class by class, so a tile's candidate range stays close to the lines
+// 256 * 2^c wavelengths), a tile range for each class, so a tile's candidate range stays close to the lines
 // that touch it; narrow classes use 64-wavelength tiles, wide ones 128.
 //
 // Core pass (k_core_fast): over the core ranges, 32-wavelength tiles x 8 depths per warp, the points where s < 196: the
@@ -25,19 +25,18 @@
 #include <cub/device/device_scan.cuh>
 #include <cuda/functional>
 #include <algorithm>
-#include <type_traits>
 
 #define CLASS_W0 128      // class c: windows of at most CLASS_W0 * 2^(c+1) wavelengths
 
-// HVoigt * LinCop in FP32 outside the table (a >= 8 or |v| >= 8, s < 196): the two-term continued
+// HVoigt in FP32 outside the table (a >= 8 or |v| >= 8, s < 196): the two-term continued
 // fraction of voigt.f90:103-107 at |v| = av
-__device__ __forceinline__ float hv_cf32(float av, float a, float cop) {
+__device__ __forceinline__ float hv_cf32(float av, float a) {
     float a2 = a * a, v2 = av * av;
     float p = v2 - a2 - 1.5f, q = 2.0f * av * a;
     float dr = av * p - a * q, di = av * q + a * p;
     float r;                                            // the denominator is of the order of v^6: no subnormals
     asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"((p + 0.5f) * di - q * dr), "f"(dr * dr + di * di));
-    return 0.56418958354775628f * r * cop;
+    return 0.56418958354775628f * r;
 }
 
 // Kahan-compensated accumulation of one value
@@ -176,6 +175,19 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
                 part[j][k] = make_float2(0.0f, 0.0f);
             }
     };
+    auto flush = [&]() {                                // the Kahan pairs onto LineOpac
+#pragma unroll
+        for (int k = 0; k < P; k++) {
+            const int pix = p0 + lane + 32 * k;
+            double *dst = J.lineopac + (size_t)pix * ntau + t0;
+#pragma unroll
+            for (int d = 0; d < D; d++) {
+                float2 &ks = S.ksum[2 * ((d >> 1) * P + k) + (d & 1)][lane];
+                if (pix < nwl && t0 + d < ntau) dst[d] += (double)ks.x - (double)ks.y;
+                ks = make_float2(0.0f, 0.0f);
+            }
+        }
+    };
     auto offsets = [&](float4 h, float (&x)[P]) {       // x = dl^2 of the lane's wavelengths
 #pragma unroll
         for (int k = 0; k < P; k++) {
@@ -241,11 +253,11 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
     // One loop, so that each of the forms above stands in the code once: lines into the queue, a group of them
     // into flight, the group before through the arithmetic.
     int head = 0, cnt = 0, sg = 0, base = 0, hi = -1;
-    bool open = false;                                  // lines of segment sg are left to look at
+    bool open = false, some = false;                    // lines of segment sg are left to look at; some are not on LineOpac
     for (;;) {
         while (cnt < WING_G) {
             if (!open) {
-                if (sg == J.nseg || (J.fold_seg && (cnt || nnext || nfold))) break;
+                if (sg == J.nseg || (J.fold_seg && (cnt || nnext || some))) break;
                 base = J.tile_lo[sg * J.seg_stride + tile];
                 hi = J.tile_hi[sg * J.seg_stride + tile];
                 sg++;
@@ -273,27 +285,20 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
         head += n;
         cnt -= n;
         if (m) work(m, mp);
+        some = some || m;
         if (!n && !m) {                               // nothing in flight: the tile's lines, or this segment's, end here
+            const bool last = sg == J.nseg && !open;
             if (nfold) fold();
-            if (sg == J.nseg && !open) break;
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < P; k++) {
-        const int pix = p0 + lane + 32 * k;
-        if (pix >= nwl) continue;
-        double *dst = J.lineopac + (size_t)pix * ntau + t0;
-#pragma unroll
-        for (int j = 0; j < NP; j++) {
-            const float2 s0 = S.ksum[2 * (j * P + k)][lane], s1 = S.ksum[2 * (j * P + k) + 1][lane];
-            if (t0 + 2 * j < ntau) dst[2 * j] += (double)s0.x - (double)s0.y;
-            if (t0 + 2 * j + 1 < ntau) dst[2 * j + 1] += (double)s1.x - (double)s1.y;
+            if (some) flush();
+            some = false;
+            if (last) break;
         }
     }
 }
 
 #define WING_D 8                      // depths per warp
 #define WING_W 4                      // warps per CTA
+#define FEW_MAX 592
 #define WING_BW 8                     // warps per CTA of the persistent form
 
 // one (tile, depth group) per warp, the groups of a tile in turn
@@ -336,11 +341,20 @@ int fsg_class_pix(int cls) { return cls <= 1 ? 2 : 4; }
 // depth groups of the wing pass
 int fsg_wing_groups(int P, int ntau) { return (ntau + WING_D - 1) / WING_D; }
 
+// Few tiles: at eight depths a warp their warps would not fill a quarter of the 148 x 16 that are resident, so the pass
+// is the latency of its longest warp.  Two depths a warp then make four times as many of them, which set out together.
+// A depth's sum is the same in either form.  300 lines, 1,001 wavelengths: core pass 51 -> 25 us, wing pass 54 -> 31 us.
+static bool few_tiles(int ntiles, int ntau) { return (int64_t)ntiles * ((ntau + 7) / 8) < FEW_MAX; }
+
 // the wing pass of one job on tiles of 32 P wavelengths
 int fsg_launch_accum_fast(cudaStream_t st, int P, const WingJob &J) {
     const int TW = 32 * P, ntiles = (J.nwl + TW - 1) / TW;
-    const unsigned grid = (unsigned)(((int64_t)ntiles * fsg_wing_groups(P, J.ntau) + WING_W - 1) / WING_W);
-    if (P == 2) k_accum_fast<WING_D, 2><<<grid, 32 * WING_W, 0, st>>>(J, ntiles);
+    const bool few = few_tiles(ntiles, J.ntau);
+    const int D = few ? 2 : WING_D;
+    const unsigned grid = (unsigned)(((int64_t)ntiles * ((J.ntau + D - 1) / D) + WING_W - 1) / WING_W);
+    if (few && P == 2) k_accum_fast<2, 2><<<grid, 32 * WING_W, 0, st>>>(J, ntiles);
+    else if (few) k_accum_fast<2, 4><<<grid, 32 * WING_W, 0, st>>>(J, ntiles);
+    else if (P == 2) k_accum_fast<WING_D, 2><<<grid, 32 * WING_W, 0, st>>>(J, ntiles);
     else k_accum_fast<WING_D, 4><<<grid, 32 * WING_W, 0, st>>>(J, ntiles);
     return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }
@@ -378,14 +392,16 @@ int fsg_launch_accum_batch(cudaStream_t st, int P, const WingJob *jobs, const in
 #define CORE_G 16                     // lines per group
 #define CORE_W 4                      // warps per CTA
 
+template <int D>
 struct __align__(16) CoreWarp {
-    CoreRec rec[2][CORE_G][CORE_D];
+    CoreRec rec[2][CORE_G][D];
     LineHdr hdr[2][CORE_G];
     uint64_t bar[2];
     int queue[64];
 };
 
-__device__ __forceinline__ void core_bars_init(CoreWarp &S, int lane) {
+template <int D>
+__device__ __forceinline__ void core_bars_init(CoreWarp<D> &S, int lane) {
     if (lane == 0) {
         mbar_init(&S.bar[0], 1);
         mbar_init(&S.bar[1], 1);
@@ -394,12 +410,14 @@ __device__ __forceinline__ void core_bars_init(CoreWarp &S, int lane) {
     __syncwarp();
 }
 
-// One tile and depth group (depths t0 .. t0 + CORE_D - 1) of one job, by one warp with its mbarriers
+// One tile and depth group (depths t0 .. t0 + D - 1) of one job, by one warp with its mbarriers
 // initialised; kk counts the groups of lines the warp has staged (their buffer and phase parity) across calls.
 // Returns false after a copy did not complete within its bound (error in *err).
-__device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, const float4 *__restrict__ vtab4, CoreWarp &S,
+template <int D>
+__device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, const float4 *__restrict__ vtab4, CoreWarp<D> &S,
                                           int lane, unsigned &kk, int *err) {
-    const int ntau = J.ntau, nwl = J.nwl, nd = min(CORE_D, ntau - t0);
+    constexpr int E = D < 4 ? D : 4;               // depths at a time
+    const int ntau = J.ntau, nwl = J.nwl, nd = min(D, ntau - t0);
     bool any = false;                              // some segment has core ranges touching the tile
     for (int sg = 0; sg < J.nseg; sg++)
         any = any || J.tile_lo[sg * J.seg_stride + tile] <= J.tile_hi[sg * J.seg_stride + tile];
@@ -408,16 +426,16 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
     const int tile_first = tile * 32 + 1, tile_last = min(tile * 32 + 32, nwl);
     const double wd = J.wave[min(p, nwl - 1)];
     const float wvh = (float)wd, wvl = (float)(wd - (double)wvh);
-    float sum[CORE_D], cmp[CORE_D];
+    float sum[D], cmp[D];
 #pragma unroll
-    for (int d = 0; d < CORE_D; d++) { sum[d] = 0.0f; cmp[d] = 0.0f; }
+    for (int d = 0; d < D; d++) { sum[d] = 0.0f; cmp[d] = 0.0f; }
     unsigned cnt = 0;
     // records past the last depth: none of their points is a core point (the copies leave them as they are)
     if (lane < CORE_G * 2)
-        for (int d = nd; d < CORE_D; d++) {
+        for (int d = nd; d < D; d++) {
             CoreRec z{};
             z.c2m1 = 3.0e38f;
-            (&S.rec[0][0][0])[lane * CORE_D + d] = z;
+            (&S.rec[0][0][0])[lane * D + d] = z;
         }
     auto work = [&](int b, int n) {
         for (int q = 0; q < n; q++) {
@@ -428,18 +446,18 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
             const double adl = fabs(wd - ((double)h.wlh + (double)h.wll)), adl125 = adl * 125.0;
             const CoreRec *__restrict__ rec = S.rec[b][q];
 #pragma unroll
-            for (int g0 = 0; g0 < CORE_D; g0 += 4) {               // depths in groups of four
-                bool core[4], tab[4], some = false, cf = false;
+            for (int g0 = 0; g0 < D; g0 += E) {
+                bool core[E], tab[E], some = false, cf = false;
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
+                for (int e = 0; e < E; e++) {
                     core[e] = fmaf(x, rec[g0 + e].vv2, rec[g0 + e].c2m1) < 195.5f;
                     some = some || core[e];
                 }
                 if (!__any_sync(0xffffffffu, some)) continue;
-                float tv[4];
-                float4 gv[4];
+                float tv[E];
+                float4 gv[E];
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
+                for (int e = 0; e < E; e++) {
                     // column and fraction: 2^52 added towards minus infinity leaves floor(v / 0.008) in the low word
                     const double fv = adl125 * rec[g0 + e].vv, m = __dadd_rd(fv, 4503599627370496.0);
                     const int iv = __double2loint(m), ia = rec[g0 + e].ia;
@@ -450,29 +468,42 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
                 }
                 cf = __any_sync(0xffffffffu, cf);
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
+                for (int e = 0; e < E; e++) {
                     const CoreRec &cr = rec[g0 + e];
                     const float c0 = gv[e].x + tv[e] * (gv[e].y - gv[e].x), c1 = gv[e].z + tv[e] * (gv[e].w - gv[e].z);
-                    float v = (c0 + cr.ua * (c1 - c0)) * cr.cop;
+                    const float h = c0 + cr.ua * (c1 - c0);
+                    float y = fmaf(h, cr.cop, -cmp[g0 + e]);     // the Kahan step takes the product unrounded
                     if (cf) {
-                        const float w = hv_cf32((float)(adl * cr.vv), cr.a, cr.cop);
-                        v = tab[e] ? v : w;
+                        const float w = hv_cf32((float)(adl * cr.vv), cr.a);
+                        const float yc = fmaf(w, cr.cop, -cmp[g0 + e]);
+                        y = tab[e] ? y : yc;
                     }
                     if (core[e]) {
-                        KAHAN(sum[g0 + e], cmp[g0 + e], v);
+                        const float t = sum[g0 + e] + y;
+                        cmp[g0 + e] = (t - sum[g0 + e]) - y;
+                        sum[g0 + e] = t;
                         cnt++;
                     }
                 }
             }
         }
     };
+    auto flush = [&]() {                                // the Kahan pairs onto LineOpac
+        double *dst = J.lineopac + (size_t)p * ntau + t0;
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+            if (p < nwl && d < nd) dst[d] = dst[d] + ((double)sum[d] - (double)cmp[d]);
+            sum[d] = 0.0f;
+            cmp[d] = 0.0f;
+        }
+    };
     const unsigned bytes = (unsigned)(nd * (int)sizeof(CoreRec));
     int head = 0, ncand = 0, sg = 0, base = 0, hi = -1, nprev = 0;
-    bool ok = true;
+    bool ok = true, some = false;                       // some: lines since the last addition to LineOpac
     for (;;) {
         while (ncand < CORE_G) {                       // lines into the queue
             if (base > hi) {
-                if (sg == J.nseg) break;
+                if (sg == J.nseg || (J.fold_seg && (ncand || nprev || some))) break;
                 base = J.tile_lo[sg * J.seg_stride + tile];
                 hi = J.tile_hi[sg * J.seg_stride + tile];
                 sg++;
@@ -509,8 +540,13 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
             if (!ok) break;
             work(g & 1, nprev);
         }
+        some = some || nprev;
         nprev = n;
-        if (!n) break;
+        if (!n) {                                       // nothing in flight: the tile's lines, or this segment's, end here
+            if (some) flush();
+            some = false;
+            if (sg == J.nseg && base > hi) break;
+        }
     }
     if (!ok) {
         if (lane == 0) {
@@ -525,31 +561,27 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if (lane == 0 && v) atomicAdd(J.nevals, v);
     }
-    if (p >= nwl) return true;
-    double *dst = J.lineopac + (size_t)p * ntau + t0;
-#pragma unroll
-    for (int d = 0; d < CORE_D; d++)
-        if (d < nd) dst[d] = dst[d] + ((double)sum[d] - (double)cmp[d]);
     return true;
 }
 
 // one (tile, depth group) per warp, the groups of a tile in turn
+template <int D>
 __global__ void __launch_bounds__(32 * CORE_W, 5)
 k_core_fast(CoreJob J, int ntiles, const float4 *__restrict__ vtab4, int *__restrict__ err) {
-    __shared__ CoreWarp S[CORE_W];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ng = fsg_core_groups(J.ntau);
+    __shared__ CoreWarp<D> S[CORE_W];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ng = (J.ntau + D - 1) / D;
     const int64_t item = (int64_t)blockIdx.x * CORE_W + warp;
     if (item >= (int64_t)ntiles * ng) return;           // warps are independent: no CTA barrier
     core_bars_init(S[warp], lane);
     unsigned kk = 0;
-    core_tile(J, (int)(item / ng), (int)(item % ng) * CORE_D, vtab4, S[warp], lane, kk, err);
+    core_tile(J, (int)(item / ng), (int)(item % ng) * D, vtab4, S[warp], lane, kk, err);
 }
 
 // persistent form: warps take (job, tile, depth group) items from the queue
 __global__ void __launch_bounds__(32 * CORE_W, 4)
 k_core_batch(const CoreJob *__restrict__ jobs, const int *__restrict__ item0, int njobs,
              const float4 *__restrict__ vtab4, unsigned *queue, int *__restrict__ err) {
-    __shared__ CoreWarp S[CORE_W];
+    __shared__ CoreWarp<CORE_D> S[CORE_W];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     core_bars_init(S[warp], lane);
     unsigned kk = 0;
@@ -569,8 +601,10 @@ k_core_batch(const CoreJob *__restrict__ jobs, const int *__restrict__ item0, in
 
 int fsg_launch_core_fast(cudaStream_t st, const CoreJob &J, const float4 *vtab4, int *err) {
     const int ntiles = (J.nwl + 31) / 32;
-    const unsigned grid = (unsigned)(((int64_t)ntiles * fsg_core_groups(J.ntau) + CORE_W - 1) / CORE_W);
-    k_core_fast<<<grid, 32 * CORE_W, 0, st>>>(J, ntiles, vtab4, err);
+    const int D = few_tiles(ntiles, J.ntau) ? 2 : CORE_D;
+    const unsigned grid = (unsigned)(((int64_t)ntiles * ((J.ntau + D - 1) / D) + CORE_W - 1) / CORE_W);
+    if (D == 2) k_core_fast<2><<<grid, 32 * CORE_W, 0, st>>>(J, ntiles, vtab4, err);
+    else k_core_fast<CORE_D><<<grid, 32 * CORE_W, 0, st>>>(J, ntiles, vtab4, err);
     return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }
 

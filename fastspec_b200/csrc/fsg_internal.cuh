@@ -133,8 +133,8 @@ struct WingJob {
     const int *tile_lo, *tile_hi;
     double *lineopac;
     int nseg, seg_stride;
-    int fold_seg;                        // the FP32 partials end with each segment (a class's sum does not depend on
-                                         // the others')
+    int fold_seg;                        // each segment's sum is added to LineOpac by itself in FP64, as a launch of its
+                                         // own would
 };
 
 // One core-pass job: as WingJob with the core records; tiles of 32 wavelengths.  nevals (may be
@@ -152,6 +152,7 @@ struct CoreJob {
     unsigned extra_tx;
     unsigned long long wait_ns;
     int nseg, seg_stride;
+    int fold_seg;                        // as WingJob
 };
 // depth groups of the core pass (8 depths per warp)
 __host__ __device__ inline int fsg_core_groups(int ntau) { return (ntau + 7) >> 3; }

@@ -13,7 +13,8 @@
 // 2 nmu of them per column and depth.  So divisions are reciprocals (rcp64) times the numerator, constants are
 // multiplied, quantities of the depth scale alone are formed once per CTA, and the two DELO branches are
 // entered only by warps that need them.  482,832 wavelengths x 71 depths x 7 angles: 2.6 ms (5.6 ms when every
-// step divided and the Taylor branch's eight divisions were paid beside the exponential).
+// step divided and the Taylor branch's eight divisions were paid beside the exponential); 40,001 wavelengths x 7 rays
+// through a spherical model 0.30 ms (0.63); the central depths of 20,000 lines 0.13 ms (0.89 with a thread per line).
 #include "fsg_fp64.cuh"
 
 #define SOLVE_C 8

@@ -73,6 +73,25 @@ def test_paired_lines(fsg, step, nwl, n, eps):
     assert np.max(np.abs(m["lineopac"] - f["lineopac"]) / (f["lineopac"] + co)) < 2e-6
 
 
+@pytest.mark.parametrize("nwl,n", [(700, 40), (8001, 1500), (40001, 3000)])
+def test_one_launch_equals_launch_per_class(fsg, nwl, n):
+    """A list that fits one block takes its window-width classes in one launch, a longer one class by class (few and
+    many depths a warp, whole groups of lines and remainders).  Sums of FP32 terms in another grouping: a rounding
+    of 6e-8 for a class, 2e-7."""
+    grid, st, co, a = case(33, nwl, n, 5)
+    out = []
+    for ram in (16.0, 0.75 * n * 1632e-9):               # the records of three quarters of the lines
+        C = fsg.Context(vmicro=1.0, limitram_gb=ram)
+        C.set_grid(grid["wmode"], grid["wstart"], grid["wend"], grid["dstep"])
+        C.set_atmosphere(st)
+        C.set_contopac(co)
+        g = C.lineop_calc(fsg.LineList.from_arrays(a))
+        out.append((g["stats"]["nblocks"], g["lineopac"]))
+        C.close()
+    assert out[0][0] == 1 and out[1][0] > 1
+    np.testing.assert_allclose(out[0][1], out[1][1], rtol=2e-7, atol=0.0)
+
+
 @pytest.mark.parametrize("n", [32769, 45001])
 def test_central_pass_forms(fsg, n):
     """Flags and windows do not depend on how the central pass spreads its lines: a list above 32,768 lines takes
