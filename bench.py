@@ -906,7 +906,8 @@ def main():
         pass
     smmax = float(peaks.get("sm_max_mhz", 1965.0))
     fp32_peak = 148 * 128 * 2 * smmax * 1e6 / 1e12
-    # one reciprocal (MUFU) per wing evaluation; 16 MUFU results per SM and clock
+    # wing evaluations against 16 MUFU results per SM and clock (a single line takes one reciprocal per evaluation,
+    # a pair of lines one for two)
     xu_peak = 148 * 16 * smmax * 1e6
     xu_achieved = wing_evals / (st["ms_wing_kernels"] / 1e3)
     # DRAM bytes of one wing launch: the LineOpac read-modify-write and one read of the records
@@ -930,13 +931,13 @@ def main():
                      "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
                      "traffic": traffic,
                      "traffic_source": "per launch: LineOpac read + write (2 x nwl x ntau x 8 B) + the records of the "
-                                       "launch's lines (ntau x 16 + 32 B each); ncu dram__bytes_read.sum + "
-                                       "dram__bytes_write.sum of the 12 wing launches of the 1e6-line case = 0.92 x "
-                                       "this model",
+                                       "launch's lines (ntau x 16 + 32 B each); for an earlier form of the kernel ncu "
+                                       "dram__bytes_read.sum + dram__bytes_write.sum of the 12 wing launches of the "
+                                       "1e6-line case = 0.92 x this model",
                      "peak_source": "derived: 148 SMs x 128 FP32 lanes x 2 x %.0f MHz (no FP32 peak is measured)" % smmax,
                      "flops_per_eval": FLOPS_PER_EVAL, "evals_per_launch": wing_evals / nl,
                      "ms_per_launch": ms_launch,
-                     "xu": {"achieved": xu_achieved, "peak": xu_peak, "unit": "reciprocals/s",
+                     "xu": {"achieved": xu_achieved, "peak": xu_peak, "unit": "evaluations/s (peak: reciprocals/s)",
                             "frac": xu_achieved / xu_peak},
                      # the same launch against the measured copy bandwidth: far from HBM-bound
                      "hbm": {"achieved": traffic / (ms_launch / 1e3) / 1e9,
