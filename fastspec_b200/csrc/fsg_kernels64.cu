@@ -312,9 +312,9 @@ k_params_fast(AtmView A, LineView L, const int64_t *__restrict__ idx, int64_t j0
         f = flags[i];
         wlc = L.wl[i] - A.wfirst;
         xline_setup(A, L, i, wlc, f, &xs[wp][lane]);
-        const int il = ileft[i], ir = iright[i];
+        const int il = max(ileft[i], 1), ir = min(iright[i], A.nwl);
         double xm = 0.0;
-        if (il >= 1 && il <= ir && ir <= A.nwl) {
+        if (il <= ir) {
             const double dl = wlc - A.wave[il - 1], dr = wlc - A.wave[ir - 1];
             xm = fmax(dl * dl, dr * dr);
         }
@@ -394,7 +394,7 @@ k_params_fast(AtmView A, LineView L, const int64_t *__restrict__ idx, int64_t j0
     LineHdr h;
     h.wlh = (float)wlc;
     h.wll = (float)(wlc - (double)h.wlh);
-    h.ileft = ileft[i]; h.iright = iright[i];
+    h.ileft = max(ileft[i], 1); h.iright = min(iright[i], A.nwl);       // given windows may reach past the grid
     h.cl = 1; h.cr = 0;
     if (f & FSG_F_WEAK) { h.ileft = 1; h.iright = 0; }    // rejected line (batched lists): empty window
     else if (hcore >= 0.0) {

@@ -143,3 +143,32 @@ def test_range_adjoints_sum_to_the_whole_gradient(fsg):
     assert np.max(np.abs(sum_lin - ref_lin)) <= 1e-6 * scale
     assert np.max(np.abs(sum_vm - ref_vm)) <= 1e-6 * np.max(np.abs(ref_vm))
     assert np.count_nonzero(ref_lin) > n // 2
+
+
+def test_given_windows_past_the_grid(fsg):
+    """Windows given to fsg_accumulate_dev may reach past either end of the grid: the sums are those of the windows
+    cut at its ends, bit for bit.  Wide steps and full windows, so that some denominators of the wing form leave the
+    range in which two lines may share a reciprocal."""
+    from fastspec_b200 import shard
+    from fastspec_b200 import workloads as W
+    ntau, nwl, step, w0 = 33, 501, 9.0, 4000.0
+    st, _ = W.batch_atmosphere(5300.0, 4.2, ntau, {})
+    wave = fsg.make_grid(0, w0, w0 + (nwl - 0.5) * step, step) + w0
+    a = W.atomic_lines(4001, wave[0], wave[-1], nwl, exact=False).arrays()
+    C = fsg.Context(vmicro=1.0, epsopac=1e-14)
+    C.set_grid(0, w0, w0 + (nwl - 0.5) * step, step)
+    C.set_atmosphere(st)
+    C.set_contopac(np.tile(1e-2 * (1.0 + np.arange(ntau)), (nwl, 1)))
+    B = shard.GpuBackend(fsg, C, {k: torch.from_numpy(np.ascontiguousarray(v)).cuda() for k, v in a.items()})
+    win = B.central(0, B.n, B.n)
+    full = ((win[0] & 1) == 0) & (win[1] == 1) & (win[2] == nwl)     # their width class stays the widest
+    past = win.clone()
+    past[1][full] = -3
+    past[2][full] = nwl + 9
+    assert int(full.sum()) > B.n // 2
+    out = []
+    for w in (win, past):
+        B.accumulate(w, 1, nwl)
+        out.append(C.lineop_get())
+    assert np.array_equal(out[0], out[1])
+    C.close()
