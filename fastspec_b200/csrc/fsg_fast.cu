@@ -430,13 +430,17 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
 #pragma unroll
     for (int d = 0; d < D; d++) { sum[d] = 0.0f; cmp[d] = 0.0f; }
     unsigned cnt = 0;
-    // records past the last depth: none of their points is a core point (the copies leave them as they are)
-    if (lane < CORE_G * 2)
-        for (int d = nd; d < D; d++) {
-            CoreRec z{};
-            z.c2m1 = 3.0e38f;
-            (&S.rec[0][0][0])[lane * D + d] = z;
-        }
+    // records past the last depth: none of their points is a core point (the copies leave them as they are).  A later
+    // tile of the warp may have more depths there: its copies, of the async proxy, come after these stores
+    if (nd < D) {
+        if (lane < CORE_G * 2)
+            for (int d = nd; d < D; d++) {
+                CoreRec z{};
+                z.c2m1 = 3.0e38f;
+                (&S.rec[0][0][0])[lane * D + d] = z;
+            }
+        fence_proxy_async_shared();
+    }
     auto work = [&](int b, int n) {
         for (int q = 0; q < n; q++) {
             const LineHdr h = S.hdr[b][q];

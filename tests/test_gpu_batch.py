@@ -177,3 +177,22 @@ def test_batch_axis_shares(fsg):
     assert mine == list(range(len(ctxs)))
     for i, f in enumerate(res):
         check(i, f)
+
+
+def test_batch_partial_and_full_depth_groups_on_the_same_warps(fsg):
+    """The persistent core pass with one CTA: its warps go from groups of eight depths to the partial last group of an
+    atmosphere and back, over the same staging buffers.  The fluxes are those of a launch that fills the device, bit
+    for bit (an item's sum does not depend on the warp that takes it)."""
+    ctxs, cases, arr = small_batch(fsg, natm=6, seed=10)
+    left = [len(state["T"]) % 8 for _, state, _ in cases]
+    assert 0 in left and any(left)
+    B = fsg.Batch(ctxs, fsg.LineList.from_arrays(arr))
+    out = []
+    for ctas in (592, 1, 1):
+        B.set_tuning({"tile_pix": 64, "wing_ctas": 148, "core_ctas": ctas})
+        B.run()
+        out.append([B.flux(i)[0] for i in range(len(ctxs))])
+    for f in out[1:]:
+        for a, b in zip(out[0], f):
+            assert np.array_equal(a, b)
+    B.close()
