@@ -6,12 +6,24 @@
 
 // 1 / d for normal d in FP64: the hardware's approximate reciprocal r (relative error e, |e| < 2^-19)
 // and one third-order step r (1 + e + e^2), e = 1 - d r, which leaves e^3
-__device__ __forceinline__ double rcp64(double d) {
+__device__ __forceinline__ double rcp64_seed(double d) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    return r;
+}
+__device__ __forceinline__ double rcp64_refine(double d, double r) {
     double e = fma(-d, r, 1.0);
     e = fma(e, e, e);
     return fma(r, e, r);
+}
+__device__ __forceinline__ double rcp64(double d) { return rcp64_refine(d, rcp64_seed(d)); }
+
+// 1 / d of an optical-depth step, which is 0 where the opacity vanishes: as rcp64, and infinite there, as the division
+// is (rcp64(0) is NaN, which CentDer's test for slopes of one sign would turn into a finite slope of 0).  With the
+// seed kept finite, e = 1 - 0 r = 1 and the step overflows to infinity.
+__device__ __forceinline__ double rcp64_step(double d) {
+    const double r = rcp64_seed(d);
+    return rcp64_refine(d, __hiloint2double(min(__double2hiint(r), 0x7fefffff), __double2loint(r)));
 }
 
 // ---- Voigt table lerp, FP64 (voigt.f90:76-110, 113-154) -------------------------------------

@@ -393,7 +393,7 @@ k_stokes_prep(AtmView A, const double *__restrict__ lineopac, const double *__re
         sa = (p0 - pm) * rcp64(step(ta - 1));
         const double sq = ta > 1 ? (pm - point(ta - 2, yq)) * rcp64(step(ta - 2)) : 0.0;
         dprev = tau(ta - 1, pm, p0, sq, sa);
-        const double id = rcp64(dprev);
+        const double id = rcp64_step(dprev);
 #pragma unroll
         for (int q = 0; q < 10; q++) gp[q] = (y0[q] - ym[q]) * id;
     } else {
@@ -407,7 +407,7 @@ k_stokes_prep(AtmView A, const double *__restrict__ lineopac, const double *__re
             const double sb = (p1 - p0) * rcp64(step(t));
             d = tau(t, p0, p1, sa, sb);
             F(21, t) = d;
-            const double id = rcp64(d), lam = t > 0 ? lambda_of(dprev, d) : 0.0;
+            const double id = rcp64_step(d), lam = t > 0 ? lambda_of(dprev, d) : 0.0;
 #pragma unroll
             for (int q = 0; q < 10; q++) {
                 const double gn = (y1[q] - y0[q]) * id;

@@ -28,10 +28,10 @@ __device__ __forceinline__ double delo_step(double d, double Y, double y0, doubl
 
 // CentDer (solver.f90:618-647) of y on the scale of the steps d, at point t of nt
 __device__ __forceinline__ double centder_at(const double *d, const double *y, int nt, int t) {
-    if (t == 0) return (y[1] - y[0]) * rcp64(d[0]);
-    if (t == nt - 1) return (y[nt - 1] - y[nt - 2]) * rcp64(d[nt - 2]);
+    if (t == 0) return (y[1] - y[0]) * rcp64_step(d[0]);
+    if (t == nt - 1) return (y[nt - 1] - y[nt - 2]) * rcp64_step(d[nt - 2]);
     const double dx = d[t - 1], dx1 = d[t];
-    return hmean((y[t] - y[t - 1]) * rcp64(dx), (y[t + 1] - y[t]) * rcp64(dx1), lambda_of(dx, dx1));
+    return hmean((y[t] - y[t - 1]) * rcp64_step(dx), (y[t + 1] - y[t]) * rcp64_step(dx1), lambda_of(dx, dx1));
 }
 
 // shared memory of a CTA: source S[c][ld], opacities X[kind][c][ld] (later the Bezier terms), steps
@@ -123,7 +123,7 @@ __device__ __forceinline__ double sweep_ray(const RayView &R, int im, const doub
     int l1 = mp[N - 1], l0 = mp[N - 2], lp = N > 2 ? mp[N - 3] : 0;
     double xc = x[l1], xb = x[l0], xa = x[lp];
     double sl1 = (xc - xb) * idm[N - 2], sl0 = N > 2 ? (xb - xa) * idm[N - 3] : 0.0;
-    double dcur = tau(N - 2, xb, xc, sl0, sl1), icur = rcp64(dcur);
+    double dcur = tau(N - 2, xb, xc, sl0, sl1), icur = rcp64_step(dcur);
     double y1 = y[l1], y0 = y[l0];
     double g1 = (y1 - y0) * icur, r1 = g1;               // slope of the source over the step; CentDer at j + 1
     double Y = R.graz[im] ? 0.0 : y1;
@@ -135,7 +135,7 @@ __device__ __forceinline__ double sweep_ray(const RayView &R, int im, const doub
             sl1 = sl0;
             sl0 = j > 1 ? (xb - xa) * idm[j - 2] : 0.0;
             dprev = tau(j - 1, xb, xc, sl0, sl1);
-            iprev = rcp64(dprev);
+            iprev = rcp64_step(dprev);
             yp = y[mp[j - 1]];
             g0 = (y0 - yp) * iprev;
             r0 = hmean(g0, g1, lambda_of(dprev, dcur));

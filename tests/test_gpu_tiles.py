@@ -164,6 +164,47 @@ def test_solver_edges(fsg, oracle_mod, ntau, nwl, nmu):
     C.close()
 
 
+@pytest.mark.parametrize("sphere", [False, True])
+def test_solver_without_opacity(fsg, oracle_mod, sphere):
+    """Layers whose opacities cancel to 0, are infinite or are no number: optical-depth steps of 0, whose reciprocals
+    are infinite.  The intensities are numbers exactly where the oracle's are; those within 1e-10 of the disk-centre
+    continuum, the bar of the intensities."""
+    ntau, nwl, nmu = 56, 160, 5
+    grid, st, co, _ = case(ntau, nwl, 1, 0)
+    x, w, _ = fsg.mu_quadrature(1, nmu)
+    lo = co * 10.0 ** np.random.default_rng(7).uniform(-2.0, 2.0, co.shape)
+    k = 0
+    for run in (1, 2, 3, 6):
+        for d in (0, 1, 7, 20, 21, 22, ntau - run - 1, ntau - run):
+            lo[k, d:d + run] = -co[k, d:d + run]
+            k += 1
+    for v in (np.inf, -np.inf, np.nan):
+        for d in (0, 1, 25, ntau - 2, ntau - 1):
+            lo[k, d] = v
+            k += 1
+    assert k < nwl
+    C = fsg.Context(vmicro=1.0)
+    C.set_grid(grid["wmode"], grid["wstart"], grid["wend"], grid["dstep"])
+    C.set_atmosphere(st)
+    C.set_contopac(co)
+    C.set_mu(x, w)
+    S = oracle_mod.State(grid, st, contopac=co, vmicro=1.0)
+    if sphere:
+        from fastspec_b200 import workloads as W
+        h = W.model_heights(st["rhox"], st["rho"])
+        radius = 250.0 * float(h[0] - h[-1])
+        C.set_geometry(radius, h)
+        S.set_sphere(radius, h, x)
+    C.lineop_set(lo)
+    spl, spc, _, _ = C.radtran()
+    ospl, ospc = oracle_mod.radtran(S, x, lo)
+    np.testing.assert_array_equal(np.isfinite(spl), np.isfinite(ospl))
+    ok = np.isfinite(ospl)
+    assert 0 < np.count_nonzero(~ok) < ok.size // 2
+    assert np.max((np.abs(spl - ospl) / ospc[:, :1])[ok]) < 1e-10
+    C.close()
+
+
 @pytest.mark.parametrize("nwl,nmu,vsini,vmacro,vgau", [(9, 2, 0.0, 0.0, 0.0), (9, 3, 30.0, 5.0, 2.0e4), (640, 7, 12.0, 0.0, 0.0),
                                                        (641, 16, 0.0, 3.0, 9.0e4), (1283, 5, 40.0, 6.0, 5.0),
                                                        (3000, 1, 7.0, 2.0, 0.0), (14001, 3, 900.0, 90.0, 3.0e3)])
