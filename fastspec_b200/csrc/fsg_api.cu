@@ -796,11 +796,9 @@ static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, int64_t nmax, fsg_s
         return WingJob{ nt, ctx->nwl, ctx->d_wave.as<double>(), hdr, wing, tlo, thi, ctx->d_lineopac.as<double>(), nseg,
                         stride, 1 };
     };
-    // the core pass adds a class's sum by itself for short lists, where the grouping of FP32 sums shows most in the flux
-    // (1e-9 of it at 100 lines, 1e-10 at 6,000); a million lines take 19 ms that way, 11 ms in one sum
     auto core_job = [&](const int *tlo, const int *thi, int nseg, int stride) {
         return CoreJob{ nt, ctx->nwl, ctx->d_wave.as<double>(), hdr, core, tlo, thi, ctx->d_lineopac.as<double>(),
-                        &dres->ncore, ctx->fault_extra_tx, ctx->fault_wait_ns, nseg, stride, nmax <= 8192 };
+                        &dres->ncore, ctx->fault_extra_tx, ctx->fault_wait_ns, nseg, stride };
     };
     // A list whose records fit one block (LIMITRAM) is one record array in window-width-class order: one launch
     // per step for all classes, each tile adding its classes in turn, and no count needed on the host.  Lists that
@@ -2540,7 +2538,7 @@ static int batch_jobs(fsg_batch *b, int P) {
                 jc.push_back(CoreJob{ c->ntau, c->nwl, c->d_wave.as<double>(), a.hdr.as<LineHdr>(),
                                       a.core.as<CoreRec>(), a.ctlo.as<int>(), a.cthi.as<int>(),
                                       c->d_lineopac.as<double>(), b->evals.as<unsigned long long>(), 0u, WAIT_NS,
-                                      nseg, cs, 0 });
+                                      nseg, cs });
                 t0.push_back(t0.back() + (c->nwl + 31) / 32 * fsg_core_groups(c->ntau));
             }
             L.nj++;

@@ -385,23 +385,30 @@ int fsg_launch_accum_batch(cudaStream_t st, int P, const WingJob *jobs, const in
 // What bounds it: instruction issue (60 to 70 % of the cycles) and the gathers, one 128-byte line of L1 a lane.  Hence
 // floor() by an addition and not by conversions (the conversion unit takes 8 cycles a warp, the FP64 one 2), the
 // continued fraction and whole depth groups left out where no lane needs them, and no barrier between depth groups.
-// Against a CTA per tile that staged all depths of a chunk: 1e6 lines, 483,000 wavelengths, 56 depths 15.4 -> 10.9 ms; a
-// batch of 24 atmospheres 19.7 -> 12.9 ms; 20,000 lines, 40,001 wavelengths 736 -> 480 us.  5 CTAs a SM (96
+// Against a CTA per tile that staged all depths of a chunk: 1e6 lines, 483,000 wavelengths, 56 depths 15.4 -> 11.5 ms; a
+// batch of 24 atmospheres 19.7 -> 12.9 ms; 20,000 lines, 40,001 wavelengths 736 -> 500 us.  5 CTAs a SM (96
 // registers): 4 take 7 % longer, 6 spill; the persistent form spills at 5.
+//
+// The segments' Kahan sums are added in FP64 (one sum over all classes of a long list is 3 % further from 64 bits: rms of
+// LineOpac 5.2e-8 against 5.05e-8 for 50,000 molecular lines), in shared memory: added to LineOpac one by one they take
+// 19.0 ms for those 1e6 lines.  Ten lines a group then, of one segment: 6 take 11.66 ms, 8 11.56, 10 11.48, 15 13.6 (less
+// L1 for the gathers).  The two-depth form adds to LineOpac itself: 31 us for 300 lines, 37 through shared memory.
 #define CORE_D 8                      // depths per warp (two groups of four gathers)
-#define CORE_G 16                     // lines per group
+#define CORE_FEW 2                    // ... where there are few tiles
+#define CORE_G 10                     // lines per group
+#define CORE_GB 16                    // ... in the persistent form, which keeps no sums in shared memory
 #define CORE_W 4                      // warps per CTA
 
-template <int D>
+template <int D, int G>
 struct __align__(16) CoreWarp {
-    CoreRec rec[2][CORE_G][D];
-    LineHdr hdr[2][CORE_G];
+    CoreRec rec[2][G][D];
+    LineHdr hdr[2][G];
     uint64_t bar[2];
     int queue[64];
 };
 
-template <int D>
-__device__ __forceinline__ void core_bars_init(CoreWarp<D> &S, int lane) {
+template <class S_>
+__device__ __forceinline__ void core_bars_init(S_ &S, int lane) {
     if (lane == 0) {
         mbar_init(&S.bar[0], 1);
         mbar_init(&S.bar[1], 1);
@@ -412,10 +419,14 @@ __device__ __forceinline__ void core_bars_init(CoreWarp<D> &S, int lane) {
 
 // One tile and depth group (depths t0 .. t0 + D - 1) of one job, by one warp with its mbarriers
 // initialised; kk counts the groups of lines the warp has staged (their buffer and phase parity) across calls.
-// Returns false after a copy did not complete within its bound (error in *err).
-template <int D>
-__device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, const float4 *__restrict__ vtab4, CoreWarp<D> &S,
-                                          int lane, unsigned &kk, int *err) {
+// PER_SEG: each segment's Kahan sums are added up in FP64, in tot (shared memory, [D][32]; null: LineOpac itself);
+// otherwise one Kahan sum runs over all segments.  Returns false after a copy did not complete within its bound (error
+// in *err).
+template <bool PER_SEG, int D, int G>
+__device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, const float4 *__restrict__ vtab4, CoreWarp<D, G> &S,
+                                          double (*tot)[32], int lane, unsigned &kk, int *err) {
+    static_assert(2 * G <= 32, "a lane fills one line's padding");
+    constexpr bool TOT = PER_SEG && D > CORE_FEW;
     constexpr int E = D < 4 ? D : 4;               // depths at a time
     const int ntau = J.ntau, nwl = J.nwl, nd = min(D, ntau - t0);
     bool any = false;                              // some segment has core ranges touching the tile
@@ -428,12 +439,16 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
     const float wvh = (float)wd, wvl = (float)(wd - (double)wvh);
     float sum[D], cmp[D];
 #pragma unroll
-    for (int d = 0; d < D; d++) { sum[d] = 0.0f; cmp[d] = 0.0f; }
+    for (int d = 0; d < D; d++) {
+        sum[d] = 0.0f;
+        cmp[d] = 0.0f;
+        if (TOT) tot[d][lane] = 0.0;
+    }
     unsigned cnt = 0;
     // records past the last depth: none of their points is a core point (the copies leave them as they are).  A later
     // tile of the warp may have more depths there: its copies, of the async proxy, come after these stores
     if (nd < D) {
-        if (lane < CORE_G * 2)
+        if (lane < G * 2)
             for (int d = nd; d < D; d++) {
                 CoreRec z{};
                 z.c2m1 = 3.0e38f;
@@ -492,25 +507,19 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
             }
         }
     };
-    auto flush = [&]() {                                // the Kahan pairs onto LineOpac
-        double *dst = J.lineopac + (size_t)p * ntau + t0;
-#pragma unroll
-        for (int d = 0; d < D; d++) {
-            if (p < nwl && d < nd) dst[d] = dst[d] + ((double)sum[d] - (double)cmp[d]);
-            sum[d] = 0.0f;
-            cmp[d] = 0.0f;
-        }
-    };
     const unsigned bytes = (unsigned)(nd * (int)sizeof(CoreRec));
+    double *dst = J.lineopac + (size_t)p * ntau + t0;
     int head = 0, ncand = 0, sg = 0, base = 0, hi = -1, nprev = 0;
-    bool ok = true, some = false;                       // some: lines since the last addition to LineOpac
+    bool ok = true;
     for (;;) {
-        while (ncand < CORE_G) {                       // lines into the queue
+        bool cut = false;                              // the group in flight is the last of its segment
+        while (ncand < G) {                            // lines into the queue
             if (base > hi) {
-                if (sg == J.nseg || (J.fold_seg && (ncand || nprev || some))) break;
+                if (sg == J.nseg || (PER_SEG && ncand)) break;     // no group of two segments
                 base = J.tile_lo[sg * J.seg_stride + tile];
                 hi = J.tile_hi[sg * J.seg_stride + tile];
                 sg++;
+                cut = true;
                 continue;
             }
             const int i = base + lane;
@@ -525,7 +534,7 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
             ncand += __popc(m);
         }
         __syncwarp();                                   // the queue is written, and the buffer's last group done with
-        const int n = min(ncand, CORE_G), b = kk & 1;
+        const int n = min(ncand, G), b = kk & 1;
         if (n) {                                        // a group into flight
             if (lane == 0) mbar_expect_tx(&S.bar[b], n * bytes + J.extra_tx);
             __syncwarp();
@@ -543,14 +552,24 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
             ok = __all_sync(0xffffffffu, mbar_wait(&S.bar[g & 1], (g >> 1) & 1, J.wait_ns));
             if (!ok) break;
             work(g & 1, nprev);
+            if (PER_SEG && (cut || !n)) {
+#pragma unroll
+                for (int d = 0; d < D; d++) {
+                    const double v = (double)sum[d] - (double)cmp[d];
+                    if (TOT) tot[d][lane] += v;
+                    else if (p < nwl && d < nd) dst[d] += v;
+                    sum[d] = 0.0f;
+                    cmp[d] = 0.0f;
+                }
+            }
         }
-        some = some || nprev;
         nprev = n;
-        if (!n) {                                       // nothing in flight: the tile's lines, or this segment's, end here
-            if (some) flush();
-            some = false;
-            if (sg == J.nseg && base > hi) break;
-        }
+        if (!n) break;                                  // nothing in flight and no line left
+    }
+    if (ok && p < nwl && (TOT || !PER_SEG)) {
+#pragma unroll
+        for (int d = 0; d < D; d++)
+            if (d < nd) dst[d] += TOT ? tot[d][lane] : (double)sum[d] - (double)cmp[d];
     }
     if (!ok) {
         if (lane == 0) {
@@ -572,20 +591,22 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
 template <int D>
 __global__ void __launch_bounds__(32 * CORE_W, 5)
 k_core_fast(CoreJob J, int ntiles, const float4 *__restrict__ vtab4, int *__restrict__ err) {
-    __shared__ CoreWarp<D> S[CORE_W];
+    __shared__ CoreWarp<D, CORE_G> S[CORE_W];
+    __shared__ double tot_s[D > CORE_FEW ? CORE_W : 1][D][32];
+    double (*tot)[32] = D > CORE_FEW ? tot_s[threadIdx.x >> 5] : nullptr;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ng = (J.ntau + D - 1) / D;
     const int64_t item = (int64_t)blockIdx.x * CORE_W + warp;
     if (item >= (int64_t)ntiles * ng) return;           // warps are independent: no CTA barrier
     core_bars_init(S[warp], lane);
     unsigned kk = 0;
-    core_tile(J, (int)(item / ng), (int)(item % ng) * D, vtab4, S[warp], lane, kk, err);
+    core_tile<true>(J, (int)(item / ng), (int)(item % ng) * D, vtab4, S[warp], tot, lane, kk, err);
 }
 
 // persistent form: warps take (job, tile, depth group) items from the queue
 __global__ void __launch_bounds__(32 * CORE_W, 4)
 k_core_batch(const CoreJob *__restrict__ jobs, const int *__restrict__ item0, int njobs,
              const float4 *__restrict__ vtab4, unsigned *queue, int *__restrict__ err) {
-    __shared__ CoreWarp<CORE_D> S[CORE_W];
+    __shared__ CoreWarp<CORE_D, CORE_GB> S[CORE_W];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     core_bars_init(S[warp], lane);
     unsigned kk = 0;
@@ -599,15 +620,15 @@ k_core_batch(const CoreJob *__restrict__ jobs, const int *__restrict__ item0, in
         while (a < b) { int m = (a + b + 1) >> 1; if (item0[m] <= item) a = m; else b = m - 1; }
         const CoreJob J = jobs[a];
         const int ng = fsg_core_groups(J.ntau), r = item - item0[a];
-        if (!core_tile(J, r / ng, (r % ng) * CORE_D, vtab4, S[warp], lane, kk, err)) break;
+        if (!core_tile<false>(J, r / ng, (r % ng) * CORE_D, vtab4, S[warp], nullptr, lane, kk, err)) break;
     }
 }
 
 int fsg_launch_core_fast(cudaStream_t st, const CoreJob &J, const float4 *vtab4, int *err) {
     const int ntiles = (J.nwl + 31) / 32;
-    const int D = few_tiles(ntiles, J.ntau) ? 2 : CORE_D;
+    const int D = few_tiles(ntiles, J.ntau) ? CORE_FEW : CORE_D;
     const unsigned grid = (unsigned)(((int64_t)ntiles * ((J.ntau + D - 1) / D) + CORE_W - 1) / CORE_W);
-    if (D == 2) k_core_fast<2><<<grid, 32 * CORE_W, 0, st>>>(J, ntiles, vtab4, err);
+    if (D == CORE_FEW) k_core_fast<CORE_FEW><<<grid, 32 * CORE_W, 0, st>>>(J, ntiles, vtab4, err);
     else k_core_fast<CORE_D><<<grid, 32 * CORE_W, 0, st>>>(J, ntiles, vtab4, err);
     return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }

@@ -152,7 +152,6 @@ struct CoreJob {
     unsigned extra_tx;
     unsigned long long wait_ns;
     int nseg, seg_stride;
-    int fold_seg;                        // as WingJob
 };
 // depth groups of the core pass (8 depths per warp)
 __host__ __device__ inline int fsg_core_groups(int ntau) { return (ntau + 7) >> 3; }

@@ -92,6 +92,29 @@ def test_one_launch_equals_launch_per_class(fsg, nwl, n):
     np.testing.assert_allclose(out[0][1], out[1][1], rtol=2e-7, atol=0.0)
 
 
+@pytest.mark.parametrize("nwl,n", [(701, 60), (4001, 900), (24001, 10500)])
+def test_class_sums_are_added_in_fp64(fsg, nwl, n):
+    """Each window-width class is one compensated FP32 sum, and the classes are added in FP64, however long the list: a
+    list in one launch for all classes equals the same list class by class (every class whole, in one block), to the
+    rounding of some twenty FP64 additions.  Few enough lines on a tile that none are paired."""
+    grid, st, co, a = case(33, nwl, n, 11)
+    out = []
+    for ram in (16.0, 0.8 * n * 1632e-9):                # all lines' records, or those of 80 % of them
+        C = fsg.Context(vmicro=1.0, epsopac=3e-3, limitram_gb=ram)
+        C.set_grid(grid["wmode"], grid["wstart"], grid["wend"], grid["dstep"])
+        C.set_atmosphere(st)
+        C.set_contopac(co)
+        g = C.lineop_calc(fsg.LineList.from_arrays(a))
+        out.append(g)
+        C.close()
+    keep = (g["flags"] & 1) == 0
+    assert (n < 8192) == (np.count_nonzero(keep) <= 8192)
+    width = (g["iright"] - g["ileft"] + 1)[keep]
+    ncls = len(np.unique(np.ceil(np.log2(np.maximum(width, 256)))))
+    assert out[0]["stats"]["nblocks"] == 1 and out[1]["stats"]["nblocks"] == ncls
+    np.testing.assert_allclose(out[0]["lineopac"], out[1]["lineopac"], rtol=1e-14, atol=0.0)
+
+
 @pytest.mark.parametrize("n", [32769, 45001])
 def test_central_pass_forms(fsg, n):
     """Flags and windows do not depend on how the central pass spreads its lines: a list above 32,768 lines takes
