@@ -756,8 +756,8 @@ static int rows64(fsg_ctx *ctx, const AtmView &A, const LineView &LV, const int6
 // mixed-precision accumulation: classes by window width, blocks within a class
 // fl/il/ir: LinFlag, Ileft, Iright of the list (device); [i0, i1]: 1-based wavelength range to fill
 // (1..nwl for the whole grid).  Lines are classed by their full windows and evaluated over the part
-// of the window inside the range, so each wavelength of the range sums the same lines in the same
-// order as in a whole-grid run.
+// of the window inside the range, so each wavelength of the range sums the same lines as in a whole-grid
+// run, and a tile inside the range in the same groups (a list that fits one block: bit for bit the same sums).
 // nmax: no more lines than these are retained (the retained count where it is known, else n).
 static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, int64_t nmax, fsg_stats *st, const int32_t *fl,
                            const int32_t *il, const int32_t *ir, int i0, int i1) {

@@ -73,16 +73,18 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // evaluation against 4 x 4, sixteen lines a group the staging against 8: a million lines, 483,000 wavelengths, 56 depths
 // 44.9 -> 40.3 ms (single, 4 x 4) -> 33.0 ms (pairs, 8 x 4, 16 lines).
 //
-// A pair rounds in other places than two single terms (the error against 64 bits is the same: 20,000 lines over
-// 200 A 7e-11 of the flux either way).  Where few lines make up a pixel the difference shows, 4e-9 of the flux at
-// 150 lines per pixel against 2e-10 at 1,000, and there the pass is short; tiles with fewer than WING_PAIR_MIN
-// candidate lines take them one at a time.
+// A pair rounds in other places than two single terms, three products more and one addition less; against 64 bits it is
+// no further off (rms of LineOpac 4.8e-8 with pairs, 5.0e-8 without, for 20,000 lines over 200 A; 3.8 and 4.0e-8 for 1e6
+// molecular lines).  The two roundings differ most where few lines make up a pixel: by 5e-9 of the flux at 140 lines per
+// pixel, 1.3e-9 at 240, 4e-10 at 500, 4e-11 at 2,100.  The pass is short there, and tiles that fewer than WING_PAIR_MIN
+// lines touch take them one at a time.  Lines are counted, not candidates, so that a tile sums alike whatever
+// part of the list and of the grid a call has; the count ends at WING_PAIR_MIN.
 
 // A line as the warp's group holds it: {wlh, wll, code, xm}.  code: first and last wavelength of the window
 // inside the tile (bits 0-7, 8-15), WING_CORE (a core range meets it); xm: the x that silences a point.
 #define WING_CORE (1 << 16)
 #define WING_G 16                     // lines per group
-#define WING_PAIR_MIN 2048
+#define WING_PAIR_MIN 1024
 
 // shared memory of one warp
 template <int D, int P>
@@ -103,7 +105,6 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
     for (int sg = 0; sg < J.nseg; sg++)
         ncand += max(J.tile_hi[sg * J.seg_stride + tile] - J.tile_lo[sg * J.seg_stride + tile] + 1, 0);
     if (!ncand) return;
-    const bool pairs = ncand >= WING_PAIR_MIN;
     const float4 *__restrict__ wing = (const float4 *)J.wing;
     const int p0 = tile * TW;
     // wavelength offsets as FP32 hi + lo: dl = (wvh - wlh) + (wvl - wll) keeps dl to FP32 relative
@@ -126,6 +127,18 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
         }
     int nfold = 0;
     const int tile_first = p0 + 1, tile_last = min(p0 + TW, nwl);
+    int touch = 0;                                      // lines that touch the tile, counted up to WING_PAIR_MIN
+    for (int sg = 0; ncand >= WING_PAIR_MIN && touch < WING_PAIR_MIN && sg < J.nseg; sg++) {
+        const int last = J.tile_hi[sg * J.seg_stride + tile];
+        for (int b = J.tile_lo[sg * J.seg_stride + tile]; b <= last && touch < WING_PAIR_MIN; b += 128)
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int i = b + 32 * u + lane;
+                const int2 w = i <= last ? *(const int2 *)&J.hdr[i].ileft : make_int2(1, 0);
+                touch += __popc(__ballot_sync(0xffffffffu, w.y >= tile_first && w.x <= tile_last));
+            }
+    }
+    const bool pairs = touch >= WING_PAIR_MIN;
     float4 rnext[U], hnext;                             // the next group's records and (lanes < n) header
     int nnext = 0, npair = 0, slot = 0;                            // lines; lane q's line's place in the group
     auto fetch = [&](int head, int n) {

@@ -172,3 +172,38 @@ def test_given_windows_past_the_grid(fsg):
         out.append(C.lineop_get())
     assert np.array_equal(out[0], out[1])
     C.close()
+
+
+@pytest.mark.parametrize("n,nwl,eps", [(600, 4001, 1e-4), (3500, 8001, 1e-4), (3500, 8001, 1e-6), (9500, 4001, 1e-4),
+                                       (9500, 4001, 1e-9)])
+def test_ranges_sum_as_the_whole_grid(fsg, n, nwl, eps):
+    """Ranges in the mixed path, with few and with many lines on a tile (enough for two lines to share a reciprocal),
+    down to a range of one tile: on tiles that lie inside a range the sums are those of the whole grid bit for bit."""
+    from fastspec_b200 import shard
+    from fastspec_b200 import workloads as W
+    ntau, step, w0 = 33, 0.011, 5100.0
+    st, _ = W.batch_atmosphere(5300.0, 4.2, ntau, {})
+    wend = w0 + (nwl - 0.5) * step
+    a = W.atomic_lines(n, w0 - 3.0, wend + 3.0, n, exact=False).arrays()
+    C = fsg.Context(vmicro=1.0, epsopac=eps)
+    C.set_grid(0, w0, wend, step)
+    C.set_atmosphere(st)
+    C.set_contopac(np.tile(1e-2 * (1.0 + np.arange(ntau)), (nwl, 1)))
+    B = shard.GpuBackend(fsg, C, {k: torch.from_numpy(np.ascontiguousarray(v)).cuda() for k, v in a.items()})
+    C.lineop_reset()
+    C.lineop_calc_dev(B.full)
+    whole = C.lineop_get()
+    win = B.central(0, B.n, B.n)
+    if eps < 1e-8:
+        keep = (win[0] & 1) == 0
+        full = keep & (win[1] <= 2000) & (win[2] >= 2100)
+        assert int(full.sum()) > 1024 and int(keep.sum()) > 8192
+    for i0, i1 in ((1, 1500), (1501, 2913), (2914, nwl), (1665, 1792), (641, 768)):
+        B.accumulate(win, i0, i1)
+        lo = C.lineop_get()
+        assert np.all(lo[:i0 - 1] == 0) and np.all(lo[i1:] == 0)
+        first = (i0 - 1 + 127) // 128 * 128                 # tiles of 128 wavelengths inside the range
+        last = nwl if i1 == nwl else i1 // 128 * 128
+        assert first < last
+        assert np.array_equal(lo[first:last], whole[first:last])
+    C.close()
