@@ -758,8 +758,8 @@ static int rows64(fsg_ctx *ctx, const AtmView &A, const LineView &LV, const int6
 // (1..nwl for the whole grid).  Lines are classed by their full windows and evaluated over the part
 // of the window inside the range, so each wavelength of the range sums the same lines as in a whole-grid
 // run, and a tile inside the range in the same groups (a list that fits one block: bit for bit the same sums).
-// nmax: no more lines than these are retained (the retained count where it is known, else n).
-static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, int64_t nmax, fsg_stats *st, const int32_t *fl,
+// nkeep: the retained lines where their number is known; < 0: the lines of the range are counted here.
+static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, int64_t nkeep, fsg_stats *st, const int32_t *fl,
                            const int32_t *il, const int32_t *ir, int i0, int i1) {
     int64_t n = LV.n;
     const int nt = ctx->ntau;
@@ -801,9 +801,25 @@ static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, int64_t nmax, fsg_s
                         &dres->ncore, ctx->fault_extra_tx, ctx->fault_wait_ns, nseg, stride };
     };
     // A list whose records fit one block (LIMITRAM) is one record array in window-width-class order: one launch
-    // per step for all classes, each tile adding its classes in turn, and no count needed on the host.  Lists that
+    // per step for all classes, each tile adding its classes in turn.  Lists that
     // do not fit take the classes one by one, in blocks: 18 launches a class and three read-backs.  The line lies where
     // memory draws it: 300 lines took 837 us by classes, 470 us this way, 20,000 6.5 and 5.1 ms, 1e6 74.9 and 61.8 ms.
+    // A range counts its lines first, so that the records of the others are neither made nor held: an eighth of the grid
+    // of 1e6 lines takes 7.8 ms and 1.0 GB, with the records of all lines 9.0 ms and 3.8 GB.
+    unsigned long long hist[32];
+    auto histogram = [&]() -> int {                    // selected lines by class, nsel in all
+        ALLOC(ctx->d_hist, sizeof hist);
+        CK(cudaMemsetAsync(ctx->d_hist.p, 0, sizeof hist, s), "hist");
+        fsg_launch_class_hist(s, n, sf, il, ir, ctx->d_hist.as<unsigned long long>());
+        ctx->launches += 1;
+        CK(cudaMemcpyAsync(hist, ctx->d_hist.p, sizeof hist, cudaMemcpyDeviceToHost, s), "hist");
+        CK(cudaStreamSynchronize(s), "hist");
+        nsel = 0;
+        for (int c = 0; c < 32; c++) nsel += (int64_t)hist[c];
+        return FSG_OK;
+    };
+    if (nkeep < 0) { const int rc = histogram(); if (rc) return rc; }
+    const int64_t nmax = nkeep < 0 ? nsel : nkeep;
     const int ncls = fsg_bclass_count(ctx->nwl);
     const int ws = (ctx->nwl + 63) / 64, cs = (ctx->nwl + 31) / 32;
     bool one = nmax <= cap && nmax > 0;
@@ -854,14 +870,7 @@ static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, int64_t nmax, fsg_s
         ctx->launches += ncls > nn ? 13 : 12;            // order 3, params, spans 6, wing 1 or 2, core
         nblocks = 1;
     } else if (nmax > 0) {
-        ALLOC(ctx->d_hist, sizeof(unsigned long long) * 32);
-        CK(cudaMemsetAsync(ctx->d_hist.p, 0, sizeof(unsigned long long) * 32, s), "hist");
-        fsg_launch_class_hist(s, n, sf, il, ir, ctx->d_hist.as<unsigned long long>());
-        ctx->launches += 1;
-        unsigned long long hist[32];
-        CK(cudaMemcpyAsync(hist, ctx->d_hist.p, sizeof hist, cudaMemcpyDeviceToHost, s), "hist");
-        CK(cudaStreamSynchronize(s), "hist");
-        for (int c = 0; c < 32; c++) nsel += (int64_t)hist[c];
+        if (nkeep >= 0) { const int rc = histogram(); if (rc) return rc; }
         ALLOC(ctx->d_counts, sizeof(int) * nblkscan);
         ALLOC(ctx->d_offs, sizeof(int64_t) * nblkscan);
         ALLOC(ctx->d_total, sizeof(int64_t));
@@ -1225,7 +1234,7 @@ int fsg_accumulate_dev(fsg_ctx *ctx, const fsg_lines *d_lines, const int32_t *d_
         CK(cudaMemcpyAsync(ctx->d_iright.p, d_iright, nb, cudaMemcpyDeviceToDevice, s), "windows");
         rc = accumulate_fp64(ctx, make_view(d_lines), -1, st, i0, i1);
     } else {
-        rc = accumulate_fast(ctx, make_view(d_lines), d_lines->n, st, d_flags, d_ileft, d_iright, i0, i1);
+        rc = accumulate_fast(ctx, make_view(d_lines), -1, st, d_flags, d_ileft, d_iright, i0, i1);
     }
     if (rc) return rc;
     CK(cudaEventRecord(ctx->ev[2], s), "event");

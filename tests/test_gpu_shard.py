@@ -207,3 +207,27 @@ def test_ranges_sum_as_the_whole_grid(fsg, n, nwl, eps):
         assert first < last
         assert np.array_equal(lo[first:last], whole[first:last])
     C.close()
+
+
+def test_a_range_holds_the_records_of_its_own_lines(fsg):
+    """A range whose lines fit one block is one launch per pass, and no buffer is larger than a third of the whole list's
+    records (1,632 bytes a line at 33 depths): the lines outside the range get none."""
+    from fastspec_b200 import shard
+    from fastspec_b200 import workloads as W
+    ntau, nwl, n, step, w0 = 33, 8001, 20000, 0.05, 5100.0
+    st, _ = W.batch_atmosphere(5300.0, 4.2, ntau, {})
+    wend = w0 + (nwl - 0.5) * step
+    a = W.atomic_lines(n, w0, wend, 3, exact=False).arrays()
+    C = fsg.Context(vmicro=1.0, epsopac=1e-2)
+    C.set_grid(0, w0, wend, step)
+    C.set_atmosphere(st)
+    C.set_contopac(np.tile(1e-2 * (1.0 + np.arange(ntau)), (nwl, 1)))
+    B = shard.GpuBackend(fsg, C, {k: torch.from_numpy(np.ascontiguousarray(v)).cuda() for k, v in a.items()})
+    C.lineop_reset()
+    win = B.central(0, B.n, B.n)
+    touch = ((win[0] & 1) == 0) & (win[1] <= 5000) & (win[2] >= 4001)
+    assert n // 8 < int(touch.sum()) < n // 4
+    C.set_fault(fsg.FAULT_ALLOC_LIMIT, n * 1632 // 3)
+    s = B.accumulate(win, 4001, 5000)
+    assert s["nlines_used"] == int(touch.sum()) and s["nblocks"] == 1 and s["accum_launches"] == 1
+    C.close()
