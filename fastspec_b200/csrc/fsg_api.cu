@@ -254,8 +254,8 @@ struct fsg_ctx {
     DBuf l_wl, l_elo, l_gf, l_grad, l_gqst, l_gvdw, l_spc, l_ismol, l_ihe;
     DBuf d_flags, d_ileft, d_iright, d_idx, d_counts, d_offs, d_total, d_hist, d_nkeep;
     // block buffers
-    DBuf d_block;                              // order, records and tile ranges of a list that fits one block
-    DBuf d_wing, d_core, d_hdr, d_hdr64, d_tlo, d_thi, d_p64, d_lstart, d_lstop, d_widx, d_pw, d_res, d_span, d_linstr, d_rflags, d_rleft, d_rright, d_gkappa, d_adjwork, d_cbuf, d_ctaps;
+    DBuf d_block;                              // a block's records; order and tile ranges too of a list that fits one
+    DBuf d_hdr64, d_tlo, d_thi, d_p64, d_lstart, d_lstop, d_widx, d_pw, d_res, d_span, d_linstr, d_rflags, d_rleft, d_rright, d_gkappa, d_adjwork, d_cbuf, d_ctaps;
     // spectra
     DBuf d_spl, d_spc, d_sfl, d_sfc, d_work, d_a, d_v, d_h, d_l;
     // magnetic
@@ -346,7 +346,7 @@ void fsg_destroy(fsg_ctx *ctx) {
                      &ctx->d_wmu, &ctx->d_lineopac, &ctx->d_maglineopac, &ctx->l_wl, &ctx->l_elo, &ctx->l_gf,
                      &ctx->l_grad, &ctx->l_gqst, &ctx->l_gvdw, &ctx->l_spc, &ctx->l_ismol, &ctx->l_ihe,
                      &ctx->d_flags, &ctx->d_ileft, &ctx->d_iright, &ctx->d_idx, &ctx->d_counts, &ctx->d_offs,
-                     &ctx->d_total, &ctx->d_hist, &ctx->d_nkeep, &ctx->d_block, &ctx->d_wing, &ctx->d_core, &ctx->d_hdr, &ctx->d_hdr64,
+                     &ctx->d_total, &ctx->d_hist, &ctx->d_nkeep, &ctx->d_block, &ctx->d_hdr64,
                      &ctx->d_tlo, &ctx->d_thi, &ctx->d_res, &ctx->d_span, &ctx->d_linstr, &ctx->d_rflags, &ctx->d_rleft, &ctx->d_rright, &ctx->d_gkappa, &ctx->d_adjwork, &ctx->d_cbuf, &ctx->d_ctaps, &ctx->d_p64, &ctx->d_lstart, &ctx->d_lstop, &ctx->d_widx,
                      &ctx->d_pw, &ctx->d_spl, &ctx->d_spc, &ctx->d_sfl, &ctx->d_sfc,
                      &ctx->d_work, &ctx->d_a, &ctx->d_v, &ctx->d_h, &ctx->d_l, &ctx->z_npi, &ctx->z_nsi,
@@ -877,6 +877,22 @@ static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, int64_t nkeep, fsg_
         ALLOC(ctx->d_idx, sizeof(int64_t) * std::max<int64_t>(n, 1));
         const int ntiles = fsg_fast_tiles(ctx->nwl);
         ALLOC(ctx->d_tlo, sizeof(int) * ntiles); ALLOC(ctx->d_thi, sizeof(int) * ntiles);
+        // blocks of at most cap lines (LIMITRAM); block b takes every nblk-th line of a class from
+        // its b-th, so each block is sorted by wavelength and spans the whole grid: every tile of a
+        // launch has work, however small the blocks
+        int64_t rows = 0;
+        for (int c = 0; c < 32; c++) {
+            const int64_t nc = (int64_t)hist[c], nblk = (nc + cap - 1) / cap;
+            if (nc) rows = std::max(rows, (nc + nblk - 1) / nblk);
+        }
+        size_t bytes = 0;
+        auto part = [&](size_t nb) { const size_t o = bytes; bytes += (nb + 255) & ~(size_t)255; return o; };
+        const size_t o_wing = part(sizeof(WingPair) * (size_t)rows * npair), o_core = part(sizeof(CoreRec) * (size_t)rows * nt);
+        const size_t o_hdr = part(sizeof(LineHdr) * (size_t)rows);
+        ALLOC(ctx->d_block, bytes);
+        ALLOC(ctx->d_span, fsg_tile_span_scratch(rows));
+        char *p = ctx->d_block.as<char>();
+        wing = (WingPair *)(p + o_wing); core = (CoreRec *)(p + o_core); hdr = (LineHdr *)(p + o_hdr);
         for (int c = 0; c < 32; c++) {
             if (!hist[c]) continue;
             int rc = fsg_select(s, n, sf, il, ir, c,
@@ -884,17 +900,7 @@ static int accumulate_fast(fsg_ctx *ctx, const LineView &LV, int64_t nkeep, fsg_
                                 ctx->d_total.as<int64_t>());
             if (rc) return cuda_fail(ctx, cudaGetLastError(), "select");
             ctx->launches += 3;
-            int64_t nc = (int64_t)hist[c];
-            // blocks of at most cap lines (LIMITRAM); block b takes every nblk-th line of the class from
-            // its b-th, so each block is sorted by wavelength and spans the whole grid: every tile of a
-            // launch has work, however small the blocks
-            const int64_t nblk = (nc + cap - 1) / cap;
-            const int64_t bcap = (nc + nblk - 1) / nblk;
-            ALLOC(ctx->d_wing, sizeof(WingPair) * (size_t)bcap * npair);
-            ALLOC(ctx->d_core, sizeof(CoreRec) * (size_t)bcap * nt);
-            ALLOC(ctx->d_hdr, sizeof(LineHdr) * (size_t)bcap);
-            ALLOC(ctx->d_span, fsg_tile_span_scratch(bcap));
-            wing = ctx->d_wing.as<WingPair>(); core = ctx->d_core.as<CoreRec>(); hdr = ctx->d_hdr.as<LineHdr>();
+            const int64_t nc = (int64_t)hist[c], nblk = (nc + cap - 1) / cap;
             for (int64_t b = 0; b < nblk; b++) {
                 const int64_t nb = (nc - b + nblk - 1) / nblk;
                 fsg_launch_params_fast(s, A, LV, ctx->d_idx.as<int64_t>(), b, nblk, nb, fl, wl_, wr_, ctx->tab, wing, core,
@@ -1462,19 +1468,20 @@ static int mag_lineop_calc_body(fsg_ctx *ctx, const fsg_lines *lines, int bframe
         ctx->launches += 3;
         const size_t per_line = fsg_mag_rec_bytes(nt) + sizeof(LineHdr);
         const int64_t bcap = std::min<int64_t>(std::max<int64_t>(nkeep, 1), block_capacity(ctx, per_line));
-        ALLOC(ctx->d_wing, fsg_mag_rec_bytes(nt) * (size_t)bcap);
-        ALLOC(ctx->d_hdr, sizeof(LineHdr) * (size_t)bcap);
+        const size_t rec_bytes = (fsg_mag_rec_bytes(nt) * (size_t)bcap + 255) & ~(size_t)255;
+        ALLOC(ctx->d_block, rec_bytes + sizeof(LineHdr) * (size_t)bcap);
+        void *rec = ctx->d_block.p;
+        LineHdr *hdr = (LineHdr *)((char *)rec + rec_bytes);
         ALLOC(ctx->d_span, fsg_tile_span_scratch(bcap));
         ALLOC(ctx->d_tlo, sizeof(int) * (size_t)fsg_fast_tiles(nwl)); ALLOC(ctx->d_thi, sizeof(int) * (size_t)fsg_fast_tiles(nwl));
         double *mlo = ctx->d_maglineopac.as<double>();
         int64_t nblocks = 0;
         for (int64_t j0 = 0; j0 < nkeep; j0 += bcap) {
             const int64_t nb = std::min(bcap, nkeep - j0);
-            fsg_launch_mag_params_fast(s, A, LV, Z, ctx->d_idx.as<int64_t>(), j0, nb, pf, pl, pr, ctx->tab, ctx->d_wing.p,
-                                       ctx->d_hdr.as<LineHdr>());
-            if (fsg_launch_tile_span_tw(s, 32, 0, nwl, nb, ctx->d_hdr.as<LineHdr>(), ctx->d_tlo.as<int>(),
+            fsg_launch_mag_params_fast(s, A, LV, Z, ctx->d_idx.as<int64_t>(), j0, nb, pf, pl, pr, ctx->tab, rec, hdr);
+            if (fsg_launch_tile_span_tw(s, 32, 0, nwl, nb, hdr, ctx->d_tlo.as<int>(),
                                         ctx->d_thi.as<int>(), ctx->d_span.p, ctx->d_span.cap) ||
-                fsg_launch_mag_fast(s, A, ctx->d_hdr.as<LineHdr>(), ctx->d_wing.p, nb, Z,
+                fsg_launch_mag_fast(s, A, hdr, rec, nb, Z,
                                     ctx->d_tlo.as<int>(), ctx->d_thi.as<int>(), ctx->tab, mlo))
                 return cuda_fail(ctx, cudaGetLastError(), "k_mag_fast");
             ctx->launches += 8;

@@ -556,3 +556,29 @@ def test_molecular_h5_lists_against_reference_pin(fsg, tmp_path, prec):
         assert np.max(np.abs(lo - ref) / (ref + d["contopac"])) < 2e-6
     spl, spc, sfl, sfc = C.radtran()
     assert np.max(np.abs(sfl[i0:i1 + 1] / d["sfl"] - 1)) < (2e-7 if prec == "fp64" else 1e-5)
+
+
+def test_short_and_long_lists_share_one_block(fsg):
+    """A list whose records fit one block and then one that does not: the context holds the records of one block
+    (LIMITRAM), not one of either kind."""
+    import torch
+    from fastspec_b200 import shard
+    from fastspec_b200 import workloads as W
+    ntau, nwl, step, w0, ram = 33, 2001, 0.05, 5100.0, 0.5
+    st, _ = W.batch_atmosphere(5300.0, 4.2, ntau, {})
+    wend = w0 + (nwl - 0.5) * step
+    lists = []
+    for n in (270000, 900000):
+        a = W.atomic_lines(n, w0, wend, n, exact=False).arrays()
+        lists.append({k: torch.from_numpy(np.ascontiguousarray(v)).cuda() for k, v in a.items()})
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    C = fsg.Context(vmicro=1.0, epsopac=1e-2, limitram_gb=ram)
+    C.set_grid(0, w0, wend, step)
+    C.set_atmosphere(st)
+    C.set_contopac(np.tile(1e-2 * (1.0 + np.arange(ntau)), (nwl, 1)))
+    blocks = [C.lineop_calc_dev(shard.GpuBackend(fsg, C, d).full)["nblocks"] for d in lists]
+    used = free - torch.cuda.mem_get_info()[0]
+    C.close()
+    assert blocks[0] == 1 and blocks[1] > 1
+    assert used < 1.4 * ram * 1e9
