@@ -2267,8 +2267,8 @@ int fsg_disk_integ_conv_dev(fsg_ctx *ctx, const double *radii, double vsini, dou
     const double *dk = ctx->d_ctaps.as<double>();
     const int rf = fsg_launch_disk_conv(s, nwl, nmu, d_spl, d_spc, dk, roff.data(), rn.data(), moff.data(), mn.data(),
                                         wmu.data(), goff, gn, tL, tC, d_sfl, d_sfc);
-    if (rf >= 0) {
-        if (rf) return cuda_fail(ctx, cudaGetLastError(), "k_disk_conv");
+    if (rf < 0) return cuda_fail(ctx, cudaGetLastError(), "k_disk_conv");
+    if (rf != CONV_WIDE) {
         ctx->launches += gn ? 2 : 1;
         CK(cudaStreamSynchronize(s), "disk integration");
         return FSG_OK;

@@ -96,11 +96,13 @@ __global__ void __launch_bounds__(CONV_TH) k_disk_conv(ConvJob J) {
 
 // The broadened flux of both kinds: intensities spl/spc [nwl][nmu], taps on the device, annulus im's kernels
 // as in ConvJob; the Gaussian taps[goff .. goff + gn) (gn = 0: none) last, through the work arrays tl, tc [nwl].
-// -1: the halo does not fit shared memory (the caller convolves annulus by annulus).
+// CONV_WIDE (positive; errors are negative): the halo does not fit shared memory, nothing was launched, the caller
+// convolves annulus by annulus.
 int fsg_launch_disk_conv(cudaStream_t s, int nwl, int nmu, const double *spl, const double *spc, const double *taps,
                          const int *roff, const int *rn, const int *moff, const int *mn, const double *wmu, int goff,
                          int gn, double *tl, double *tc, double *sfl, double *sfc) {
     ConvJob J;
+    if (nmu > (int)(sizeof J.rn / sizeof *J.rn)) return CONV_WIDE;
     J.nwl = nwl; J.stride = nmu; J.nann = nmu; J.rh = J.mh = 0; J.taps = taps;
     for (int im = 0; im < nmu; im++) {
         J.roff[im] = roff[im]; J.rn[im] = rn[im]; J.moff[im] = moff[im]; J.mn[im] = mn[im]; J.w[im] = wmu[im];
@@ -108,7 +110,7 @@ int fsg_launch_disk_conv(cudaStream_t s, int nwl, int nmu, const double *spl, co
         J.mh = mn[im] / 2 > J.mh ? mn[im] / 2 : J.mh;
     }
     const size_t sm1 = conv_smem(J.rh, J.mh), sm2 = conv_smem(0, gn / 2), most = 200 * 1024;
-    if (nmu > 16 || sm1 > most || sm2 > most) return -1;
+    if (sm1 > most || sm2 > most) return CONV_WIDE;
     const size_t sm = sm1 > sm2 ? sm1 : sm2;
     if (sm > 48 * 1024 &&
         cudaFuncSetAttribute(k_disk_conv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess)
@@ -123,5 +125,5 @@ int fsg_launch_disk_conv(cudaStream_t s, int nwl, int nmu, const double *spl, co
         J.in[0] = tl; J.in[1] = tc; J.out[0] = sfl; J.out[1] = sfc;
         k_disk_conv<<<grid, CONV_TH, sm2, s>>>(J);
     }
-    return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
+    return cudaPeekAtLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }

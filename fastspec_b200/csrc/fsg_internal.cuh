@@ -166,6 +166,9 @@ struct RayView {
     const double *m, *dm, *idm, *lam;
 };
 
+// fsg_launch_disk_conv: kernels too wide for the fused pass (not an error code, which are negative)
+#define CONV_WIDE 1
+
 // Error reporting
 std::string fsg_cuda_msg(cudaError_t e, const char *what);
 

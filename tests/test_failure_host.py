@@ -102,3 +102,26 @@ def test_rank_leaving_between_steps_is_noticed(tmp_path, world):
         seen, flux = open(out + ".rank%d" % r).read().split("\n")
         assert seen == "lost:%d" % (world - 1), seen
         assert np.isfinite(float(flux))
+
+
+def test_disk_convolution_tells_wide_kernels_from_errors():
+    """The launcher of the fused disk integration: kernels too wide for shared memory, or more annuli than its job holds,
+    are a positive answer (nothing is launched, the caller convolves annulus by annulus); a launch that fails (here: no
+    wavelengths, so no grid) is a negative error code."""
+    import ctypes as C
+    import fastspec_b200 as F
+    f = F.lib()["_Z20fsg_launch_disk_convP11CUstream_stiiPKdS2_S2_PKiS4_S4_S4_S2_iiPdS5_S5_S5_"]
+    f.restype = C.c_int
+    p = C.c_void_p
+
+    def launch(nwl, nmu, rn, mn):
+        off = (C.c_int * nmu)()
+        w = (C.c_double * nmu)(*[1.0 / nmu] * nmu)
+        null = p(None)
+        return f(null, C.c_int(nwl), C.c_int(nmu), null, null, null, off, (C.c_int * nmu)(*[rn] * nmu), off,
+                 (C.c_int * nmu)(*[mn] * nmu), w, C.c_int(0), C.c_int(0), null, null, null, null)
+
+    assert launch(100000, 7, 40001, 101) > 0
+    assert launch(100000, 7, 101, 40001) > 0
+    assert launch(100000, 17, 3, 3) > 0
+    assert launch(0, 7, 3, 3) < 0
