@@ -96,8 +96,16 @@ __global__ void __launch_bounds__(CONV_TH) k_disk_conv(ConvJob J) {
 
 // The broadened flux of both kinds: intensities spl/spc [nwl][nmu], taps on the device, annulus im's kernels
 // as in ConvJob; the Gaussian taps[goff .. goff + gn) (gn = 0: none) last, through the work arrays tl, tc [nwl].
-// CONV_WIDE (positive; errors are negative): the halo does not fit shared memory, nothing was launched, the caller
-// convolves annulus by annulus.
+// CONV_WIDE (positive; errors are negative): kernels too wide, nothing was launched, the caller convolves annulus by
+// annulus.
+//
+// Where that is: a CTA rotates the halo of the macroturbulence too, rn (CONV_T + 2 mh) products for rn CONV_T, and wide
+// kernels leave room for few CTAs on an SM and little L1 for the taps.  Time annulus by annulus over fused, 200,001
+// wavelengths, 3 and 9 annuli, by the half-widths (rotation, macroturbulence); the fused pass's products over the
+// others; CTAs per SM:
+//   (100, 600) 3.3, 3.8 x; 1.3; 7    (1200, 600) 1.6, 1.8 x; 2.3; 4    (600, 2000) 1.2, 1.3 x; 2.4; 2
+//   (1200, 2000) 0.96, 1.1 x; 3.3; 2    (2500, 2000) 0.48, 0.58 x; 4.5; 2    (6000, 200) 1.1, 1.3 x; 1.6; 2
+//   (0, 6000) 1.3, 1.6 x; 1.0; 1    (100, 5000) 1.1, 1.1 x; 1.3; 1    (300, 5000) 0.96, 1.0 x; 1.9; 1
 int fsg_launch_disk_conv(cudaStream_t s, int nwl, int nmu, const double *spl, const double *spc, const double *taps,
                          const int *roff, const int *rn, const int *moff, const int *mn, const double *wmu, int goff,
                          int gn, double *tl, double *tc, double *sfl, double *sfc) {
@@ -111,6 +119,13 @@ int fsg_launch_disk_conv(cudaStream_t s, int nwl, int nmu, const double *spl, co
     }
     const size_t sm1 = conv_smem(J.rh, J.mh), sm2 = conv_smem(0, gn / 2), most = 200 * 1024;
     if (sm1 > most || sm2 > most) return CONV_WIDE;
+    double fused = 0.0, apart = 0.0;                     // products of a CTA's wavelengths
+    for (int im = 0; im < nmu; im++) {
+        fused += (double)rn[im] * (CONV_T + mn[im]) + (double)mn[im] * CONV_T;
+        apart += ((double)rn[im] + mn[im]) * CONV_T;
+    }
+    const int ctas = (int)((227 * 1024) / (sm1 + 1024)), taps_most = 2 * (J.rh > J.mh ? J.rh : J.mh);
+    if (fused > (ctas < 2 ? 1.4 : ctas == 2 && taps_most > 4096 ? 1.65 : 2.5) * apart) return CONV_WIDE;
     const size_t sm = sm1 > sm2 ? sm1 : sm2;
     if (sm > 48 * 1024 &&
         cudaFuncSetAttribute(k_disk_conv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess)

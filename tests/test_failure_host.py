@@ -125,3 +125,8 @@ def test_disk_convolution_tells_wide_kernels_from_errors():
     assert launch(100000, 7, 101, 40001) > 0
     assert launch(100000, 17, 3, 3) > 0
     assert launch(0, 7, 3, 3) < 0
+    # the rule between the two (no wavelengths: what it would launch is an error): (rotation, macroturbulence) half-widths
+    for rh, mh in ((25, 28), (100, 600), (1200, 600), (3000, 200), (6000, 200), (600, 2000), (0, 6000), (10000, 0)):
+        assert launch(0, 7, 2 * rh + 1 if rh else 0, 2 * mh + 1 if mh else 0) < 0, (rh, mh)
+    for rh, mh in ((1200, 2000), (2500, 2000), (2001, 2830), (1000, 4244), (400, 5660), (300, 5000), (0, 6400)):
+        assert launch(0, 7, 2 * rh + 1 if rh else 0, 2 * mh + 1) > 0, (rh, mh)
