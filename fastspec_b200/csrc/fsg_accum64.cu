@@ -33,8 +33,10 @@
 struct Wing64 { double vv2, c2m1, twoA, c1; };
 struct Core64 { double vv, a, ua, cop; int ia, pad; };
 
-__device__ __forceinline__ double wing64(double t, const Wing64 &w) {
-    return fma(w.c1, t, w.c1) * rcp64(fma(t, t, w.twoA));
+// acc + the wing term, one rounding: the same in every branch that takes it, so that a point's sum does not depend
+// on how its tile or range cuts the line's window
+__device__ __forceinline__ double wing64(double acc, double t, const Wing64 &w) {
+    return fma(fma(w.c1, t, w.c1), rcp64(fma(t, t, w.twoA)), acc);
 }
 
 // HVoigt (voigt.f90:81-107) where s < 196, table row and weight of a given
@@ -46,11 +48,11 @@ __device__ __forceinline__ double core64(const float *__restrict__ vtab, const C
         const float *p0 = vtab + (c.ia - 1) * FSG_NV1 + iv, *p1 = p0 + FSG_NV1;
         const float t00 = __ldg(p0), t01 = __ldg(p0 + 1), t10 = __ldg(p1), t11 = __ldg(p1 + 1);
         const double c0 = (double)t00 + tv * (double)(t01 - t00), c1 = (double)t10 + tv * (double)(t11 - t10);
-        return (c0 + c.ua * (c1 - c0)) * c.cop;
+        return c0 + c.ua * (c1 - c0);
     }
     const double a2 = c.a * c.a, v2 = av * av, p = v2 - a2 - 1.5, q = 2.0 * av * c.a;
     const double dr = av * p - c.a * q, di = av * q + c.a * p;
-    return FSG_SQRTPIINV * ((p + 0.5) * di - q * dr) / (dr * dr + di * di) * c.cop;
+    return FSG_SQRTPIINV * ((p + 0.5) * di - q * dr) / (dr * dr + di * di);
 }
 
 // table row and weight of a as HVoigt takes them (voigt.f90:84-92); ia = 0: a >= 8
@@ -138,8 +140,8 @@ __global__ void __launch_bounds__(32 * A64_W, 6) k_accum64(Accum64Job J) {
                         if (pix[k] < g.il || pix[k] > g.ir) continue;
                         const double dk = dl[k] - sh, t = fma(dk * dk, w.vv2, w.c2m1);
                         const Core64 &c = core_s[warp][q][d];
-                        if (t >= 195.5) acc[k][d] += wing64(t, w);
-                        else acc[k][d] += core64(J.vtab, c, fabs(dk) * c.vv);
+                        if (t >= 195.5) acc[k][d] = wing64(acc[k][d], t, w);
+                        else acc[k][d] = fma(core64(J.vtab, c, fabs(dk) * c.vv), c.cop, acc[k][d]);
                     }
                 }
             } else if (g.il <= first && g.ir >= last) {
@@ -147,7 +149,7 @@ __global__ void __launch_bounds__(32 * A64_W, 6) k_accum64(Accum64Job J) {
                 for (int d = 0; d < A64_D; d++) {
                     const Wing64 w = wing_s[warp][q][d];
 #pragma unroll
-                    for (int k = 0; k < A64_P; k++) acc[k][d] += wing64(fma(x[k], w.vv2, w.c2m1), w);
+                    for (int k = 0; k < A64_P; k++) acc[k][d] = wing64(acc[k][d], fma(x[k], w.vv2, w.c2m1), w);
                 }
             } else {
                 bool in[A64_P];
@@ -158,8 +160,8 @@ __global__ void __launch_bounds__(32 * A64_W, 6) k_accum64(Accum64Job J) {
                     const Wing64 w = wing_s[warp][q][d];
 #pragma unroll
                     for (int k = 0; k < A64_P; k++) {
-                        const double v = wing64(fma(x[k], w.vv2, w.c2m1), w);
-                        if (in[k]) acc[k][d] += v;
+                        const double v = wing64(acc[k][d], fma(x[k], w.vv2, w.c2m1), w);
+                        if (in[k]) acc[k][d] = v;
                     }
                 }
             }
