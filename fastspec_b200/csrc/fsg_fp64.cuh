@@ -1,11 +1,16 @@
 // fsg_fp64.cuh -- FP64 device functions restating voigt.f90 / opacity.f90 / solver.f90.
-// Included only by translation units built with -fmad=false: every a*b+c below must stay an
-// unfused multiply and add, as the reference's SSE2 build evaluates it.
+// In the units built with -fmad=false (fsg_kernels64, fsg_solve, fsg_mag, fsg_adjoint) every a*b+c below stays an
+// unfused multiply and add, as the reference's SSE2 build evaluates it; fused ones are written fma.  The tile
+// kernels' units (fsg_accum64, fsg_magfast, fsg_adjoint_line) are built with -fmad=true and take rcp64 and the line
+// parameters from here.
 #pragma once
 #include "fsg_internal.cuh"
 
-// 1 / d for normal d in FP64: the hardware's approximate reciprocal r (relative error e, |e| < 2^-19)
-// and one third-order step r (1 + e + e^2), e = 1 - d r, which leaves e^3
+// 1 / d in FP64 for normal d: the hardware's approximate reciprocal r and one step of the hyperpower iteration of order
+// three (Altman 1960), r (1 + e + e^2) with e = 1 - d r, which leaves e^3 of the result.  The seed comes with the low word
+// 0, that is 20 fraction bits, from the high word of d: |e| < 2^-19, so e^3 < 2^-57 is a sixteenth of an ulp, and
+// the result within 0.5 + 0.0625 ulp (measured over 4e6 arguments: |e| < 2^-19.9, 0.507 ulp; a division 0.5).
+// NaN for d = 0 or infinite.
 __device__ __forceinline__ double rcp64_seed(double d) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));

@@ -44,6 +44,3 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, unsign
     }
     return false;
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(bar)) : "memory");
-}

@@ -225,3 +225,50 @@ def test_stokes_prf_pp(fsg, oracle_mod):
     with pytest.raises(fsg.FsgError):
         C.stokes_prf_pp(np.array([0], np.int32), src[:1], *geo)
     C.close()
+
+
+def test_reciprocal_by_iteration(tmp_path):
+    """rcp64 and rcp64_step (fsg_fp64.cuh) against 1 / d.  The seed's low word is 0: 20 fraction bits of a value formed from
+    as many of d, an error below 2^-19; the third-order step leaves its cube, 2^-57 or 0.0625 ulp, beside its own
+    rounding of 0.5 ulp (the fma that forms 1 + e + e^2 - 1 adds 2^-72).  0 and infinity as the callers count on."""
+    import ctypes
+    import os
+    import subprocess
+    from fastspec_b200 import build as B
+    src, so = str(tmp_path / "r.cu"), str(tmp_path / "r.so")
+    with open(src, "w") as f:
+        f.write('#include "fsg_fp64.cuh"\n'
+                "__global__ void k(int n, const double *d, double *s, double *q, double *z) {\n"
+                "    const int i = blockIdx.x * 256 + threadIdx.x;\n"
+                "    if (i < n) { s[i] = rcp64_seed(d[i]); q[i] = rcp64(d[i]); z[i] = rcp64_step(d[i]); }\n"
+                "}\n"
+                'extern "C" int run(int n, const double *d, double *s, double *q, double *z) {\n'
+                "    k<<<(n + 255) / 256, 256>>>(n, d, s, q, z);\n"
+                "    return (int)cudaDeviceSynchronize();\n"
+                "}\n")
+    subprocess.run([B.NVCC] + B.COMMON + ["-fmad=false", "-I", B.CSRC, "-I", os.path.join(B.HERE, "..", "include"), "-shared",
+                                          "-o", so, src], check=True)
+    import torch
+    run = ctypes.CDLL(so).run
+    rng = np.random.default_rng(5)
+    d = np.ldexp(rng.uniform(1.0, 2.0, 1 << 22), rng.integers(-1000, 1000, 1 << 22)) * rng.choice([-1.0, 1.0], 1 << 22)
+    edge = np.concatenate([1.0 + np.arange(4096) * 2.0 ** -20, 1.0 + np.arange(4096) * 2.0 ** -20 + 2.0 ** -20 - 2.0 ** -52,
+                           2.0 - np.arange(1, 4097) * 2.0 ** -52])
+    special = np.array([0.0, np.inf, -np.inf, np.nan, 5e-324, 1e-310])
+    d = np.concatenate([d, edge, special])
+    t = torch.from_numpy(d).cuda()
+    out = [torch.empty_like(t) for _ in range(3)]
+    torch.cuda.synchronize()
+    assert run(len(d), *[ctypes.c_void_p(x.data_ptr()) for x in (t, *out)]) == 0
+    seed, q, z = (x.cpu().numpy() for x in out)
+    n = len(d) - len(special)
+    exact = np.longdouble(1.0) / d[:n].astype(np.longdouble)
+    ulp = np.spacing(np.abs(1.0 / d[:n])).astype(np.longdouble)
+    e = np.max(np.abs(seed[:n].astype(np.longdouble) / exact - 1))
+    err = np.max(np.abs(q[:n].astype(np.longdouble) - exact) / ulp)
+    print("seed error 2^%.2f, result %.4f ulp" % (np.log2(float(e)), float(err)))
+    assert e < 2.0 ** -19
+    assert err < 0.5 + 0.0625 + 1e-3
+    assert np.array_equal(q[:n], z[:n])
+    assert np.isnan(q[n:n + 4]).all()
+    assert z[n] == np.inf and np.isnan(z[n + 3]) and z[n + 4] == np.inf and z[n + 5] == np.inf
