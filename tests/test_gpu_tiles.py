@@ -164,6 +164,35 @@ def test_magnetic_tile_edges(fsg, oracle_mod, prec, ntau, nwl, n):
     C.close()
 
 
+@pytest.mark.parametrize("prec,j", [("fp64", 5.0), ("fp64", 6.0), ("fp64", 17.0), ("mixed", 5.0), ("mixed", 6.0), ("mixed", 9.0)])
+def test_many_zeeman_components(fsg, oracle_mod, prec, j):
+    """Lines with more components than the tile kernel stages (32; a line J - J has 6 J, at J 17 the pi components
+    alone are more).  Errors on the scale of the depth's peak absorption profile: FP64 as above; mixed, the FP32 sum of
+    a profile's components, 6e-8 each, and ten operations a term."""
+    from fastspec_b200 import workloads as W
+    ntau, nwl, n = 33, 200, 12
+    grid, st, co, _ = case(ntau, nwl, 1, 0)
+    L = W.zeeman_lines(n, grid["wstart"], grid["wend"], int(j))
+    few = L.zeeman
+    L.zeeman = (np.where(np.arange(n) % 3 == 2, few[0], np.float32(j)), np.where(np.arange(n) % 3 == 2, few[1], np.float32(j)),
+                few[2], few[3])
+    z = W.zeeman_components(L, oracle_mod.zeeman_pattern)
+    assert (z[0] + z[1]).max() == 6 * j
+    C = fsg.Context(precision=fsg.PREC_FP64 if prec == "fp64" else fsg.PREC_MIXED, vmicro=1.0)
+    C.set_grid(grid["wmode"], grid["wstart"], grid["wend"], grid["dstep"])
+    C.set_atmosphere(st)
+    C.set_contopac(co)
+    b = np.array([3000.0, 50.0, 20.0])
+    g = C.mag_lineop_calc(fsg.LineList.from_arrays(L.arrays(), zeeman=z), 1, b)
+    S = oracle_mod.State(grid, st, contopac=co, vmicro=1.0)
+    r = oracle_mod.mag_lineop_calc(S, oracle_mod.Lines(**L.arrays(), kind=2, zeeman=z), 1, b)
+    om = r["maglineopac"]
+    scale = np.maximum(om[..., :3].max(axis=(0, 2)), 1e-300)[None, :, None]
+    tol = 1e-12 if prec == "fp64" else 6e-8 * (10 + 2 * j + 1)
+    assert np.max(np.abs(g["maglineopac"] - om) / scale) < tol
+    C.close()
+
+
 @pytest.mark.parametrize("ntau,nwl,nmu", [(3, 2, 1), (4, 7, 2), (64, 9, 9), (65, 17, 16), (128, 8, 5)])
 def test_solver_edges(fsg, oracle_mod, ntau, nwl, nmu):
     """The formal solver around its CTA's eight wavelengths and its thread counts, on a line opacity spread over
