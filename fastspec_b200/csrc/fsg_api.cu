@@ -90,11 +90,9 @@ void fsg_launch_params_fast(cudaStream_t, const AtmView &, const LineView &, con
 void fsg_launch_params_fp64(cudaStream_t, const AtmView &, const LineView &, const int64_t *, int64_t, int64_t, int,
                             const int32_t *, const int32_t *, const int32_t *, const ZView *, const int64_t *, double3 *,
                             LineHdr64 *);
-int fsg_mag64_tile();
 int fsg_launch_mag64(cudaStream_t, const AtmView &, const LineHdr64 *, const double3 *, const ZView &, const int *,
                      const int *, int, int, const VoigtTables &, double *);
 int fsg_launch_tile_span64(cudaStream_t, int, int, int64_t, const LineHdr64 *, int *, int *, void *, size_t);
-int fsg_accum64_tile();
 int fsg_launch_accum64(cudaStream_t, const AtmView &, const LineHdr64 *, const double3 *, const int *, const int *, int,
                        int, const VoigtTables &, double *);
 void fsg_launch_span(cudaStream_t, int64_t, const int32_t *, const int32_t *, const int32_t *, int *, int *);
@@ -733,8 +731,8 @@ static int central_pass(fsg_ctx *ctx, const LineView &LV, int64_t *nkeep) {
     return FSG_OK;
 }
 
-// FP64 rows of the lines list[0 .. nb) (list null: i0 .. i0 + nb) with their headers (d_hdr64) and the tile
-// ranges (d_tlo, d_thi) of k_accum64, or of k_mag64 when the list's Zeeman components are given (line i's at
+// FP64 rows of the lines list[0 .. nb) (list null: i0 .. i0 + nb) with their headers (d_hdr64) and the row
+// ranges of each 32 wavelengths (d_tlo, d_thi) for k_accum64, or for k_mag64 when the list's Zeeman components are given (line i's at
 // zmap[i]); lines with any flag of skip get an empty window
 static int rows64(fsg_ctx *ctx, const AtmView &A, const LineView &LV, const int64_t *list, int64_t i0, int64_t nb,
                   int skip, const int32_t *fl, const int32_t *il, const int32_t *ir, DBuf &p64,
@@ -746,7 +744,7 @@ static int rows64(fsg_ctx *ctx, const AtmView &A, const LineView &LV, const int6
     ALLOC(ctx->d_tlo, sizeof(int) * ntiles); ALLOC(ctx->d_thi, sizeof(int) * ntiles);
     fsg_launch_params_fp64(ctx->stream, A, LV, list, i0, nb, skip, fl, il, ir, Z, zmap, p64.as<double3>(),
                            ctx->d_hdr64.as<LineHdr64>());
-    if (fsg_launch_tile_span64(ctx->stream, Z ? fsg_mag64_tile() : fsg_accum64_tile(), ctx->nwl, nb, ctx->d_hdr64.as<LineHdr64>(),
+    if (fsg_launch_tile_span64(ctx->stream, 32, ctx->nwl, nb, ctx->d_hdr64.as<LineHdr64>(),
                                ctx->d_tlo.as<int>(), ctx->d_thi.as<int>(), ctx->d_span.p, ctx->d_span.cap))
         return cuda_fail(ctx, cudaGetLastError(), "FP64 tile span");
     ctx->launches += 7;

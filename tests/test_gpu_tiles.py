@@ -329,3 +329,29 @@ def test_adjoint_tile_edges(fsg, ntau, nwl, n):
     for q in range(2):
         assert float((out[0][q] - out[1][q] - out[2][q]).abs().max()) < 2e-6 * max(scale, float(out[0][q].abs().sum()))
     C.close()
+
+
+@pytest.mark.parametrize("ntau,nwl", [(5, 3000), (56, 7501), (71, 8001)])
+def test_fp64_forms_sum_alike(fsg, ntau, nwl):
+    """The FP64 tile kernel takes fewer points a warp where there are few wavelengths: ranges short enough for each of
+    its forms give the sums of the whole grid bit for bit."""
+    import torch
+    from fastspec_b200.shard import GpuBackend
+    grid, st, co, a = case(ntau, nwl, 300, 9)
+    C = fsg.Context(precision=fsg.PREC_FP64, vmicro=1.0)
+    C.set_grid(grid["wmode"], grid["wstart"], grid["wend"], grid["dstep"])
+    C.set_atmosphere(st)
+    C.set_contopac(co)
+    B = GpuBackend(fsg, C, {k: torch.from_numpy(np.ascontiguousarray(v)).cuda() for k, v in a.items()})
+    C.lineop_reset()
+    C.lineop_calc_dev(B.full)
+    whole = C.lineop_get()
+    win = B.central(0, B.n, B.n)
+    warps = lambda n: ((n - 1) // 64 + 1) * ((ntau + 3) // 4)        # noqa: E731
+    used = set()
+    for i0, i1 in ((1, 1), (17, 80), (33, 1003), (100, 2999), (60, min(5500, nwl)), (1, nwl)):
+        used.add((warps(i1 - i0 + 1) >= 660) + (warps(i1 - i0 + 1) >= 1600))
+        B.accumulate(win, i0, i1)
+        assert np.array_equal(C.lineop_get()[i0 - 1:i1], whole[i0 - 1:i1])
+    assert len(used) == (1 if ntau == 5 else 3)
+    C.close()
