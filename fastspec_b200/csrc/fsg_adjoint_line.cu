@@ -47,8 +47,7 @@ size_t fsg_tile_span_scratch(int64_t);
 int fsg_launch_tile_span_tw(cudaStream_t, int, int, int, int64_t, const LineHdr *, int *, int *, void *, size_t);
 
 #define ADJ_SETUP_WARPS 8
-#define ADJ_P 4                        // wavelengths per lane
-#define ADJ_TW (32 * ADJ_P)            // wavelengths per tile
+#define ADJ_P 4                        // wavelengths per lane; 1 where there are few tiles
 #define ADJ_G 8                        // lines per group
 #define ADJ_W 4                        // warps per CTA
 
@@ -266,10 +265,10 @@ __device__ __forceinline__ void core_h_hd(const float4 *__restrict__ ftab2, floa
 }
 
 // wing form over the warp's depth pairs and the lane's wavelengths (MASK: some lanes outside the window)
-template <int KD, bool MASK>
-__device__ __forceinline__ void wing_line(const float4 *__restrict__ rp, const float2 (&g)[ADJ_P][KD / 2],
-                                          const float (&X)[ADJ_P], const float (&XX)[ADJ_P],
-                                          const bool (&in)[ADJ_P], float2 &s1, float2 &s2) {
+template <int KD, bool MASK, int P>
+__device__ __forceinline__ void wing_line(const float4 *__restrict__ rp, const float2 (&g)[P][KD / 2],
+                                          const float (&X)[P], const float (&XX)[P],
+                                          const bool (&in)[P], float2 &s1, float2 &s2) {
 #pragma unroll
     for (int j = 0; j < KD / 2; j++) {
         const float4 r0 = rp[4 * j], r1 = rp[4 * j + 1], r2 = rp[4 * j + 2], r3 = rp[4 * j + 3];
@@ -278,7 +277,7 @@ __device__ __forceinline__ void wing_line(const float4 *__restrict__ rp, const f
         const float2 e0 = make_float2(r2.x, r2.y), f2 = make_float2(r2.z, r2.w);
         const float2 f0 = make_float2(r3.x, r3.y), K2 = make_float2(r3.z, r3.w);
 #pragma unroll
-        for (int k = 0; k < ADJ_P; k++) {
+        for (int k = 0; k < P; k++) {
             const float2 x2 = make_float2(X[k], X[k]), xx2 = make_float2(XX[k], XX[k]);
             const float2 D = __ffma2_rn(__ffma2_rn(c4, x2, c2), x2, B0);
             const float2 rD = make_float2(rcp_approx(D.x), rcp_approx(D.y));
@@ -296,8 +295,9 @@ __device__ __forceinline__ void wing_line(const float4 *__restrict__ rp, const f
 
 // point by point: lines whose core range meets the tile.  A loop over depths that reads its weights from memory
 // again: unrolled over the warp's depths the three profile forms outgrew the instruction cache.
-__device__ __forceinline__ void core_line(const AdjTileJob &J, int line, int t0, int t1, const int (&pix)[ADJ_P],
-                                          const float (&dl)[ADJ_P], const bool (&in)[ADJ_P], float2 &s1,
+template <int P>
+__device__ __forceinline__ void core_line(const AdjTileJob &J, int line, int t0, int t1, const int (&pix)[P],
+                                          const float (&dl)[P], const bool (&in)[P], float2 &s1,
                                           float2 &s2) {
 #pragma unroll 1
     for (int t = t0; t < t1; t++) {
@@ -306,7 +306,7 @@ __device__ __forceinline__ void core_line(const AdjTileJob &J, int line, int t0,
         const float a = cr.y, a2 = a * a;
         float h1 = 0.0f, h2 = 0.0f;
 #pragma unroll
-        for (int k = 0; k < ADJ_P; k++) {
+        for (int k = 0; k < P; k++) {
             if (!in[k]) continue;
             const float v = dl[k] * cr.x, s = fmaf(v, v, a2);
             float H, Hd;
@@ -329,8 +329,9 @@ __device__ __forceinline__ void core_line(const AdjTileJob &J, int line, int t0,
 }
 
 // one (tile, depth group) per warp, the groups of a tile in turn
-template <int KD>
+template <int KD, int P>
 __global__ void __launch_bounds__(32 * ADJ_W) k_adj_tiles(AdjTileJob J) {
+    constexpr int TW = 32 * P;
     constexpr int R = 2 * KD;                             // 16-byte record parts of a line at the warp's depths
     __shared__ int queue_s[ADJ_W][64];
     __shared__ LineHdr hdr_s[ADJ_W][ADJ_G];
@@ -343,14 +344,14 @@ __global__ void __launch_bounds__(32 * ADJ_W) k_adj_tiles(AdjTileJob J) {
     const int tile = (int)(item / J.ngrp), t0 = (int)(item % J.ngrp) * KD;
     const int lo = J.tlo[tile], hi = J.thi[tile];
     if (lo > hi) return;
-    const int f1 = tile * ADJ_TW + 1, l1 = min(tile * ADJ_TW + ADJ_TW, nwl);     // 1-based wavelengths
+    const int f1 = tile * TW + 1, l1 = min(tile * TW + TW, nwl);     // 1-based wavelengths
     const int *queue = queue_s[warp];
-    float2 g[ADJ_P][KD / 2];
-    float wh[ADJ_P], wl[ADJ_P];
-    int pix[ADJ_P];
+    float2 g[P][KD / 2];
+    float wh[P], wl[P];
+    int pix[P];
 #pragma unroll
-    for (int k = 0; k < ADJ_P; k++) {
-        pix[k] = tile * ADJ_TW + lane + 32 * k;
+    for (int k = 0; k < P; k++) {
+        pix[k] = tile * TW + lane + 32 * k;
         const bool pin = pix[k] < nwl;
         // past the grid: the last wavelength's offsets (zero weights, finite wing values)
         wh[k] = J.wvh[min(pix[k], nwl - 1)];
@@ -371,10 +372,10 @@ __global__ void __launch_bounds__(32 * ADJ_W) k_adj_tiles(AdjTileJob J) {
         __syncwarp();
         for (int m = 0; m < n; m++) {
             const LineHdr h = hdr_s[warp][m];
-            float dl[ADJ_P], X[ADJ_P], XX[ADJ_P];
-            bool in[ADJ_P];
+            float dl[P], X[P], XX[P];
+            bool in[P];
 #pragma unroll
-            for (int k = 0; k < ADJ_P; k++) {
+            for (int k = 0; k < P; k++) {
                 dl[k] = (wh[k] - h.wlh) + (wl[k] - h.wll);
                 X[k] = dl[k] * dl[k];
                 XX[k] = X[k] * X[k];
@@ -383,8 +384,8 @@ __global__ void __launch_bounds__(32 * ADJ_W) k_adj_tiles(AdjTileJob J) {
             float2 s1 = make_float2(0.0f, 0.0f), s2 = make_float2(0.0f, 0.0f);
             const float4 *rp = rec_s[warp][m];
             if (!(h.cr < f1 || h.cl > l1)) core_line(J, queue[(head + m) & 63], t0, min(t0 + KD, nt), pix, dl, in, s1, s2);
-            else if (h.ileft <= f1 && h.iright >= l1) wing_line<KD, false>(rp, g, X, XX, in, s1, s2);
-            else wing_line<KD, true>(rp, g, X, XX, in, s1, s2);
+            else if (h.ileft <= f1 && h.iright >= l1) wing_line<KD, false, P>(rp, g, X, XX, in, s1, s2);
+            else wing_line<KD, true, P>(rp, g, X, XX, in, s1, s2);
             part_s[warp][m][lane] = make_float2(s1.x + s1.y, s2.x + s2.y);
         }
         __syncwarp();
@@ -416,19 +417,26 @@ static size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // workspace of the line pass for n lines
 size_t fsg_line_adjoint_work(int nwl, int nt, int64_t n) {
-    const int ntiles = (nwl + ADJ_TW - 1) / ADJ_TW;
+    const int ntiles = (nwl + 31) / 32;                  // of the narrowest tiles
     return al256(sizeof(float) * 8 * (size_t)n * adj_ntp(nt)) + al256(sizeof(float4) * (size_t)n * nt) +
            al256(sizeof(float2) * (size_t)n * nt) + al256(sizeof(LineHdr) * (size_t)n) +
            2 * al256(sizeof(int) * (size_t)ntiles) + al256(fsg_tile_span_scratch(n)) + 256;
 }
 
+// Few tiles: the warps of 128 wavelengths x 4 depths are few, and the pass is the latency of one warp's lines; 32 x 2 points
+// a warp make eight times as many.  Whole adjoint, ms: 301 wavelengths, 20,000 lines, 8 depths 59 -> 9.5 (29 with CTAs of
+// one producer and two consumer warps on 64 wavelengths), 56 depths 62 -> 10.8; 8,001 wavelengths, 5,000 lines, 56 depths
+// (882 warps) 1.99 and 1.85; 40,001, 20,000, 8 depths (626 warps) 1.51 and 1.63; 16,001, 8,000, 56 depths (1,764) 2.1
+// and 2.9.
+#define ADJ_FEW 600
 int fsg_launch_line_adjoint(cudaStream_t s, const AtmView &A, const LineView &L, const VoigtTables &T,
                             const int32_t *flags, const int32_t *ileft, const int32_t *iright, const double *gkappa,
                             const float *gk32, const float *wvh, const float *wvl, double vmic, double *glin,
                             double *gvmic, void *work, int i0, int i1) {
     const int nt = A.ntau, nwl = A.nwl, ntp = adj_ntp(nt), kd = adj_kd(nt);
     const int64_t n = L.n;
-    const int ntiles = (nwl + ADJ_TW - 1) / ADJ_TW;
+    const bool few = (int64_t)((i1 - i0) / (32 * ADJ_P) + 1) * (ntp / kd) < ADJ_FEW;
+    const int KD = few ? 2 : kd, P = few ? 1 : ADJ_P, ntiles = (nwl + 32 * P - 1) / (32 * P);
     char *w = (char *)(((uintptr_t)work + 255) & ~(uintptr_t)255);
     float *prec = (float *)w; w += al256(sizeof(float) * 8 * (size_t)n * ntp);
     float4 *crec = (float4 *)w; w += al256(sizeof(float4) * (size_t)n * nt);
@@ -442,14 +450,15 @@ int fsg_launch_line_adjoint(cudaStream_t s, const AtmView &A, const LineView &L,
     k_adj_setup<<<(unsigned)((n + ADJ_SETUP_WARPS - 1) / ADJ_SETUP_WARPS), 32 * ADJ_SETUP_WARPS, smem, s>>>(
         A, L, T.vtab, T.fvtab, T.anode, T.aida, flags, ileft, iright, gkappa, vmic, ntp, prec, crec, tabi, hdr, glin,
         gvmic, i0, i1);
-    int rc = fsg_launch_tile_span_tw(s, ADJ_TW, 0, nwl, n, hdr, tlo, thi, span, span_bytes);
+    int rc = fsg_launch_tile_span_tw(s, 32 * P, 0, nwl, n, hdr, tlo, thi, span, span_bytes);
     if (rc) return rc;
     AdjTileJob J;
-    J.nwl = nwl; J.nt = nt; J.ntp = ntp; J.ntiles = ntiles; J.ngrp = ntp / kd; J.gk32 = gk32; J.wvh = wvh; J.wvl = wvl;
+    J.nwl = nwl; J.nt = nt; J.ntp = ntp; J.ntiles = ntiles; J.ngrp = (nt + KD - 1) / KD; J.gk32 = gk32; J.wvh = wvh; J.wvl = wvl;
     J.prec = (const float4 *)prec; J.crec = crec; J.tabi = tabi; J.hdr = hdr; J.tlo = tlo; J.thi = thi;
     J.fvtab2 = T.fvtab2; J.glin = glin; J.gvmic = gvmic;
     const unsigned grid = (unsigned)(((int64_t)J.ntiles * J.ngrp + ADJ_W - 1) / ADJ_W);
-    if (kd == 4) k_adj_tiles<4><<<grid, 32 * ADJ_W, 0, s>>>(J);
-    else k_adj_tiles<2><<<grid, 32 * ADJ_W, 0, s>>>(J);
+    if (few) k_adj_tiles<2, 1><<<grid, 32 * ADJ_W, 0, s>>>(J);
+    else if (kd == 4) k_adj_tiles<4, ADJ_P><<<grid, 32 * ADJ_W, 0, s>>>(J);
+    else k_adj_tiles<2, ADJ_P><<<grid, 32 * ADJ_W, 0, s>>>(J);
     return cudaGetLastError() == cudaSuccess ? FSG_OK : FSG_E_CUDA;
 }

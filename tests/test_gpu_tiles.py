@@ -287,6 +287,37 @@ def test_broadening_edges(fsg, oracle_mod, nwl, nmu, vsini, vmacro, vgau):
     C.close()
 
 
+@pytest.mark.parametrize("ntau,nwl", [(9, 31000), (56, 6001), (64, 4801)])
+def test_adjoint_forms_agree(fsg, ntau, nwl):
+    """The adjoint's line pass takes fewer points a warp where there are few tiles: the gradients of ranges short enough
+    for that, summed, against the whole grid's.  FP32 profiles summed in other groups, both signs: 2e-6 of the sum of
+    magnitudes, as at the tile edges."""
+    import torch
+    from fastspec_b200.shard import GpuBackend
+    grid, st, co, a = case(ntau, nwl, 150, 13)
+    C = fsg.Context(vmicro=1.0)
+    C.set_grid(grid["wmode"], grid["wstart"], grid["wend"], grid["dstep"])
+    C.set_atmosphere(st)
+    C.set_contopac(co)
+    x, w, _ = fsg.mu_quadrature(1, 2)
+    C.set_mu(x, w)
+    B = GpuBackend(fsg, C, {k: torch.from_numpy(np.ascontiguousarray(v)).cuda() for k, v in a.items()})
+    C.lineop_reset()
+    C.lineop_calc_dev(B.full)
+    win = B.central(0, B.n, B.n)
+    g = torch.from_numpy(np.random.default_rng(3).normal(0.0, 1.0, nwl)).cuda()
+    whole = B.adjoint(win, 1, nwl, g)
+    warps = lambda n: ((n - 1) // 128 + 1) * ((ntau + 3) // 4)       # noqa: E731
+    cut = nwl // 3
+    ranges = ((1, cut), (cut + 1, 2 * cut + 5), (2 * cut + 6, nwl))
+    assert warps(nwl) >= 600 and all(warps(j - i + 1) < 600 for i, j in ranges)
+    parts = [B.adjoint(win, i, j, g) for i, j in ranges]
+    for q in range(2):
+        total = sum(p[q] for p in parts)
+        assert float((total - whole[q]).abs().max()) < 2e-6 * float(whole[q].abs().sum())
+    C.close()
+
+
 @pytest.mark.parametrize("ntau,nwl,n", [(3, 2, 1), (7, 127, 8), (9, 129, 9), (33, 300, 33), (65, 640, 70)])
 def test_adjoint_tile_edges(fsg, ntau, nwl, n):
     """The line pass of the adjoint around its tiles and depth groups: the whole-grid gradients against the sum of
