@@ -263,14 +263,15 @@ __global__ void __launch_bounds__(128) k_center_warp(AtmView A, LineView L, cons
     if (lane == 0 && center_result(A, c, mx1, mx2, dWwin, i, flags, ileft, iright)) atomicAdd(nkeep, 1ull);
 }
 
-// A thread's sweep over the depths takes 125 us whatever the number of lines (the latency of an FP64 chain), and
+// A thread's sweep over the depths takes 2.3 us a depth whatever the number of lines (the latency of an FP64 chain), and
 // a list fills the GPU with threads from 150,000 lines on; a warp per line repeats the line's set-up in every
-// lane.  300 lines: 126 us by threads, 11 us by warps; 20,000: 133 and 66 us, 3.3 us more per thousand, so the two
-// meet near 40,000.
+// lane, 1.7 us more per thousand lines up to 32 depths, 2.7 up to 64, 3.7 up to 96.  56 depths, with the call's own 25 us:
+// 300 lines 140 us by threads, 32 us by warps; 20,000: 144 and 81 us.  The two meet near 8,000 lines at 8 depths (42 and
+// 45 us), 20,000 at 20 (69 us), 31,000 at 33 (105 us).
 void fsg_launch_center(cudaStream_t s, const AtmView &A, const LineView &L, const VoigtTables &T,
                        int32_t *flags, int32_t *ileft, int32_t *iright, unsigned long long *nkeep) {
     if (L.n <= 0) return;
-    if (L.n <= 32768)
+    if (L.n <= std::min(32768, 950 * A.ntau))
         k_center_warp<<<(unsigned)((L.n + 3) / 4), 128, 0, s>>>(A, L, T.vtab, T.anode, T.aida, flags, ileft, iright, nkeep);
     else
         k_center<<<(unsigned)((L.n + 127) / 128), 128, 0, s>>>(A, L, T.vtab, T.anode, T.aida, flags, ileft, iright, nkeep);

@@ -216,6 +216,21 @@ def test_solver_edges(fsg, oracle_mod, ntau, nwl, nmu):
     C.close()
 
 
+def test_central_pass_forms_shallow(fsg):
+    """The same in a shallow model, where shorter lists take a thread per line (8 depths: above 7,600)."""
+    from fastspec_b200 import workloads as W
+    grid, st, co, _ = case(8, 64, 1, 0)
+    a = W.atomic_lines(9001, grid["wstart"] - 40.0, grid["wend"] + 40.0, 2, exact=False).arrays()
+    C = fsg.Context(vmicro=1.0)
+    C.set_grid(grid["wmode"], grid["wstart"], grid["wend"], grid["dstep"])
+    C.set_atmosphere(st)
+    C.set_contopac(co)
+    out = [C.lineop_calc(fsg.LineList.from_arrays({k: v[i:j] for k, v in a.items()})) for i, j in ((0, 9001), (0, 5000), (5000, 9001))]
+    for k in ("flags", "ileft", "iright"):
+        np.testing.assert_array_equal(out[0][k], np.concatenate([out[1][k], out[2][k]]))
+    C.close()
+
+
 @pytest.mark.parametrize("sphere", [False, True])
 def test_solver_without_opacity(fsg, oracle_mod, sphere):
     """Layers whose opacities cancel to 0, are infinite or are no number: optical-depth steps of 0, whose reciprocals
