@@ -523,6 +523,7 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
     const unsigned bytes = (unsigned)(nd * (int)sizeof(CoreRec));
     double *dst = J.lineopac + (size_t)p * ntau + t0;
     int head = 0, ncand = 0, sg = 0, base = 0, hi = -1, nprev = 0;
+    const unsigned kk0 = kk;
     bool ok = true;
     for (;;) {
         bool cut = false;                              // the group in flight is the last of its segment
@@ -565,7 +566,9 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
             ok = __all_sync(0xffffffffu, mbar_wait(&S.bar[g & 1], (g >> 1) & 1, J.wait_ns));
             if (!ok) break;
             work(g & 1, nprev);
-            if (PER_SEG && (cut || !n)) {
+            // (the last sums are added here too: with a copy of this behind the loop the sparse tiles of a batch took 0.27 ms
+            // for 0.20)
+            if ((PER_SEG && cut) || !n) {
 #pragma unroll
                 for (int d = 0; d < D; d++) {
                     const double v = (double)sum[d] - (double)cmp[d];
@@ -579,10 +582,10 @@ __device__ __forceinline__ bool core_tile(const CoreJob &J, int tile, int t0, co
         nprev = n;
         if (!n) break;                                  // nothing in flight and no line left
     }
-    if (ok && p < nwl && (TOT || !PER_SEG)) {
+    if (TOT && ok && kk != kk0 && p < nwl) {            // some line has points here
 #pragma unroll
         for (int d = 0; d < D; d++)
-            if (d < nd) dst[d] += TOT ? tot[d][lane] : (double)sum[d] - (double)cmp[d];
+            if (d < nd) dst[d] += tot[d][lane];
     }
     if (!ok) {
         if (lane == 0) {
