@@ -159,7 +159,7 @@ __global__ void k_solver_adjoint(AtmView A, const double *__restrict__ lineopac,
 }
 
 // Spherical models: the same chain along each ray of LocPrfSph (solver.f90:182-261, the forward is
-// delo_ray): per ray the TauStep steps on the ray's column mass, CentDer of the source, the Bezier
+// sweep_ray in fsg_solve.cu): per ray the TauStep steps on the ray's column mass, CentDer of the source, the Bezier
 // terms and the sweep (grazing rays start from zero at the far side), run backwards from dL/dI_ray =
 // Wmu dL/dSfL; a ray point's derivative goes to the layer it samples.  One thread per wavelength; work:
 // per wavelength X, Y, GX by layer (3 nt) and D, R, U, YS, GD, GR, GU by ray point (7 x 2 nt).

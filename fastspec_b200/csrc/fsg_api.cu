@@ -105,7 +105,7 @@ void fsg_launch_locprf(cudaStream_t, int, int, const double *, int, const double
                        double *, double *);
 int fsg_launch_accum_fast(cudaStream_t, int, const WingJob &);
 int fsg_launch_core_fast(cudaStream_t, const CoreJob &, const float4 *, int *);
-int fsg_wing_groups(int, int);
+int fsg_wing_groups(int);
 int fsg_launch_accum_batch(cudaStream_t, int, const WingJob *, const int *, int, int, unsigned *);
 int fsg_launch_core_batch(cudaStream_t, int, const CoreJob *, const int *, int, int, const float4 *, unsigned *,
                           int *);
@@ -2547,7 +2547,7 @@ static int batch_jobs(fsg_batch *b, int P) {
                 jw.push_back(WingJob{ c->ntau, c->nwl, c->d_wave.as<double>(), a.hdr.as<LineHdr>(),
                                       a.wing.as<WingPair>(), a.wtlo.as<int>() + (size_t)c0 * ws,
                                       a.wthi.as<int>() + (size_t)c0 * ws, c->d_lineopac.as<double>(), nseg, ws, 0 });
-                t0.push_back(t0.back() + (c->nwl + 32 * Pk - 1) / (32 * Pk) * fsg_wing_groups(Pk, c->ntau));
+                t0.push_back(t0.back() + (c->nwl + 32 * Pk - 1) / (32 * Pk) * fsg_wing_groups(c->ntau));
             } else {
                 jc.push_back(CoreJob{ c->ntau, c->nwl, c->d_wave.as<double>(), a.hdr.as<LineHdr>(),
                                       a.core.as<CoreRec>(), a.ctlo.as<int>(), a.cthi.as<int>(),

@@ -156,8 +156,8 @@ __device__ __forceinline__ void wing_tile(const WingJob &J, int tile, int t0, Wi
             const bool full = h.ileft <= tile_first && h.iright >= tile_last && !core_hit;
             const int l = max(h.ileft - tile_first, 0), r = min(h.iright - tile_first, TW - 1);
             hnext = make_float4(h.wlh, h.wll, __int_as_float(l | r << 8 | (core_hit ? WING_CORE : 0)),
-                                __int_as_float(h.pad0));
-            pair = pairs && full && h.pad1;
+                                __int_as_float(h.silent));
+            pair = pairs && full && h.pairable;
         }
         // the lines to be paired first
         const unsigned pm = __ballot_sync(0xffffffffu, pair), before = __popc(pm & ((1u << lane) - 1u));
@@ -352,7 +352,7 @@ k_accum_batch(const WingJob *__restrict__ jobs, const int *__restrict__ item0, i
 int fsg_class_pix(int cls) { return cls <= 1 ? 2 : 4; }
 
 // depth groups of the wing pass
-int fsg_wing_groups(int P, int ntau) { return (ntau + WING_D - 1) / WING_D; }
+int fsg_wing_groups(int ntau) { return (ntau + WING_D - 1) / WING_D; }
 
 // Few tiles: at eight depths a warp their warps would not fill a quarter of the 148 x 16 that are resident, so the pass
 // is the latency of its longest warp.  Two depths a warp then make four times as many of them, which set out together.

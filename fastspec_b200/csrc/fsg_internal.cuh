@@ -91,11 +91,11 @@ static_assert(sizeof(CoreRec) == 32, "core record: 32 bytes");
 // Line header of a retained line inside a block (fast path).  The centre offset Wlcent is split
 // into FP32 wlh + wll (wlh = fl32(Wlcent), wll = fl32(Wlcent - wlh)).  [cl, cr] is the core range:
 // every wavelength index of the window where some depth may have s < 196 lies inside it
-// (cl > cr when no depth has a core).  pad0 holds, in the wing pass's headers, the FP32 bits of the
+// (cl > cr when no depth has a core).  silent: in the wing pass's headers, the FP32 bits of the
 // x = dl^2 that makes every depth's wing term exactly 0 (points outside the window or inside the core
-// range of a partly covered tile), pad1 whether the line may share a reciprocal with another; the magnetic pass
-// keeps its He I table index in pad0.
-struct __align__(16) LineHdr { float wlh, wll; int ileft, iright; int cl, cr, pad0, pad1; };
+// range of a partly covered tile); in the magnetic pass's, the He I table index (0: none).  pairable: the line may
+// share a reciprocal with another (wing pass).
+struct __align__(16) LineHdr { float wlh, wll; int ileft, iright; int cl, cr, silent, pairable; };
 
 // Line header of the FP64 tile kernels: the centre offset Wlcent, the window, the core range [cl, cr]
 // (every wavelength of the window where some depth may have s < 196, He I shifts included; cl > cr:

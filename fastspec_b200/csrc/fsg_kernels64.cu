@@ -407,13 +407,13 @@ k_params_fast(AtmView A, LineView L, const int64_t *__restrict__ idx, int64_t j0
         int cl = max(a - 1, h.ileft), cr = min(b + 1, h.iright);
         if (cl <= cr) { h.cl = cl; h.cr = cr; }
     }
-    // pad1: the line may share a reciprocal in the wing pass (no depth's denominator above 2^62, no coefficient
+    // pairable: the line may share a reciprocal in the wing pass (no depth's denominator above 2^62, no coefficient
     // above 2^30: the product of two stays below 2^126, its numerator finite)
     // x offset that silences a point in the wing pass: with dl^2 replaced by 1e19 / min vv2, every
     // depth has t >= 1e19, so t^2 >= 1e38 and the FP32 reciprocal (flush-to-zero) is exactly 0 while
     // c1 (t + 1) stays finite; the point then adds exactly 0
-    h.pad0 = __float_as_int(1.0e19f / vv2min);
-    h.pad1 = !big[wp][lane];
+    h.silent = __float_as_int(1.0e19f / vv2min);
+    h.pairable = !big[wp][lane];
     hdr[jb + lane] = h;
 }
 

@@ -101,8 +101,8 @@ k_mag_params_fast(AtmView A, LineView L, ZView Z, const int64_t *__restrict__ id
         const int cl = max(a - 1, h.ileft), cr = min(b + 1, h.iright);
         if (cl <= cr) { h.cl = cl; h.cr = cr; }
     }
-    h.pad0 = ihe;                                     // He I table index (0: none)
-    h.pad1 = 0;
+    h.silent = ihe;                                   // He I table index (0: none)
+    h.pairable = 0;
     hdr[j] = h;
     comp[j] = MagComp{ Z.pi_off[i], Z.si_off[i], Z.npi[i], Z.nsi[i], { 0, 0 } };
 }
@@ -229,8 +229,8 @@ __global__ void __launch_bounds__(32 * MAG_W) k_mag_fast(MagJob J, ZView Z) {
                 const MagPair &m = pair_s[warp][q][j];
                 vv[j] = make_float2(m.vv[0], m.vv[1]);
                 float2 d2 = make_float2(dl, dl);
-                if (h.pad0 > 0) {
-                    const double *sh = J.heshf + (size_t)(h.pad0 - 1) * ntau;
+                if (h.silent > 0) {
+                    const double *sh = J.heshf + (size_t)(h.silent - 1) * ntau;
                     d2.x -= (float)sh[min(t0 + 2 * j, ntau - 1)];
                     d2.y -= (float)sh[min(t0 + 2 * j + 1, ntau - 1)];
                 }

@@ -171,10 +171,11 @@ int fsg_lineop_calc_dev(fsg_ctx *ctx, const fsg_lines *d_lines, fsg_stats *stats
  * list into caller-owned device arrays LinFlag / Ileft / Iright (n each) and returns the retained
  * count; fsg_accumulate_dev accumulates a device list whose windows are given onto the device
  * LineOpac, over wavelength indices i0..i1 (1-based, inclusive) only.  Each wavelength of the range
- * sums the same lines in the same order as a whole-grid fsg_lineop_calc_dev (mixed precision: equal
- * to rounding, as the Kahan groups of a tile cut by the range ends, and the blocks of a class, may
- * differ; FP64: the same segments and order, so equal bit for bit); other wavelengths are left as
- * they are. */
+ * sums the same lines as a whole-grid fsg_lineop_calc_dev (mixed precision: equal to rounding, as the
+ * groups of lines summed together differ in a tile of 128 wavelengths that a range end cuts, and where
+ * the records of the list or of the range do not fit one block, LIMITRAM; FP64: the same segments and
+ * order, so equal bit for bit); other wavelengths are left as they are.  Windows may reach past the
+ * ends of the grid. */
 int fsg_central_dev(fsg_ctx *ctx, const fsg_lines *d_lines, int32_t *d_flags, int32_t *d_ileft,
                     int32_t *d_iright, int64_t *nkeep);
 int fsg_accumulate_dev(fsg_ctx *ctx, const fsg_lines *d_lines, const int32_t *d_flags,
