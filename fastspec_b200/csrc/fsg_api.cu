@@ -1230,12 +1230,13 @@ int fsg_accumulate_dev(fsg_ctx *ctx, const fsg_lines *d_lines, const int32_t *d_
     cudaStream_t s = ctx->stream;
     CK(cudaEventRecord(ctx->ev[1], s), "event");
     if (ctx->cfg.precision == FSG_PREC_FP64) {
-        // the FP64 path marks wide lines in its own copy of the windows
+        // the FP64 path marks wide lines in its own copy of the windows, and reads the grid at their ends: the parts of
+        // them inside the grid
         const size_t nb = sizeof(int32_t) * (size_t)d_lines->n;
         ALLOC(ctx->d_flags, nb); ALLOC(ctx->d_ileft, nb); ALLOC(ctx->d_iright, nb);
-        CK(cudaMemcpyAsync(ctx->d_flags.p, d_flags, nb, cudaMemcpyDeviceToDevice, s), "windows");
-        CK(cudaMemcpyAsync(ctx->d_ileft.p, d_ileft, nb, cudaMemcpyDeviceToDevice, s), "windows");
-        CK(cudaMemcpyAsync(ctx->d_iright.p, d_iright, nb, cudaMemcpyDeviceToDevice, s), "windows");
+        fsg_launch_range_clip(s, d_lines->n, d_flags, d_ileft, d_iright, 1, ctx->nwl, ctx->d_flags.as<int32_t>(),
+                              ctx->d_ileft.as<int32_t>(), ctx->d_iright.as<int32_t>());
+        ctx->launches += 1;
         rc = accumulate_fp64(ctx, make_view(d_lines), -1, st, i0, i1);
     } else {
         rc = accumulate_fast(ctx, make_view(d_lines), -1, st, d_flags, d_ileft, d_iright, i0, i1);

@@ -145,7 +145,8 @@ def test_range_adjoints_sum_to_the_whole_gradient(fsg):
     assert np.count_nonzero(ref_lin) > n // 2
 
 
-def test_given_windows_past_the_grid(fsg):
+@pytest.mark.parametrize("prec,ram", [("mixed", 16.0), ("fp64", 16.0), ("fp64", 2.0e-3)])
+def test_given_windows_past_the_grid(fsg, prec, ram):
     """Windows given to fsg_accumulate_dev may reach past either end of the grid: the sums are those of the windows
     cut at its ends, bit for bit.  Wide steps and full windows, so that some denominators of the wing form leave the
     range in which two lines may share a reciprocal."""
@@ -155,7 +156,7 @@ def test_given_windows_past_the_grid(fsg):
     st, _ = W.batch_atmosphere(5300.0, 4.2, ntau, {})
     wave = fsg.make_grid(0, w0, w0 + (nwl - 0.5) * step, step) + w0
     a = W.atomic_lines(4001, wave[0], wave[-1], nwl, exact=False).arrays()
-    C = fsg.Context(vmicro=1.0, epsopac=1e-14)
+    C = fsg.Context(precision=fsg.PREC_FP64 if prec == "fp64" else fsg.PREC_MIXED, vmicro=1.0, epsopac=1e-14, limitram_gb=ram)
     C.set_grid(0, w0, w0 + (nwl - 0.5) * step, step)
     C.set_atmosphere(st)
     C.set_contopac(np.tile(1e-2 * (1.0 + np.arange(ntau)), (nwl, 1)))
